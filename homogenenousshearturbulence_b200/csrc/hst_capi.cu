@@ -348,17 +348,14 @@ static int choose_geometry(const hst_gpu_params& p, Geometry& g, std::string& wh
     why = "ny too large for one line-solver group's shared memory";
     return HST_EARG;
   }
-  // FFT points per thread: 8 selects the low-register plans (lengths 192,
-  // 384, 768; the x kernel then moves its tiles by TMA).  Measured at
-  // 384^2 x 256: x 8 (1.31 against 2.41 ms), z 16 (0.26/0.50 against
-  // 0.29/0.52 ms); at 768^2 x 512 the z kernels need 8 (2.4/4.9 against
-  // 4.0/14.0 ms).  HST_FFT_PPT_X / HST_FFT_PPT_Z override.
+  // z FFT points per thread: 8 selects the low-register plans (lengths 192,
+  // 384, 768).  Measured: 16 at 384^2 x 256 (0.26/0.50 against 0.29/0.52 ms),
+  // 8 at 768^2 x 512 (2.4/4.9 against 4.0/14.0 ms).  HST_FFT_PPT_Z overrides.
   auto ppt_of = [](const char* name, int dflt) {
     const char* e = std::getenv(name);
     int v = e ? std::atoi(e) : dflt;
     return (v == 8 || v == 16) ? v : dflt;
   };
-  g.pptx = ppt_of("HST_FFT_PPT_X", 8);
   g.pptz = ppt_of("HST_FFT_PPT_Z", g.nzd >= 768 ? 8 : 16);
   // mixed precision: the FP32 transforms of the lengths it compiles
   // (8 points a thread, 16 at 96) and the streamed right-hand sides
@@ -372,7 +369,6 @@ static int choose_geometry(const hst_gpu_params& p, Geometry& g, std::string& wh
       why = "mixed precision needs 2 nxd and nzd in {96, 192, 384, 768, 1536} and ny a multiple of 32";
       return HST_EARG;
     }
-    g.pptx = 8;
     // 16 points a thread for the FP32 z transforms (zfwd 0.29 against 0.34 ms at 384)
     g.pptz = g.nzd == 768 ? 8 : ppt_of("HST_FFT_PPT_Z", 16);
   }
@@ -576,8 +572,8 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ctx->ps.beta0 = p.beta0;
   ctx->ps.ni = 1.0 / p.re;
   ctx->ps.S = p.S;
-  ctx->ps.dx = PI / (p.alfa0 * g.nxd);
-  ctx->ps.dz = 2.0 * PI / (p.beta0 * g.nzd);
+  ctx->ps.rdx = p.alfa0 * g.nxd / PI;
+  ctx->ps.rdz = p.beta0 * g.nzd / (2.0 * PI);
   ctx->ps.factor = 1.0 / (2.0 * g.nxd * g.nzd);
   // grid (src/hst_setup.f90:42-71)
   const int ny = p.ny;
@@ -626,9 +622,9 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ok = ok && alloc((void**)&d.y, sizeof(double) * (ny + 4));
   ok = ok && alloc((void**)&d.dyl, sizeof(double) * ny);
   ok = ok && alloc((void**)&d.gdamp, sizeof(double) * g.ncol);
-  ok = ok && alloc((void**)&d.twx, sizeof(double2) * 4 * g.nxd);
+  ok = ok && alloc((void**)&d.twx, sizeof(double2) * 6 * g.nxd);
   ok = ok && alloc((void**)&d.twz, sizeof(double2) * g.nzd);
-  ok = ok && alloc((void**)&d.twxf, sizeof(float2) * 4 * g.nxd);
+  ok = ok && alloc((void**)&d.twxf, sizeof(float2) * 6 * g.nxd);
   ok = ok && alloc((void**)&d.twzf, sizeof(float2) * g.nzd);
   // outstats scratch (sized for the largest reduction grid, 4 blocks an SM of up to 256 SMs)
   ok = ok && alloc((void**)&d.stats, sizeof(double) * ((hst::stats_partials() + 3) * 4 * 256 + 24));
@@ -662,17 +658,17 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   cudaMemcpy(d.y, ctx->y.data(), sizeof(double) * (ny + 4), cudaMemcpyHostToDevice);
   cudaMemcpy(d.dyl, ctx->dyl.data(), sizeof(double) * ny, cudaMemcpyHostToDevice);
   cudaMemcpy(d.gdamp, ctx->gdamp.data(), sizeof(double) * g.ncol, cudaMemcpyHostToDevice);
-  tx.resize((size_t)4 * g.nxd, make_double2(0.0, 0.0));
-  hst::staged_twiddles(2 * g.nxd, tx.data() + 2 * g.nxd);
+  tx.resize((size_t)6 * g.nxd, make_double2(0.0, 0.0));
+  hst::x_twiddles(2 * g.nxd, tx.data() + 2 * g.nxd);
   cudaMemcpy(d.twx, tx.data(), sizeof(double2) * tx.size(), cudaMemcpyHostToDevice);
   {
     // FP32 copies (rounded from the long double values)
-    std::vector<float2> fx((size_t)4 * g.nxd, make_float2(0.f, 0.f)), fz(g.nzd);
+    std::vector<float2> fx((size_t)6 * g.nxd, make_float2(0.f, 0.f)), fz(g.nzd);
     for (int k = 0; k < 2 * g.nxd; ++k) {
       long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)(2 * g.nxd);
       fx[k] = make_float2((float)cosl(a), (float)sinl(a));
     }
-    hst::staged_twiddles(2 * g.nxd, fx.data() + 2 * g.nxd);
+    hst::x_twiddles(2 * g.nxd, fx.data() + 2 * g.nxd);
     for (int k = 0; k < g.nzd; ++k) {
       long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)g.nzd;
       fz[k] = make_float2((float)cosl(a), (float)sinl(a));
@@ -682,15 +678,13 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   }
   cudaMemcpy(d.twz, tz.data(), sizeof(double2) * tz.size(), cudaMemcpyHostToDevice);
   cudaError_t e = etab;
-  if (e == cudaSuccess) e = hst::set_fft_constants();
-  // the base of all members (maps over nmem members), then member 0's view
+  // the base of all members; d is member 0's view
   ctx->gb = g;
   ctx->gb.nmem = nmem;
-  if (e == cudaSuccess) {
-    ctx->db = d;
-    e = hst::make_transform_maps(ctx->gb, ctx->db);
-  }
-  if (e == cudaSuccess) e = hst::make_transform_maps(g, d);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, p.device);
+  ctx->db = d;
+  if (e == cudaSuccess) e = hst::make_x_maps(ctx->gb, ctx->db);
+  if (e == cudaSuccess) e = hst::make_x_maps(g, d);
   if (e == cudaSuccess) e = ensure_facg(ctx);
   if (e == cudaSuccess) ctx->db.facg = d.facg, ctx->db.facg_doubles = d.facg_doubles;
   {
@@ -743,8 +737,7 @@ extern "C" int hst_gpu_select_member(hst_ctx* ctx, int m) {
   d.Zg = off(b.Zg, 3 * (size_t)g.nzd * g.nxB * 4);
   d.Ppg = off(b.Ppg, 6 * (size_t)g.nzd * g.nxB * 4);
   d.Qg = off(b.Qg, 6 * (size_t)g.ncol * 4);
-  CK(cudaStreamSynchronize(ctx->stream));  // the maps are kernel arguments of work already queued
-  CK(hst::make_transform_maps(g, d));
+  CK(hst::make_x_maps(g, d));
   ctx->member = m;
   return HST_OK;
 }
@@ -1079,7 +1072,7 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat);
 
 // ------------------------------------------------------------ autotune ----
 // Tries the launch choices that leave every buffer's layout unchanged -- the
-// lanes of a line-solver group (P) and the points a thread of the x and z
+// lanes of a line-solver group (P) and the points a thread of the z
 // FFT plans -- on this context's own sizes, `steps` time steps each after
 // one untimed step, keeps the fastest, and puts the fields and the time back
 // as they were.  The report lists every candidate with its time a step.
@@ -1118,14 +1111,7 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
     t.MS = t.m | 1;
     if (hst::column_smem_bytes(t, 1) <= 200 * 1024) lanes.push_back(c);
   }
-  const int NX = 2 * g0.nxd;
-  std::vector<int> px, pz;
-  if (g0.mp) {
-    px.push_back(8);
-  } else {
-    px.push_back(16);
-    if (NX == 192 || NX == 384 || NX == 768) px.push_back(8);
-  }
+  std::vector<int> pz;
   for (int v : {16, 8}) {
     if (g0.mp && g0.nzd == 768 && v == 16) continue;
     if (v == 8 && !(g0.nzd == 192 || g0.nzd == 384 || g0.nzd == 768)) continue;
@@ -1145,41 +1131,38 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
     auto ds = slab_major(ctx->der, g.ny, g.P, g.m);
     cudaError_t e = cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * 20 * g.ny, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = hst::launch_d0_table(g, ctx->d, ctx->stream);
-    if (e == cudaSuccess) e = hst::make_transform_maps(g, ctx->d);
     if (e == cudaSuccess) e = ensure_facg(ctx);
     return e;
   };
   for (int P : lanes)
-    for (int a : px)
-      for (int b : pz) {
-        Geometry t = g0;
-        t.P = P;
-        t.m = g0.ny / P;
-        t.MS = t.m | 1;
-        t.pptx = a;
-        t.pptz = b;
-        if (apply(t) != cudaSuccess) continue;
-        for (int i = 0; i < 5 && rc == HST_OK; ++i)
-          if (cudaMemcpyAsync(ctx->d.F[i], save[i], fb, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-            rc = HST_ECUDA;
-        double tt = time0;
-        if (rc == HST_OK) rc = queue_timestep(ctx, &tt, deltat);
-        if (rc == HST_OK && cudaEventRecord(e0, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
-        for (int k = 0; k < steps && rc == HST_OK; ++k) rc = queue_timestep(ctx, &tt, deltat);
-        if (rc == HST_OK && cudaEventRecord(e1, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
-        if (rc == HST_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = HST_ECUDA;
-        if (rc != HST_OK) break;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        const double per = ms / steps;
-        char line[128];
-        std::snprintf(line, sizeof line, "P=%d x=%d z=%d: %.4f ms a step\n", P, a, b, per);
-        rep += line;
-        if (per < best) {
-          best = per;
-          gbest = t;
-        }
+    for (int b : pz) {
+      Geometry t = g0;
+      t.P = P;
+      t.m = g0.ny / P;
+      t.MS = t.m | 1;
+      t.pptz = b;
+      if (apply(t) != cudaSuccess) continue;
+      for (int i = 0; i < 5 && rc == HST_OK; ++i)
+        if (cudaMemcpyAsync(ctx->d.F[i], save[i], fb, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
+          rc = HST_ECUDA;
+      double tt = time0;
+      if (rc == HST_OK) rc = queue_timestep(ctx, &tt, deltat);
+      if (rc == HST_OK && cudaEventRecord(e0, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
+      for (int k = 0; k < steps && rc == HST_OK; ++k) rc = queue_timestep(ctx, &tt, deltat);
+      if (rc == HST_OK && cudaEventRecord(e1, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
+      if (rc == HST_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = HST_ECUDA;
+      if (rc != HST_OK) break;
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, e0, e1);
+      const double per = ms / steps;
+      char line[128];
+      std::snprintf(line, sizeof line, "P=%d z=%d: %.4f ms a step\n", P, b, per);
+      rep += line;
+      if (per < best) {
+        best = per;
+        gbest = t;
       }
+    }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   // the winner, and the state as it was
@@ -1194,7 +1177,7 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   }
   if (rc != HST_OK) return rc;
   char line[128];
-  std::snprintf(line, sizeof line, "chosen: P=%d x=%d z=%d\n", g.P, g.pptx, g.pptz);
+  std::snprintf(line, sizeof line, "chosen: P=%d z=%d\n", g.P, g.pptz);
   rep += line;
   if (report && report_len > 0) std::snprintf(report, (size_t)report_len, "%s", rep.c_str());
   return HST_OK;

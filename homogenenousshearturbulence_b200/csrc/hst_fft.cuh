@@ -11,10 +11,10 @@
 // three stages.  Threads are mapped line-fastest so that global accesses of
 // consecutive threads touch consecutive lines (the y rows, contiguous in
 // memory); shared lines have an odd stride against bank conflicts.
-// Stage twiddles come from W[e] = exp(-2 pi i e / N) in global memory, the
-// twiddles inside a register DFT from a 48-entry table in constant memory
-// (all threads read the same entry).  Both tables are computed on the host
-// in extended precision.  Unnormalised both ways, like the reference's FFTW
+// Stage twiddles come from W[e] = exp(-2 pi i e / N) in global memory
+// (computed on the host in extended precision), the twiddles inside a
+// register DFT from a 48-entry table in constant memory (all threads read
+// the same entry).  Unnormalised both ways, like the reference's FFTW
 // and cuFFT plans (src/hst_fft.f90:98-121): S = -1 forward, S = +1 backward.
 #pragma once
 #include <type_traits>
@@ -25,16 +25,73 @@ namespace hst {
 
 #define HST_SQRT3_2 0.86602540378443864676
 
-// exp(-2 pi i k / 48), k = 0..47, in both precisions (set per device by
-// set_fft_constants; this header is included by one translation unit only)
-__constant__ double2 c_w48[48];
-__constant__ float2 c_w48f[48];
+// exp(-2 pi i k / 48), k = 0..47, rounded from extended precision (one copy
+// in the constant memory of each translation unit that includes this header)
+static __constant__ double2 c_w48[48] = {
+    {1.0, 0.0}, {0.9914448613738104, -0.1305261922200516},
+    {0.9659258262890683, -0.25881904510252074}, {0.9238795325112867, -0.3826834323650898},
+    {0.8660254037844386, -0.5}, {0.7933533402912352, -0.6087614290087207},
+    {0.7071067811865476, -0.7071067811865476}, {0.6087614290087207, -0.7933533402912352},
+    {0.5, -0.8660254037844386}, {0.3826834323650898, -0.9238795325112867},
+    {0.25881904510252074, -0.9659258262890683}, {0.1305261922200516, -0.9914448613738104},
+    {0.0, -1.0}, {-0.1305261922200516, -0.9914448613738104},
+    {-0.25881904510252074, -0.9659258262890683}, {-0.3826834323650898, -0.9238795325112867},
+    {-0.5, -0.8660254037844386}, {-0.6087614290087207, -0.7933533402912352},
+    {-0.7071067811865476, -0.7071067811865476}, {-0.7933533402912352, -0.6087614290087207},
+    {-0.8660254037844386, -0.5}, {-0.9238795325112867, -0.3826834323650898},
+    {-0.9659258262890683, -0.25881904510252074}, {-0.9914448613738104, -0.1305261922200516},
+    {-1.0, 0.0}, {-0.9914448613738104, 0.1305261922200516},
+    {-0.9659258262890683, 0.25881904510252074}, {-0.9238795325112867, 0.3826834323650898},
+    {-0.8660254037844386, 0.5}, {-0.7933533402912352, 0.6087614290087207},
+    {-0.7071067811865476, 0.7071067811865476}, {-0.6087614290087207, 0.7933533402912352},
+    {-0.5, 0.8660254037844386}, {-0.3826834323650898, 0.9238795325112867},
+    {-0.25881904510252074, 0.9659258262890683}, {-0.1305261922200516, 0.9914448613738104},
+    {0.0, 1.0}, {0.1305261922200516, 0.9914448613738104},
+    {0.25881904510252074, 0.9659258262890683}, {0.3826834323650898, 0.9238795325112867},
+    {0.5, 0.8660254037844386}, {0.6087614290087207, 0.7933533402912352},
+    {0.7071067811865476, 0.7071067811865476}, {0.7933533402912352, 0.6087614290087207},
+    {0.8660254037844386, 0.5}, {0.9238795325112867, 0.3826834323650898},
+    {0.9659258262890683, 0.25881904510252074}, {0.9914448613738104, 0.1305261922200516}};
+static __constant__ float2 c_w48f[48] = {
+    {1.0f, 0.0f}, {0.991444886f, -0.130526185f}, {0.965925813f, -0.258819044f}, {0.923879504f, -0.382683426f},
+    {0.866025388f, -0.5f}, {0.793353319f, -0.60876143f}, {0.707106769f, -0.707106769f}, {0.60876143f, -0.793353319f},
+    {0.5f, -0.866025388f}, {0.382683426f, -0.923879504f}, {0.258819044f, -0.965925813f}, {0.130526185f, -0.991444886f},
+    {0.0f, -1.0f}, {-0.130526185f, -0.991444886f}, {-0.258819044f, -0.965925813f}, {-0.382683426f, -0.923879504f},
+    {-0.5f, -0.866025388f}, {-0.60876143f, -0.793353319f}, {-0.707106769f, -0.707106769f}, {-0.793353319f, -0.60876143f},
+    {-0.866025388f, -0.5f}, {-0.923879504f, -0.382683426f}, {-0.965925813f, -0.258819044f}, {-0.991444886f, -0.130526185f},
+    {-1.0f, 0.0f}, {-0.991444886f, 0.130526185f}, {-0.965925813f, 0.258819044f}, {-0.923879504f, 0.382683426f},
+    {-0.866025388f, 0.5f}, {-0.793353319f, 0.60876143f}, {-0.707106769f, 0.707106769f}, {-0.60876143f, 0.793353319f},
+    {-0.5f, 0.866025388f}, {-0.382683426f, 0.923879504f}, {-0.258819044f, 0.965925813f}, {-0.130526185f, 0.991444886f},
+    {0.0f, 1.0f}, {0.130526185f, 0.991444886f}, {0.258819044f, 0.965925813f}, {0.382683426f, 0.923879504f},
+    {0.5f, 0.866025388f}, {0.60876143f, 0.793353319f}, {0.707106769f, 0.707106769f}, {0.793353319f, 0.60876143f},
+    {0.866025388f, 0.5f}, {0.923879504f, 0.382683426f}, {0.965925813f, 0.258819044f}, {0.991444886f, 0.130526185f}};
 template <typename C>
 __device__ __forceinline__ C w48(int i);
 template <>
 __device__ __forceinline__ double2 w48<double2>(int i) { return c_w48[i]; }
 template <>
 __device__ __forceinline__ float2 w48<float2>(int i) { return c_w48f[i]; }
+
+// t exp(S 2 pi i e / 48), e known at compile time: quarter turns are free and
+// odd eighths take two multiplications
+template <int S, typename C>
+__device__ __forceinline__ C mul_w48(C t, int e) {
+  typedef typename RealOf<C>::T T;
+  if (e == 0) return t;
+  if (e == 12) return S < 0 ? C{t.y, -t.x} : C{-t.y, t.x};
+  if (e == 24) return C{-t.x, -t.y};
+  if (e == 36) return S < 0 ? C{-t.y, t.x} : C{t.y, -t.x};
+  if (e % 6 == 0) {
+    const T h = T(0.70710678118654752440);
+    const T p = h * (t.x + t.y), m = h * (t.y - t.x);
+    const int q = e / 6;  // exp(-i pi q / 4) = (+-1 -+ i) / sqrt 2
+    if (S < 0) return q == 1 ? C{p, m} : (q == 3 ? C{m, -p} : (q == 5 ? C{-p, -m} : C{-m, p}));
+    return q == 1 ? C{-m, p} : (q == 3 ? C{-p, -m} : (q == 5 ? C{m, -p} : C{p, m}));
+  }
+  C w = w48<C>(e);
+  if (S > 0) w.y = -w.y;
+  return cmul(t, w);
+}
 
 template <int R, int S>
 struct DFT;
@@ -87,13 +144,7 @@ __device__ __forceinline__ void dft_ab(C* v) {
     DFT<A, S>::run(t);
 #pragma unroll
     for (int ka = 0; ka < A; ++ka) {
-      if (b * ka == 0) {
-        v[b + B * ka] = t[ka];
-      } else {
-        C w = w48<C>((b * ka * (48 / (A * B))) % 48);
-        if (S > 0) w.y = -w.y;
-        v[b + B * ka] = cmul(t[ka], w);
-      }
+      v[b + B * ka] = mul_w48<S>(t[ka], (b * ka * (48 / (A * B))) % 48);
     }
   }
 #pragma unroll
@@ -170,12 +221,9 @@ struct ShLinesT {
   __device__ __forceinline__ C operator()(int l, int i) const { return p[l * LS + i]; }
   __device__ __forceinline__ void operator()(int l, int i, C v) const { p[l * LS + i] = v; }
 };
-typedef ShLinesT<cxd> ShLines;
-// The same with one pad element after every 8: with butterflies mapped
-// index-fastest (JF) the radix-8/6/12 exchanges of the 8-point plans are
-// then free of bank conflicts.  Line stride ls_padded(N).
-// (SH: one pad element in 2^SH; 3 for the 8-point plans, 4 for the
-// 16-point plans of the z kernels, whose first radix is 16)
+// The same with one pad element after every 2^SH (3 for the 8-point plans, 4
+// for the 16-point plans of the z kernels, whose first radix is 16), at the
+// line stride ls_lines
 template <typename C, int SH = 3>
 struct ShLinesPT {
   C* p;
@@ -183,9 +231,7 @@ struct ShLinesPT {
   __device__ __forceinline__ C operator()(int l, int i) const { return p[l * LS + i + (i >> SH)]; }
   __device__ __forceinline__ void operator()(int l, int i, C v) const { p[l * LS + i + (i >> SH)] = v; }
 };
-typedef ShLinesPT<cxd> ShLinesP;
-__host__ __device__ constexpr int ls_padded(int N) { return N + N / 8 + 1; }
-// The line stride of the same padded layout under the line-fastest mapping
+// The line stride of the padded layout under the line-fastest mapping
 // of the z kernels (butterfly b: line b % nl, index b / nl, so that the
 // global loads and stores of nl adjacent rows coalesce): a wavefront's
 // lanes cover nl lines times S/nl consecutive indices (S = 128 / sizeof(C)
@@ -204,10 +250,7 @@ __host__ __device__ inline int ls_lines(int N, int nl) {
 // j = b / nl.  Inputs ld(l, j + r N/R), outputs st(l, (j/Ns) Ns R + j%Ns + r Ns).
 // SYNC: the stage reads and writes the same shared lines (all reads, then
 // a barrier, then all writes).
-// JF also selects the staged twiddle table: tw points at this stage's
-// block [r - 1][kk] of W^(kk r N/(Ns R)), r = 1..R-1, kk = 0..Ns-1, so that
-// a warp's twiddle loads are contiguous.
-template <int R, int S, int PPT, bool SYNC, typename LD, typename ST, bool JF = false, typename C = cxd>
+template <int R, int S, int PPT, bool SYNC, typename LD, typename ST, typename C = cxd>
 __device__ __forceinline__ void fft_stage_io(int N, int nl, int Ns, const C* __restrict__ tw, const LD& ld,
                                              const ST& st) {
   constexpr int MAXB = (PPT + R - 1) / R;
@@ -221,13 +264,13 @@ __device__ __forceinline__ void fft_stage_io(int N, int nl, int Ns, const C* __r
     int b = threadIdx.x + k * blockDim.x;
     lj[k] = -1;
     if (b < total) {
-      int l = JF ? b / nb : b % nl, j = JF ? b % nb : b / nl;
+      int l = b % nl, j = b / nl;
       int kk = j % Ns;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         C x = ld(l, j + r * nb);
         if (r > 0 && kk > 0) {
-          C w = JF ? __ldg(tw + (r - 1) * Ns + kk) : __ldg(tw + kk * r * tstride);
+          C w = __ldg(tw + kk * r * tstride);
           if (S > 0) w.y = -w.y;
           x = cmul(x, w);
         }
@@ -241,7 +284,7 @@ __device__ __forceinline__ void fft_stage_io(int N, int nl, int Ns, const C* __r
 #pragma unroll
   for (int k = 0; k < MAXB; ++k) {
     if (lj[k] >= 0) {
-      int l = JF ? lj[k] / nb : lj[k] % nl, j = JF ? lj[k] % nb : lj[k] / nl;
+      int l = lj[k] % nl, j = lj[k] / nl;
       int kk = j % Ns;
       int base = (j / Ns) * Ns * R + kk;
 #pragma unroll
@@ -322,57 +365,37 @@ template <> struct Plan8<384> { static constexpr int n = 3, r0 = 8, r1 = 8, r2 =
 template <> struct Plan8<768> { static constexpr int n = 3, r0 = 8, r1 = 8, r2 = 12; };
 
 // PZ: the padded lines at stride ls_lines under the line-fastest mapping.
-// PP (three-stage plans): the second stage writes a second set of nl lines
-// at sh2 and the third reads them, so that neither stage reads and writes
-// the same lines (two barriers fewer); src must not overlap the lines at sh
-// and dst not those at sh2.
-// XSH > 0: the caller's padded layout, one pad in 2^XSH at line stride lsx;
-// with JF, lsx > 0 is the stride of the padded lines (at least ls_padded).
-template <int N, int S, int PPT, bool SRC_SH, bool DST_SH, bool JF, bool PZ, bool PP, int XSH, typename LD,
-          typename ST, typename C>
-__device__ __forceinline__ void fft_fixed(int nl, const C* __restrict__ tw, C* sh, const LD& src, const ST& dst,
-                                          C* sh2, int lsx) {
+template <int N, int S, int PPT, bool PZ, typename LD, typename ST, typename C>
+__device__ __forceinline__ void fft_fixed(int nl, const C* __restrict__ tw, C* sh, const LD& src, const ST& dst) {
   using PL = std::conditional_t<(PPT <= 8), Plan8<N>, Plan<N>>;
   static_assert(PL::n > 0, "no compile-time plan for this length and points per thread");
-  static_assert(!(JF && (PZ || XSH > 0)), "PZ and XSH are the line-fastest mapping's layouts");
-  // the pad follows the plan's first radix (8 or 16), or the caller's
-  constexpr int PSH = XSH > 0 ? XSH : (PPT <= 8 ? 3 : 4);
-  using LT = std::conditional_t<JF, ShLinesPT<C>, std::conditional_t<(PZ || XSH > 0), ShLinesPT<C, PSH>, ShLinesT<C>>>;
-  const LT L = {sh, JF ? (lsx > 0 ? lsx : ls_padded(N)) : (XSH > 0 ? lsx : (PZ ? ls_lines<C, PSH>(N, nl) : N + 1))};
+  constexpr int PSH = PPT <= 8 ? 3 : 4;  // the pad follows the plan's first radix (8 or 16)
+  using LT = std::conditional_t<PZ, ShLinesPT<C, PSH>, ShLinesT<C>>;
+  const LT L = {sh, PZ ? ls_lines<C, PSH>(N, nl) : N + 1};
   if constexpr (PL::n == 1) {
-    fft_stage_io<PL::r0, S, PPT, SRC_SH && DST_SH, LD, ST, JF, C>(N, nl, 1, tw, src, dst);
+    fft_stage_io<PL::r0, S, PPT, false>(N, nl, 1, tw, src, dst);
   } else if constexpr (PL::n == 2) {
-    fft_stage_io<PL::r0, S, PPT, SRC_SH, LD, LT, JF, C>(N, nl, 1, tw, src, L);
+    fft_stage_io<PL::r0, S, PPT, false>(N, nl, 1, tw, src, L);
     __syncthreads();
-    fft_stage_io<PL::r1, S, PPT, DST_SH, LT, ST, JF, C>(N, nl, PL::r0, tw, L, dst);
+    fft_stage_io<PL::r1, S, PPT, false>(N, nl, PL::r0, tw, L, dst);
   } else {
-    // staged table (JF): stage 2's block first, then stage 3's
-    const C* tw3 = JF ? tw + (PL::r1 - 1) * PL::r0 : tw;
-    fft_stage_io<PL::r0, S, PPT, SRC_SH, LD, LT, JF, C>(N, nl, 1, tw, src, L);
+    fft_stage_io<PL::r0, S, PPT, false>(N, nl, 1, tw, src, L);
     __syncthreads();
-    if constexpr (PP) {
-      const LT L2 = {sh2, L.LS};
-      fft_stage_io<PL::r1, S, PPT, false, LT, LT, JF, C>(N, nl, PL::r0, tw, L, L2);
-      __syncthreads();
-      fft_stage_io<PL::r2, S, PPT, false, LT, ST, JF, C>(N, nl, PL::r0 * PL::r1, tw3, L2, dst);
-    } else {
-      fft_stage_io<PL::r1, S, PPT, true, LT, LT, JF, C>(N, nl, PL::r0, tw, L, L);
-      __syncthreads();
-      fft_stage_io<PL::r2, S, PPT, DST_SH, LT, ST, JF, C>(N, nl, PL::r0 * PL::r1, tw3, L, dst);
-    }
+    fft_stage_io<PL::r1, S, PPT, true>(N, nl, PL::r0, tw, L, L);
+    __syncthreads();
+    fft_stage_io<PL::r2, S, PPT, false>(N, nl, PL::r0 * PL::r1, tw, L, dst);
   }
 }
 
 // NT > 0: the compile-time plan of length NT; NT = 0: the runtime plan of N.
-template <int NT, int S, int PPT, bool SRC_SH, bool DST_SH, bool JF = false, bool PZ = false, bool PP = false,
-          int XSH = 0, typename LD, typename ST, typename C>
+template <int NT, int S, int PPT, bool PZ, typename LD, typename ST, typename C>
 __device__ __forceinline__ void fft_sel(int N, int nl, const C* __restrict__ tw, C* sh, const LD& src,
-                                        const ST& dst, C* sh2 = nullptr, int lsx = 0) {
-  static_assert(!(PZ || PP || XSH > 0) || NT > 0, "PZ, PP and XSH need a compile-time plan");
+                                        const ST& dst) {
+  static_assert(!PZ || NT > 0, "PZ needs a compile-time plan");
   if constexpr (NT > 0) {
-    fft_fixed<NT, S, PPT, SRC_SH, DST_SH, JF, PZ, PP, XSH>(nl, tw, sh, src, dst, sh2, lsx);
+    fft_fixed<NT, S, PPT, PZ>(nl, tw, sh, src, dst);
   } else {
-    fft_global<S, PPT, SRC_SH, DST_SH>(N, nl, tw, sh, src, dst);
+    fft_global<S, PPT, false, false>(N, nl, tw, sh, src, dst);
   }
 }
 

@@ -21,7 +21,7 @@ struct Geometry {
   long nf;             // complex elements of one field (ncol * rows)
   int P, m, MS;        // line-solve group: P lanes, m rows per lane, slab stride
   int Ty;              // y tile of the transforms (divides ny)
-  int pptx, pptz;      // FFT points per thread of the x and z transforms (8: the low-register plans)
+  int pptz;            // FFT points per thread of the z transforms (8: the low-register plans)
   int mp;              // mixed precision: Z, Pp, Q and their transforms in FP32 (complex64)
   // 0, or (in the view of the four ghost rows that the edge transforms take)
   // ny: the z-inverse then reads rows -2, -1, ny, ny+1 of V
@@ -48,22 +48,18 @@ struct DeviceState {
   double* y;            // y(-2:ny+1)
   double* dyl;          // dyl(0:ny-1)
   double* gdamp;        // gdamp(-nz:nz, 0:nx)
-  double2* twx;         // exp(-2 pi i e / (2 nxd)), then the staged table of the x kernel's 8-point plan
+  double2* twx;         // exp(-2 pi i e / (2 nxd)), then the x plan's tables (x_twiddles)
   double2* twz;         // exp(-2 pi i e / nzd)
   float2* twxf;         // the same tables in FP32 (mixed precision)
   float2* twzf;
   unsigned long long* cfl;  // running max (bits of a non-negative double)
   int* err;                 // set by a kernel whose bounded wait ran out
-  // TMA maps of Z and Pp as 4-D f64 tensors {2 Ty, nxB, nzd ny/Ty, comps}
-  // (set by make_transform_maps when the x kernel's 8-point plan uses them)
-  CUtensorMap tmZ, tmPp;
-  bool maps;
+  CUtensorMap tmZ, tmPp, tmZg, tmPpg;  // TMA maps of Z, Pp and the ghost rows' buffers (make_x_maps)
   // The products of the four ghost rows (-2, -1, ny, ny+1) transformed like
   // the interior ones (null when their shear-periodic images are exact):
   // Zg [3][nzd][nxB][4], Ppg [6][nzd][nxB][4], Qg [6][ncol][4], in the
-  // transforms' precision, with their TMA maps
+  // transforms' precision
   double2 *Zg, *Ppg, *Qg;
-  CUtensorMap tmZg, tmPpg;
   int nsm;        // SMs of the device
   double* stats;  // outstats scratch: block partials of the moments (stats_partials() a block),
                   // of the three gradients (one a block each), then the 24 results
@@ -126,7 +122,7 @@ struct SubstepScalars {
 
 struct PhysScalars {
   double alfa0, beta0, ni, S;
-  double dx, dz, factor;
+  double rdx, rdz, factor;  // 1/dx, 1/dz, 1/(2 nxd nzd)
 };
 
 cudaError_t launch_zinv(const Geometry& g, const DeviceState& d, cudaStream_t st);
@@ -187,16 +183,15 @@ cudaError_t launch_shift_default(const Geometry& g, const DeviceState& d, const 
 // nzd = 3 nz, the retained modes iz = +-nz alias product modes -+2nz, whose
 // wrap phases differ
 bool edge_rows_needed(const Geometry& g, bool s2_active);
-// the TMA maps of Z and Pp for the x kernel (d.maps false when not used)
-cudaError_t make_transform_maps(const Geometry& g, DeviceState& d);
-// the stage-ordered twiddles of the 8-point plan of N into out (at most N
-// entries); returns their number, 0 for a length without such a plan
-int staged_twiddles(int N, double2* out);
-int staged_twiddles(int N, float2* out);
+// the x stage of the lengths with a compiled plan (hst_xprod.cu), the TMA maps
+// of Z and Pp that it uses, its twiddle tables (at most 2 N entries into out; their number, 0 without one)
+bool x_compiled(int N, bool fp32);
+cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, cudaStream_t st);
+cudaError_t make_x_maps(const Geometry& g, DeviceState& d);
+int x_twiddles(int N, double2* out);
+int x_twiddles(int N, float2* out);
 // a transform length of the mixed-precision form
 bool mp_length_ok(int n);
-// the constant twiddles of the register DFTs, once per device
-cudaError_t set_fft_constants();
 // a transform length the FFT kernels support
 bool fft_length_ok(int n);
 

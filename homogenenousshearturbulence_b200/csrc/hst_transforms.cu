@@ -22,19 +22,6 @@
 
 namespace hst {
 
-cudaError_t set_fft_constants() {
-  double2 w[48];
-  float2 wf[48];
-  for (int k = 0; k < 48; ++k) {
-    long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / 48.0L;
-    w[k] = make_double2((double)cosl(a), (double)sinl(a));
-    wf[k] = make_float2((float)cosl(a), (float)sinl(a));
-  }
-  cudaError_t e = cudaMemcpyToSymbol(c_w48, w, sizeof w);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_w48f, wf, sizeof wf);
-  return e;
-}
-
 bool fft_length_ok(int n) { return plan_ok(n); }
 
 #ifndef ZPAD16
@@ -122,7 +109,7 @@ __device__ __forceinline__ void zinv_body(const Geometry& g, const double2* __re
   const ZinvSrc<C> src = {V + (size_t)ix * g.nzT * g.rows + (g.edge_gap ? 0 : 2) + yt * Ty, g.rows, g.nz, NZ,
                           g.edge_gap};
   const TileDst<C> dst = {Z + (((size_t)c * nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
-  fft_sel<NT, +1, PPT, false, false, false, z_padded<NT, PPT, C>()>(NZ, Ty, twz, sh, src, dst);
+  fft_sel<NT, +1, PPT, z_padded<NT, PPT, C>()>(NZ, Ty, twz, sh, src, dst);
 }
 template <int NT, int PPT, typename C>
 __global__ void __launch_bounds__(PPT <= 8 ? 512 : 256)
@@ -182,7 +169,7 @@ __global__ void __launch_bounds__(PPT <= 8 ? 384 : (PPT == 32 && NT > 0 ? 192 : 
   Q += (size_t)mem * 6 * g.ncol * g.ny;
   const TileSrc<C> src = {Pp + (((size_t)p * nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
   const ZfwdDst<C> dst = {Q + ((size_t)p * g.ncol + (size_t)ix * g.nzT) * g.ny + yt * Ty, g.ny, g.nz, NZ};
-  fft_sel<NT, -1, PPT, false, false, false, z_padded<NT, PPT, C>()>(NZ, Ty, twz, sh, src, dst);
+  fft_sel<NT, -1, PPT, z_padded<NT, PPT, C>()>(NZ, Ty, twz, sh, src, dst);
 }
 
 // -------------------------------------------------------------- k_xprod ----
@@ -218,31 +205,6 @@ struct XinvSrc {
     return C{a.x + b.y, b.x - a.y};  // conj(a) + i conj(b)
   }
 };
-// The same from the block's staging copy of the tile, [comp 3][nxB][row 2]
-// (landed by TMA)
-template <typename C>
-struct XinvSh {
-  const C* s;
-  int nxB, nx, NX;
-  __device__ __forceinline__ C operator()(int l, int k) const {
-    const int m = k <= nx ? k : (k >= NX - nx ? NX - k : -1);
-    if (m < 0) return C{0, 0};
-    C a, b;
-    if (l == 0) {
-      a = s[2 * m];
-      b = s[2 * (nxB + m)];
-    } else if (l == 1) {
-      a = s[2 * m + 1];
-      b = s[2 * (nxB + m) + 1];
-    } else {
-      a = s[2 * (2 * nxB + m)];
-      b = s[2 * (2 * nxB + m) + 1];
-    }
-    if (k == 0) return C{a.x, b.x};
-    if (k <= nx) return C{a.x - b.y, a.y + b.x};
-    return C{a.x + b.y, b.x - a.y};
-  }
-};
 // the products of row yy, pair pl (0: uu, vv; 1: ww, uv; 2: vw, uw) at x
 template <typename LT, typename C>
 struct ProdSrc {
@@ -259,80 +221,16 @@ struct ProdSrc {
   }
 };
 
-#ifndef XPROD_MINB
-#define XPROD_MINB 3
-#endif
-#ifndef XPROD_PP
-#define XPROD_PP 1
-#endif
-#ifndef XPAD1536
-#define XPAD1536 1
-#endif
-// line stride of the padded 1536-point x lines: 1728 + 3 (FP64) or + 11
-// (FP32), the strides that a CPU count of the plan's shared accesses ranks
-// best for three and six lines side by side
-__host__ __device__ constexpr int xls_1536(int elem) { return elem == 16 ? 1731 : 1739; }
-// launch bounds of k_xprod: 6 NX / PPT threads; the 8-point plan at 384
-// is held to 72 registers so that three 288-thread blocks fit an SM, the
-// FP32 32-point plan at 1536 to two blocks
-constexpr int xprod_threads(int NT, int PPT) {
-  return PPT <= 8 ? (NT == 384 ? 288 : (NT == 768 ? 576 : 640)) : (NT == 1536 ? 288 : 320);
-}
-#ifndef XPROD_MINB_768
-#define XPROD_MINB_768 2
-#endif
-#ifndef XPROD_MINB_F32
-#define XPROD_MINB_F32 4
-#endif
-constexpr int xprod_min_blocks(int NT, int PPT, int es) {
-  return PPT <= 8 && NT == 384 ? (es == 8 ? XPROD_MINB_F32 : XPROD_MINB) : ((NT == 1536 || NT == 768) && es == 8 ? 2 : (NT == 768 && PPT <= 8 ? XPROD_MINB_768 : 1));
-}
-
-constexpr int XPROD_WAIT_LIMIT = 1 << 22;  // polls of the tile's TMA barrier before giving up
-
-// shared layout of the TMA variant (double2 units): the six padded lines,
-// then the staging tile (in: [3][nxB][2], out: [6][nxB][2]) rounded up to
-// the next 128-byte address (tensor copies need 128-byte aligned shared
-// addresses, and the dynamic shared base is only known to be 16-byte
-// aligned), then the mbarrier and the tile flag
-// the x kernel's padded line stride: at least ls_padded(NX), and 3 LS half
-// a bank row modulo a bank row (S = 128 / elem elements), for the
-// separation's alternating reads of lines pl and pl + 3
-__host__ __device__ constexpr int ls_x(int NX, int elem) {
-  const int S = 128 / elem, base = ls_padded(NX);
-  return elem == 16 ? base + (((S / 2 - base) % S) + S) % S : base;
-}
-__host__ __device__ inline int xprod_stage_off(int NX, int elem) { return 6 * ls_x(NX, elem); }
-__host__ __device__ inline size_t xprod_tma_smem(int NX, int nxB, size_t elem) {
-  return ((size_t)xprod_stage_off(NX, (int)elem) + 12 * (size_t)nxB + 2) * elem + 128;
-}
-// At 768 points the staging tiles live inside the six lines instead (the
-// tile in where lines 3..5 are, which the three inverse lines never touch;
-// the tile out over the lines once they have been read), so that a block
-// needs 6 padded lines of shared memory and two blocks share an SM
-__host__ __device__ constexpr bool xprod_alias(int NT, int PPT) { return PPT <= 8 && NT == 768; }
-__host__ __device__ inline size_t xprod_alias_smem(int NX, size_t elem) {
-  return (size_t)6 * ls_x(NX, (int)elem) * elem + 128;
-}
-
-template <int NT, int PPT, typename C>
-__global__ void __launch_bounds__(xprod_threads(NT, PPT), xprod_min_blocks(NT, PPT, (int)sizeof(C)))
-    k_xprod(Geometry g, const C* __restrict__ Z, C* __restrict__ Pp, const C* __restrict__ twx,
-            const double* __restrict__ dyl, PhysScalars ps, int want_cfl, unsigned long long* __restrict__ cflmax,
-            const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmP, int* __restrict__ err) {
-  typedef typename RealOf<C>::T T;
-  extern __shared__ double2 sh_d[];
-  C* sh = reinterpret_cast<C*>(sh_d);
-  // 8-point plans: butterflies index-fastest over padded shared lines, the
-  // tile in and out by TMA
-  constexpr bool JF = (PPT <= 8 && NT > 0);
-  // the 1536-point plan (butterflies line-fastest): lines padded one in
-  // eight at the stride xls_1536 (fewer bank conflicts for both the three
-  // inverse and the six forward lines)
-  constexpr int XSH = (!JF && NT == 1536 && XPAD1536) ? 3 : 0;
-  using LT = std::conditional_t<JF, ShLinesPT<C>, std::conditional_t<XSH != 0, ShLinesPT<C, 3>, ShLinesT<C>>>;
+// The x stage of the lengths without a compiled plan (hst_xprod.cu), FP64,
+// with the runtime plan (PPT points a thread)
+template <int PPT>
+__global__ void __launch_bounds__(320)
+    k_xprod(Geometry g, const double2* __restrict__ Z, double2* __restrict__ Pp, const double2* __restrict__ twx,
+            const double* __restrict__ dyl, PhysScalars ps, int want_cfl, unsigned long long* __restrict__ cflmax) {
+  typedef double2 C;
+  extern __shared__ double2 sh[];
+  typedef ShLinesT<C> LT;
   const int NX = 2 * g.nxd, nx = g.nx, nxB = g.nxB, NZ = g.nzd, Ty = g.Ty;
-  const int LS = JF ? ls_x(NX, (int)sizeof(C)) : (XSH ? xls_1536((int)sizeof(C)) : NX + 1);
   const int nyT = g.ny / Ty;
   const int y0 = 2 * blockIdx.x, kz = blockIdx.y % g.nzd, mem = blockIdx.y / g.nzd;
   Z += (size_t)mem * 3 * g.nzd * g.ny * g.nxB;
@@ -340,55 +238,18 @@ __global__ void __launch_bounds__(xprod_threads(NT, PPT), xprod_min_blocks(NT, P
   const int yt = y0 / Ty, yi0 = y0 - yt * Ty;
   const size_t cs = (size_t)NZ * nyT * nxB * Ty;
   const size_t tile = ((size_t)yt * NZ + kz) * nxB * Ty;
-  const LT L = {sh, LS};
-  constexpr bool ALIAS = xprod_alias(NT, PPT);
-  auto align128 = [](C* q) { return q + ((128u - (smem_u32(q) & 127u)) & 127u) / sizeof(C); };
-  C* stg = ALIAS ? sh + 3 * LS : sh + xprod_stage_off(NX, (int)sizeof(C));
-  if constexpr (JF) stg = align128(stg);
-  C* const stg_out = ALIAS ? align128(sh) : stg;
-  __shared__ uint64_t bar_al;
-  __shared__ int tile_ok_al;
+  const LT L = {sh, NX + 1};
   // u + i v of both rows and w0 + i w1 on the physical x grid
-  if constexpr (JF) {
-    uint64_t* bar = ALIAS ? &bar_al : reinterpret_cast<uint64_t*>(stg + 12 * nxB);
-    int& tile_ok = ALIAS ? tile_ok_al : *reinterpret_cast<int*>(stg + 12 * nxB + 1);
-    if ((smem_u32(stg) & 127u) != 0) {  // never taken: the staging tile is aligned above
-      if (threadIdx.x == 0) atomicExch(err, 1);
-      return;
-    }
-    if (threadIdx.x == 0) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
-      mbar_arrive_expect_tx(bar, 3u * nxB * 2u * (unsigned)sizeof(C));
-      tma_load_4d(stg, &tmZ, 2 * yi0, 0, yt * NZ + kz, 3 * mem, bar);
-      bool ok = mbar_wait_bounded(bar, 0, XPROD_WAIT_LIMIT);
-      if (!ok) {
-        // record the failure and give the copy a second bounded wait
-        // before the block (and its shared memory) goes away
-        atomicExch(err, 1);
-        mbar_wait_bounded(bar, 0, XPROD_WAIT_LIMIT);
-      }
-      tile_ok = ok;
-    }
-    __syncthreads();
-    if (!tile_ok) return;
-    // the three inverse lines ping-pong between lines 0..2 and 3..5 (the
-    // tile in lies in 3..5 at 768 points, read by the first stage only)
-    const XinvSh<C> xs = {stg, nxB, nx, NX};
-    constexpr bool PP = XPROD_PP && Plan8<NT>::n == 3;
-    fft_sel<NT, +1, PPT, false, true, JF, false, PP>(NX, 3, twx + NX, sh, xs, L, sh + 3 * LS, LS);
-  } else {
-    const XinvSrc<C> xs = {Z + tile + yi0, cs, Ty, nx, NX};
-    fft_sel<NT, +1, PPT, false, true, JF, false, false, XSH>(NX, 3, twx, sh, xs, L, sh, LS);
-  }
+  const XinvSrc<C> xs = {Z + tile + yi0, cs, Ty, nx, NX};
+  fft_global<+1, PPT, false, true>(NX, 3, twx, sh, xs, L);
   __syncthreads();
   if (want_cfl) {
     double cm = 0.0;
-    const double rdy0 = dyl[y0], rdy1 = dyl[y0 + 1];
+    const double rdy0 = 1.0 / dyl[y0], rdy1 = 1.0 / dyl[y0 + 1];
     for (int x = threadIdx.x; x < NX; x += blockDim.x) {
       const C a0 = L(0, x), a1 = L(1, x), b = L(2, x);
-      double c0 = fabs((double)a0.x) / ps.dx + fabs((double)a0.y) / rdy0 + fabs((double)b.x) / ps.dz;
-      double c1 = fabs((double)a1.x) / ps.dx + fabs((double)a1.y) / rdy1 + fabs((double)b.y) / ps.dz;
+      double c0 = fabs(a0.x) * ps.rdx + fabs(a0.y) * rdy0 + fabs(b.x) * ps.rdz;
+      double c1 = fabs(a1.x) * ps.rdx + fabs(a1.y) * rdy1 + fabs(b.y) * ps.rdz;
       cm = nan_max(cm, nan_max(c0, c1));
     }
     for (int o = 16; o > 0; o >>= 1) cm = nan_max(cm, __shfl_xor_sync(0xffffffffu, cm, o));
@@ -398,111 +259,19 @@ __global__ void __launch_bounds__(xprod_threads(NT, PPT), xprod_min_blocks(NT, P
     if ((threadIdx.x & 31) == 0) atomicMax(cflmax, (unsigned long long)__double_as_longlong(cm));
   }
   // the six product lines, transformed forward in place
-  const ProdSrc<LT, C> ps6 = {L, (T)ps.factor};
-  fft_sel<NT, -1, PPT, true, true, JF, false, false, XSH>(NX, 6, JF ? twx + NX : twx, sh, ps6, L, sh, LS);
+  const ProdSrc<LT, C> ps6 = {L, ps.factor};
+  fft_global<-1, PPT, true, true>(NX, 6, twx, sh, ps6, L);
   __syncthreads();
-  // separate the two real transforms of each line, keep kx = 0..nx.  In
-  // FP64, with the tile out ([comp][ix][row]), item e is (row e & 1, mode
-  // e >> 1), so that a warp's stores are consecutive; the lines' stride
-  // (ls_x: 3 LS is half a bank row modulo a bank row) keeps the alternating
-  // reads of lines pl and pl + 3 on distinct banks too (384^2 x 256: 1.151
-  // -> 1.102 ms; in FP32 the same measured slower at 768 points, 7.66
-  // against 7.29 ms, and the items stay (mode, both rows)).
-  constexpr bool ALT = sizeof(C) == 16;
-  if constexpr (ALIAS && !ALT) {
-    // the tile out overlays the lines: every thread reads its (at most two,
-    // as 3 nxB <= NX <= 2 blockDim) entries first, then writes
-    C zk[2][2], zm[2][2];
+  // separate the two real transforms of each line, keep kx = 0..nx
+  for (int e = threadIdx.x; e < nxB * 3; e += blockDim.x) {
+    const int pl = e / nxB, ix = e - pl * nxB;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int e = threadIdx.x + k * blockDim.x;
-      if (e < nxB * 3) {
-        const int pl = e / nxB, ix = e - pl * nxB;
-#pragma unroll
-        for (int yy = 0; yy < 2; ++yy) {
-          zk[k][yy] = L(pl + 3 * yy, ix);
-          zm[k][yy] = L(pl + 3 * yy, ix == 0 ? 0 : NX - ix);
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int e = threadIdx.x + k * blockDim.x;
-      if (e < nxB * 3) {
-        const int pl = e / nxB, ix = e - pl * nxB;
-#pragma unroll
-        for (int yy = 0; yy < 2; ++yy) {
-          const C Zk = zk[k][yy], Zm = zm[k][yy];
-          const T h = T(0.5);
-          stg_out[((2 * pl) * nxB + ix) * 2 + yy] = C{h * (Zk.x + Zm.x), h * (Zk.y - Zm.y)};
-          stg_out[((2 * pl + 1) * nxB + ix) * 2 + yy] = C{h * (Zk.y + Zm.y), h * (Zm.x - Zk.x)};
-        }
-      }
-    }
-  } else if constexpr (ALIAS) {
-    // the tile out overlays the lines: every thread reads its (at most
-    // three, as 6 nxB <= 3 blockDim) entries first, then writes
-    C zk[3], zm[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int e = threadIdx.x + k * blockDim.x;
-      if (e < nxB * 6) {
-        const int yy = e & 1, q = e >> 1, pl = q / nxB, ix = q - pl * nxB;
-        zk[k] = L(pl + 3 * yy, ix);
-        zm[k] = L(pl + 3 * yy, ix == 0 ? 0 : NX - ix);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int e = threadIdx.x + k * blockDim.x;
-      if (e < nxB * 6) {
-        const int yy = e & 1, q = e >> 1, pl = q / nxB, ix = q - pl * nxB;
-        const C Zk = zk[k], Zm = zm[k];
-        const T h = T(0.5);
-        stg_out[((2 * pl) * nxB + ix) * 2 + yy] = C{h * (Zk.x + Zm.x), h * (Zk.y - Zm.y)};
-        stg_out[((2 * pl + 1) * nxB + ix) * 2 + yy] = C{h * (Zk.y + Zm.y), h * (Zm.x - Zk.x)};
-      }
-    }
-  } else if constexpr (JF && ALT) {
-    for (int e = threadIdx.x; e < nxB * 6; e += blockDim.x) {
-      const int yy = e & 1, q = e >> 1, pl = q / nxB, ix = q - pl * nxB;
+    for (int yy = 0; yy < 2; ++yy) {
       const int ln = pl + 3 * yy;
       const C Zk = L(ln, ix), Zm = L(ln, ix == 0 ? 0 : NX - ix);
-      const T h = T(0.5);
-      stg[((2 * pl) * nxB + ix) * 2 + yy] = C{h * (Zk.x + Zm.x), h * (Zk.y - Zm.y)};
-      stg[((2 * pl + 1) * nxB + ix) * 2 + yy] = C{h * (Zk.y + Zm.y), h * (Zm.x - Zk.x)};
-    }
-  } else {
-    for (int e = threadIdx.x; e < nxB * 3; e += blockDim.x) {
-      int pl = e / nxB, ix = e - pl * nxB;
-#pragma unroll
-      for (int yy = 0; yy < 2; ++yy) {
-        const int ln = pl + 3 * yy;
-        const C Zk = L(ln, ix), Zm = L(ln, ix == 0 ? 0 : NX - ix);
-        const T h = T(0.5);
-        const C X = C{h * (Zk.x + Zm.x), h * (Zk.y - Zm.y)};
-        const C Y = C{h * (Zk.y + Zm.y), h * (Zm.x - Zk.x)};
-        if constexpr (JF) {
-          stg[((2 * pl) * nxB + ix) * 2 + yy] = X;
-          stg[((2 * pl + 1) * nxB + ix) * 2 + yy] = Y;
-        } else {
-          size_t o = tile + (size_t)ix * Ty + yi0 + yy;
-          Pp[(size_t)(2 * pl) * cs + o] = X;
-          Pp[(size_t)(2 * pl + 1) * cs + o] = Y;
-        }
-      }
-    }
-  }
-  if constexpr (JF) {
-    // the six spectra of both rows in one tensor store
-    fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      tma_store_4d(&tmP, 2 * yi0, 0, yt * NZ + kz, 6 * mem, stg_out);
-      bulk_commit();
-      bulk_wait_read_all();
+      const size_t o = tile + (size_t)ix * Ty + yi0 + yy;
+      Pp[(size_t)(2 * pl) * cs + o] = C{0.5 * (Zk.x + Zm.x), 0.5 * (Zk.y - Zm.y)};
+      Pp[(size_t)(2 * pl + 1) * cs + o] = C{0.5 * (Zk.y + Zm.y), 0.5 * (Zm.x - Zk.x)};
     }
   }
 }
@@ -582,98 +351,6 @@ cudaError_t launch_piece_lines(const DeviceState& d, double2* base, size_t strid
     k_piece_lines<-1><<<blocks, threads, smem, st>>>(P, nlines, lpb, tw);
   }
   return cudaGetLastError();
-}
-
-// ------------------------------------------------------- staged twiddles ----
-// The twiddles of the 8-point plan of N in stage order (see fft_stage_io):
-// for each stage after the first, [r - 1][kk] = W_N^(kk r N/(Ns R)).
-template <int N, typename C>
-static int staged_twiddles_t(C* out) {
-  using PL = Plan8<N>;
-  const int rad[3] = {PL::r0, PL::r1, PL::r2};
-  int n = 0, Ns = 1;
-  for (int st = 0; st < PL::n; ++st) {
-    const int R = rad[st];
-    if (Ns > 1)
-      for (int r = 1; r < R; ++r)
-        for (int kk = 0; kk < Ns; ++kk) {
-          const long e = (long)kk * r * (N / (Ns * R)) % N;
-          long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)e / (long double)N;
-          out[n].x = (typename RealOf<C>::T)cosl(a);
-          out[n++].y = (typename RealOf<C>::T)sinl(a);
-        }
-    Ns *= R;
-  }
-  return n;
-}
-
-int staged_twiddles(int N, double2* out) {
-  switch (N) {
-    case 192: return staged_twiddles_t<192>(out);
-    case 384: return staged_twiddles_t<384>(out);
-    case 768: return staged_twiddles_t<768>(out);
-  }
-  return 0;
-}
-int staged_twiddles(int N, float2* out) {
-  switch (N) {
-    case 192: return staged_twiddles_t<192>(out);
-    case 384: return staged_twiddles_t<384>(out);
-    case 768: return staged_twiddles_t<768>(out);
-  }
-  return 0;
-}
-
-// ------------------------------------------------------------- TMA maps ----
-// Z and Pp seen as 4-D f64 tensors: d0 = the 2 Ty doubles of one y tile
-// (innermost), d1 = ix, d2 = (y tile, kz) as yt nzd + kz, d3 = component.
-// The x kernel's box is {4 doubles (two rows), nxB, 1, comps}.
-static bool xprod_uses_maps(const Geometry& g) {
-  const int NX = 2 * g.nxd;
-  return (g.pptx == 8 || g.mp) && (NX == 192 || NX == 384 || NX == 768) && g.nxB <= 256;
-}
-
-typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-cudaError_t make_transform_maps(const Geometry& g, DeviceState& d) {
-  d.maps = false;
-  {
-    int dev = 0;
-    cudaError_t e0 = cudaGetDevice(&dev);
-    if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e0 != cudaSuccess) return e0;
-  }
-  if (!xprod_uses_maps(g)) return cudaSuccess;
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-  if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) return e != cudaSuccess ? e : cudaErrorNotSupported;
-  const EncodeTiled enc = reinterpret_cast<EncodeTiled>(fn);
-  const int nyT = g.ny / g.Ty;
-  for (int which = 0; which < 2; ++which) {
-    const cuuint32_t comps = which == 0 ? 3 : 6;
-    cuuint64_t dims[4] = {(cuuint64_t)2 * g.Ty, (cuuint64_t)g.nxB, (cuuint64_t)g.nzd * nyT, (cuuint64_t)comps * g.nmem};
-    const cuuint64_t es = g.mp ? 8 : 16;  // bytes of one complex element
-    cuuint64_t strides[3] = {es * g.Ty, es * g.Ty * g.nxB, es * g.Ty * g.nxB * g.nzd * nyT};
-    cuuint32_t box[4] = {4, (cuuint32_t)g.nxB, 1, comps};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = enc(which == 0 ? &d.tmZ : &d.tmPp, g.mp ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
-                     which == 0 ? (void*)d.Z : (void*)d.Pp, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    if (d.Zg) {  // the ghost rows' buffers: one tile of four rows
-      cuuint64_t dg[4] = {8, (cuuint64_t)g.nxB, (cuuint64_t)g.nzd, (cuuint64_t)comps * g.nmem};
-      cuuint64_t sg[3] = {es * 4, es * 4 * g.nxB, es * 4 * g.nxB * g.nzd};
-      r = enc(which == 0 ? &d.tmZg : &d.tmPpg, g.mp ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
-              which == 0 ? (void*)d.Zg : (void*)d.Ppg, dg, sg, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    }
-  }
-  d.maps = true;
-  return cudaSuccess;
 }
 
 bool edge_rows_needed(const Geometry& g, bool s2_active) { return s2_active && g.nzd <= 3 * g.nz; }
@@ -818,39 +495,17 @@ static cudaError_t launch_zfwd_main(const Geometry& g, const DeviceState& d, cud
 static cudaError_t launch_xprod_main(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl,
                                      cudaStream_t st) {
   const int NX = 2 * g.nxd;
-  const int pts = 6 * NX;
-  if (xprod_uses_maps(g) != d.maps) return cudaErrorInvalidValue;
+  if (x_compiled(NX, g.mp != 0)) return launch_x(g, d, ph, want_cfl, st);
+  if (g.mp) return cudaErrorInvalidValue;
   const dim3 grid(g.ny / 2, g.nzd * g.nmem);
-  if (g.mp) {
-    typedef float2 C;
-    const size_t lines = (size_t)6 * (NX == 1536 && XPAD1536 ? xls_1536(8) : NX + 1) * sizeof(C);
-    const size_t smem = !xprod_uses_maps(g) ? lines
-                        : (NX == 768 ? xprod_alias_smem(NX, sizeof(C)) : xprod_tma_smem(NX, g.nxB, sizeof(C)));
-    const C* Z = reinterpret_cast<const C*>(d.Z);
-    C* Pp = reinterpret_cast<C*>(d.Pp);
-#define HST_XPROD(NT, PPT)                                                                                    \
-  {                                                                                                           \
-    big_smem(d, k_xprod<NT, PPT, C>);                                                                            \
-    k_xprod<NT, PPT, C><<<grid, fft_threads(pts, PPT), smem, st>>>(g, Z, Pp, d.twxf, d.dyl, ph, want_cfl,     \
-                                                                    d.cfl, d.tmZ, d.tmPp, d.err);             \
+  const size_t smem = (size_t)6 * (NX + 1) * sizeof(double2);
+  if (6 * NX <= 16 * 256) {
+    big_smem(d, k_xprod<16>);
+    k_xprod<16><<<grid, fft_threads(6 * NX, 16), smem, st>>>(g, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
+  } else {
+    big_smem(d, k_xprod<32>);
+    k_xprod<32><<<grid, fft_threads(6 * NX, 32), smem, st>>>(g, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
   }
-    HST_FFT_DISPATCH_MP(NX, false, HST_XPROD);
-#undef HST_XPROD
-    return cudaGetLastError();
-  }
-  typedef double2 C;
-  const size_t lines = (size_t)6 * (NX == 1536 && XPAD1536 ? xls_1536(16) : NX + 1) * sizeof(C);
-  const size_t smem = !xprod_uses_maps(g) ? lines
-                      : (NX == 768 && g.pptx == 8 ? xprod_alias_smem(NX, sizeof(C))
-                                                  : xprod_tma_smem(NX, g.nxB, sizeof(C)));
-#define HST_XPROD(NT, PPT)                                                                                    \
-  {                                                                                                           \
-    big_smem(d, k_xprod<NT, PPT, C>);                                                                            \
-    k_xprod<NT, PPT, C><<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl,  \
-                                                                    d.cfl, d.tmZ, d.tmPp, d.err);             \
-  }
-  HST_FFT_DISPATCH(NX, pts, g.pptx == 8, HST_XPROD);
-#undef HST_XPROD
   return cudaGetLastError();
 }
 

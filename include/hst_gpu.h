@@ -191,7 +191,7 @@ int hst_gpu_outstats(hst_ctx* ctx, double time, double* out);
 int hst_gpu_outstats_sums(hst_ctx* ctx, double time, double* sums, double* exz);
 
 /* Tries the launch choices that keep every buffer's layout -- the lanes of
- * a line-solver group and the points a thread of the x and z FFT plans --
+ * a line-solver group and the points a thread of the z FFT plans --
  * on this context's sizes (`steps` time steps of `deltat` each, after one
  * untimed step), keeps the fastest and restores the fields (V, OLD) and
  * the damping state.  A report of the candidates' times a step goes to
