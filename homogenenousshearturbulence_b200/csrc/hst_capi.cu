@@ -163,6 +163,7 @@ struct hst_ctx {
   // forces it
   bool shift_split;
   bool solve_halves;  // the solve stage as two one-line passes
+  bool y_uniform;  // y(r) = r ly / ny to rounding, y(0) = 0
   // per-kernel-class CUDA-event accounting (hst_gpu_set_profiling)
   bool prof_on;
   std::vector<cudaEvent_t> ev;
@@ -518,6 +519,15 @@ static cudaError_t ensure_facg(hst_ctx* ctx) {
   return cudaSuccess;
 }
 
+// whether the y table is the uniform grid r ly / ny to rounding
+static void check_uniform(hst_ctx* ctx) {
+  const int ny = ctx->p.ny;
+  const double dy = ctx->p.ly / ny;
+  ctx->y_uniform = ctx->p.ystretch <= 1.0e-10;
+  for (int r = 0; r < ny; ++r)
+    if (!(std::fabs(ctx->y[r + 2] - r * dy) <= 4.0e-16 * std::fabs(ctx->p.ly))) ctx->y_uniform = false;
+}
+
 static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   if (!pin || !out || nmem < 1 || nmem > 4096) return HST_EARG;
   *out = nullptr;
@@ -584,6 +594,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   }
   ctx->dyl.resize(ny);
   for (int iy = 0; iy < ny; ++iy) ctx->dyl[iy] = 0.5 * (ctx->y[iy + 3] - ctx->y[iy + 1]);
+  check_uniform(ctx);
   setup_derivatives(ny, ctx->y, ctx->der);
   ctx->gdamp.assign((size_t)g.ncol, 0.0);
   ctx->theta_last = -1.0e308;
@@ -804,6 +815,7 @@ extern "C" int hst_gpu_set_tables(hst_ctx* ctx, const double* der, const double*
   }
   if (y) {
     std::memcpy(ctx->y.data(), y, sizeof(double) * (ny + 4));
+    check_uniform(ctx);
     CK(cudaMemcpyAsync(ctx->d.y, ctx->y.data(), sizeof(double) * (ny + 4), cudaMemcpyHostToDevice, ctx->stream));
   }
   if (dyl) {
@@ -1336,7 +1348,7 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
     sc.damp_hard = (p.damp_hard && damp) ? 1 : 0;
     sc.dgx = p.S * dt_sub;
     sc.dgz = s2_integral(p, t, t + dt_sub);
-    sc.yuni = p.ystretch <= 1.0e-10 ? 1 : 0;
+    sc.yuni = ctx->y_uniform ? 1 : 0;
     sc.ytile = p.ly * 32.0 / p.ny;
     shear_shifts(ctx, t, &sc.sx_t, &sc.sz_t);
     shear_shifts(ctx, t + dt_sub, &sc.sx_n, &sc.sz_n);
@@ -1600,7 +1612,7 @@ extern "C" int hst_gpu_shear_shift(hst_ctx* ctx, double dt_sub, double time) {
   SubstepScalars sc = {};
   sc.dgx = dgx;
   sc.dgz = dgz;
-  sc.yuni = p.ystretch <= 1.0e-10 ? 1 : 0;
+  sc.yuni = ctx->y_uniform ? 1 : 0;
   sc.ytile = p.ly * 32.0 / p.ny;
   shear_shifts(ctx, time, &sc.sx_t, &sc.sz_t);
   shear_shifts(ctx, time + dt_sub, &sc.sx_n, &sc.sz_n);

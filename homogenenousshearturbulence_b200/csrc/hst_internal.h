@@ -134,6 +134,9 @@ cudaError_t launch_zfwd(const Geometry& g, const DeviceState& d, cudaStream_t st
 // 4 the right-hand-side stage in its untiled FP64 form
 cudaError_t launch_column(const Geometry& g, const DeviceState& d, const PhysScalars& ph, const SubstepScalars& sc,
                           int exact, int nonlin, int part, cudaStream_t st);
+// the right-hand sides streamed through shared memory (hst_rhs.cu)
+cudaError_t launch_rhs_tiled(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
+                             int exact, int nonlin, cudaStream_t st);
 cudaError_t launch_line_solve(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int sys, double lambda,
                               int src, int dst, double sx, double sz, cudaStream_t st);
 cudaError_t launch_fill_ghosts(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int field, double sx,

@@ -1,12 +1,11 @@
-// The column kernels of the hst substep on sm_100a (FP64); the transforms
-// (k_zinv, k_xprod, k_zfwd) are in hst_transforms.cu.
+// The column kernels of the hst substep on sm_100a (FP64); the transforms are
+// in hst_transforms.cu and hst_xprod.cu, the streamed right-hand sides in
+// hst_rhs.cu.
 //
 //   k_column     one warp group per Fourier column: the right-hand sides of
 //                buildrhs_prepare and buildrhs, the hard damping mask, the
 //                mean-shear phase shift (both forms), the D2V, ETA and DY
 //                line solves, u and w, all ghost rows; or either half of it
-//   k_rhs_tiled  the right-hand-side half as a streaming kernel fed by TMA
-//                bulk copies
 //   k_line_solve, k_fill_ghosts: the single operations for the drop-in
 //                interface and the tests
 //
@@ -36,14 +35,9 @@ struct ColumnArgs {
   const double2* Qg;  // the ghost rows' product spectra [6][ncol][4] (null: their wrap images)
   const double* der;
   const double* derS;
-  const double* derU;  // the distinct rows of der (DerRows), or null
-  const int* derI;
-  int nderU;
   const double* d0tab;
   const double* y;
   const double* gdamp;
-  int* err;   // set to 1 by a kernel whose bounded wait ran out
-  int tiled;  // the right-hand sides through k_rhs_tiled
   const DeviceState* dstate;  // host side only: the launch's context state
   double* facg;               // global factor scratch of the persistent form (null: shared memory)
   int fac_groups;             // groups that scratch holds
@@ -747,137 +741,6 @@ __global__ void k_fill_ghosts(Geometry g, PhysScalars ps, double2* __restrict__ 
   c[-2] = cmul(c[ny - 2], cconj(ph));
 }
 
-// ----------------------------------------------------------- k_rhs_tiled ----
-// The right-hand-side stage as a streaming kernel: one warp per Fourier
-// column walks its rows in tiles of 32; the 36-row windows of the three
-// velocity components and of the six product spectra, and the carried terms
-// of each tile are fetched with TMA bulk copies into shared memory (two
-// stages: the next tile is in flight while this one computes), so the warp
-// issues a handful of copy instructions per tile instead of one load per
-// stencil tap.  Needs ny a multiple of 32.
-constexpr int RT_W = 36;                                 // window rows
-constexpr int RT_STAGE = 3 * RT_W + 6 * RT_W + 2 * 32;  // double2 per stage: V[3][36], Q[6][36], old[2][32]
-constexpr int RT_WARPS = 4;
-#ifndef RT_MINB
-#define RT_MINB 4  // 128 registers: four 4-warp blocks an SM (0.52 against 0.69 ms at 384^2 x 256)
-#endif
-constexpr int RT_WAIT_LIMIT = 1 << 22;
-
-// QT: the complex type of the product spectra Q (float2 in the mixed-
-// precision form: the window lands as FP32 and each value is widened to
-// FP64 where it is read)
-template <bool EXACT, bool NONLIN, typename QT>
-__global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(ColumnArgs a, int* __restrict__ err) {
-  extern __shared__ __align__(128) double2 smt[];
-  __shared__ __align__(8) uint64_t bars[RT_WARPS][2];
-  const Geometry& g = a.g;
-  const int ny = g.ny;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cgl = blockIdx.x * RT_WARPS + warp;  // the column over all members
-  if (cgl >= g.ncol * g.nmem) return;
-  const int mem = cgl / g.ncol, col = cgl - mem * g.ncol;
-  double2* st0 = smt + (size_t)warp * 2 * RT_STAGE;
-  uint64_t* bar = bars[warp];
-  if (lane == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    fence_mbar_init();
-  }
-  __syncwarp();
-  const int ntile = ny / 32;
-  const size_t cbase = (size_t)cgl * g.rows;  // row -2 of the column
-  const double2* Vg[3] = {a.V1, a.V2, a.V3};
-  // lane 0 queues the copies of tile t into stage t & 1
-  const QT* Qg = reinterpret_cast<const QT*>(a.Q);
-  const QT* Qgg = reinterpret_cast<const QT*>(a.Qg);
-  constexpr unsigned QE = sizeof(QT);
-  auto issue = [&](int t) {
-    const int stg = t & 1;
-    double2* S = st0 + stg * RT_STAGE;
-    const int r0 = t * 32;
-    mbar_arrive_expect_tx(&bar[stg], (3 * RT_W + 2 * 32) * 16 + 6 * RT_W * QE);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) bulk_g2s(S + c * RT_W, Vg[c] + cbase + r0, RT_W * 16, &bar[stg]);
-#pragma unroll 1
-    for (int p = 0; p < 6; ++p) {
-      const QT* Qc = Qg + (((size_t)mem * 6 + p) * g.ncol + col) * ny;
-      QT* D = reinterpret_cast<QT*>(S + 3 * RT_W) + p * RT_W;
-      const int lo = r0 - 2, hi = r0 + 34;
-      const int m0 = lo < 0 ? 0 : lo, m1 = hi > ny ? ny : hi;
-      // the rows beyond the box: the wrapped interior rows (their phase is
-      // applied in tq), or the ghost rows' own spectra
-      const QT* Qgc = Qgg ? Qgg + (((size_t)mem * 6 + p) * g.ncol + col) * 4 : nullptr;
-      if (lo < 0) bulk_g2s(D, Qgc ? Qgc : Qc + ny + lo, (unsigned)(-lo) * QE, &bar[stg]);
-      bulk_g2s(D + (m0 - lo), Qc + m0, (unsigned)(m1 - m0) * QE, &bar[stg]);
-      if (hi > ny) bulk_g2s(D + (ny - lo), Qgc ? Qgc + 2 : Qc, (unsigned)(hi - ny) * QE, &bar[stg]);
-    }
-    bulk_g2s(S + 9 * RT_W, a.O1 + cbase + 2 + r0, 32 * 16, &bar[stg]);
-    bulk_g2s(S + 9 * RT_W + 32, a.O2 + cbase + 2 + r0, 32 * 16, &bar[stg]);
-  };
-  if (lane == 0) {
-    issue(0);
-    if (ntile > 1) issue(1);
-  }
-  const ColConst cc = col_const(col, g, a.ps, a.sc, a.gdamp);
-  const SubstepScalars& sc = a.sc;
-  typedef typename RealOf<QT>::T QR;
-  const QT ph_q = QT{(QR)cc.ph_t.x, (QR)cc.ph_t.y};  // the ghost-row phase in the spectra's precision
-  // the default-form shift factor of row t 32 + lane on a uniform grid:
-  // exp(-i g y(lane)) times exp(-i g 32 dy)^t, one product a tile instead
-  // of a sine and cosine a row (mixed precision only: in the FP64 form the
-  // two extra live values cost this 128-register kernel more than the
-  // sines save, 0.57 against 0.52 ms at 384^2 x 256)
-  constexpr bool REC = !EXACT && sizeof(QT) == 8;
-  cxd fbase = mkc(1.0, 0.0), fstep = mkc(1.0, 0.0);
-  if (REC && sc.yuni) {
-    const double gsh = cc.al * sc.dgx + cc.be * sc.dgz;
-    fbase = cexpi(-gsh * a.y[lane + 2]);
-    fstep = cexpi(-gsh * sc.ytile);
-  }
-  for (int t = 0; t < ntile; ++t) {
-    const int stg = t & 1;
-    if (!mbar_wait_bounded(&bar[stg], (t >> 1) & 1, RT_WAIT_LIMIT)) {
-      // record the failure, give this warp's copies still in flight a
-      // second bounded wait to land, and leave
-      if (lane == 0) atomicExch(err, 1);
-      mbar_wait_bounded(&bar[stg], (t >> 1) & 1, RT_WAIT_LIMIT);
-      if (t + 1 < ntile) mbar_wait_bounded(&bar[stg ^ 1], ((t + 1) >> 1) & 1, RT_WAIT_LIMIT);
-      return;
-    }
-    const double2* S = st0 + stg * RT_STAGE;
-    const int r = t * 32 + lane;
-    auto tv = [&](int c, int j) -> cxd { return S[c * RT_W + lane + j]; };
-    const QT* SQ = reinterpret_cast<const QT*>(S + 3 * RT_W);
-    auto tq = [&](int p, int j) -> QT {
-      const QT q = SQ[p * RT_W + lane + j];
-      const int row = r + j - 2;
-      if (Qgg) return q;
-      if (row < 0) return cmul(q, cconj(ph_q));
-      if (row >= ny) return cmul(q, ph_q);
-      return q;
-    };
-    cxd r1, r2, o1, o2;
-    const double yr = a.y[r + 2];
-    auto fsh = [&]() -> cxd {
-      if (REC && sc.yuni) return fbase;
-      return cexpi(-(cc.al * sc.dgx + cc.be * sc.dgz) * yr);
-    };
-    rhs_point<NONLIN, EXACT>(cc, sc, DerRows{a.derU, a.derI, a.nderU}, ny, r, fsh, tv, tq, S[9 * RT_W + lane],
-                             S[9 * RT_W + 32 + lane], r1, r2, o1, o2);
-    if (REC) fbase = cmul(fbase, fstep);
-    const size_t ro = cbase + 2 + r;
-    a.O1[ro] = o1;
-    a.O2[ro] = o2;
-    a.R1[ro] = r1;
-    a.R2[ro] = r2;
-    __syncwarp();
-    if (lane == 0 && t + 2 < ntile) {
-      fence_proxy_async();
-      issue(t + 2);
-    }
-  }
-}
-
 // -------------------------------------------------------------- launchers ----
 size_t column_lines_bytes(const Geometry& g) { return (size_t)2 * g.P * g.MS * sizeof(double2); }
 
@@ -891,18 +754,6 @@ size_t column_smem_bytes(const Geometry& g, int exact) {
 template <int P, bool EXACT, bool NONLIN, int MODE>
 static cudaError_t launch_column_t(const ColumnArgs& a, cudaStream_t st) {
   const Geometry& g = a.g;
-  if (MODE == COL_RHS && g.ny % 32 == 0 && a.tiled) {  // TMA-staged tiles
-    const size_t smem = (size_t)RT_WARPS * 2 * RT_STAGE * sizeof(double2);
-    const int blocks = (g.ncol * g.nmem + RT_WARPS - 1) / RT_WARPS;
-    if (g.mp) {
-      smem_limit(*a.dstate, k_rhs_tiled<EXACT, NONLIN, float2>, (int)smem);
-      k_rhs_tiled<EXACT, NONLIN, float2><<<blocks, 32 * RT_WARPS, smem, st>>>(a, a.err);
-    } else {
-      smem_limit(*a.dstate, k_rhs_tiled<EXACT, NONLIN, double2>, (int)smem);
-      k_rhs_tiled<EXACT, NONLIN, double2><<<blocks, 32 * RT_WARPS, smem, st>>>(a, a.err);
-    }
-    return cudaGetLastError();
-  }
   // the untiled and fused forms read FP64 product spectra only (the
   // linear right-hand sides read none)
   if (MODE != COL_SOLVE && MODE != COL_SHIFT && MODE != COL_SOLVE_V && MODE != COL_SOLVE_ETA && g.mp && NONLIN)
@@ -1030,24 +881,19 @@ cudaError_t launch_column(const Geometry& g, const DeviceState& d, const PhysSca
   a.Qg = d.Qg;
   a.der = d.der;
   a.derS = d.derS;
-  a.derU = d.derU;
-  a.derI = d.derI;
-  a.nderU = d.nderU;
   a.d0tab = d.d0tab;
   a.y = d.y;
   a.gdamp = d.gdamp;
-  a.err = d.err;
   a.dstate = &d;
   a.facg = d.facg;
   a.fac_groups = d.facg ? (int)std::min<size_t>(d.facg_doubles / column_fac_doubles(g), 1u << 30) : 0;
   if (a.fac_groups < 1) a.facg = nullptr;
-  {
+  // the right-hand sides: streamed, or untiled (HST_RHS_TILED=0, and part 4,
+  // the per-piece prepare)
+  if (part == 4) part = COL_RHS;
+  else if (part == COL_RHS) {
     const char* e = std::getenv("HST_RHS_TILED");
-    a.tiled = !(e && std::atoi(e) == 0);
-  }
-  if (part == 4) {  // the right-hand-side stage, untiled (the per-piece prepare)
-    a.tiled = 0;
-    part = COL_RHS;
+    if (!(e && std::atoi(e) == 0)) return launch_rhs_tiled(g, d, ph, sc, exact, nonlin, st);
   }
   switch (g.P) {
     case 2: return launch_column_p<2>(a, exact, nonlin, part, st);
