@@ -151,18 +151,8 @@ struct hst_ctx {
   Geometry gb;
   DeviceState db;
   std::unordered_set<const void*> configured;  // kernels whose shared-memory limit is raised
-  std::unordered_map<uint64_t, int> occupancy;  // resident blocks an SM, per launch shape
   long long launches;
   int device;
-  // the column stage as two kernels (right-hand sides streamed row by row,
-  // then the solves) or one; HST_COLUMN_FUSED=1 selects the single kernel
-  bool column_split;
-  // with exact_shift, the shift as a third kernel before the solves: on with
-  // the persistent solve stage (slabs of 16 rows or more; 768^2 x 512: shift
-  // 4.4 + solves 4.9 ms against 10.3 ms in one kernel), HST_SHIFT_SPLIT=0 / 1
-  // forces it
-  bool shift_split;
-  bool solve_halves;  // the solve stage as two one-line passes
   bool y_uniform;  // y(r) = r ly / ny to rounding, y(0) = 0
   // per-kernel-class CUDA-event accounting (hst_gpu_set_profiling)
   bool prof_on;
@@ -289,7 +279,7 @@ static bool damping_update(hst_ctx* c, double t) {
 }
 
 // ------------------------------------------------------ geometry ----
-static int choose_geometry(const hst_gpu_params& p, Geometry& g, std::string& why) {
+static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::string& why) {
   g.nx = p.nx;
   g.ny = p.ny;
   g.nz = p.nz;
@@ -322,32 +312,28 @@ static int choose_geometry(const hst_gpu_params& p, Geometry& g, std::string& wh
   g.rows = p.ny + 4;
   g.ncol = g.nxB * g.nzT;
   g.nf = (long)g.ncol * g.rows;
-  // line-solve group: P lanes of m rows; the widest group with m >= 8
-  // (measured best at 384^2 x 256), else m >= 4
-  int P = 0;
-  const char* env = std::getenv("HST_LINE_LANES");
-  if (env) {
+  // the most rows: what a group of P lanes dividing ny, with its lines and
+  // factors in shared memory, has room for
+  {
+    int P = 0;
+    for (int mmin : {8, 4})
+      for (int c = 32; c >= 2 && !P; c >>= 1)
+        if (p.ny % c == 0 && p.ny / c >= mmin) P = c;
+    if (!P) {
+      why = "ny must be a multiple of 2 with at least 4 rows per lane";
+      return HST_EARG;
+    }
+    const size_t m = p.ny / P;
+    if ((6 * P * (m | 1) + 4 * (m - 2) * P) * sizeof(double) > 200 * 1024) {
+      why = "ny too large for one line-solver group's shared memory";
+      return HST_EARG;
+    }
+  }
+  // the line-solver group (HST_LINE_LANES overrides)
+  g.P = hst::line_lanes(p.ny, (long)g.ncol * nmem);
+  if (const char* env = std::getenv("HST_LINE_LANES")) {
     int e = std::atoi(env);
-    if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && p.ny % e == 0 && p.ny / e >= 4) P = e;
-  }
-  for (int mmin : {8, 4}) {
-    if (P) break;
-    for (int c = 32; c >= 2; c >>= 1)
-      if (p.ny % c == 0 && p.ny / c >= mmin) {
-        P = c;
-        break;
-      }
-  }
-  if (!P) {
-    why = "ny must be a multiple of 2 with at least 4 rows per lane";
-    return HST_EARG;
-  }
-  g.P = P;
-  g.m = p.ny / P;
-  g.MS = g.m | 1;
-  if (hst::column_smem_bytes(g, 1) > 200 * 1024) {
-    why = "ny too large for one line-solver group's shared memory";
-    return HST_EARG;
+    if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && p.ny % e == 0 && p.ny / e >= 4) g.P = e;
   }
   // z FFT points per thread: 8 selects the low-register plans (lengths 192,
   // 384, 768).  Measured: 16 at 384^2 x 256 (0.26/0.50 against 0.29/0.52 ms),
@@ -403,19 +389,8 @@ static double dev_bytes(const Geometry& g) {
 extern "C" double hst_gpu_device_bytes(const hst_gpu_params* p) {
   Geometry g;
   std::string why;
-  if (!p || choose_geometry(*p, g, why) != HST_OK) return 0.0;
+  if (!p || choose_geometry(*p, 1, g, why) != HST_OK) return 0.0;
   return dev_bytes(g);
-}
-
-// der in the slab-major order of hst::SlabDer
-static std::vector<double> slab_major(const std::vector<double>& der, int ny, int P, int m) {
-  std::vector<double> o((size_t)20 * ny);
-  for (int n = 0; n < 4; ++n)
-    for (int j = 0; j < 5; ++j)
-      for (int i = 0; i < m; ++i)
-        for (int s = 0; s < P; ++s)
-          o[((size_t)(n * 5 + j) * m + i) * P + s] = der[(size_t)(s * m + i) + (size_t)ny * (n + 4 * j)];
-  return o;
 }
 
 // der's distinct rows (equal bits) coefficient-major, and each row's index
@@ -474,34 +449,15 @@ static void free_device(hst_ctx* c) {
   if (d.facg) cudaFree(d.facg);
   std::memset(&d, 0, sizeof d);
   d.configured = &c->configured;
-  d.occupancy = &c->occupancy;
 }
 
-// The column kernels' factor scratch in global memory: one slice of
-// (m-2) x 4 x P doubles per solver group that can be resident at once (at
-// most 16 warps an SM), sized for the current group width.  It is used (and
-// with it the persistent solve stage, k_column_solve) for slabs of 16 rows
-// or more, where the scratch would otherwise take half a warp's shared memory
-// (768^2 x 512: column 10.2 against 11.1 ms); at 8 rows a lane the one-column
-// kernel with the scratch in shared memory measured faster (384^2 x 256:
-// 0.54 against 0.75 ms).  HST_COLUMN_GFAC=1 / 0 forces either.
+// The line solves' factor scratch for the current group width: a slice for
+// every solver group that can be resident (sixteen warps an SM), or for as
+// many as the device has room for (the solves then run on fewer groups).
 static cudaError_t ensure_facg(hst_ctx* ctx) {
-  const Geometry& g = ctx->g;
-  const char* e = std::getenv("HST_COLUMN_GFAC");
-  const bool want = e ? std::atoi(e) == 1 : g.m >= 16;
-  if (!want) {
-    if (ctx->d.facg) {
-      cudaError_t r = cudaStreamSynchronize(ctx->stream);
-      if (r != cudaSuccess) return r;
-      cudaFree(ctx->d.facg);
-      ctx->d.facg = nullptr;
-      ctx->d.facg_doubles = 0;
-    }
-    return cudaSuccess;
-  }
   const int nsm = ctx->d.nsm > 0 ? ctx->d.nsm : 148;
-  const size_t need = (size_t)nsm * 16 * (32 / std::min(g.P, 32)) * hst::column_fac_doubles(g);
-  if (ctx->d.facg && ctx->d.facg_doubles >= need) return cudaSuccess;
+  const size_t need = hst::solve_scratch_bytes(ctx->g, nsm);
+  if (ctx->d.facg && ctx->d.facg_doubles * sizeof(double) >= need) return cudaSuccess;
   if (ctx->d.facg) {
     cudaError_t r = cudaStreamSynchronize(ctx->stream);
     if (r != cudaSuccess) return r;
@@ -509,14 +465,19 @@ static cudaError_t ensure_facg(hst_ctx* ctx) {
     ctx->d.facg = nullptr;
     ctx->d.facg_doubles = 0;
   }
-  cudaError_t r = cudaMalloc((void**)&ctx->d.facg, need * sizeof(double));
-  if (r != cudaSuccess) {
+  cudaError_t r = cudaSuccess;
+  for (size_t bytes = need; bytes >= need / nsm / 16; bytes /= 2) {
+    r = cudaMalloc((void**)&ctx->d.facg, bytes);
+    if (r == cudaSuccess) {
+      ctx->d.facg_doubles = bytes / sizeof(double);
+      break;
+    }
     cudaGetLastError();
-    ctx->d.facg = nullptr;  // fall back to the scratch in shared memory
-    return cudaSuccess;
+    ctx->d.facg = nullptr;
   }
-  ctx->d.facg_doubles = need;
-  return cudaSuccess;
+  ctx->db.facg = ctx->d.facg;
+  ctx->db.facg_doubles = ctx->d.facg_doubles;
+  return r;
 }
 
 // whether the y table is the uniform grid r ly / ny to rounding
@@ -536,12 +497,6 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ctx->p = *pin;
   ctx->nmem = nmem;
   ctx->launches = 0;
-  {
-    const char* e = std::getenv("HST_COLUMN_FUSED");
-    ctx->column_split = !(e && std::atoi(e) == 1);
-    ctx->shift_split = false;  // decided once the geometry is known
-    ctx->solve_halves = false;
-  }
   ctx->prof_on = false;
   for (int k = 0; k < HST_KC_N; ++k) {
     ctx->prof_ms[k] = 0.0;
@@ -552,9 +507,8 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ctx->h_cfl = nullptr;
   std::memset(&ctx->d, 0, sizeof ctx->d);
   ctx->d.configured = &ctx->configured;
-  ctx->d.occupancy = &ctx->occupancy;
   std::string why;
-  int rc = choose_geometry(*pin, ctx->g, why);
+  int rc = choose_geometry(*pin, nmem, ctx->g, why);
   if (rc != HST_OK) {
     std::fprintf(stderr, "hst_gpu_create: %s\n", why.c_str());
     delete ctx;
@@ -565,9 +519,8 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   if (ctx->g.mp) {
     // the FP32 product spectra are read only by the streamed right-hand-side kernel
     const char* t = std::getenv("HST_RHS_TILED");
-    if (!ctx->column_split || (t && std::atoi(t) == 0)) {
-      std::fprintf(stderr, "hst_gpu_create: mixed precision needs the split column stage and the streamed "
-                           "right-hand sides (HST_COLUMN_FUSED, HST_RHS_TILED unset)\n");
+    if (t && std::atoi(t) == 0) {
+      std::fprintf(stderr, "hst_gpu_create: mixed precision needs the streamed right-hand sides (HST_RHS_TILED unset)\n");
       delete ctx;
       return HST_EARG;
     }
@@ -626,7 +579,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
     ok = ok && alloc((void**)&d.Qg, es * 6 * (size_t)g.ncol * 4 * nm);
   }
   ok = ok && alloc((void**)&d.der, sizeof(double) * 20 * (size_t)ny);
-  ok = ok && alloc((void**)&d.derS, sizeof(double) * 20 * (size_t)ny);
+  ok = ok && alloc((void**)&d.derS, sizeof(double) * hst::slab_der_doubles(ny));
   ok = ok && alloc((void**)&d.derU, sizeof(double) * 20 * (size_t)ny);
   ok = ok && alloc((void**)&d.derI, sizeof(int) * (size_t)ny);
   ok = ok && alloc((void**)&d.d0tab, sizeof(double) * hst::d0_table_doubles(ny));
@@ -661,8 +614,8 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   cudaMemcpy(d.der, ctx->der.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice);
   cudaError_t etab;
   {
-    auto ds = slab_major(ctx->der, ny, g.P, g.m);
-    cudaMemcpy(d.derS, ds.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice);
+    auto ds = hst::slab_major(ctx->der, ny, g.P);
+    cudaMemcpy(d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
     etab = hst::launch_d0_table(g, d, ctx->stream);
     if (etab == cudaSuccess) etab = upload_der_rows(ctx);
   }
@@ -697,14 +650,6 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   if (e == cudaSuccess) e = hst::make_x_maps(ctx->gb, ctx->db);
   if (e == cudaSuccess) e = hst::make_x_maps(g, d);
   if (e == cudaSuccess) e = ensure_facg(ctx);
-  if (e == cudaSuccess) ctx->db.facg = d.facg, ctx->db.facg_doubles = d.facg_doubles;
-  {
-    const char* f = std::getenv("HST_SHIFT_SPLIT");
-    ctx->shift_split = f ? std::atoi(f) == 1 : ctx->d.facg != nullptr;
-    // the solves in two one-line passes (needs the global factor scratch)
-    const char* h = std::getenv("HST_SOLVE_HALVES");
-    ctx->solve_halves = ctx->d.facg != nullptr && (h ? std::atoi(h) == 1 : true);
-  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -808,8 +753,8 @@ extern "C" int hst_gpu_set_tables(hst_ctx* ctx, const double* der, const double*
   if (der) {
     std::memcpy(ctx->der.data(), der, sizeof(double) * 20 * ny);
     CK(cudaMemcpy(ctx->d.der, ctx->der.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice));
-    auto ds = slab_major(ctx->der, ny, ctx->g.P, ctx->g.m);
-    CK(cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice));
+    auto ds = hst::slab_major(ctx->der, ny, ctx->g.P);
+    CK(cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice));
     CK(hst::launch_d0_table(ctx->g, ctx->d, ctx->stream));
     CK(upload_der_rows(ctx));
   }
@@ -1115,14 +1060,9 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   const std::vector<double> gdamp0 = ctx->gdamp;
   // candidates
   std::vector<int> lanes;
-  for (int c = 32; c >= 4; c >>= 1) {
-    Geometry t = g0;
-    if (g0.ny % c != 0 || g0.ny / c < 4) continue;
-    t.P = c;
-    t.m = g0.ny / c;
-    t.MS = t.m | 1;
-    if (hst::column_smem_bytes(t, 1) <= 200 * 1024) lanes.push_back(c);
-  }
+  for (int c = 32; c >= 4; c >>= 1)
+    if (g0.ny / c >= 4) lanes.push_back(c);
+  if (lanes.empty()) lanes.push_back(g0.P);
   std::vector<int> pz;
   for (int v : {16, 8}) {
     if (g0.mp && g0.nzd == 768 && v == 16) continue;
@@ -1140,8 +1080,8 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   int rc = HST_OK;
   auto apply = [&](const Geometry& t) -> cudaError_t {
     g = t;
-    auto ds = slab_major(ctx->der, g.ny, g.P, g.m);
-    cudaError_t e = cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * 20 * g.ny, cudaMemcpyHostToDevice);
+    auto ds = hst::slab_major(ctx->der, g.ny, g.P);
+    cudaError_t e = cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = hst::launch_d0_table(g, ctx->d, ctx->stream);
     if (e == cudaSuccess) e = ensure_facg(ctx);
     return e;
@@ -1150,8 +1090,6 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
     for (int b : pz) {
       Geometry t = g0;
       t.P = P;
-      t.m = g0.ny / P;
-      t.MS = t.m | 1;
       t.pptz = b;
       if (apply(t) != cudaSuccess) continue;
       for (int i = 0; i < 5 && rc == HST_OK; ++i)
@@ -1296,19 +1234,16 @@ extern "C" int hst_gpu_read_restart(hst_ctx* ctx, const char* path, double* time
   return HST_OK;
 }
 
-// the solve stage of a substep whose right-hand sides (and exact_shift
-// shift) are done: one kernel, or its two one-line halves
+// the implicit solves of a substep: their two passes
 static cudaError_t solve_stage(hst_ctx* ctx, const hst::Geometry& G, const hst::DeviceState& D,
-                               const hst::SubstepScalars& sc, int nonlin) {
-  if (ctx->solve_halves)
-    return timed(
-        ctx, HST_KC_COLUMN,
-        [&] {
-          cudaError_t e = hst::launch_column(G, D, ctx->ps, sc, 0, nonlin, 5, ctx->stream);
-          return e == cudaSuccess ? hst::launch_column(G, D, ctx->ps, sc, 0, nonlin, 6, ctx->stream) : e;
-        },
-        2);
-  return timed(ctx, HST_KC_COLUMN, [&] { return hst::launch_column(G, D, ctx->ps, sc, 0, nonlin, 2, ctx->stream); });
+                               const hst::SubstepScalars& sc) {
+  return timed(
+      ctx, HST_KC_COLUMN,
+      [&] {
+        cudaError_t e = hst::launch_solve_half(G, D, ctx->ps, sc, 0, ctx->stream);
+        return e == cudaSuccess ? hst::launch_solve_half(G, D, ctx->ps, sc, 1, ctx->stream) : e;
+      },
+      2);
 }
 
 // One time step (src/hst_equations.f90:56-87) queued on the stream.
@@ -1320,6 +1255,8 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
   // every member of an ensemble at once (the base buffers); the field itself otherwise
   const Geometry& G = ctx->nmem > 1 ? ctx->gb : ctx->g;
   const DeviceState& D = ctx->nmem > 1 ? ctx->db : ctx->d;
+  const char* env = std::getenv("HST_RHS_TILED");
+  const bool tiled = !(env && std::atoi(env) == 0);
   for (int i = 0; i < 3; ++i) {
     const double* ODE = RK[i];
     const double t = *time;
@@ -1352,26 +1289,12 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
     sc.ytile = p.ly * 32.0 / p.ny;
     shear_shifts(ctx, t, &sc.sx_t, &sc.sz_t);
     shear_shifts(ctx, t + dt_sub, &sc.sx_n, &sc.sz_n);
-    if (ctx->column_split) {
-      CK(timed(ctx, HST_KC_RHS,
-               [&] { return hst::launch_column(G, D, ctx->ps, sc, p.exact_shift, !p.linear, 1, ctx->stream); }));
-      if (p.exact_shift && ctx->shift_split) {
-        // the exact_shift shift as a kernel of its own (one line a group,
-        // no factor scratch: more warps an SM), then the solves
-        CK(timed(ctx, HST_KC_SHIFT,
-                 [&] { return hst::launch_column(G, D, ctx->ps, sc, 1, 0, 3, ctx->stream); }));
-        CK(solve_stage(ctx, G, D, sc, !p.linear));
-      } else if (!p.exact_shift && ctx->solve_halves) {
-        CK(solve_stage(ctx, G, D, sc, !p.linear));
-      } else {
-        CK(timed(ctx, HST_KC_COLUMN, [&] {
-          return hst::launch_column(G, D, ctx->ps, sc, p.exact_shift, !p.linear, 2, ctx->stream);
-        }));
-      }
-    } else {
-      CK(timed(ctx, HST_KC_COLUMN,
-               [&] { return hst::launch_column(G, D, ctx->ps, sc, p.exact_shift, !p.linear, 0, ctx->stream); }));
-    }
+    CK(timed(ctx, HST_KC_RHS, [&] {
+      return tiled ? hst::launch_rhs_tiled(G, D, ctx->ps, sc, p.exact_shift, !p.linear, ctx->stream)
+                   : hst::launch_rhs_rows(G, D, ctx->ps, sc, p.exact_shift, !p.linear, ctx->stream);
+    }));
+    if (p.exact_shift) CK(timed(ctx, HST_KC_SHIFT, [&] { return hst::launch_shift(G, D, ctx->ps, sc, ctx->stream); }));
+    CK(solve_stage(ctx, G, D, sc));
     *time = t + dt_sub;
   }
   return HST_OK;
@@ -1566,7 +1489,7 @@ extern "C" int hst_gpu_buildrhs_prepare(hst_ctx* ctx, const double* ODE, double 
   sc.damp_hard = 0;  // the mask is its own piece (hst_gpu_damping_mask)
   shear_shifts(ctx, time, &sc.sx_t, &sc.sz_t);
   CK(timed(ctx, HST_KC_RHS,
-           [&] { return hst::launch_column(ctx->g, ctx->d, ctx->ps, sc, 1, 0, 4, ctx->stream); }));
+           [&] { return hst::launch_rhs_rows(ctx->g, ctx->d, ctx->ps, sc, 1, 0, ctx->stream); }));
   return HST_OK;
 }
 
@@ -1616,7 +1539,7 @@ extern "C" int hst_gpu_shear_shift(hst_ctx* ctx, double dt_sub, double time) {
   sc.ytile = p.ly * 32.0 / p.ny;
   shear_shifts(ctx, time, &sc.sx_t, &sc.sz_t);
   shear_shifts(ctx, time + dt_sub, &sc.sx_n, &sc.sz_n);
-  CK(timed(ctx, HST_KC_COLUMN, [&] { return hst::launch_column(ctx->g, ctx->d, ctx->ps, sc, 1, 0, 3, ctx->stream); }));
+  CK(timed(ctx, HST_KC_COLUMN, [&] { return hst::launch_shift(ctx->g, ctx->d, ctx->ps, sc, ctx->stream); }));
   return HST_OK;
 }
 
@@ -1626,8 +1549,7 @@ extern "C" int hst_gpu_linsolve(hst_ctx* ctx, double lambda, double time) {
   SubstepScalars sc = {};
   sc.lambda = lambda;
   shear_shifts(ctx, time, &sc.sx_n, &sc.sz_n);
-  CK(timed(ctx, HST_KC_COLUMN,
-           [&] { return hst::launch_column(ctx->g, ctx->d, ctx->ps, sc, 0, !ctx->p.linear, 2, ctx->stream); }));
+  CK(solve_stage(ctx, ctx->g, ctx->d, sc));
   return HST_OK;
 }
 

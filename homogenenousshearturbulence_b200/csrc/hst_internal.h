@@ -1,12 +1,12 @@
 // Internal interface between the C ABI (hst_capi.cu) and the kernels
-// (hst_kernels.cu).  Not installed; the public interface is include/hst_gpu.h.
+// (hst_*.cu).  Not installed; the public interface is include/hst_gpu.h.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <unordered_map>
 #include <unordered_set>
+#include <vector>
 
 #include "../../include/hst_gpu.h"
 
@@ -19,7 +19,7 @@ struct Geometry {
   int nxB, nzT, rows;  // nx+1, 2nz+1, ny+4
   int ncol;            // nxB * nzT Fourier columns
   long nf;             // complex elements of one field (ncol * rows)
-  int P, m, MS;        // line-solve group: P lanes, m rows per lane, slab stride
+  int P;               // lanes of a line-solve group
   int Ty;              // y tile of the transforms (divides ny)
   int pptz;            // FFT points per thread of the z transforms (8: the low-register plans)
   int mp;              // mixed precision: Z, Pp, Q and their transforms in FP32 (complex64)
@@ -40,7 +40,7 @@ struct DeviceState {
   double2* Pp;          // x-forward of the products: [6][nzd][ny/Ty][nxB][Ty]
   double2* Q;           // spectral products: [6][ncol][ny]
   double* der;          // der(0:ny-1, 0:3, -2:2)
-  double* derS;         // the same, slab-major for the line-solve groups (SlabDer)
+  double* derS;         // the same, slab-major for the line-solve groups (slab_major)
   double* derU;         // der's distinct rows, coefficient-major (DerRows); nderU of them, 0: not used
   int* derI;            // the distinct row of each row
   int nderU;
@@ -69,32 +69,10 @@ struct DeviceState {
   // kernels whose shared-memory limit has been raised in this context
   // (owned by the context; null: raise it at every launch)
   std::unordered_set<const void*>* configured;
-  // resident blocks an SM of (kernel, threads, shared bytes) launches, asked
-  // once (owned by the context; null: asked at every launch)
-  std::unordered_map<uint64_t, int>* occupancy;
-  // the column kernels' factor scratch in global memory (one slice per
-  // resident solver group; null: the scratch stays in shared memory)
+  // the line solves' factor scratch (a slice a resident solver group)
   double* facg;
   size_t facg_doubles;
 };
-
-// Resident blocks an SM of kernel k with T threads and `smem` dynamic
-// shared bytes (cudaOccupancyMaxActiveBlocksPerMultiprocessor, cached).
-template <typename K>
-inline int blocks_per_sm(const DeviceState& d, K k, int T, size_t smem) {
-  const uint64_t key = (uint64_t)(uintptr_t)reinterpret_cast<const void*>(k) * 1000003ull ^ ((uint64_t)T << 40) ^ smem;
-  if (d.occupancy) {
-    auto it = d.occupancy->find(key);
-    if (it != d.occupancy->end()) return it->second;
-  }
-  int n = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, T, smem) != cudaSuccess || n < 1) {
-    cudaGetLastError();
-    n = 1;
-  }
-  if (d.occupancy) (*d.occupancy)[key] = n;
-  return n;
-}
 
 // Raises kernel k's dynamic shared-memory limit to `bytes`, once per context
 // (the attribute belongs to the function in the current context; setting it
@@ -128,24 +106,31 @@ struct PhysScalars {
 cudaError_t launch_zinv(const Geometry& g, const DeviceState& d, cudaStream_t st);
 cudaError_t launch_xprod(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl, cudaStream_t st);
 cudaError_t launch_zfwd(const Geometry& g, const DeviceState& d, cudaStream_t st);
-// part: 0 the fused column kernel, 1 its right-hand-side stage alone (row
-// streaming, into RHS1/RHS2), 2 the rest (shift, solves, u, w) from RHS1/RHS2,
-// 3 (exact only, nonlin 0) the exact_shift shift of RHS1/2, OLD1/2 alone,
-// 4 the right-hand-side stage in its untiled FP64 form
-cudaError_t launch_column(const Geometry& g, const DeviceState& d, const PhysScalars& ph, const SubstepScalars& sc,
-                          int exact, int nonlin, int part, cudaStream_t st);
 // the right-hand sides streamed through shared memory (hst_rhs.cu)
 cudaError_t launch_rhs_tiled(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
                              int exact, int nonlin, cudaStream_t st);
+// the same row by row from global memory (hst_kernels.cu)
+cudaError_t launch_rhs_rows(const Geometry& g, const DeviceState& d, const PhysScalars& ph, const SubstepScalars& sc,
+                            int exact, int nonlin, cudaStream_t st);
+// the implicit half (hst_solve.cu): the exact_shift shift of RHS1/2, OLD1/2,
+// and the solves in two passes (half 0, then 1) from RHS1/2 into V1..V3
+cudaError_t launch_shift(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
+                         cudaStream_t st);
+cudaError_t launch_solve_half(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
+                              int half, cudaStream_t st);
+// lanes of a solver group for ny rows and this many columns
+int line_lanes(int ny, long columns);
+// der(0:ny-1, 0:3, -2:2) in the slab-major order of groups of P lanes; the
+// doubles that any P takes
+std::vector<double> slab_major(const std::vector<double>& der, int ny, int P);
+size_t slab_der_doubles(int ny);
+// bytes of the solves' factor scratch (DeviceState::facg)
+size_t solve_scratch_bytes(const Geometry& g, int nsm);
 cudaError_t launch_line_solve(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int sys, double lambda,
                               int src, int dst, double sx, double sz, cudaStream_t st);
 cudaError_t launch_fill_ghosts(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int field, double sx,
                                double sz, cudaStream_t st);
-size_t column_smem_bytes(const Geometry& g, int exact);
-// the two line buffers of a solver group, and its factor scratch (doubles)
-size_t column_lines_bytes(const Geometry& g);
-size_t column_fac_doubles(const Geometry& g);
-// the factored D0 matrix of the line-solve group (P, m of g) into d.d0tab,
+// the factored D0 matrix of the line-solve group (P of g) into d.d0tab,
 // from d.derS; d0_table_doubles: the table's size for any group of ny rows
 cudaError_t launch_d0_table(const Geometry& g, const DeviceState& d, cudaStream_t st);
 size_t d0_table_doubles(int ny);

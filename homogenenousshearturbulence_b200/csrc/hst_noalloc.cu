@@ -39,25 +39,27 @@
 #include <cstdlib>
 #include <cstdio>
 
-#include "hst_dev.cuh"
 #include "hst_internal.h"
+#include "hst_line.cuh"
 
 #define HST_NOALLOC_MAX_NY 2048
 
 namespace {
 
-// der(0:ny-1, 0:3, -2:2) reordered slab-major (the order of hst::SlabDer)
+// der(0:ny-1, 0:3, -2:2) reordered slab-major (the order of hst::slab_major)
 __device__ __align__(256) double g_line_der[20 * HST_NOALLOC_MAX_NY];
 
-// out[((n*5 + j)*m + i)*P + s] = der(s*m + i, n, j - 2)
-__global__ void k_slab_major(const double* __restrict__ der, double* __restrict__ out, int ny, int P, int m) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 20 * ny) return;
+// out[((n*5 + j)*mM + i)*P + s] = der(first(s) + i, n, j - 2); the place past
+// the end of a shorter slab repeats its last row
+__global__ void k_slab_major(const double* __restrict__ der, double* __restrict__ out, int ny, int P) {
+  const int mM = hst::slab_rows(ny, P), e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 20 * mM * P) return;
+  const hst::LineGeom G = hst::line_geom(ny, P);
   const int s = e % P;
-  const int i = (e / P) % m;
-  const int nj = e / (P * m);  // n * 5 + j
+  const int i = (e / P) % mM;
+  const int nj = e / (P * mM);  // n * 5 + j
   const int n = nj / 5, j = nj - 5 * n;
-  out[e] = der[(size_t)(s * m + i) + (size_t)ny * (n + 4 * j)];
+  out[e] = der[(size_t)(G.first(s) + min(i, G.rows(s) - 1)) + (size_t)ny * (n + 4 * j)];
 }
 
 int fail(char* msg, int len, int rc, const char* fmt, ...) {
@@ -70,21 +72,17 @@ int fail(char* msg, int len, int rc, const char* fmt, ...) {
   return rc;
 }
 
-// lanes of a solver group: the rule of the context's default geometry (the
-// widest power of two up to 32 that leaves at least 8 rows per lane, else 4;
-// HST_LINE_LANES overrides), so the results are identical to those of a
+// lanes of a solver group: the rule of a context of one field of these sizes
+// (HST_LINE_LANES overrides), so the results are identical to those of such a
 // context that has not been autotuned; hst_gpu_autotune may give a context
 // another group width, and the two then agree up to rounding
-int line_lanes(int ny) {
+int lanes_of(int ny, long columns) {
   const char* env = std::getenv("HST_LINE_LANES");
   if (env) {
     int e = std::atoi(env);
     if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && ny % e == 0 && ny / e >= 4) return e;
   }
-  for (int mmin : {8, 4})
-    for (int c = 32; c >= 2; c >>= 1)
-      if (ny % c == 0 && ny / c >= mmin) return c;
-  return 0;
+  return hst::line_lanes(ny, columns);
 }
 
 }  // namespace
@@ -110,8 +108,7 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
     if (a < b + bytes && b < a + bytes) return fail(msg, msg_len, HST_EARG, "src and dst overlap");
     if (c < b + bytes && b < c + dbytes) return fail(msg, msg_len, HST_EARG, "der and dst overlap");
   }
-  const int P = line_lanes(ny);
-  if (!P) return fail(msg, msg_len, HST_EARG, "ny = %d: no solver group with at least 4 rows per lane", ny);
+  const int P = lanes_of(ny, (long)(nx + 1) * (2 * nz + 1));
 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -131,8 +128,6 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
   g.ncol = g.nxB * g.nzT;
   g.nf = (long)g.ncol * g.rows;
   g.P = P;
-  g.m = ny / P;
-  g.MS = g.m | 1;
   hst::PhysScalars ps = {};
   ps.alfa0 = alfa0;
   ps.beta0 = beta0;
@@ -144,8 +139,9 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
   d.derS = scratch;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-  const int n = 20 * ny, T = 256;
-  k_slab_major<<<(n + T - 1) / T, T, 0, st>>>(der, scratch, ny, P, g.m);
+  const int n = 20 * hst::slab_rows(ny, P) * P, T = 256;
+  if (n > 20 * HST_NOALLOC_MAX_NY) return fail(msg, msg_len, HST_EARG, "ny = %d exceeds the static scratch", ny);
+  k_slab_major<<<(n + T - 1) / T, T, 0, st>>>(der, scratch, ny, P);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = hst::launch_line_solve(g, d, ps, sys, lambda, 0, 1, shift_x, shift_z, st);
   if (e != cudaSuccess) return fail(msg, msg_len, HST_ECUDA, "launch: %s", cudaGetErrorString(e));

@@ -1,0 +1,434 @@
+// The implicit half of the substep, one Fourier column a group of P lanes
+// (hst_line.cuh), the line in shared memory:
+//
+//   k_shift       the exact_shift shear shift (shift_unweighted,
+//                 src/hst_equations.f90:263-293) of rhs1, rhs2, old1, old2: D0
+//                 solve with the wrap at t, node phase exp(-i gx y), D0 stencil
+//                 with the ghost images at t + dt_sub
+//   k_solve_half  linsolve (src/hst_equations.f90:298-326) in two passes of
+//                 one line: 0 the D2V solve, V2 with its ghost rows, dv/dy (the
+//                 DY solve of its D1 stencil) into the interior rows of V1,
+//                 scratch until the second pass; 1 the ETA solve, u and w,
+//                 V1 and V3 with their ghost rows
+//   k_line_solve  line_solve (src/hst_linsolve.f90:147-233) of one field
+//   k_d0_table    the factored D0 matrix
+//
+// k_shift and k_solve_half run on a persistent grid of one block an SM whose
+// warps share the tables in shared memory; the factors of the D2V and ETA
+// solves go to a slice of global scratch a group, rewritten column after
+// column (so that it stays in L2): without them in shared memory sixteen
+// warps' lines fit an SM.
+#include <algorithm>
+
+#include "hst_internal.h"
+#include "hst_line.cuh"
+
+namespace hst {
+
+struct SolveArgs {
+  Geometry g;
+  PhysScalars ps;
+  SubstepScalars sc;
+  double2 *V1, *V2, *V3, *O1, *O2, *R1, *R2;
+  const double* derS;
+  const double* d0tab;
+  const double* y;
+  double2* fac;  // factor scratch, facn double2 a group
+  int facn;
+};
+
+// a group's lanes within its warp
+template <int P>
+__device__ __forceinline__ unsigned group_mask() {
+  if (P == 32) return 0xffffffffu;
+  return ((1u << (P & 31)) - 1u) << ((threadIdx.x & 31) / P * P);
+}
+
+// a column's place and wave numbers
+struct Column {
+  double al, be, kk;
+  bool c00;
+  size_t cb;  // row 0 of the column
+};
+__device__ __forceinline__ Column column_of(const Geometry& g, const PhysScalars& ps, int cg) {
+  Column c;
+  const int col = g.nmem > 1 ? cg % g.ncol : cg;
+  const int ix = col / g.nzT, iz = col - ix * g.nzT - g.nz;
+  c.c00 = ix == 0 && iz == 0;
+  c.al = ps.alfa0 * ix;
+  c.be = ps.beta0 * iz;
+  c.kk = c.al * c.al + c.be * c.be;
+  c.cb = (size_t)cg * g.rows + 2;
+  return c;
+}
+
+template <int P>
+__device__ __forceinline__ void load_line(const double2* __restrict__ src, cxd* buf, const LineGeom& G, int s) {
+#pragma unroll 4
+  for (int r = s; r < G.n; r += P) buf[G.at(r)] = src[r];
+}
+template <int P>
+__device__ __forceinline__ void store_line(double2* __restrict__ dst, const cxd* buf, const LineGeom& G, int s) {
+#pragma unroll 4
+  for (int r = s; r < G.n; r += P) dst[r] = buf[G.at(r)];
+}
+// the four ghost rows of a column (row 0 at dst) from its line (wrap_rows,
+// src/hst_mpi.f90:340-355)
+template <int P>
+__device__ __forceinline__ void store_ghosts(double2* __restrict__ dst, const cxd* buf, const LineGeom& G, cxd ph, int s) {
+  for (int k = s; k < 4; k += P) {
+    // k = 0: row ny (row 0 ph), 1: row ny+1 (row 1 ph), 2: row -1 (row ny-1 conj), 3: row -2
+    const int srow = k < 2 ? k : G.n + 1 - k, drow = k < 2 ? G.n + k : 1 - k;
+    dst[drow] = cmul(buf[G.at(srow)], k < 2 ? ph : cconj(ph));
+  }
+}
+
+// SH: the tables in shared memory (the most rows have no room there)
+template <int P, bool SH>
+__global__ void __launch_bounds__(512, 1) k_shift(SolveArgs a) {
+  extern __shared__ __align__(16) double smem_d[];
+  const Geometry& g = a.g;
+  const SubstepScalars& sc = a.sc;
+  const LineGeom G = line_geom(g.ny, P);
+  const int mM = slab_rows(g.ny, P);
+  const int groups = blockDim.x / P, grp = threadIdx.x / P, s = threadIdx.x % P;
+  const unsigned gmask = group_mask<P>();
+  const int ntab = SH ? d0_fields(mM, P) * P : 0, nder = SH ? 5 * mM * P : 0;
+  double* const d0s = smem_d;
+  double* const der0s = d0s + ntab;
+  for (int i = threadIdx.x; i < ntab; i += blockDim.x) d0s[i] = a.d0tab[i];
+  for (int i = threadIdx.x; i < nder; i += blockDim.x) der0s[i] = a.derS[i];
+  if (SH) __syncthreads();
+  cxd* const buf = reinterpret_cast<cxd*>(der0s + nder) + (size_t)grp * P * G.MS;
+  cxd* const sb = buf + s * G.MS;
+  const int m = G.rows(s), r0 = G.first(s);
+  const SlabDerT<SH> DS = {SH ? der0s : a.derS, mM, P};
+  for (int cg = blockIdx.x * groups + grp; cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
+    const Column c = column_of(g, a.ps, cg);
+    const cxd pt = cexpi(-(c.al * sc.sx_t + c.be * sc.sz_t)), pn = cexpi(-(c.al * sc.sx_n + c.be * sc.sz_n));
+    const double gx = c.al * sc.dgx + c.be * sc.dgz;
+    // the node phase of the slab's last row; on a uniform grid the rows
+    // below follow by one complex product each (dy = ly / ny apart)
+    const cxd e0 = sc.yuni ? cexpi(-gx * a.y[r0 + m + 1]) : mkc(1.0, 0.0);
+    const cxd step = sc.yuni ? cexpi(gx * (sc.ytile / 32.0)) : mkc(1.0, 0.0);
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      double2* const f = (q == 0 ? a.O1 : (q == 1 ? a.O2 : (q == 2 ? a.R1 : a.R2))) + c.cb;
+      load_line<P>(f, buf, G, s);
+      __syncwarp(gmask);
+      line_solve_d0<P, SH, true>(pt, SH ? d0s : a.d0tab, mM, m, sb, s, gmask, e0, step);
+      if (!sc.yuni)
+        for (int i = 0; i < m; ++i) sb[i] = cmul(sb[i], cexpi(-gx * a.y[r0 + i + 2]));
+      slab_stencil<P>(0, DS, sb, m, s, pn, gmask);
+      __syncwarp(gmask);
+      store_line<P>(f, buf, G, s);
+      __syncwarp(gmask);
+    }
+  }
+}
+
+__host__ __device__ constexpr int half_slices(int half) { return half == 0 ? 4 : 3; }
+// SH: der's slices (HALF 0: all four, 1: the first three) in shared memory
+template <int P, int HALF, bool SH>
+__global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
+  extern __shared__ __align__(16) double smem_d[];
+  const Geometry& g = a.g;
+  const SubstepScalars& sc = a.sc;
+  const LineGeom G = line_geom(g.ny, P);
+  const int mM = slab_rows(g.ny, P), ny = g.ny;
+  const int groups = blockDim.x / P, grp = threadIdx.x / P, s = threadIdx.x % P;
+  const unsigned gmask = group_mask<P>();
+  const int nder = SH ? half_slices(HALF) * 5 * mM * P : 0;
+  if (SH) {
+    for (int i = threadIdx.x; i < nder; i += blockDim.x) smem_d[i] = a.derS[i];
+    __syncthreads();
+  }
+  cxd* const buf = reinterpret_cast<cxd*>(smem_d + nder) + (size_t)grp * P * G.MS;
+  cxd* const sb = buf + s * G.MS;
+  const int m = G.rows(s);
+  const SlabDerT<SH> DS = {SH ? smem_d : a.derS, mM, P};
+  const int slot = blockIdx.x * groups + grp;
+  double2* const fac = a.fac + (size_t)slot * a.facn + s;
+  for (int cg = slot; cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
+    const Column c = column_of(g, a.ps, cg);
+    const cxd pn = cexpi(-(c.al * sc.sx_n + c.be * sc.sz_n));
+    double2* const v1 = a.V1 + c.cb;
+    load_line<P>((HALF == 0 ? a.R2 : a.R1) + c.cb, buf, G, s);
+    __syncwarp(gmask);
+    if constexpr (HALF == 0) {
+      line_solve<P, 3>(band_const(K_D2V, sc.lambda, a.ps.ni, c.kk), pn, DS, m, sb, fac, s, gmask);
+      if (c.c00)  // the (0,0) column's v is zero
+        for (int i = 0; i < m; ++i) sb[i] = mkc(0, 0);
+      __syncwarp(gmask);
+      double2* const v2 = a.V2 + c.cb;
+      store_line<P>(v2, buf, G, s);
+      store_ghosts<P>(v2, buf, G, pn, s);
+      __syncwarp(gmask);
+      // D1 v, then D0 (dv/dy) = D1 v (KIND_DY)
+      slab_stencil<P>(1, DS, sb, m, s, pn, gmask);
+      line_solve_d0<P, false, false>(pn, a.d0tab, mM, m, sb, s, gmask);
+      __syncwarp(gmask);
+      store_line<P>(v1, buf, G, s);
+    } else {
+      line_solve<P, 2>(band_const(K_ETA, sc.lambda, a.ps.ni, c.kk), pn, DS, m, sb, fac, s, gmask);
+      __syncwarp(gmask);
+      const double rkk = c.c00 ? 0.0 : 1.0 / c.kk, ar = c.al * rkk, br = c.be * rkk;
+      double2* const v3 = a.V3 + c.cb;
+      // dv/dy eight rows at a time, every load issued before the first use
+      for (int r0 = s; r0 < ny; r0 += 8 * P) {
+        cxd dvb[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dvb[k] = r0 + k * P < ny ? v1[r0 + k * P] : mkc(0, 0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = r0 + k * P;
+          if (r >= ny) break;
+          const cxd eta = buf[G.at(r)], dv = dvb[k];
+          // (i alfa dv - i beta eta) / k2, (i beta dv + i alfa eta) / k2
+          const cxd u = c.c00 ? mkc(eta.x, 0.0) : mkc(br * eta.y - ar * dv.y, ar * dv.x - br * eta.x);
+          const cxd w = c.c00 ? mkc(eta.y, 0.0) : mkc(-br * dv.y - ar * eta.y, br * dv.x + ar * eta.x);
+          v1[r] = u;
+          v3[r] = w;
+          if (r < 2) {
+            v1[ny + r] = cmul(u, pn);
+            v3[ny + r] = cmul(w, pn);
+          }
+          if (r >= ny - 2) {
+            v1[r - ny] = cmul(u, cconj(pn));
+            v3[r - ny] = cmul(w, cconj(pn));
+          }
+        }
+      }
+    }
+    __syncwarp(gmask);
+  }
+}
+
+// line_solve for every Fourier column of one field, the factors in shared
+// memory (a caller's own arrays come with no scratch)
+template <int P>
+__global__ void __launch_bounds__(64) k_line_solve(Geometry g, PhysScalars ps, int sys, double lambda,
+                                                   const double2* __restrict__ src, double2* __restrict__ dst, double sx,
+                                                   double sz, const double* __restrict__ der,
+                                                   const double* __restrict__ derS) {
+  extern __shared__ __align__(16) double smem_d[];
+  const LineGeom G = line_geom(g.ny, P);
+  const int mM = slab_rows(g.ny, P), ny = g.ny;
+  const SlabDerT<false> DS = {derS, mM, P};
+  const int groups = blockDim.x / P, grp = threadIdx.x / P, s = threadIdx.x % P;
+  const int col = blockIdx.x * groups + grp;
+  if (col >= g.ncol) return;
+  const unsigned gmask = group_mask<P>();
+  double2* const buf = reinterpret_cast<double2*>(smem_d) + (size_t)grp * P * (G.MS + 2 * (mM - 2));
+  double2* const fac = buf + P * G.MS + s;
+  const Column c = column_of(g, ps, col);
+  const double2* const sc = src + c.cb;
+  double2* const dc = dst + c.cb;
+  if (sys == K_DY) {
+    for (int r = s; r < ny; r += P) {
+      cxd v = mkc(0, 0);
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const double d1 = derv(der, ny, r, 1, j - 2);
+        const cxd q = sc[r + j - 2];
+        v = mkc(v.x + d1 * q.x, v.y + d1 * q.y);
+      }
+      buf[G.at(r)] = v;
+    }
+  } else {
+    load_line<P>(sc, buf, G, s);
+  }
+  __syncwarp(gmask);
+  const BandConst bc = band_const(sys, lambda, ps.ni, c.kk);
+  const cxd ph = cexpi(-(c.al * sx + c.be * sz));
+  cxd* const sb = buf + s * G.MS;
+  if (sys == K_D2V)
+    line_solve<P, 3>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
+  else if (sys == K_ETA || sys == K_POISSON)
+    line_solve<P, 2>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
+  else
+    line_solve<P, 1>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
+  __syncwarp(gmask);
+  if (c.c00 && sys == K_POISSON) return;
+  if (c.c00 && sys == K_D2V)
+    for (int r = s; r < ny; r += P) dc[r] = mkc(0, 0);
+  else
+    store_line<P>(dc, buf, G, s);
+}
+
+// d0_factor of the group of P lanes: one warp, lanes 0..P-1
+template <int P>
+__global__ void k_d0_table(const double* __restrict__ derS, int ny, double* __restrict__ tab) {
+  const int s = threadIdx.x;
+  if (s >= P) return;
+  const int mM = slab_rows(ny, P);
+  const SlabDerT<false> DS = {derS, mM, P};
+  d0_factor<P>(DS, line_geom(ny, P).rows(s), mM, s, group_mask<P>(), tab);
+}
+
+// -------------------------------------------------------------- launchers ----
+// The lanes of a solver group: as many as leave at least four rows a lane,
+// then half of them while a lane has fewer than twelve rows and the columns
+// still give each of the chip's 148 SMs twelve warps: the reduction across
+// the lanes costs as much as some ten rows.  Measured for the solves: 64 rows of
+// 2080 columns 25.0 us with 16 lanes, 29.0 with 8; 128 rows of 8128 columns
+// 59 us with 8 lanes, 73 with 16, 97 with 32; 256 rows of 32896 columns 384 us
+// with 16 lanes, 434 with 32, 487 with 8; 512 rows 3.10 ms with 32, 3.71 with 16.
+int line_lanes(int ny, long columns) {
+  int P = 2;
+  for (int c = 32; c > 2; c >>= 1)
+    if (ny / c >= 4) {
+      P = c;
+      break;
+    }
+  while (P > 4 && ny / P < 12 && columns >= 148L * 12 * (32 / (P / 2))) P >>= 1;
+  return P;
+}
+
+size_t slab_der_doubles(int ny) { return (size_t)20 * (ny + 32); }
+size_t d0_table_doubles(int ny) {
+  // d0_fields(mM, P) P, mM P < ny + P
+  return (size_t)9 * (ny + 32) + 32 * (31 + 8 * 4);
+}
+std::vector<double> slab_major(const std::vector<double>& der, int ny, int P) {
+  const int mM = slab_rows(ny, P);
+  const LineGeom G = line_geom(ny, P);
+  std::vector<double> o((size_t)20 * mM * P, 0.0);
+  for (int s = 0; s < P; ++s) {
+    const int m = G.m + (s < G.rem ? 1 : 0), r0 = s * G.m + std::min(s, G.rem);
+    for (int n = 0; n < 4; ++n)
+      for (int j = 0; j < 5; ++j)
+        for (int i = 0; i < m; ++i)
+          o[((size_t)(n * 5 + j) * mM + i) * P + s] = der[(size_t)(r0 + i) + (size_t)ny * (n + 4 * j)];
+  }
+  return o;
+}
+
+static size_t line_bytes(int ny, int P) { return (size_t)P * line_geom(ny, P).MS * sizeof(double2); }
+// double2 of factor scratch a group
+static int fac_elems(int ny, int P) { return 2 * (slab_rows(ny, P) - 2) * P; }
+
+// warps a block (one block an SM): as many as sixteen whose lines fit beside
+// `tabs` bytes of tables, and no more than spread the columns over the SMs;
+// 0 when not even one fits
+static int solve_warps(const Geometry& g, int nsm, size_t tabs) {
+  const size_t warp = line_bytes(g.ny, g.P) * (32 / g.P);
+  if (tabs + warp > 227 * 1024) return 0;
+  const long groups = ((long)g.ncol * g.nmem + nsm - 1) / nsm;  // columns an SM
+  const long want = (groups * g.P + 31) / 32;
+  return (int)std::min<long>({16, want, (long)((227 * 1024 - tabs) / warp)});
+}
+
+size_t solve_scratch_bytes(const Geometry& g, int nsm) {
+  return (size_t)nsm * 16 * (32 / g.P) * fac_elems(g.ny, g.P) * sizeof(double2);
+}
+
+static SolveArgs solve_args(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc) {
+  return {g,      ps,     sc,     d.F[0], d.F[1],  d.F[2], d.F[3],
+          d.F[4], d.F[5], d.F[6], d.derS, d.d0tab, d.y,    reinterpret_cast<double2*>(d.facg), fac_elems(g.ny, g.P)};
+}
+static int sm_count(const DeviceState& d) { return d.nsm > 0 ? d.nsm : 148; }
+
+template <int P>
+static cudaError_t launch_shift_t(const SolveArgs& a, const DeviceState& d, cudaStream_t st) {
+  const Geometry& g = a.g;
+  const int mM = slab_rows(g.ny, P), nsm = sm_count(d);
+  size_t tabs = ((size_t)d0_fields(mM, P) * P + (size_t)5 * mM * P) * sizeof(double);
+  int W = solve_warps(g, nsm, tabs);
+  const bool sh = W >= 4 || W == solve_warps(g, nsm, 0);
+  if (!sh) {  // the tables through L1
+    tabs = 0;
+    W = solve_warps(g, nsm, 0);
+  }
+  if (W < 1) return cudaErrorInvalidValue;
+  const int groups = W * 32 / P;
+  const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
+  auto k = sh ? k_shift<P, true> : k_shift<P, false>;
+  smem_limit(d, k, 227 * 1024);
+  k<<<nb, 32 * W, tabs + W * line_bytes(g.ny, P) * (32 / P), st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int P, int HALF>
+static cudaError_t launch_half_t(const SolveArgs& a, const DeviceState& d, cudaStream_t st) {
+  const Geometry& g = a.g;
+  const int mM = slab_rows(g.ny, P), nsm = sm_count(d);
+  size_t tabs = (size_t)half_slices(HALF) * 5 * mM * P * sizeof(double);
+  int W = solve_warps(g, nsm, tabs);
+  const bool sh = W >= 4 || W == solve_warps(g, nsm, 0);
+  if (!sh) {  // der through L1
+    tabs = 0;
+    W = solve_warps(g, nsm, 0);
+  }
+  if (W < 1 || !a.fac) return cudaErrorInvalidValue;
+  int groups = W * 32 / P;
+  // no more groups than the scratch has slices for
+  const long slices = (long)(d.facg_doubles / 2 / a.facn);
+  while (W > 1 && slices < groups) groups = --W * 32 / P;
+  const int nb = (int)std::min<long>({nsm, (g.ncol * g.nmem + groups - 1) / groups, slices / groups});
+  if (nb < 1) return cudaErrorInvalidValue;
+  const size_t smem = tabs + W * line_bytes(g.ny, P) * (32 / P);
+  auto k = sh ? k_solve_half<P, HALF, true> : k_solve_half<P, HALF, false>;
+  smem_limit(d, k, 227 * 1024);
+  k<<<nb, 32 * W, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int P>
+static cudaError_t launch_line_solve_t(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int sys,
+                                       double lambda, int src, int dst, double sx, double sz, cudaStream_t st) {
+  const size_t per = line_bytes(g.ny, P) + fac_elems(g.ny, P) * sizeof(double2);
+  int groups = 32 / P;
+  while (groups > 1 && per * groups > 200 * 1024) groups >>= 1;
+  if (per * groups > 200 * 1024) return cudaErrorInvalidValue;
+  smem_limit(d, k_line_solve<P>, 200 * 1024);
+  k_line_solve<P><<<(g.ncol + groups - 1) / groups, groups * P, per * groups, st>>>(g, ps, sys, lambda, d.F[src],
+                                                                                   d.F[dst], sx, sz, d.der, d.derS);
+  return cudaGetLastError();
+}
+
+#define HST_LANES(P_, CALL)                \
+  switch (P_) {                            \
+    case 2: return CALL(2);                \
+    case 4: return CALL(4);                \
+    case 8: return CALL(8);                \
+    case 16: return CALL(16);              \
+    case 32: return CALL(32);              \
+  }                                        \
+  return cudaErrorInvalidValue
+
+cudaError_t launch_shift(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
+                         cudaStream_t st) {
+  const SolveArgs a = solve_args(g, d, ps, sc);
+#define HST_CALL(P) launch_shift_t<P>(a, d, st)
+  HST_LANES(g.P, HST_CALL);
+#undef HST_CALL
+}
+
+cudaError_t launch_solve_half(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
+                              int half, cudaStream_t st) {
+  const SolveArgs a = solve_args(g, d, ps, sc);
+#define HST_CALL(P) (half == 0 ? launch_half_t<P, 0>(a, d, st) : launch_half_t<P, 1>(a, d, st))
+  HST_LANES(g.P, HST_CALL);
+#undef HST_CALL
+}
+
+cudaError_t launch_line_solve(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int sys, double lambda,
+                              int src, int dst, double sx, double sz, cudaStream_t st) {
+#define HST_CALL(P) launch_line_solve_t<P>(g, d, ps, sys, lambda, src, dst, sx, sz, st)
+  HST_LANES(g.P, HST_CALL);
+#undef HST_CALL
+}
+
+template <int P>
+static cudaError_t launch_d0_t(const Geometry& g, const DeviceState& d, cudaStream_t st) {
+  k_d0_table<P><<<1, 32, 0, st>>>(d.derS, g.ny, d.d0tab);
+  return cudaGetLastError();
+}
+cudaError_t launch_d0_table(const Geometry& g, const DeviceState& d, cudaStream_t st) {
+#define HST_CALL(P) launch_d0_t<P>(g, d, st)
+  HST_LANES(g.P, HST_CALL);
+#undef HST_CALL
+}
+
+}  // namespace hst
