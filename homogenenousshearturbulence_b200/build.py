@@ -15,7 +15,7 @@ PKG = pathlib.Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libhst_gpu.so"
-SOURCES = ["hst_kernels.cu", "hst_transforms.cu", "hst_xprod.cu", "hst_rhs.cu", "hst_solve.cu", "hst_capi.cu", "hst_noalloc.cu", "hst_stats.cu", "hst_pieces.cu"]
+SOURCES = ["hst_kernels.cu", "hst_transforms.cu", "hst_z.cu", "hst_xprod.cu", "hst_rhs.cu", "hst_solve.cu", "hst_capi.cu", "hst_noalloc.cu", "hst_stats.cu", "hst_pieces.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -335,17 +335,8 @@ static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::
     int e = std::atoi(env);
     if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && p.ny % e == 0 && p.ny / e >= 4) g.P = e;
   }
-  // z FFT points per thread: 8 selects the low-register plans (lengths 192,
-  // 384, 768).  Measured: 16 at 384^2 x 256 (0.26/0.50 against 0.29/0.52 ms),
-  // 8 at 768^2 x 512 (2.4/4.9 against 4.0/14.0 ms).  HST_FFT_PPT_Z overrides.
-  auto ppt_of = [](const char* name, int dflt) {
-    const char* e = std::getenv(name);
-    int v = e ? std::atoi(e) : dflt;
-    return (v == 8 || v == 16) ? v : dflt;
-  };
-  g.pptz = ppt_of("HST_FFT_PPT_Z", g.nzd >= 768 ? 8 : 16);
-  // mixed precision: the FP32 transforms of the lengths it compiles
-  // (8 points a thread, 16 at 96) and the streamed right-hand sides
+  // mixed precision: the FP32 transforms of the lengths it compiles and the
+  // streamed right-hand sides
   g.mp = p.precision == HST_PREC_MIXED;
   if (p.precision != HST_PREC_FP64 && p.precision != HST_PREC_MIXED) {
     why = "precision must be HST_PREC_FP64 or HST_PREC_MIXED";
@@ -356,23 +347,24 @@ static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::
       why = "mixed precision needs 2 nxd and nzd in {96, 192, 384, 768, 1536} and ny a multiple of 32";
       return HST_EARG;
     }
-    // 16 points a thread for the FP32 z transforms (zfwd 0.29 against 0.34 ms at 384)
-    g.pptz = g.nzd == 768 ? 8 : ppt_of("HST_FFT_PPT_Z", 16);
   }
-  // 1536 points: one plan in both precisions, 32 points a thread
-  if (g.nzd == 1536) g.pptz = 32;
-  // transform y tile (at most 512 threads for the 8-point z plans)
-  g.Ty = 2;
-  for (int t : {8, 4}) {
-    // (the lines are padded, one element in eight for the 8-point plans, in
-    // sixteen for the others: two blocks of up to 112 KB share an SM)
-    const size_t line = g.pptz == 8 ? g.nzd + g.nzd / 8 + 8 : g.nzd + g.nzd / 16 + 8;
-    if (p.ny % t == 0 && (size_t)t * line * 16 <= 112 * 1024 && (g.pptz != 8 || t * g.nzd / 8 <= 384)) {
-      g.Ty = t;
-      break;
+  // y tiles of the transforms: what the z plan takes, the last one reaching
+  // beyond ny where it does not divide it; of the runtime plan, divisors of ny
+  // whose lines fit half an SM's shared memory
+  g.Ty = hst::z_rows(g.nzd, g.mp != 0);
+  if (!g.Ty) {
+    g.Ty = 2;
+    for (int t : {8, 4}) {
+      if (p.ny % t == 0 && (size_t)t * (g.nzd + 1) * 16 <= 112 * 1024) {
+        g.Ty = t;
+        break;
+      }
     }
   }
-  if (!hst::fft_length_ok(2 * g.nxd) || !hst::fft_length_ok(g.nzd) || g.Ty * g.nzd > 32 * 256 ||
+  g.nyT = (p.ny + g.Ty - 1) / g.Ty;
+  g.EY = hst::z_rows(g.nzd, g.mp != 0) ? g.Ty : 4;
+  if (!hst::fft_length_ok(2 * g.nxd) || !hst::fft_length_ok(g.nzd) ||
+      (!hst::z_rows(g.nzd, g.mp != 0) && g.Ty * g.nzd > 32 * 256) ||
       6 * 2 * g.nxd > 32 * 320) {
     why = "transform length not supported (2 nxd <= 1536, radices 2, 3, 4, 6, 8, 12, 16, 24)";
     return HST_EARG;
@@ -382,7 +374,7 @@ static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::
 
 static double dev_bytes(const Geometry& g) {
   double nf = (double)g.nf;
-  double z = 3.0 * g.nzd * g.ny * g.nxB, pp = 6.0 * g.nzd * g.ny * g.nxB, q = 6.0 * g.ncol * g.ny;
+  double z = 3.0 * g.nzd * g.nyT * g.Ty * g.nxB, pp = 2.0 * z, q = 6.0 * g.ncol * g.ny;
   return 16.0 * 7.0 * nf + (g.mp ? 8.0 : 16.0) * (z + pp + q) + 8.0 * (20.0 * g.ny + 2.0 * g.ny + 4 + g.ncol);
 }
 
@@ -570,12 +562,12 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   const size_t nm = (size_t)nmem;  // the per-field buffers hold every member
   for (int i = 0; i < 7 && ok; ++i) ok = alloc((void**)&d.F[i], sizeof(double2) * g.nf * nm);
   const size_t es = g.mp ? sizeof(float2) : sizeof(double2);  // the transforms' complex element
-  ok = ok && alloc((void**)&d.Z, es * 3 * (size_t)g.nzd * g.ny * g.nxB * nm);
-  ok = ok && alloc((void**)&d.Pp, es * 6 * (size_t)g.nzd * g.ny * g.nxB * nm);
+  ok = ok && alloc((void**)&d.Z, es * 3 * (size_t)g.nzd * g.nyT * g.Ty * g.nxB * nm);
+  ok = ok && alloc((void**)&d.Pp, es * 6 * (size_t)g.nzd * g.nyT * g.Ty * g.nxB * nm);
   ok = ok && alloc((void**)&d.Q, es * 6 * (size_t)g.ncol * g.ny * nm);
   if (hst::edge_rows_needed(g, p.s2_amplitude != 0.0 || p.s2_mean != 0.0)) {
-    ok = ok && alloc((void**)&d.Zg, es * 3 * (size_t)g.nzd * g.nxB * 4 * nm);
-    ok = ok && alloc((void**)&d.Ppg, es * 6 * (size_t)g.nzd * g.nxB * 4 * nm);
+    ok = ok && alloc((void**)&d.Zg, es * 3 * (size_t)g.nzd * g.nxB * g.EY * nm);
+    ok = ok && alloc((void**)&d.Ppg, es * 6 * (size_t)g.nzd * g.nxB * g.EY * nm);
     ok = ok && alloc((void**)&d.Qg, es * 6 * (size_t)g.ncol * 4 * nm);
   }
   ok = ok && alloc((void**)&d.der, sizeof(double) * 20 * (size_t)ny);
@@ -587,9 +579,9 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ok = ok && alloc((void**)&d.dyl, sizeof(double) * ny);
   ok = ok && alloc((void**)&d.gdamp, sizeof(double) * g.ncol);
   ok = ok && alloc((void**)&d.twx, sizeof(double2) * 6 * g.nxd);
-  ok = ok && alloc((void**)&d.twz, sizeof(double2) * g.nzd);
+  ok = ok && alloc((void**)&d.twz, sizeof(double2) * 3 * g.nzd);
   ok = ok && alloc((void**)&d.twxf, sizeof(float2) * 6 * g.nxd);
-  ok = ok && alloc((void**)&d.twzf, sizeof(float2) * g.nzd);
+  ok = ok && alloc((void**)&d.twzf, sizeof(float2) * 3 * g.nzd);
   // outstats scratch (sized for the largest reduction grid, 4 blocks an SM of up to 256 SMs)
   ok = ok && alloc((void**)&d.stats, sizeof(double) * ((hst::stats_partials() + 3) * 4 * 256 + 24));
   // two words: the CFL maximum and the bounded-wait error flag
@@ -627,7 +619,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   cudaMemcpy(d.twx, tx.data(), sizeof(double2) * tx.size(), cudaMemcpyHostToDevice);
   {
     // FP32 copies (rounded from the long double values)
-    std::vector<float2> fx((size_t)6 * g.nxd, make_float2(0.f, 0.f)), fz(g.nzd);
+    std::vector<float2> fx((size_t)6 * g.nxd, make_float2(0.f, 0.f)), fz((size_t)3 * g.nzd, make_float2(0.f, 0.f));
     for (int k = 0; k < 2 * g.nxd; ++k) {
       long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)(2 * g.nxd);
       fx[k] = make_float2((float)cosl(a), (float)sinl(a));
@@ -637,9 +629,12 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
       long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)g.nzd;
       fz[k] = make_float2((float)cosl(a), (float)sinl(a));
     }
+    hst::z_twiddles(g.nzd, fz.data() + g.nzd);
     cudaMemcpy(d.twxf, fx.data(), sizeof(float2) * fx.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(d.twzf, fz.data(), sizeof(float2) * fz.size(), cudaMemcpyHostToDevice);
   }
+  tz.resize((size_t)3 * g.nzd, make_double2(0.0, 0.0));
+  hst::z_twiddles(g.nzd, tz.data() + g.nzd);
   cudaMemcpy(d.twz, tz.data(), sizeof(double2) * tz.size(), cudaMemcpyHostToDevice);
   cudaError_t e = etab;
   // the base of all members; d is member 0's view
@@ -649,6 +644,8 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ctx->db = d;
   if (e == cudaSuccess) e = hst::make_x_maps(ctx->gb, ctx->db);
   if (e == cudaSuccess) e = hst::make_x_maps(g, d);
+  if (e == cudaSuccess) e = hst::make_z_maps(ctx->gb, ctx->db);
+  if (e == cudaSuccess) e = hst::make_z_maps(g, d);
   if (e == cudaSuccess) e = ensure_facg(ctx);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -687,13 +684,14 @@ extern "C" int hst_gpu_select_member(hst_ctx* ctx, int m) {
     return g.mp ? reinterpret_cast<double2*>(reinterpret_cast<float2*>(base) + mm * elems) : base + mm * elems;
   };
   (void)es;
-  d.Z = off(b.Z, 3 * (size_t)g.nzd * g.ny * g.nxB);
-  d.Pp = off(b.Pp, 6 * (size_t)g.nzd * g.ny * g.nxB);
+  d.Z = off(b.Z, 3 * (size_t)g.nzd * g.nyT * g.Ty * g.nxB);
+  d.Pp = off(b.Pp, 6 * (size_t)g.nzd * g.nyT * g.Ty * g.nxB);
   d.Q = off(b.Q, 6 * (size_t)g.ncol * g.ny);
-  d.Zg = off(b.Zg, 3 * (size_t)g.nzd * g.nxB * 4);
-  d.Ppg = off(b.Ppg, 6 * (size_t)g.nzd * g.nxB * 4);
+  d.Zg = off(b.Zg, 3 * (size_t)g.nzd * g.nxB * g.EY);
+  d.Ppg = off(b.Ppg, 6 * (size_t)g.nzd * g.nxB * g.EY);
   d.Qg = off(b.Qg, 6 * (size_t)g.ncol * 4);
   CK(hst::make_x_maps(g, d));
+  CK(hst::make_z_maps(g, d));
   ctx->member = m;
   return HST_OK;
 }
@@ -1063,15 +1061,6 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   for (int c = 32; c >= 4; c >>= 1)
     if (g0.ny / c >= 4) lanes.push_back(c);
   if (lanes.empty()) lanes.push_back(g0.P);
-  std::vector<int> pz;
-  for (int v : {16, 8}) {
-    if (g0.mp && g0.nzd == 768 && v == 16) continue;
-    if (v == 8 && !(g0.nzd == 192 || g0.nzd == 384 || g0.nzd == 768)) continue;
-    if (v == 8 && g0.Ty * g0.nzd / 8 > 384) continue;
-    if (v == 16 && g0.Ty * g0.nzd / 16 > 256) continue;
-    pz.push_back(v);
-  }
-  if (pz.empty()) pz.push_back(g0.pptz);  // one plan only (1536 points)
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -1086,32 +1075,30 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
     if (e == cudaSuccess) e = ensure_facg(ctx);
     return e;
   };
-  for (int P : lanes)
-    for (int b : pz) {
-      Geometry t = g0;
-      t.P = P;
-      t.pptz = b;
-      if (apply(t) != cudaSuccess) continue;
-      for (int i = 0; i < 5 && rc == HST_OK; ++i)
-        if (cudaMemcpyAsync(ctx->d.F[i], save[i], fb, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-          rc = HST_ECUDA;
-      double tt = time0;
-      if (rc == HST_OK) rc = queue_timestep(ctx, &tt, deltat);
-      if (rc == HST_OK && cudaEventRecord(e0, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
-      for (int k = 0; k < steps && rc == HST_OK; ++k) rc = queue_timestep(ctx, &tt, deltat);
-      if (rc == HST_OK && cudaEventRecord(e1, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
-      if (rc == HST_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = HST_ECUDA;
-      if (rc != HST_OK) break;
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      const double per = ms / steps;
-      char line[128];
-      std::snprintf(line, sizeof line, "P=%d z=%d: %.4f ms a step\n", P, b, per);
-      rep += line;
-      if (per < best) {
-        best = per;
-        gbest = t;
-      }
+  for (int P : lanes) {
+    Geometry t = g0;
+    t.P = P;
+    if (apply(t) != cudaSuccess) continue;
+    for (int i = 0; i < 5 && rc == HST_OK; ++i)
+      if (cudaMemcpyAsync(ctx->d.F[i], save[i], fb, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
+        rc = HST_ECUDA;
+    double tt = time0;
+    if (rc == HST_OK) rc = queue_timestep(ctx, &tt, deltat);
+    if (rc == HST_OK && cudaEventRecord(e0, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
+    for (int k = 0; k < steps && rc == HST_OK; ++k) rc = queue_timestep(ctx, &tt, deltat);
+    if (rc == HST_OK && cudaEventRecord(e1, ctx->stream) != cudaSuccess) rc = HST_ECUDA;
+    if (rc == HST_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = HST_ECUDA;
+    if (rc != HST_OK) break;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    const double per = ms / steps;
+    char line[128];
+    std::snprintf(line, sizeof line, "P=%d: %.4f ms a step\n", P, per);
+    rep += line;
+    if (per < best) {
+      best = per;
+      gbest = t;
+    }
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1127,7 +1114,7 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   }
   if (rc != HST_OK) return rc;
   char line[128];
-  std::snprintf(line, sizeof line, "chosen: P=%d z=%d\n", g.P, g.pptz);
+  std::snprintf(line, sizeof line, "chosen: P=%d\n", g.P);
   rep += line;
   if (report && report_len > 0) std::snprintf(report, (size_t)report_len, "%s", rep.c_str());
   return HST_OK;

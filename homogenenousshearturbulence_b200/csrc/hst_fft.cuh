@@ -1,20 +1,19 @@
-// Stockham FFTs for the 3/2-dealiased x and z transforms.
+// The register DFTs of the 3/2-dealiased x and z transforms (radices up to 24,
+// built from radix-2/3/4 pieces), and a Stockham FFT with a runtime plan for
+// the lengths without a compiled plan.
 //
-// A block transforms nl lines of length N = 2^a 3^b.  Each radix-R stage
-// is one pass: a thread gathers the R inputs of its butterflies into
-// registers, applies the stage twiddles, computes a radix-R DFT in
-// registers (R up to 24, built from radix-2/3/4 pieces), and scatters the
-// outputs.  The first stage reads through a caller's loader (global memory,
-// or a function of other lines) and the last stage writes through a
-// caller's storer, so only the exchanges between stages go through shared
-// memory: N = 384 is two stages (16 x 24) with one shared exchange, N = 768
-// three stages.  Threads are mapped line-fastest so that global accesses of
-// consecutive threads touch consecutive lines (the y rows, contiguous in
-// memory); shared lines have an odd stride against bank conflicts.
-// Stage twiddles come from W[e] = exp(-2 pi i e / N) in global memory
-// (computed on the host in extended precision), the twiddles inside a
-// register DFT from a 48-entry table in constant memory (all threads read
-// the same entry).  Unnormalised both ways, like the reference's FFTW
+// In the runtime plan a block transforms nl lines of length N = 2^a 3^b.  Each
+// radix-R stage is one pass: a thread gathers the R inputs of its butterflies
+// into registers, applies the stage twiddles, computes a radix-R DFT in
+// registers, and scatters the outputs.  The first stage reads through a
+// caller's loader (global memory, or a function of other lines) and the last
+// stage writes through a caller's storer, so only the exchanges between
+// stages go through shared memory.  Threads are mapped line-fastest so that
+// global accesses of consecutive threads touch consecutive lines (the y rows,
+// contiguous in memory).  Stage twiddles come from W[e] = exp(-2 pi i e / N) in
+// global memory (computed on the host in extended precision), the twiddles
+// inside a register DFT from a 48-entry table in constant memory (all threads
+// read the same entry).  Unnormalised both ways, like the reference's FFTW
 // and cuFFT plans (src/hst_fft.f90:98-121): S = -1 forward, S = +1 backward.
 #pragma once
 #include <type_traits>
@@ -221,31 +220,6 @@ struct ShLinesT {
   __device__ __forceinline__ C operator()(int l, int i) const { return p[l * LS + i]; }
   __device__ __forceinline__ void operator()(int l, int i, C v) const { p[l * LS + i] = v; }
 };
-// The same with one pad element after every 2^SH (3 for the 8-point plans, 4
-// for the 16-point plans of the z kernels, whose first radix is 16), at the
-// line stride ls_lines
-template <typename C, int SH = 3>
-struct ShLinesPT {
-  C* p;
-  int LS;
-  __device__ __forceinline__ C operator()(int l, int i) const { return p[l * LS + i + (i >> SH)]; }
-  __device__ __forceinline__ void operator()(int l, int i, C v) const { p[l * LS + i + (i >> SH)] = v; }
-};
-// The line stride of the padded layout under the line-fastest mapping
-// of the z kernels (butterfly b: line b % nl, index b / nl, so that the
-// global loads and stores of nl adjacent rows coalesce): a wavefront's
-// lanes cover nl lines times S/nl consecutive indices (S = 128 / sizeof(C)
-// elements a bank row), and a stride of S/nl (mod S) with the pad in eight
-// spreads them over distinct banks in every stage of the 8-point plans
-// (nl in {2, 4, 8}).
-template <typename C, int SH = 3>
-__host__ __device__ inline int ls_lines(int N, int nl) {
-  const int S = 128 / (int)sizeof(C);
-  const int target = (S / nl) % S;
-  const int base = N + (N >> SH);
-  return base + ((target - base) % S + S) % S;
-}
-
 // One radix-R stage.  Butterfly b of the block: line l = b % nl, index
 // j = b / nl.  Inputs ld(l, j + r N/R), outputs st(l, (j/Ns) Ns R + j%Ns + r Ns).
 // SYNC: the stage reads and writes the same shared lines (all reads, then
@@ -332,71 +306,6 @@ __device__ void fft_global(int N, int nl, const C* __restrict__ tw, C* sh, const
     __syncthreads();
   }
   fft_stage_r<S, PPT, DST_SH>(P.r[P.n - 1], N, nl, Ns, tw, L, dst);
-}
-
-// Compile-time plans of the lengths the configurations use (the 3/2-padded
-// sizes 2^a 3 from 12 to 1536), so that each kernel instantiates only the
-// radices it runs.
-template <int N>
-struct Plan {
-  static constexpr int n = 0, r0 = 1, r1 = 1, r2 = 1;
-};
-template <> struct Plan<12> { static constexpr int n = 1, r0 = 12, r1 = 1, r2 = 1; };
-template <> struct Plan<24> { static constexpr int n = 1, r0 = 24, r1 = 1, r2 = 1; };
-template <> struct Plan<48> { static constexpr int n = 2, r0 = 16, r1 = 3, r2 = 1; };
-template <> struct Plan<96> { static constexpr int n = 2, r0 = 16, r1 = 6, r2 = 1; };
-template <> struct Plan<192> { static constexpr int n = 2, r0 = 16, r1 = 12, r2 = 1; };
-template <> struct Plan<384> { static constexpr int n = 2, r0 = 16, r1 = 24, r2 = 1; };
-template <> struct Plan<768> { static constexpr int n = 3, r0 = 16, r1 = 16, r2 = 3; };
-template <> struct Plan<1536> { static constexpr int n = 3, r0 = 16, r1 = 16, r2 = 6; };
-
-// Plans of at most radix 12 for 8 points a thread: more stages (one more
-// shared exchange) for far fewer registers, hence more resident warps.
-template <int N>
-struct Plan8 {
-  static constexpr int n = 0, r0 = 1, r1 = 1, r2 = 1;
-};
-template <> struct Plan8<12> { static constexpr int n = 1, r0 = 12, r1 = 1, r2 = 1; };
-template <> struct Plan8<24> { static constexpr int n = 2, r0 = 4, r1 = 6, r2 = 1; };
-template <> struct Plan8<48> { static constexpr int n = 2, r0 = 8, r1 = 6, r2 = 1; };
-template <> struct Plan8<96> { static constexpr int n = 2, r0 = 8, r1 = 12, r2 = 1; };
-template <> struct Plan8<192> { static constexpr int n = 3, r0 = 8, r1 = 4, r2 = 6; };
-template <> struct Plan8<384> { static constexpr int n = 3, r0 = 8, r1 = 8, r2 = 6; };
-template <> struct Plan8<768> { static constexpr int n = 3, r0 = 8, r1 = 8, r2 = 12; };
-
-// PZ: the padded lines at stride ls_lines under the line-fastest mapping.
-template <int N, int S, int PPT, bool PZ, typename LD, typename ST, typename C>
-__device__ __forceinline__ void fft_fixed(int nl, const C* __restrict__ tw, C* sh, const LD& src, const ST& dst) {
-  using PL = std::conditional_t<(PPT <= 8), Plan8<N>, Plan<N>>;
-  static_assert(PL::n > 0, "no compile-time plan for this length and points per thread");
-  constexpr int PSH = PPT <= 8 ? 3 : 4;  // the pad follows the plan's first radix (8 or 16)
-  using LT = std::conditional_t<PZ, ShLinesPT<C, PSH>, ShLinesT<C>>;
-  const LT L = {sh, PZ ? ls_lines<C, PSH>(N, nl) : N + 1};
-  if constexpr (PL::n == 1) {
-    fft_stage_io<PL::r0, S, PPT, false>(N, nl, 1, tw, src, dst);
-  } else if constexpr (PL::n == 2) {
-    fft_stage_io<PL::r0, S, PPT, false>(N, nl, 1, tw, src, L);
-    __syncthreads();
-    fft_stage_io<PL::r1, S, PPT, false>(N, nl, PL::r0, tw, L, dst);
-  } else {
-    fft_stage_io<PL::r0, S, PPT, false>(N, nl, 1, tw, src, L);
-    __syncthreads();
-    fft_stage_io<PL::r1, S, PPT, true>(N, nl, PL::r0, tw, L, L);
-    __syncthreads();
-    fft_stage_io<PL::r2, S, PPT, false>(N, nl, PL::r0 * PL::r1, tw, L, dst);
-  }
-}
-
-// NT > 0: the compile-time plan of length NT; NT = 0: the runtime plan of N.
-template <int NT, int S, int PPT, bool PZ, typename LD, typename ST, typename C>
-__device__ __forceinline__ void fft_sel(int N, int nl, const C* __restrict__ tw, C* sh, const LD& src,
-                                        const ST& dst) {
-  static_assert(!PZ || NT > 0, "PZ needs a compile-time plan");
-  if constexpr (NT > 0) {
-    fft_fixed<NT, S, PPT, PZ>(nl, tw, sh, src, dst);
-  } else {
-    fft_global<S, PPT, false, false>(N, nl, tw, sh, src, dst);
-  }
 }
 
 }  // namespace hst

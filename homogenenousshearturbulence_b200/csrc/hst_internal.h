@@ -20,15 +20,15 @@ struct Geometry {
   int ncol;            // nxB * nzT Fourier columns
   long nf;             // complex elements of one field (ncol * rows)
   int P;               // lanes of a line-solve group
-  int Ty;              // y tile of the transforms (divides ny)
-  int pptz;            // FFT points per thread of the z transforms (8: the low-register plans)
+  int Ty, nyT;         // rows and number of the transforms' y tiles (the last may reach beyond ny)
+  int EY;              // rows of the y tile that holds the four ghost rows (Ty of a z plan, else 4)
   int mp;              // mixed precision: Z, Pp, Q and their transforms in FP32 (complex64)
   // 0, or (in the view of the four ghost rows that the edge transforms take)
   // ny: the z-inverse then reads rows -2, -1, ny, ny+1 of V
   int edge_gap;
   // members of an ensemble advanced together (1 for a single field): every
   // per-field buffer holds nmem members one after another (fields nf
-  // elements a member, Z 3 ny nzd nxB, Pp 6 ny nzd nxB, Q 6 ncol ny), the
+  // elements a member, Z 3 nyT Ty nzd nxB, Pp 6 nyT Ty nzd nxB, Q 6 ncol ny), the
   // tables are shared, and the substep's kernels cover all members in one
   // launch each
   int nmem;
@@ -36,8 +36,8 @@ struct Geometry {
 
 struct DeviceState {
   double2* F[7];        // V1 V2 V3 OLD1 OLD2 RHS1 RHS2, (iy fastest, ghost rows included)
-  double2* Z;           // z-inverse of V: [3][nzd][ny/Ty][nxB][Ty]
-  double2* Pp;          // x-forward of the products: [6][nzd][ny/Ty][nxB][Ty]
+  double2* Z;           // z-inverse of V: [3][nyT][nzd][nxB][Ty]
+  double2* Pp;          // x-forward of the products: [6][nyT][nzd][nxB][Ty]
   double2* Q;           // spectral products: [6][ncol][ny]
   double* der;          // der(0:ny-1, 0:3, -2:2)
   double* derS;         // the same, slab-major for the line-solve groups (slab_major)
@@ -49,15 +49,16 @@ struct DeviceState {
   double* dyl;          // dyl(0:ny-1)
   double* gdamp;        // gdamp(-nz:nz, 0:nx)
   double2* twx;         // exp(-2 pi i e / (2 nxd)), then the x plan's tables (x_twiddles)
-  double2* twz;         // exp(-2 pi i e / nzd)
+  double2* twz;         // exp(-2 pi i e / nzd), then the z plan's tables (z_twiddles)
   float2* twxf;         // the same tables in FP32 (mixed precision)
   float2* twzf;
   unsigned long long* cfl;  // running max (bits of a non-negative double)
   int* err;                 // set by a kernel whose bounded wait ran out
   CUtensorMap tmZ, tmPp, tmZg, tmPpg;  // TMA maps of Z, Pp and the ghost rows' buffers (make_x_maps)
+  CUtensorMap tmPz, tmPgz;             // of Pp and Ppg for the z-forward kernel (make_z_maps)
   // The products of the four ghost rows (-2, -1, ny, ny+1) transformed like
   // the interior ones (null when their shear-periodic images are exact):
-  // Zg [3][nzd][nxB][4], Ppg [6][nzd][nxB][4], Qg [6][ncol][4], in the
+  // Zg [3][nzd][nxB][EY], Ppg [6][nzd][nxB][EY], Qg [6][ncol][4], in the
   // transforms' precision
   double2 *Zg, *Ppg, *Qg;
   int nsm;        // SMs of the device
@@ -176,6 +177,20 @@ bool edge_rows_needed(const Geometry& g, bool s2_active);
 bool x_compiled(int N, bool fp32);
 cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, cudaStream_t st);
 cudaError_t make_x_maps(const Geometry& g, DeviceState& d);
+// cuTensorMapEncodeTiled (null: the driver has none)
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled();
+// the z transforms of the lengths with a compiled plan (hst_z.cu): the rows of
+// their y tile (0: no plan), the TMA maps of the forward kernel, its twiddle
+// tables (at most 2 N entries into out; their number)
+int z_rows(int N, bool fp32);
+cudaError_t make_z_maps(const Geometry& g, DeviceState& d);
+int z_twiddles(int N, double2* out);
+int z_twiddles(int N, float2* out);
+cudaError_t launch_z_inv(const Geometry& g, const DeviceState& d, cudaStream_t st);
+cudaError_t launch_z_fwd(const Geometry& g, const DeviceState& d, cudaStream_t st);
 int x_twiddles(int N, double2* out);
 int x_twiddles(int N, float2* out);
 // a transform length of the mixed-precision form

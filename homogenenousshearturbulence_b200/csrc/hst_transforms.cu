@@ -1,19 +1,22 @@
-// The transform kernels of the hst substep (FP64):
+// The transforms of the hst substep for the lengths without a compiled plan
+// (FP64, the runtime plan), the launches of the three transform stages, and
+// the line transforms of the per-piece path:
 //
-//   k_zinv   V (u, v, w) -> zero-padded z-inverse transform (Z)
-//   k_xprod  Z -> x-inverse (c2r) of u, v, w; the six products times
-//            1/(2 nxd nzd); the CFL maximum; x-forward (r2c) of the products
-//            truncated to the nx+1 retained modes (Pp)
-//   k_zfwd   Pp -> z-forward transform truncated to the 2nz+1 modes (Q)
+//   zinv    V (u, v, w) -> zero-padded z-inverse transform (Z)
+//   xprod   Z -> x-inverse (c2r) of u, v, w; the six products times
+//           1/(2 nxd nzd); the CFL maximum; x-forward (r2c) of the products
+//           truncated to the nx+1 retained modes (Pp)
+//   zfwd    Pp -> z-forward transform truncated to the 2nz+1 modes (Q)
 //
-// Together they are transform_to_physical + build_products (both groups) +
+// (hst_z.cu and hst_xprod.cu for the compiled lengths.)  Together they are
+// transform_to_physical + build_products (both groups) +
 // products_to_spectral + compute_cfl of the reference
 // (src/hst_transforms.f90:33-179, src/hst_fft.f90:181-237), with the local
 // transposes (src/hst_mpi.f90:615-669) absorbed into the index maps.  Only
-// the ny interior rows are transformed (see k_column for the ghost-row
-// products).  Z and Pp are stored [component][y tile][kz][ix][Ty]: a block
-// of k_zinv / k_zfwd (one x mode, one y tile, all kz) then spans a few
-// huge pages instead of one page per kz.
+// the ny interior rows are transformed (see hst_rhs.cu for the ghost-row
+// products).  Z and Pp are stored [component][y tile][kz][ix][Ty]: the z
+// lines of one x mode and one y tile then span a few huge pages instead of
+// one page per kz.
 #include <cmath>
 
 #include "hst_dev.cuh"
@@ -24,35 +27,12 @@ namespace hst {
 
 bool fft_length_ok(int n) { return plan_ok(n); }
 
-#ifndef ZPAD16
-#define ZPAD16 1  // 0: the 16- and 32-point z plans on unpadded lines
-#endif
-// The order of the z kernels' blocks: IXF = 1 runs the x modes of one y tile
-// side by side (consecutive blocks read, or write, adjacent 64-byte runs of
-// the [yt][kz][ix][Ty] tiles of Z and Pp), 0 the y tiles of one x mode.
-// Measured at 768^2 x 512: the z-inverse 2.18 against 2.26 ms with 1 (1.75
-// against 1.85 in FP32); the z-forward 4.82 against 4.68 ms (FP64) and 3.03
-// against 3.14 ms (FP32), 0.327 against 0.302 ms at 384^2 x 256 (FP32).
-#ifndef ZINV_IXF
-#define ZINV_IXF 1
-#endif
-#ifndef ZFWD_IXF
-#define ZFWD_IXF 0
-#endif
-
 // --------------------------------------------------------------- k_zinv ----
 // assemble_vvdz + IFT (src/hst_transforms.f90:33-54, src/hst_fft.f90:195-207):
 // line yi of the block is row y0 + yi of one x mode of one component; the
 // z modes -nz..nz sit at padded index iz (iz >= 0) or nzd + iz.
-// C: the complex type of the transforms (double2; float2 in the
-// mixed-precision form, where V is read as FP64 and rounded once)
-template <typename C>
-__device__ __forceinline__ C to_c(double2 v) {
-  typedef typename RealOf<C>::T T;
-  return C{(T)v.x, (T)v.y};
-}
-template <typename C>
 struct ZinvSrc {
+  typedef double2 C;
   const double2* __restrict__ col;  // V + (ix nzT) rows + 2 + y0: row y0 of iz = -nz
   int rows, nz, NZ;
   int gap;  // the edge view: rows -2, -1 at 0, 1 and ny, ny+1 at gap + 2, gap + 3
@@ -61,84 +41,40 @@ struct ZinvSrc {
     if (kz <= nz) iz = kz;
     else if (kz >= NZ - nz) iz = kz - NZ;
     else return C{0, 0};
-    return to_c<C>(col[(size_t)(iz + nz) * rows + yi + (yi >= 2 ? gap : 0)]);
+    return col[(size_t)(iz + nz) * rows + yi + (yi >= 2 ? gap : 0)];
   }
 };
-template <typename C>
-struct TileDst {  // one (component, y tile, x mode) z-line set of Z / Pp
+struct TileDst {
+  typedef double2 C;  // one (component, y tile, x mode) z-line set of Z / Pp
   C* __restrict__ base;
   size_t zstride;
   __device__ __forceinline__ void operator()(int yi, int kz, C v) const { base[(size_t)kz * zstride + yi] = v; }
 };
-template <typename C>
 struct TileSrc {
+  typedef double2 C;
   const C* __restrict__ base;
   size_t zstride;
   __device__ __forceinline__ C operator()(int yi, int kz) const { return base[(size_t)kz * zstride + yi]; }
 };
 
-// the z kernels' compile-time plans keep their lines padded (ls_lines: one
-// pad in 8 for the 8-point plans, in 16 for the 16- and 32-point plans),
-// free of bank conflicts under the line-fastest mapping
-// (FP64 16- and 32-point plans stay unpadded: at 384 points their eight
-// rows a block are conflict-free anyway, and at 1536 the pad measured
-// slower, 15.8 against 12.5 ms z-inverse and 27.0 against 23.6 ms
-// z-forward, where in FP32 it gains, 12.2 against 13.2 and 15.6 against
-// 17.8 ms)
-template <int NT, int PPT, typename C>
-__host__ __device__ constexpr bool z_padded() {
-  return NT > 0 && (PPT <= 8 || (ZPAD16 && sizeof(C) == 8));
-}
-template <int NT, int PPT, typename C>
-__host__ __device__ inline size_t z_smem(int nzd, int Ty) {
-  const int ls = !z_padded<NT, PPT, C>() ? nzd + 1 : (PPT <= 8 ? ls_lines<C, 3>(nzd, Ty) : ls_lines<C, 4>(nzd, Ty));
-  return (size_t)Ty * ls * sizeof(C);
-}
-
-template <int NT, int PPT, typename C>
-__device__ __forceinline__ void zinv_body(const Geometry& g, const double2* __restrict__ V0,
-                                          const double2* __restrict__ V1, const double2* __restrict__ V2,
-                                          C* __restrict__ Z, const C* __restrict__ twz) {
-  extern __shared__ double2 sh_d[];
-  C* sh = reinterpret_cast<C*>(sh_d);
-  const int yt = ZINV_IXF ? blockIdx.y : blockIdx.x, ix = ZINV_IXF ? blockIdx.x : blockIdx.y;
-  const int c = blockIdx.z % 3, mem = blockIdx.z / 3;
-  const int Ty = g.Ty, NZ = g.nzd, nyT = g.ny / Ty;
-  const double2* V = (c == 0 ? V0 : (c == 1 ? V1 : V2)) + (size_t)mem * g.nf;
-  Z += (size_t)mem * 3 * NZ * g.ny * g.nxB;
-  const ZinvSrc<C> src = {V + (size_t)ix * g.nzT * g.rows + (g.edge_gap ? 0 : 2) + yt * Ty, g.rows, g.nz, NZ,
-                          g.edge_gap};
-  const TileDst<C> dst = {Z + (((size_t)c * nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
-  fft_sel<NT, +1, PPT, z_padded<NT, PPT, C>()>(NZ, Ty, twz, sh, src, dst);
-}
-template <int NT, int PPT, typename C>
-__global__ void __launch_bounds__(PPT <= 8 ? 512 : 256)
+template <int PPT>
+__global__ void __launch_bounds__(256)
     k_zinv(Geometry g, const double2* __restrict__ V0, const double2* __restrict__ V1, const double2* __restrict__ V2,
-           C* __restrict__ Z, const C* __restrict__ twz) {
-  zinv_body<NT, PPT, C>(g, V0, V1, V2, Z, twz);
-}
-// the FP64 32-point plans (192 threads) held to two blocks an SM (1536
-// points: 16.5 -> 12.5 ms at 1536^2 x 512; an explicit block minimum on
-// the kernel above made the 384-point plan slower, 0.42 against 0.25 ms)
-template <int NT>
-__global__ void __launch_bounds__(192, 2) k_zinv_32(Geometry g, const double2* __restrict__ V0,
-                                                    const double2* __restrict__ V1, const double2* __restrict__ V2,
-                                                    double2* __restrict__ Z, const double2* __restrict__ twz) {
-  zinv_body<NT, 32, double2>(g, V0, V1, V2, Z, twz);
-}
-// the FP32 1536-point plan (192 threads) held to three blocks an SM (an
-// explicit block minimum on the kernel above made the 384-point plan slower)
-__global__ void __launch_bounds__(192, 3) k_zinv_1536f(Geometry g, const double2* __restrict__ V0,
-                                                       const double2* __restrict__ V1, const double2* __restrict__ V2,
-                                                       float2* __restrict__ Z, const float2* __restrict__ twz) {
-  zinv_body<1536, 32, float2>(g, V0, V1, V2, Z, twz);
+           double2* __restrict__ Z, const double2* __restrict__ twz) {
+  extern __shared__ double2 sh[];
+  const int ix = blockIdx.x, yt = blockIdx.y, c = blockIdx.z % 3, mem = blockIdx.z / 3;
+  const int Ty = g.Ty, NZ = g.nzd;
+  const double2* V = (c == 0 ? V0 : (c == 1 ? V1 : V2)) + (size_t)mem * g.nf;
+  const ZinvSrc src = {V + (size_t)ix * g.nzT * g.rows + (g.edge_gap ? 0 : 2) + yt * Ty, g.rows, g.nz, NZ, g.edge_gap};
+  const TileDst dst = {Z + ((((size_t)mem * 3 + c) * g.nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
+  fft_global<+1, PPT, false, false>(NZ, Ty, twz, sh, src, dst);
 }
 
 // --------------------------------------------------------------- k_zfwd ----
 // transpose_xTOz + FFT (src/hst_transforms.f90:135-139, src/hst_fft.f90:181-193)
 // keeping the 2nz+1 retained modes, stored without ghost rows.
-template <typename C>
 struct ZfwdDst {
+  typedef double2 C;
   C* __restrict__ base;  // Q + (p ncol + ix nzT) ny + y0
   int ny, nz, NZ;
   __device__ __forceinline__ void operator()(int yi, int k, C v) const {
@@ -150,26 +86,15 @@ struct ZfwdDst {
   }
 };
 
-// (the explicit one-block minimum lets the compiler take 160 registers
-// for the 16-point plans, which measured 0.46 against 0.50 ms at 384^2 x
-// 256; the same on k_zinv measured slower; the 8-point plans are held to
-// three blocks an SM: at 768^2 x 512 4.68 against 5.19 ms for two in FP64,
-// where the kernel waits on its global loads, while the z-inverse measured
-// slower held to two or three)
-template <int NT, int PPT, typename C>
-__global__ void __launch_bounds__(PPT <= 8 ? 384 : (PPT == 32 && NT > 0 ? 192 : 256),
-                                  PPT <= 8 ? 3 : (PPT == 32 && NT > 0 ? 2 : 1))
-    k_zfwd(Geometry g, const C* __restrict__ Pp, C* __restrict__ Q, const C* __restrict__ twz) {
-  extern __shared__ double2 sh_d[];
-  C* sh = reinterpret_cast<C*>(sh_d);
-  const int yt = ZFWD_IXF ? blockIdx.y : blockIdx.x, ix = ZFWD_IXF ? blockIdx.x : blockIdx.y;
-  const int p = blockIdx.z % 6, mem = blockIdx.z / 6;
-  const int Ty = g.Ty, NZ = g.nzd, nyT = g.ny / Ty;
-  Pp += (size_t)mem * 6 * NZ * g.ny * g.nxB;
-  Q += (size_t)mem * 6 * g.ncol * g.ny;
-  const TileSrc<C> src = {Pp + (((size_t)p * nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
-  const ZfwdDst<C> dst = {Q + ((size_t)p * g.ncol + (size_t)ix * g.nzT) * g.ny + yt * Ty, g.ny, g.nz, NZ};
-  fft_sel<NT, -1, PPT, z_padded<NT, PPT, C>()>(NZ, Ty, twz, sh, src, dst);
+template <int PPT>
+__global__ void __launch_bounds__(256)
+    k_zfwd(Geometry g, const double2* __restrict__ Pp, double2* __restrict__ Q, const double2* __restrict__ twz) {
+  extern __shared__ double2 sh[];
+  const int yt = blockIdx.x, ix = blockIdx.y, pm = blockIdx.z;
+  const int Ty = g.Ty, NZ = g.nzd;
+  const TileSrc src = {Pp + (((size_t)pm * g.nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
+  const ZfwdDst dst = {Q + ((size_t)pm * g.ncol + (size_t)ix * g.nzT) * g.ny + yt * Ty, g.ny, g.nz, NZ};
+  fft_global<-1, PPT, false, false>(NZ, Ty, twz, sh, src, dst);
 }
 
 // -------------------------------------------------------------- k_xprod ----
@@ -231,10 +156,10 @@ __global__ void __launch_bounds__(320)
   extern __shared__ double2 sh[];
   typedef ShLinesT<C> LT;
   const int NX = 2 * g.nxd, nx = g.nx, nxB = g.nxB, NZ = g.nzd, Ty = g.Ty;
-  const int nyT = g.ny / Ty;
+  const int nyT = g.nyT;
   const int y0 = 2 * blockIdx.x, kz = blockIdx.y % g.nzd, mem = blockIdx.y / g.nzd;
-  Z += (size_t)mem * 3 * g.nzd * g.ny * g.nxB;
-  Pp += (size_t)mem * 6 * g.nzd * g.ny * g.nxB;
+  Z += (size_t)mem * 3 * g.nzd * nyT * Ty * g.nxB;
+  Pp += (size_t)mem * 6 * g.nzd * nyT * Ty * g.nxB;
   const int yt = y0 / Ty, yi0 = y0 - yt * Ty;
   const size_t cs = (size_t)NZ * nyT * nxB * Ty;
   const size_t tile = ((size_t)yt * NZ + kz) * nxB * Ty;
@@ -355,12 +280,13 @@ cudaError_t launch_piece_lines(const DeviceState& d, double2* base, size_t strid
 
 bool edge_rows_needed(const Geometry& g, bool s2_active) { return s2_active && g.nzd <= 3 * g.nz; }
 
-// The view of the four ghost rows: the same transforms with ny = Ty = 4 on
-// the edge buffers
+// The view of the four ghost rows: the same transforms with ny = 4 and one y
+// tile on the edge buffers
 static void edge_view(const Geometry& g, const DeviceState& d, Geometry& ge, DeviceState& de) {
   ge = g;
   ge.ny = 4;
-  ge.Ty = 4;
+  ge.Ty = g.EY;
+  ge.nyT = 1;
   ge.edge_gap = g.ny;
   de = d;
   de.Z = d.Zg;
@@ -368,6 +294,7 @@ static void edge_view(const Geometry& g, const DeviceState& d, Geometry& ge, Dev
   de.Q = d.Qg;
   de.tmZ = d.tmZg;
   de.tmPp = d.tmPpg;
+  de.tmPz = d.tmPgz;
 }
 
 // -------------------------------------------------------------- launchers ----
@@ -382,113 +309,35 @@ static void big_smem(const DeviceState& d, K k) {
   smem_limit(d, k, 220 * 1024);
 }
 
-// Dispatch on the transform length: compile-time plans for the lengths the
-// workloads use, with 8 points a thread (radix <= 12, P8) or 16 up to 384
-// and 32 above (radix 16/24), the runtime plan otherwise.
-#define HST_FFT_DISPATCH(N, PTS, P8, CALL)                  \
-  do {                                                      \
-    switch (N) {                                            \
-      case 12: CALL(12, 16) break;                          \
-      case 24: CALL(24, 16) break;                          \
-      case 48: CALL(48, 16) break;                          \
-      case 96: CALL(96, 16) break;                          \
-      case 192:                                             \
-        if (P8) CALL(192, 8) else CALL(192, 16) break;      \
-      case 384:                                             \
-        if (P8) CALL(384, 8) else CALL(384, 16) break;      \
-      case 768:                                             \
-        if (P8) CALL(768, 8) else CALL(768, 32) break;      \
-      case 1536: CALL(1536, 32) break;                      \
-      default:                                              \
-        if ((PTS) <= 16 * 256) CALL(0, 16) else CALL(0, 32) \
-        break;                                              \
-    }                                                       \
-  } while (0)
-
-// The mixed-precision form compiles the transforms for the lengths its
-// workloads use: 8 points a thread at 192, 384 and 768, 16 at 96, 32 (the
-// radix 16, 16, 6 plan) at 1536.
-#define HST_FFT_DISPATCH_MP(N, P16, CALL)          \
-  do {                                             \
-    switch (N) {                                   \
-      case 96: CALL(96, 16) break;                 \
-      case 192:                                    \
-        if (P16) CALL(192, 16) else CALL(192, 8) break; \
-      case 384:                                    \
-        if (P16) CALL(384, 16) else CALL(384, 8) break; \
-      case 768: CALL(768, 8) break;                \
-      case 1536: CALL(1536, 32) break;             \
-      default:                                     \
-        return cudaErrorInvalidValue;              \
-    }                                              \
-  } while (0)
-
-bool mp_length_ok(int n) { return n == 96 || n == 192 || n == 384 || n == 768 || n == 1536; }
+bool mp_length_ok(int n) { return x_compiled(n, true) && z_rows(n, true) > 0; }
 
 static cudaError_t launch_zinv_main(const Geometry& g, const DeviceState& d, cudaStream_t st) {
+  if (z_rows(g.nzd, g.mp != 0)) return launch_z_inv(g, d, st);
   const int pts = g.nzd * g.Ty;
-  const dim3 grid(ZINV_IXF ? g.nxB : g.ny / g.Ty, ZINV_IXF ? g.ny / g.Ty : g.nxB, 3 * g.nmem);
-  if (g.mp) {
-    typedef float2 C;
-    C* Z = reinterpret_cast<C*>(d.Z);
-#define HST_ZINV(NT, PPT)                                                                                     \
-  {                                                                                                           \
-    const size_t smem = z_smem<NT, PPT, C>(g.nzd, g.Ty);                                                      \
-    if (NT == 1536) {                                                                                         \
-      big_smem(d, k_zinv_1536f);                                                                                 \
-      k_zinv_1536f<<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.F[0], d.F[1], d.F[2], Z, d.twzf);          \
-    } else {                                                                                                  \
-      big_smem(d, k_zinv<NT, PPT, C>);                                                                           \
-      k_zinv<NT, PPT, C><<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.F[0], d.F[1], d.F[2], Z, d.twzf);    \
-    }                                                                                                         \
+  const dim3 grid(g.nxB, g.nyT, 3 * g.nmem);
+  const size_t smem = (size_t)g.Ty * (g.nzd + 1) * sizeof(double2);
+  if (pts <= 16 * 256) {
+    big_smem(d, k_zinv<16>);
+    k_zinv<16><<<grid, fft_threads(pts, 16), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz);
+  } else {
+    big_smem(d, k_zinv<32>);
+    k_zinv<32><<<grid, fft_threads(pts, 32), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz);
   }
-    HST_FFT_DISPATCH_MP(g.nzd, g.pptz == 16, HST_ZINV);
-#undef HST_ZINV
-    return cudaGetLastError();
-  }
-  typedef double2 C;
-#define HST_ZINV(NT, PPT)                                                                                     \
-  {                                                                                                           \
-    const size_t smem = z_smem<NT, PPT, C>(g.nzd, g.Ty);                                                      \
-    if (PPT == 32 && NT > 0) {                                                                                \
-      big_smem(d, k_zinv_32<NT>);                                                                             \
-      k_zinv_32<NT><<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz);        \
-    } else {                                                                                                  \
-      big_smem(d, k_zinv<NT, PPT, C>);                                                                        \
-      k_zinv<NT, PPT, C><<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz);   \
-    }                                                                                                         \
-  }
-  HST_FFT_DISPATCH(g.nzd, pts, g.pptz == 8, HST_ZINV);
-#undef HST_ZINV
   return cudaGetLastError();
 }
 
 static cudaError_t launch_zfwd_main(const Geometry& g, const DeviceState& d, cudaStream_t st) {
+  if (z_rows(g.nzd, g.mp != 0)) return launch_z_fwd(g, d, st);
   const int pts = g.nzd * g.Ty;
-  const dim3 grid(ZFWD_IXF ? g.nxB : g.ny / g.Ty, ZFWD_IXF ? g.ny / g.Ty : g.nxB, 6 * g.nmem);
-  if (g.mp) {
-    typedef float2 C;
-    const C* Pp = reinterpret_cast<const C*>(d.Pp);
-    C* Q = reinterpret_cast<C*>(d.Q);
-#define HST_ZFWD(NT, PPT)                                                                  \
-  {                                                                                        \
-    const size_t smem = z_smem<NT, PPT, C>(g.nzd, g.Ty);                                   \
-    big_smem(d, k_zfwd<NT, PPT, C>);                                                          \
-    k_zfwd<NT, PPT, C><<<grid, fft_threads(pts, PPT), smem, st>>>(g, Pp, Q, d.twzf);       \
+  const dim3 grid(g.nyT, g.nxB, 6 * g.nmem);
+  const size_t smem = (size_t)g.Ty * (g.nzd + 1) * sizeof(double2);
+  if (pts <= 16 * 256) {
+    big_smem(d, k_zfwd<16>);
+    k_zfwd<16><<<grid, fft_threads(pts, 16), smem, st>>>(g, d.Pp, d.Q, d.twz);
+  } else {
+    big_smem(d, k_zfwd<32>);
+    k_zfwd<32><<<grid, fft_threads(pts, 32), smem, st>>>(g, d.Pp, d.Q, d.twz);
   }
-    HST_FFT_DISPATCH_MP(g.nzd, g.pptz == 16, HST_ZFWD);
-#undef HST_ZFWD
-    return cudaGetLastError();
-  }
-  typedef double2 C;
-#define HST_ZFWD(NT, PPT)                                                                  \
-  {                                                                                        \
-    const size_t smem = z_smem<NT, PPT, C>(g.nzd, g.Ty);                                   \
-    big_smem(d, k_zfwd<NT, PPT, C>);                                                          \
-    k_zfwd<NT, PPT, C><<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.Pp, d.Q, d.twz);    \
-  }
-  HST_FFT_DISPATCH(g.nzd, pts, g.pptz == 8, HST_ZFWD);
-#undef HST_ZFWD
   return cudaGetLastError();
 }
 

@@ -437,15 +437,21 @@ int x_twiddles(int N, float2* out) {
 // Z and Pp seen as 4-D real tensors: d0 = the 2 Ty reals of one y tile
 // (innermost), d1 = ix, d2 = (y tile, kz) as yt nzd + kz, d3 = component.
 // The box is {the rows of a tile, modes, 1, three components}.
-typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+  static const EncodeTiled enc = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<EncodeTiled>(fn) : nullptr;
+  }();
+  return enc;
+}
 
-static cudaError_t encode_map(EncodeTiled enc, const Geometry& g, void* base, int comps, int ny, int Ty, int rp,
+static cudaError_t encode_map(EncodeTiled enc, const Geometry& g, void* base, int comps, int Ty, int nyT, int rp,
                               CUtensorMap* map) {
   const cuuint64_t es = g.mp ? 8 : 16;  // bytes of one complex element
-  cuuint64_t dims[4] = {(cuuint64_t)2 * Ty, (cuuint64_t)g.nxB, (cuuint64_t)g.nzd * (ny / Ty), (cuuint64_t)comps * g.nmem};
-  cuuint64_t strides[3] = {es * Ty, es * Ty * g.nxB, es * Ty * g.nxB * g.nzd * (ny / Ty)};
+  cuuint64_t dims[4] = {(cuuint64_t)2 * Ty, (cuuint64_t)g.nxB, (cuuint64_t)g.nzd * nyT, (cuuint64_t)comps * g.nmem};
+  cuuint64_t strides[3] = {es * Ty, es * Ty * g.nxB, es * Ty * g.nxB * g.nzd * nyT};
   cuuint32_t box[4] = {(cuuint32_t)(4 * rp), (cuuint32_t)x_box(g.nxB), 1, 3};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(map, g.mp ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, base, dims,
@@ -456,17 +462,14 @@ static cudaError_t encode_map(EncodeTiled enc, const Geometry& g, void* base, in
 
 cudaError_t make_x_maps(const Geometry& g, DeviceState& d) {
   if (!x_compiled(2 * g.nxd, g.mp != 0)) return cudaSuccess;
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-  if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) return e != cudaSuccess ? e : cudaErrorNotSupported;
-  const EncodeTiled enc = reinterpret_cast<EncodeTiled>(fn);
+  const EncodeTiled enc = encode_tiled();
+  if (!enc) return cudaErrorNotSupported;
   const int rp = x_row_pairs(2 * g.nxd, g.mp != 0);
-  e = encode_map(enc, g, d.Z, 3, g.ny, g.Ty, rp, &d.tmZ);
-  if (e == cudaSuccess) e = encode_map(enc, g, d.Pp, 6, g.ny, g.Ty, rp, &d.tmPp);
-  if (e == cudaSuccess && d.Zg) {  // the ghost rows' buffers: one tile of four rows
-    e = encode_map(enc, g, d.Zg, 3, 4, 4, rp, &d.tmZg);
-    if (e == cudaSuccess) e = encode_map(enc, g, d.Ppg, 6, 4, 4, rp, &d.tmPpg);
+  cudaError_t e = encode_map(enc, g, d.Z, 3, g.Ty, g.nyT, rp, &d.tmZ);
+  if (e == cudaSuccess) e = encode_map(enc, g, d.Pp, 6, g.Ty, g.nyT, rp, &d.tmPp);
+  if (e == cudaSuccess && d.Zg) {  // the ghost rows' buffers: one tile
+    e = encode_map(enc, g, d.Zg, 3, g.EY, 1, rp, &d.tmZg);
+    if (e == cudaSuccess) e = encode_map(enc, g, d.Ppg, 6, g.EY, 1, rp, &d.tmPpg);
   }
   return e;
 }
