@@ -938,11 +938,10 @@ extern "C" int hst_gpu_compute_cfl(hst_ctx* ctx, double* cfl) {
   return read_cfl(ctx, cfl);
 }
 
-// outstats (src/hst_stats.f90:136-285) of the resident field at `time`:
-// the three DY solves go through RHS1, which is scratch between steps (as
-// the reference's rhs is).  res (24 doubles on the host): the 8 box averages,
-// then the 16 sums of the reference's `sums` array; exz (ncol doubles, may
-// be NULL): the column energies, computed into RHS1 after the solves.
+// outstats (src/hst_stats.f90:136-285) of the resident field at `time`.  res
+// (24 doubles on the host): the 8 box averages, then the 16 sums of the
+// reference's `sums` array; exz (ncol doubles, may be NULL): the column
+// energies, staged in RHS1, which is scratch between steps.
 static int outstats_all(hst_ctx* ctx, double time, double* res_h, double* exz_h) {
   CK(cudaSetDevice(ctx->device));
   const Geometry& g = ctx->g;
@@ -950,27 +949,19 @@ static int outstats_all(hst_ctx* ctx, double time, double* res_h, double* exz_h)
   if (nblk > 4 * 256) return fail(ctx, HST_EARG, "outstats: %d reduction blocks exceed the scratch", nblk);
   double* pm = ctx->d.stats;
   double* pg = pm + (size_t)hst::stats_partials() * nblk;
-  double* res = pg + (size_t)3 * nblk;
+  double* res = pg + (size_t)3 * 4 * 256;
   double sx, sz;
   shear_shifts(ctx, time, &sx, &sz);
-  for (int c = 0; c < 3; ++c) {
-    CK(timed(ctx, HST_KC_LINE_SOLVE, [&] {
-      return hst::launch_line_solve(g, ctx->d, ctx->ps, hst::K_DY, 0.0, c, HST_RHS1, sx, sz, ctx->stream);
-    }));
-    CK(hst::launch_stats_grad(g, ctx->d, HST_RHS1, pg + (size_t)c * nblk, ctx->stream));
-    ctx->launches++;
-  }
+  int nblk_dy = 0;
+  CK(timed(ctx, HST_KC_LINE_SOLVE,
+           [&] { return hst::launch_dy_sums(g, ctx->d, ctx->ps, sx, sz, pg, &nblk_dy, ctx->stream); }));
   const double gsoft = (damping_active(ctx->p) && !ctx->p.damp_hard) ? 1.0 : 0.0;
-  CK(hst::launch_stats_moments(g, ctx->d, ctx->ps, gsoft, pm, ctx->stream));
+  double* exz_d = exz_h ? reinterpret_cast<double*>(ctx->d.F[HST_RHS1]) : nullptr;
+  CK(hst::launch_stats_moments(g, ctx->d, ctx->ps, gsoft, pm, exz_d, ctx->stream));
   double ly_w = 0.0;
   for (int iy = 0; iy < g.ny; ++iy) ly_w += ctx->dyl[iy];
-  CK(hst::launch_stats_final(g, ctx->d, pm, pg, ly_w, ctx->ps.ni, ctx->p.ly, res, ctx->stream));
+  CK(hst::launch_stats_final(g, ctx->d, pm, pg, nblk_dy, ly_w, ctx->ps.ni, ctx->p.ly, res, ctx->stream));
   ctx->launches += 2;
-  double* exz_d = reinterpret_cast<double*>(ctx->d.F[HST_RHS1]);
-  if (exz_h) {
-    CK(hst::launch_stats_columns(g, ctx->d, exz_d, ctx->stream));
-    ctx->launches++;
-  }
   CK(cudaMemcpyAsync(res_h, res, 24 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (exz_h) CK(cudaMemcpyAsync(exz_h, exz_d, sizeof(double) * g.ncol, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));

@@ -135,18 +135,18 @@ cudaError_t launch_fill_ghosts(const Geometry& g, const DeviceState& d, const Ph
 // from d.derS; d0_table_doubles: the table's size for any group of ny rows
 cudaError_t launch_d0_table(const Geometry& g, const DeviceState& d, cudaStream_t st);
 size_t d0_table_doubles(int ny);
-// outstats (src/hst_stats.f90:136-285): block count of the reductions and
-// the three kernels (hst_stats.cu)
+// outstats (src/hst_stats.f90:136-285): block count of the moments' reduction,
+// the moments and (exz not null) the column energies exz(-nz:nz, 0:nx), the
+// wall-normal gradients (hst_solve.cu; *blocks: its block count), the results
 int stats_blocks(const Geometry& g, int nsm);
 cudaError_t launch_stats_moments(const Geometry& g, const DeviceState& d, const PhysScalars& ps, double gsoft,
-                                 double* partial, cudaStream_t st);
-// the column energies exz(-nz:nz, 0:nx) of outstats into exz (ncol doubles)
-cudaError_t launch_stats_columns(const Geometry& g, const DeviceState& d, double* exz, cudaStream_t st);
+                                 double* partial, double* exz, cudaStream_t st);
+cudaError_t launch_dy_sums(const Geometry& g, const DeviceState& d, const PhysScalars& ps, double sx, double sz,
+                           double* partial, int* blocks, cudaStream_t st);
+cudaError_t launch_stats_final(const Geometry& g, const DeviceState& d, const double* pm, const double* pg, int nblk_dy,
+                               double ly_w, double ni, double ly, double* out, cudaStream_t st);
 // moment partials a reduction block writes
 int stats_partials();
-cudaError_t launch_stats_grad(const Geometry& g, const DeviceState& d, int field, double* partial, cudaStream_t st);
-cudaError_t launch_stats_final(const Geometry& g, const DeviceState& d, const double* pm, const double* pg,
-                               double ly_w, double ni, double ly, double* out, cudaStream_t st);
 // compute_pressure (src/hst_pressure.f90:35-110): the right-hand side into
 // RHS1 (after the transforms), and the (0,0) mode into dst (after the
 // POISSON solve)

@@ -513,10 +513,12 @@ __device__ __forceinline__ void line_solve_d0(cxd ph, const double* __restrict__
 // sliding window, the two rows beyond each end of the slab from the
 // neighbouring lanes (by shuffle, taken before anything is written) and,
 // across the box edge, the shear-periodic ghost images f(ny + k) = f(k) ph,
-// f(-k) = f(ny - k) conj(ph) (wrap_rows, src/hst_mpi.f90:340-355).  The sum
-// runs over j = -2..2 in order, as the reference's stencils do.
+// f(-k) = f(ny - k) conj(ph) (wrap_rows, src/hst_mpi.f90:340-355), or, with
+// `ghosts` (rows -2, -1, ny, ny + 1), those rows.  The sum runs over j = -2..2
+// in order, as the reference's stencils do.
 template <int P, class DST>
-__device__ __forceinline__ void slab_stencil(int n, const DST& DS, cxd* sb, int m, int s, cxd ph, unsigned gmask) {
+__device__ __forceinline__ void slab_stencil(int n, const DST& DS, cxd* sb, int m, int s, cxd ph, unsigned gmask,
+                                             const cxd* ghosts = nullptr) {
   const cxd f0 = sb[0], f1 = sb[1], l0 = sb[m - 2], l1 = sb[m - 1];
   const int up = (s + 1) & (P - 1), dn = (s - 1) & (P - 1);
   cxd a0 = shfl_c(gmask, f0, up, P), a1 = shfl_c(gmask, f1, up, P);  // rows m, m + 1 of the slab
@@ -528,6 +530,10 @@ __device__ __forceinline__ void slab_stencil(int n, const DST& DS, cxd* sb, int 
   if (s == 0) {
     b0 = cmul(b0, cconj(ph));
     b1 = cmul(b1, cconj(ph));
+  }
+  if (ghosts) {
+    if (s == 0) b0 = ghosts[0], b1 = ghosts[1];
+    if (s == P - 1) a0 = ghosts[2], a1 = ghosts[3];
   }
   cxd w0 = b0, w1 = b1, w2 = f0, w3 = f1, w4 = sb[2];
 #pragma unroll 2

@@ -10,6 +10,7 @@
 //                 DY solve of its D1 stencil) into the interior rows of V1,
 //                 scratch until the second pass; 1 the ETA solve, u and w,
 //                 V1 and V3 with their ghost rows
+//   k_dy_sums     the wall-normal gradients' part of outstats
 //   k_line_solve  line_solve (src/hst_linsolve.f90:147-233) of one field
 //   k_d0_table    the factored D0 matrix
 //
@@ -204,6 +205,66 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
   }
 }
 
+// The weighted sums of |du/dy|^2, |dv/dy|^2, |dw/dy|^2 over every column and
+// row (outstats, src/hst_stats.f90:136-285): D1 with the stored ghost rows, the
+// DY solve, nothing written but the blocks' partials [component][block]
+// SH: the tables in shared memory (the most rows have no room there)
+template <int P, bool SH>
+__global__ void __launch_bounds__(512, 1) k_dy_sums(SolveArgs a, double sx, double sz, const double* __restrict__ dyl,
+                                                    double* __restrict__ partial) {
+  extern __shared__ __align__(16) double smem_d[];
+  __shared__ double part[16][3];
+  const Geometry& g = a.g;
+  const LineGeom G = line_geom(g.ny, P);
+  const int mM = slab_rows(g.ny, P), ny = g.ny;
+  const int groups = blockDim.x / P, grp = threadIdx.x / P, s = threadIdx.x % P;
+  const unsigned gmask = group_mask<P>();
+  const int nd1 = 5 * mM * P, ntab = SH ? d0_fields(mM, P) * P : 0, nder = SH ? nd1 : 0;
+  double* const d0s = smem_d;
+  double* const der1s = d0s + ntab;
+  for (int i = threadIdx.x; i < ntab; i += blockDim.x) d0s[i] = a.d0tab[i];
+  for (int i = threadIdx.x; i < nder; i += blockDim.x) der1s[i] = a.derS[nd1 + i];
+  if (SH) __syncthreads();
+  cxd* const buf = reinterpret_cast<cxd*>(der1s + nder) + (size_t)grp * P * G.MS;
+  cxd* const sb = buf + s * G.MS;
+  const int m = G.rows(s), r0 = G.first(s);
+  const SlabDerT<SH> DS = {SH ? der1s : a.derS + nd1, mM, P};
+  double sum[3] = {0.0, 0.0, 0.0};
+  for (int cg = blockIdx.x * groups + grp; cg < g.ncol; cg += gridDim.x * groups) {
+    const Column c = column_of(g, a.ps, cg);
+    const cxd ph = cexpi(-(c.al * sx + c.be * sz));
+    const double wc = cg < g.nzT ? 1.0 : 2.0;  // ix > 0: the conjugate half
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double2* const f = (q == 0 ? a.V1 : (q == 1 ? a.V2 : a.V3)) + c.cb;
+      load_line<P>(f, buf, G, s);
+      cxd gh[4] = {mkc(0, 0), mkc(0, 0), mkc(0, 0), mkc(0, 0)};
+      if (s == 0) gh[0] = f[-2], gh[1] = f[-1];
+      if (s == P - 1) gh[2] = f[ny], gh[3] = f[ny + 1];
+      __syncwarp(gmask);
+      slab_stencil<P>(0, DS, sb, m, s, ph, gmask, gh);
+      line_solve_d0<P, SH, false>(ph, SH ? d0s : a.d0tab, mM, m, sb, s, gmask);
+      for (int i = 0; i < m; ++i) {
+        const cxd d = sb[i];
+        sum[q] += wc * __ldg(dyl + r0 + i) * (d.x * d.x + d.y * d.y);
+      }
+      __syncwarp(gmask);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], o);
+  if ((threadIdx.x & 31) == 0)
+    for (int q = 0; q < 3; ++q) part[threadIdx.x >> 5][q] = sum[q];
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) t += part[w][threadIdx.x];
+    partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
+  }
+}
+
 // line_solve for every Fourier column of one field, the factors in shared
 // memory (a caller's own arrays come with no scratch)
 template <int P>
@@ -349,6 +410,27 @@ static cudaError_t launch_shift_t(const SolveArgs& a, const DeviceState& d, cuda
   return cudaGetLastError();
 }
 
+template <int P>
+static cudaError_t launch_dy_sums_t(const SolveArgs& a, const DeviceState& d, double sx, double sz, double* partial,
+                                    int* blocks, cudaStream_t st) {
+  const Geometry& g = a.g;
+  const int mM = slab_rows(g.ny, P), nsm = sm_count(d);
+  size_t tabs = ((size_t)d0_fields(mM, P) * P + (size_t)5 * mM * P) * sizeof(double);
+  int W = solve_warps(g, nsm, tabs + 1024);
+  const bool sh = W >= 4 || W == solve_warps(g, nsm, 1024);
+  if (!sh) {
+    tabs = 0;
+    W = solve_warps(g, nsm, 1024);
+  }
+  if (W < 1) return cudaErrorInvalidValue;
+  const int groups = W * 32 / P;
+  *blocks = std::min(nsm, (g.ncol + groups - 1) / groups);
+  auto k = sh ? k_dy_sums<P, true> : k_dy_sums<P, false>;
+  smem_limit(d, k, 226 * 1024);
+  k<<<*blocks, 32 * W, tabs + W * line_bytes(g.ny, P) * (32 / P), st>>>(a, sx, sz, d.dyl, partial);
+  return cudaGetLastError();
+}
+
 template <int P, int HALF>
 static cudaError_t launch_half_t(const SolveArgs& a, const DeviceState& d, cudaStream_t st) {
   const Geometry& g = a.g;
@@ -401,6 +483,14 @@ cudaError_t launch_shift(const Geometry& g, const DeviceState& d, const PhysScal
                          cudaStream_t st) {
   const SolveArgs a = solve_args(g, d, ps, sc);
 #define HST_CALL(P) launch_shift_t<P>(a, d, st)
+  HST_LANES(g.P, HST_CALL);
+#undef HST_CALL
+}
+
+cudaError_t launch_dy_sums(const Geometry& g, const DeviceState& d, const PhysScalars& ps, double sx, double sz,
+                           double* partial, int* blocks, cudaStream_t st) {
+  const SolveArgs a = solve_args(g, d, ps, SubstepScalars{});
+#define HST_CALL(P) launch_dy_sums_t<P>(a, d, sx, sz, partial, blocks, st)
   HST_LANES(g.P, HST_CALL);
 #undef HST_CALL
 }

@@ -8,10 +8,11 @@
 //                    moments with the y weights dyl (twice for ix > 0, the
 //                    conjugate half), k^2 |u|^2 for the dissipation, and the
 //                    mean-flow sums of the (0,0) column
-//   k_stats_grad     per column, the weighted |dq/dy|^2 of one component
-//                    (its compact derivative comes from the DY line solve)
+//                    and the column energies of the 2-D spectrum
 //   k_stats_final    the block partials summed in order, the mean flow
 //                    removed from the (0,0) variances, everything over ly
+//
+// (the weighted |dq/dy|^2: k_dy_sums in hst_solve.cu)
 #include "hst_dev.cuh"
 #include "hst_internal.h"
 
@@ -53,7 +54,8 @@ __global__ void __launch_bounds__(32 * ST_WARPS) k_stats_moments(Geometry g, Phy
                                                                  const double2* __restrict__ V3,
                                                                  const double* __restrict__ dyl,
                                                                  const double* __restrict__ gdamp, double gsoft,
-                                                                 double* __restrict__ partial) {
+                                                                 double* __restrict__ partial,
+                                                                 double* __restrict__ exz) {
   double v[ST_NM] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int col = blockIdx.x * ST_WARPS + warp; col < g.ncol; col += gridDim.x * ST_WARPS) {
@@ -61,10 +63,14 @@ __global__ void __launch_bounds__(32 * ST_WARPS) k_stats_moments(Geometry g, Phy
     const double al = ps.alfa0 * ix, be = ps.beta0 * iz, kk = al * al + be * be;
     const double gd = gdamp[col];
     const size_t cb = (size_t)col * g.rows + 2;
+    // the column's energy exz(iz, ix) = sum_y w |u|^2 (src/hst_stats.f90:225-240)
+    double ec = 0.0;
+#pragma unroll 2
     for (int iy = lane; iy < g.ny; iy += 32) {
       const cxd u = V1[cb + iy], vv = V2[cb + iy], w = V3[cb + iy];
       const double d = dyl[iy];
       if (ix == 0 && iz == 0) {
+        ec += d * ((u.x * u.x + u.y * u.y) + (vv.x * vv.x + vv.y * vv.y) + (w.x * w.x + w.y * w.y));
         v[7] += u.x * d;
         v[8] += w.x * d;
         if (gd > 0.0) {
@@ -92,64 +98,38 @@ __global__ void __launch_bounds__(32 * ST_WARPS) k_stats_moments(Geometry g, Phy
       v[6] += wt * (u.x * w.x + u.y * w.y);
       v[0] += wt * kk * (pu + pv + pw);
       v[9] += wt * (pu + pv + pw);
+      ec += wt * (pu + pv + pw);
+    }
+    if (exz) {
+      for (int o = 16; o > 0; o >>= 1) ec += __shfl_xor_sync(0xffffffffu, ec, o);
+      if (lane == 0) exz[col] = ec;
     }
   }
   block_sums<ST_NM>(v, partial);
-}
-
-// the column energies exz(iz, ix) = sum_y w |u|^2 (src/hst_stats.f90:225-240),
-// one warp per column, lanes over rows, a fixed order
-__global__ void __launch_bounds__(32 * ST_WARPS) k_stats_columns(Geometry g, const double2* __restrict__ V1,
-                                                                 const double2* __restrict__ V2,
-                                                                 const double2* __restrict__ V3,
-                                                                 const double* __restrict__ dyl,
-                                                                 double* __restrict__ exz) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * ST_WARPS + warp;
-  if (col >= g.ncol) return;
-  const int ix = col / g.nzT;
-  const size_t cb = (size_t)col * g.rows + 2;
-  double q = 0.0;
-  for (int iy = lane; iy < g.ny; iy += 32) {
-    const cxd u = V1[cb + iy], vv = V2[cb + iy], w = V3[cb + iy];
-    const double wt = ix == 0 ? dyl[iy] : 2.0 * dyl[iy];
-    q += wt * ((u.x * u.x + u.y * u.y) + (vv.x * vv.x + vv.y * vv.y) + (w.x * w.x + w.y * w.y));
-  }
-  for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-  if (lane == 0) exz[col] = q;
-}
-
-// the weighted sum of |q|^2 over every column (q: the DY solve of one component)
-__global__ void __launch_bounds__(32 * ST_WARPS) k_stats_grad(Geometry g, const double2* __restrict__ Q,
-                                                              const double* __restrict__ dyl,
-                                                              double* __restrict__ partial) {
-  double v[1] = {0.0};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int col = blockIdx.x * ST_WARPS + warp; col < g.ncol; col += gridDim.x * ST_WARPS) {
-    const int ix = col / g.nzT;
-    const size_t cb = (size_t)col * g.rows + 2;
-    for (int iy = lane; iy < g.ny; iy += 32) {
-      const cxd q = Q[cb + iy];
-      const double wt = ix == 0 ? dyl[iy] : 2.0 * dyl[iy];
-      v[0] += wt * (q.x * q.x + q.y * q.y);
-    }
-  }
-  block_sums<1>(v, partial);
 }
 
 // out[0..7]: energy, dissipation, uv, vw, uu, vv, ww, uw (the order of the
 // Runtimedata columns the reference writes); out[8..23]: the reference's
 // sums array before the box-mean correction (eps, uv, uu, vv, ww, vw, uw,
 // mfx, mfz, q_in, q_out, e_in, e_out, ed, pd; ncol_damped is the host's)
-__global__ void k_stats_final(int nblk, const double* __restrict__ pm, const double* __restrict__ pg, double ly_w,
-                              double ni, double ly, double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s[ST_NM] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int b = 0; b < nblk; ++b)
-    for (int k = 0; k < ST_NM; ++k) s[k] += pm[(size_t)b * ST_NM + k];
+// One warp a sum: lanes over the blocks, then over the lanes, a fixed order.
+__global__ void __launch_bounds__(32 * (ST_NM + 3)) k_stats_final(int nblk, int nblk_dy, const double* __restrict__ pm,
+                                                                  const double* __restrict__ pg, double ly_w, double ni,
+                                                                  double ly, double* __restrict__ out) {
+  __shared__ double tot[ST_NM + 3];
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double t = 0.0;
+  if (k < ST_NM)
+    for (int b = lane; b < nblk; b += 32) t += pm[(size_t)b * ST_NM + k];
+  else
+    for (int b = lane; b < nblk_dy; b += 32) t += pg[(size_t)(k - ST_NM) * nblk_dy + b];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) tot[k] = t;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const double* const s = tot;
   double eps = s[0];
-  for (int c = 0; c < 3; ++c)
-    for (int b = 0; b < nblk; ++b) eps += pg[(size_t)c * nblk + b];
+  for (int c = 0; c < 3; ++c) eps += tot[ST_NM + c];
   double* raw = out + 8;
   raw[0] = eps;
   for (int k = 1; k < 9; ++k) raw[k] = s[k];
@@ -284,27 +264,17 @@ int stats_blocks(const Geometry& g, int nsm) {
 }
 
 cudaError_t launch_stats_moments(const Geometry& g, const DeviceState& d, const PhysScalars& ps, double gsoft,
-                                 double* partial, cudaStream_t st) {
+                                 double* partial, double* exz, cudaStream_t st) {
   k_stats_moments<<<stats_blocks(g, d.nsm), 32 * ST_WARPS, 0, st>>>(g, ps, d.F[0], d.F[1], d.F[2], d.dyl, d.gdamp,
-                                                                     gsoft, partial);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_stats_columns(const Geometry& g, const DeviceState& d, double* exz, cudaStream_t st) {
-  k_stats_columns<<<(g.ncol + ST_WARPS - 1) / ST_WARPS, 32 * ST_WARPS, 0, st>>>(g, d.F[0], d.F[1], d.F[2], d.dyl, exz);
+                                                                     gsoft, partial, exz);
   return cudaGetLastError();
 }
 
 int stats_partials() { return ST_NM; }
 
-cudaError_t launch_stats_grad(const Geometry& g, const DeviceState& d, int field, double* partial, cudaStream_t st) {
-  k_stats_grad<<<stats_blocks(g, d.nsm), 32 * ST_WARPS, 0, st>>>(g, d.F[field], d.dyl, partial);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_stats_final(const Geometry& g, const DeviceState& d, const double* pm, const double* pg,
+cudaError_t launch_stats_final(const Geometry& g, const DeviceState& d, const double* pm, const double* pg, int nblk_dy,
                                double ly_w, double ni, double ly, double* out, cudaStream_t st) {
-  k_stats_final<<<1, 32, 0, st>>>(stats_blocks(g, d.nsm), pm, pg, ly_w, ni, ly, out);
+  k_stats_final<<<1, 32 * (ST_NM + 3), 0, st>>>(stats_blocks(g, d.nsm), nblk_dy, pm, pg, ly_w, ni, ly, out);
   return cudaGetLastError();
 }
 
