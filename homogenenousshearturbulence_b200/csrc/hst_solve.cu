@@ -84,9 +84,14 @@ __device__ __forceinline__ void store_ghosts(double2* __restrict__ dst, const cx
   }
 }
 
+// The four lines of a column one after another.  What bounds it is the
+// shared-memory traffic of the tables and the lines; two lines at a time,
+// sharing the table loads, leave nine warps an SM and measured slower (3.42
+// against 2.62 ms at 768^2 x 512).
+constexpr int SHIFT_LINES = 1, SHIFT_WARPS = 16;
 // SH: the tables in shared memory (the most rows have no room there)
 template <int P, bool SH>
-__global__ void __launch_bounds__(512, 1) k_shift(SolveArgs a) {
+__global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
   extern __shared__ __align__(16) double smem_d[];
   const Geometry& g = a.g;
   const SubstepScalars& sc = a.sc;
@@ -100,29 +105,43 @@ __global__ void __launch_bounds__(512, 1) k_shift(SolveArgs a) {
   for (int i = threadIdx.x; i < ntab; i += blockDim.x) d0s[i] = a.d0tab[i];
   for (int i = threadIdx.x; i < nder; i += blockDim.x) der0s[i] = a.derS[i];
   if (SH) __syncthreads();
-  cxd* const buf = reinterpret_cast<cxd*>(der0s + nder) + (size_t)grp * P * G.MS;
-  cxd* const sb = buf + s * G.MS;
+  const int lineN = P * G.MS;
+  cxd* const buf = reinterpret_cast<cxd*>(der0s + nder) + (size_t)grp * SHIFT_LINES * lineN;
+  cxd* sb[SHIFT_LINES];
+#pragma unroll
+  for (int k = 0; k < SHIFT_LINES; ++k) sb[k] = buf + k * lineN + s * G.MS;
   const int m = G.rows(s), r0 = G.first(s);
   const SlabDerT<SH> DS = {SH ? der0s : a.derS, mM, P};
+  const D0Table<P, SH> T = {(SH ? d0s : a.d0tab) + s};
   for (int cg = blockIdx.x * groups + grp; cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
     const Column c = column_of(g, a.ps, cg);
     const cxd pt = cexpi(-(c.al * sc.sx_t + c.be * sc.sz_t)), pn = cexpi(-(c.al * sc.sx_n + c.be * sc.sz_n));
     const double gx = c.al * sc.dgx + c.be * sc.dgz;
     // the node phase of the slab's last row; on a uniform grid the rows
     // below follow by one complex product each (dy = ly / ny apart)
-    const cxd e0 = sc.yuni ? cexpi(-gx * a.y[r0 + m + 1]) : mkc(1.0, 0.0);
+    const cxd etop = sc.yuni ? cexpi(-gx * a.y[r0 + m + 1]) : mkc(1.0, 0.0);
     const cxd step = sc.yuni ? cexpi(gx * (sc.ytile / 32.0)) : mkc(1.0, 0.0);
 #pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-      double2* const f = (q == 0 ? a.O1 : (q == 1 ? a.O2 : (q == 2 ? a.R1 : a.R2))) + c.cb;
-      load_line<P>(f, buf, G, s);
+    for (int q = 0; q < 4; q += SHIFT_LINES) {
+      double2* f[SHIFT_LINES];
+#pragma unroll
+      for (int k = 0; k < SHIFT_LINES; ++k) {
+        const int l = q + k;
+        f[k] = (l == 0 ? a.O1 : (l == 1 ? a.O2 : (l == 2 ? a.R1 : a.R2))) + c.cb;
+        load_line<P>(f[k], buf + k * lineN, G, s);
+      }
       __syncwarp(gmask);
-      line_solve_d0<P, SH, true>(pt, SH ? d0s : a.d0tab, mM, m, sb, s, gmask, e0, step);
-      if (!sc.yuni)
-        for (int i = 0; i < m; ++i) sb[i] = cmul(sb[i], cexpi(-gx * a.y[r0 + i + 2]));
-      slab_stencil<P>(0, DS, sb, m, s, pn, gmask);
+      cxd e = etop;
+      auto node = [&](int i) -> cxd {
+        if (!sc.yuni) return cexpi(-gx * a.y[r0 + i + 2]);
+        const cxd v = e;
+        e = cmul(e, step);
+        return v;
+      };
+      shift_lines<P, SHIFT_LINES>(pt, pn, T, DS, mM, m, sb, s, gmask, node);
       __syncwarp(gmask);
-      store_line<P>(f, buf, G, s);
+#pragma unroll
+      for (int k = 0; k < SHIFT_LINES; ++k) store_line<P>(f[k], buf + k * lineN, G, s);
       __syncwarp(gmask);
     }
   }
@@ -167,7 +186,7 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
       __syncwarp(gmask);
       // D1 v, then D0 (dv/dy) = D1 v (KIND_DY)
       slab_stencil<P>(1, DS, sb, m, s, pn, gmask);
-      line_solve_d0<P, false, false>(pn, a.d0tab, mM, m, sb, s, gmask);
+      line_solve_d0<P, false>(pn, a.d0tab, mM, m, sb, s, gmask);
       __syncwarp(gmask);
       store_line<P>(v1, buf, G, s);
     } else {
@@ -243,7 +262,7 @@ __global__ void __launch_bounds__(512, 1) k_dy_sums(SolveArgs a, double sx, doub
       if (s == P - 1) gh[2] = f[ny], gh[3] = f[ny + 1];
       __syncwarp(gmask);
       slab_stencil<P>(0, DS, sb, m, s, ph, gmask, gh);
-      line_solve_d0<P, SH, false>(ph, SH ? d0s : a.d0tab, mM, m, sb, s, gmask);
+      line_solve_d0<P, SH>(ph, SH ? d0s : a.d0tab, mM, m, sb, s, gmask);
       for (int i = 0; i < m; ++i) {
         const cxd d = sb[i];
         sum[q] += wc * __ldg(dyl + r0 + i) * (d.x * d.x + d.y * d.y);
@@ -369,15 +388,15 @@ static size_t line_bytes(int ny, int P) { return (size_t)P * line_geom(ny, P).MS
 // double2 of factor scratch a group
 static int fac_elems(int ny, int P) { return 2 * (slab_rows(ny, P) - 2) * P; }
 
-// warps a block (one block an SM): as many as sixteen whose lines fit beside
-// `tabs` bytes of tables, and no more than spread the columns over the SMs;
-// 0 when not even one fits
-static int solve_warps(const Geometry& g, int nsm, size_t tabs) {
-  const size_t warp = line_bytes(g.ny, g.P) * (32 / g.P);
+// warps a block (one block an SM): as many as `most` whose groups' lines fit
+// beside `tabs` bytes of tables, and no more than spread the columns over the
+// SMs; 0 when not even one fits
+static int solve_warps(const Geometry& g, int nsm, size_t tabs, int lines = 1, int most = 16) {
+  const size_t warp = lines * line_bytes(g.ny, g.P) * (32 / g.P);
   if (tabs + warp > 227 * 1024) return 0;
   const long groups = ((long)g.ncol * g.nmem + nsm - 1) / nsm;  // columns an SM
   const long want = (groups * g.P + 31) / 32;
-  return (int)std::min<long>({16, want, (long)((227 * 1024 - tabs) / warp)});
+  return (int)std::min<long>({most, want, (long)((227 * 1024 - tabs) / warp)});
 }
 
 size_t solve_scratch_bytes(const Geometry& g, int nsm) {
@@ -395,18 +414,18 @@ static cudaError_t launch_shift_t(const SolveArgs& a, const DeviceState& d, cuda
   const Geometry& g = a.g;
   const int mM = slab_rows(g.ny, P), nsm = sm_count(d);
   size_t tabs = ((size_t)d0_fields(mM, P) * P + (size_t)5 * mM * P) * sizeof(double);
-  int W = solve_warps(g, nsm, tabs);
-  const bool sh = W >= 4 || W == solve_warps(g, nsm, 0);
+  int W = solve_warps(g, nsm, tabs, SHIFT_LINES, SHIFT_WARPS);
+  const bool sh = W >= 4 || W == solve_warps(g, nsm, 0, SHIFT_LINES, SHIFT_WARPS);
   if (!sh) {  // the tables through L1
     tabs = 0;
-    W = solve_warps(g, nsm, 0);
+    W = solve_warps(g, nsm, 0, SHIFT_LINES, SHIFT_WARPS);
   }
   if (W < 1) return cudaErrorInvalidValue;
   const int groups = W * 32 / P;
   const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
   auto k = sh ? k_shift<P, true> : k_shift<P, false>;
   smem_limit(d, k, 227 * 1024);
-  k<<<nb, 32 * W, tabs + W * line_bytes(g.ny, P) * (32 / P), st>>>(a);
+  k<<<nb, 32 * W, tabs + W * SHIFT_LINES * line_bytes(g.ny, P) * (32 / P), st>>>(a);
   return cudaGetLastError();
 }
 
