@@ -141,7 +141,13 @@ struct hst_ctx {
   std::vector<double> y, dyl, der, gdamp;
   double theta_last;
   cudaStream_t stream;
-  double* h_gdamp;                // pinned staging of gdamp uploads
+  // pinned staging of gdamp uploads: GD_SLOTS copies of the table's first
+  // gd_nix x modes (the others are never damped), each with the event after
+  // its copy to the device
+  static constexpr int GD_SLOTS = 4;
+  double* h_gdamp;
+  int gd_nix, gd_next;
+  cudaEvent_t ev_gd[GD_SLOTS] = {nullptr, nullptr, nullptr, nullptr};
   unsigned long long* h_cfl;      // pinned CFL read-back
   std::string err;
   // an ensemble of nmem members in one context (hst_gpu_create_batch): gb, db
@@ -248,16 +254,31 @@ static void shear_shifts(const hst_ctx* c, double t, double* sx, double* sz) {  
 static bool damping_active(const hst_gpu_params& p) {  // src/hst_damping.f90:46-48
   return p.damp_kpar > 0.0 && p.damp_kperp > 0.0 && (p.damp_hard || p.damp_rate > 0.0);
 }
+// The modes |ix| <= nix, |iz| <= niz outside which the damping rate is zero at
+// any angle: it needs |kpar| < damp_kpar and |kperp| < damp_kperp, so k^2 <
+// damp_kpar^2 + damp_kperp^2 (for a positive norm).
+static void damping_box(const hst_gpu_params& p, int* nix, int* niz) {
+  *nix = p.nx;
+  *niz = p.nz;
+  if (!(p.damp_norm > 0.0)) return;
+  const double K = std::sqrt(p.damp_kpar * p.damp_kpar + p.damp_kperp * p.damp_kperp) * (1.0 + 1.0e-9);
+  if (K < std::fabs(p.alfa0) * p.nx) *nix = (int)(K / std::fabs(p.alfa0)) + 1;
+  if (K < std::fabs(p.beta0) * p.nz) *niz = (int)(K / std::fabs(p.beta0)) + 1;
+  *nix = std::min(*nix, p.nx);
+  *niz = std::min(*niz, p.nz);
+}
 // damping_update (src/hst_damping.f90:80-115); true when the table changed
 static bool damping_update(hst_ctx* c, double t) {
   const hst_gpu_params& p = c->p;
   double theta = p.damp_follow ? std::atan2(s2_of(p, t), p.S) : p.damp_angle * PI / 180.0;
   if (theta == c->theta_last) return false;
   c->theta_last = theta;
+  int nix, niz;
+  damping_box(p, &nix, &niz);
   double cs = std::cos(theta), sn = std::sin(theta);
-  for (int ix = 0; ix <= p.nx; ++ix) {
+  for (int ix = 0; ix <= nix; ++ix) {
     double kx = p.alfa0 * ix;
-    for (int iz = -p.nz; iz <= p.nz; ++iz) {
+    for (int iz = -niz; iz <= niz; ++iz) {
       double kz = p.beta0 * iz;
       double kpar = kx * cs + kz * sn, kperp = -kx * sn + kz * cs;
       double r = std::pow(std::pow(std::fabs(kpar) / p.damp_kpar, p.damp_norm) + std::pow(std::fabs(kperp) / p.damp_kperp, p.damp_norm),
@@ -276,6 +297,30 @@ static bool damping_update(hst_ctx* c, double t) {
     }
   }
   return true;
+}
+
+// The damping table's x modes that can be damped, uploaded in stream order (an
+// oscillating S2 turns the damped region every substep): one of GD_SLOTS pinned
+// copies is refilled, once the copy from it GD_SLOTS updates ago has gone out,
+// so that the host does not wait for the stream.
+static int upload_gdamp(hst_ctx* ctx) {
+  const size_t nzT = 2 * (size_t)ctx->p.nz + 1;
+  if (!ctx->h_gdamp) {
+    int niz;
+    damping_box(ctx->p, &ctx->gd_nix, &niz);
+    ctx->gd_nix += 1;
+    CK(cudaMallocHost((void**)&ctx->h_gdamp, sizeof(double) * nzT * ctx->gd_nix * hst_ctx::GD_SLOTS));
+  }
+  const int k = ctx->gd_next;
+  ctx->gd_next = (k + 1) % hst_ctx::GD_SLOTS;
+  const size_t n = nzT * ctx->gd_nix;
+  double* const slot = ctx->h_gdamp + n * k;
+  if (ctx->ev_gd[k]) CK(cudaEventSynchronize(ctx->ev_gd[k]));
+  else CK(cudaEventCreateWithFlags(&ctx->ev_gd[k], cudaEventDisableTiming));
+  std::memcpy(slot, ctx->gdamp.data(), sizeof(double) * n);
+  CK(cudaMemcpyAsync(ctx->d.gdamp, slot, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaEventRecord(ctx->ev_gd[k], ctx->stream));
+  return HST_OK;
 }
 
 // ------------------------------------------------------ geometry ----
@@ -496,6 +541,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   }
   ctx->stream = nullptr;
   ctx->h_gdamp = nullptr;
+  ctx->gd_nix = ctx->gd_next = 0;
   ctx->h_cfl = nullptr;
   std::memset(&ctx->d, 0, sizeof ctx->d);
   ctx->d.configured = &ctx->configured;
@@ -594,7 +640,6 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
     return HST_ENOMEM;
   }
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMallocHost((void**)&ctx->h_gdamp, sizeof(double) * g.ncol) != cudaSuccess ||
       cudaMallocHost((void**)&ctx->h_cfl, 2 * sizeof(unsigned long long)) != cudaSuccess) {
     free_device(ctx);
     delete ctx;
@@ -718,6 +763,8 @@ extern "C" int hst_gpu_destroy(hst_ctx* ctx) {
   for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
   free_device(ctx);
   if (ctx->h_gdamp) cudaFreeHost(ctx->h_gdamp);
+  for (cudaEvent_t e : ctx->ev_gd)
+    if (e) cudaEventDestroy(e);
   if (ctx->h_cfl) cudaFreeHost(ctx->h_cfl);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -1245,11 +1292,8 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
       if (!p.linear) CK(timed(ctx, HST_KC_ZFWD, [&] { return hst::launch_zfwd(G, D, ctx->stream); }));
     }
     if (damp && damping_update(ctx, t)) {
-      // stream-ordered upload of the new table (the previous copy has been
-      // consumed once the stream reaches it, so wait before refilling)
-      CK(cudaStreamSynchronize(ctx->stream));
-      std::memcpy(ctx->h_gdamp, ctx->gdamp.data(), sizeof(double) * ctx->g.ncol);
-      CK(cudaMemcpyAsync(D.gdamp, ctx->h_gdamp, sizeof(double) * ctx->g.ncol, cudaMemcpyHostToDevice, ctx->stream));
+      int rc = upload_gdamp(ctx);
+      if (rc != HST_OK) return rc;
     }
     SubstepScalars sc;
     sc.ode0 = ODE[0];
@@ -1485,10 +1529,7 @@ extern "C" int hst_gpu_damping_update(hst_ctx* ctx, double time) {
   if (!ctx) return HST_EARG;
   if (!damping_active(ctx->p) || !damping_update(ctx, time)) return HST_OK;
   CK(cudaSetDevice(ctx->device));
-  CK(cudaStreamSynchronize(ctx->stream));
-  std::memcpy(ctx->h_gdamp, ctx->gdamp.data(), sizeof(double) * ctx->g.ncol);
-  CK(cudaMemcpyAsync(ctx->d.gdamp, ctx->h_gdamp, sizeof(double) * ctx->g.ncol, cudaMemcpyHostToDevice, ctx->stream));
-  return HST_OK;
+  return upload_gdamp(ctx);
 }
 
 extern "C" int hst_gpu_damping_mask(hst_ctx* ctx) {

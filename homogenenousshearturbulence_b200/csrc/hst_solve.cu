@@ -400,7 +400,8 @@ static int solve_warps(const Geometry& g, int nsm, size_t tabs, int lines = 1, i
 }
 
 size_t solve_scratch_bytes(const Geometry& g, int nsm) {
-  return (size_t)nsm * 16 * (32 / g.P) * fac_elems(g.ny, g.P) * sizeof(double2);
+  const size_t most = (size_t)nsm * 16 * (32 / g.P), cols = (size_t)g.ncol * g.nmem + 16 * (32 / g.P);
+  return std::min(most, cols) * fac_elems(g.ny, g.P) * sizeof(double2);
 }
 
 static SolveArgs solve_args(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc) {
