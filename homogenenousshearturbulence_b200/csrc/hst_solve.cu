@@ -284,13 +284,13 @@ __global__ void __launch_bounds__(512, 1) k_dy_sums(SolveArgs a, double sx, doub
   }
 }
 
-// line_solve for every Fourier column of one field, the factors in shared
-// memory (a caller's own arrays come with no scratch)
+// line_solve of KIND_D2V, KIND_ETA or KIND_POISSON for every Fourier column of
+// one field, the factors in shared memory (a caller's own arrays come with no
+// scratch)
 template <int P>
 __global__ void __launch_bounds__(64) k_line_solve(Geometry g, PhysScalars ps, int sys, double lambda,
                                                    const double2* __restrict__ src, double2* __restrict__ dst, double sx,
-                                                   double sz, const double* __restrict__ der,
-                                                   const double* __restrict__ derS) {
+                                                   double sz, const double* __restrict__ derS) {
   extern __shared__ __align__(16) double smem_d[];
   const LineGeom G = line_geom(g.ny, P);
   const int mM = slab_rows(g.ny, P), ny = g.ny;
@@ -304,12 +304,45 @@ __global__ void __launch_bounds__(64) k_line_solve(Geometry g, PhysScalars ps, i
   const Column c = column_of(g, ps, col);
   const double2* const sc = src + c.cb;
   double2* const dc = dst + c.cb;
-  if (sys == K_DY) {
-    for (int r = s; r < ny; r += P) {
+  load_line<P>(sc, buf, G, s);
+  __syncwarp(gmask);
+  const BandConst bc = band_const(sys, lambda, ps.ni, c.kk);
+  const cxd ph = cexpi(-(c.al * sx + c.be * sz));
+  cxd* const sb = buf + s * G.MS;
+  if (sys == K_D2V)
+    line_solve<P, 3>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
+  else
+    line_solve<P, 2>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
+  __syncwarp(gmask);
+  if (c.c00 && sys == K_POISSON) return;
+  if (c.c00 && sys == K_D2V)
+    for (int r = s; r < ny; r += P) dc[r] = mkc(0, 0);
+  else
+    store_line<P>(dc, buf, G, s);
+}
+
+// line_solve of KIND_D0 or (dy) KIND_DY, whose right-hand side is D1 src, from
+// the factored table
+template <int P>
+__global__ void __launch_bounds__(128) k_line_solve_d0(Geometry g, PhysScalars ps, int dy,
+                                                       const double2* __restrict__ src, double2* __restrict__ dst,
+                                                       double sx, double sz, const double* __restrict__ der,
+                                                       const double* __restrict__ d0tab) {
+  extern __shared__ __align__(16) double smem_d[];
+  const LineGeom G = line_geom(g.ny, P);
+  const int groups = blockDim.x / P, grp = threadIdx.x / P, s = threadIdx.x % P;
+  const int col = blockIdx.x * groups + grp;
+  if (col >= g.ncol) return;
+  const unsigned gmask = group_mask<P>();
+  cxd* const buf = reinterpret_cast<cxd*>(smem_d) + (size_t)grp * P * G.MS;
+  const Column c = column_of(g, ps, col);
+  const double2* const sc = src + c.cb;
+  if (dy) {
+    for (int r = s; r < G.n; r += P) {
       cxd v = mkc(0, 0);
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
-        const double d1 = derv(der, ny, r, 1, j - 2);
+        const double d1 = derv(der, G.n, r, 1, j - 2);
         const cxd q = sc[r + j - 2];
         v = mkc(v.x + d1 * q.x, v.y + d1 * q.y);
       }
@@ -319,21 +352,9 @@ __global__ void __launch_bounds__(64) k_line_solve(Geometry g, PhysScalars ps, i
     load_line<P>(sc, buf, G, s);
   }
   __syncwarp(gmask);
-  const BandConst bc = band_const(sys, lambda, ps.ni, c.kk);
-  const cxd ph = cexpi(-(c.al * sx + c.be * sz));
-  cxd* const sb = buf + s * G.MS;
-  if (sys == K_D2V)
-    line_solve<P, 3>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
-  else if (sys == K_ETA || sys == K_POISSON)
-    line_solve<P, 2>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
-  else
-    line_solve<P, 1>(bc, ph, DS, G.rows(s), sb, fac, s, gmask);
+  line_solve_d0<P, false>(cexpi(-(c.al * sx + c.be * sz)), d0tab, slab_rows(g.ny, P), G.rows(s), buf + s * G.MS, s, gmask);
   __syncwarp(gmask);
-  if (c.c00 && sys == K_POISSON) return;
-  if (c.c00 && sys == K_D2V)
-    for (int r = s; r < ny; r += P) dc[r] = mkc(0, 0);
-  else
-    store_line<P>(dc, buf, G, s);
+  store_line<P>(dst + c.cb, buf, G, s);
 }
 
 // d0_factor of the group of P lanes: one warp, lanes 0..P-1
@@ -479,13 +500,22 @@ static cudaError_t launch_half_t(const SolveArgs& a, const DeviceState& d, cudaS
 template <int P>
 static cudaError_t launch_line_solve_t(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int sys,
                                        double lambda, int src, int dst, double sx, double sz, cudaStream_t st) {
+  if (sys == K_D0 || sys == K_DY) {
+    const size_t line = line_bytes(g.ny, P);
+    int groups = 128 / P;
+    while (groups > 1 && line * groups > 56 * 1024) groups >>= 1;
+    smem_limit(d, k_line_solve_d0<P>, 200 * 1024);
+    k_line_solve_d0<P><<<(g.ncol + groups - 1) / groups, groups * P, line * groups, st>>>(
+        g, ps, sys == K_DY, d.F[src], d.F[dst], sx, sz, d.der, d.d0tab);
+    return cudaGetLastError();
+  }
   const size_t per = line_bytes(g.ny, P) + fac_elems(g.ny, P) * sizeof(double2);
   int groups = 32 / P;
   while (groups > 1 && per * groups > 200 * 1024) groups >>= 1;
   if (per * groups > 200 * 1024) return cudaErrorInvalidValue;
   smem_limit(d, k_line_solve<P>, 200 * 1024);
   k_line_solve<P><<<(g.ncol + groups - 1) / groups, groups * P, per * groups, st>>>(g, ps, sys, lambda, d.F[src],
-                                                                                   d.F[dst], sx, sz, d.der, d.derS);
+                                                                                   d.F[dst], sx, sz, d.derS);
   return cudaGetLastError();
 }
 
