@@ -376,9 +376,10 @@ static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::
   }
   // the line-solver group (HST_LINE_LANES overrides)
   g.P = hst::line_lanes(p.ny, (long)g.ncol * nmem);
+  g.PL = hst::line_lanes_shared(p.ny);
   if (const char* env = std::getenv("HST_LINE_LANES")) {
     int e = std::atoi(env);
-    if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && p.ny % e == 0 && p.ny / e >= 4) g.P = e;
+    if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && p.ny % e == 0 && p.ny / e >= 4) g.P = g.PL = e;
   }
   // mixed precision: the FP32 transforms of the lengths it compiles and the
   // streamed right-hand sides
@@ -480,7 +481,8 @@ static void free_device(hst_ctx* c) {
   for (int i = 0; i < 7; ++i)
     if (d.F[i]) cudaFree(d.F[i]);
   void* ps[] = {d.Z,    d.Pp,   d.Q,    d.der,  d.derS,  d.d0tab, d.y,    d.dyl,  d.gdamp, d.twx, d.twz,
-                d.twxf, d.twzf, d.cfl,  d.stats, d.vvdz, d.vvdx,  d.vvdp, d.Zg,   d.Ppg,  d.Qg,  d.derU, d.derI};
+                d.twxf, d.twzf, d.cfl,  d.stats, d.vvdz, d.vvdx,  d.vvdp, d.Zg,   d.Ppg,  d.Qg,  d.derU, d.derI,
+                d.derL};
   for (void* q : ps)
     if (q) cudaFree(q);
   if (d.facg) cudaFree(d.facg);
@@ -618,6 +620,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   }
   ok = ok && alloc((void**)&d.der, sizeof(double) * 20 * (size_t)ny);
   ok = ok && alloc((void**)&d.derS, sizeof(double) * hst::slab_der_doubles(ny));
+  ok = ok && alloc((void**)&d.derL, sizeof(double) * hst::slab_der_doubles(ny));
   ok = ok && alloc((void**)&d.derU, sizeof(double) * 20 * (size_t)ny);
   ok = ok && alloc((void**)&d.derI, sizeof(int) * (size_t)ny);
   ok = ok && alloc((void**)&d.d0tab, sizeof(double) * hst::d0_table_doubles(ny));
@@ -653,6 +656,8 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   {
     auto ds = hst::slab_major(ctx->der, ny, g.P);
     cudaMemcpy(d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
+    ds = hst::slab_major(ctx->der, ny, g.PL);
+    cudaMemcpy(d.derL, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
     etab = hst::launch_d0_table(g, d, ctx->stream);
     if (etab == cudaSuccess) etab = upload_der_rows(ctx);
   }
@@ -800,6 +805,8 @@ extern "C" int hst_gpu_set_tables(hst_ctx* ctx, const double* der, const double*
     CK(cudaMemcpy(ctx->d.der, ctx->der.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice));
     auto ds = hst::slab_major(ctx->der, ny, ctx->g.P);
     CK(cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice));
+    ds = hst::slab_major(ctx->der, ny, ctx->g.PL);
+    CK(cudaMemcpy(ctx->d.derL, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice));
     CK(hst::launch_d0_table(ctx->g, ctx->d, ctx->stream));
     CK(upload_der_rows(ctx));
   }

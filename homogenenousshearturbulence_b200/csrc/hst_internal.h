@@ -19,7 +19,7 @@ struct Geometry {
   int nxB, nzT, rows;  // nx+1, 2nz+1, ny+4
   int ncol;            // nxB * nzT Fourier columns
   long nf;             // complex elements of one field (ncol * rows)
-  int P;               // lanes of a line-solve group
+  int P, PL;           // lanes of a line-solve group: in the substep, in hst_gpu_line_solve's factored kinds
   int Ty, nyT;         // rows and number of the transforms' y tiles (the last may reach beyond ny)
   int EY;              // rows of the y tile that holds the four ghost rows (Ty of a z plan, else 4)
   int mp;              // mixed precision: Z, Pp, Q and their transforms in FP32 (complex64)
@@ -41,6 +41,7 @@ struct DeviceState {
   double2* Q;           // spectral products: [6][ncol][ny]
   double* der;          // der(0:ny-1, 0:3, -2:2)
   double* derS;         // the same, slab-major for the line-solve groups (slab_major)
+  double* derL;         // the same for groups of PL lanes
   double* derU;         // der's distinct rows, coefficient-major (DerRows); nderU of them, 0: not used
   int* derI;            // the distinct row of each row
   int nderU;
@@ -121,6 +122,8 @@ cudaError_t launch_solve_half(const Geometry& g, const DeviceState& d, const Phy
                               int half, cudaStream_t st);
 // lanes of a solver group for ny rows and this many columns
 int line_lanes(int ny, long columns);
+// of k_line_solve, whose factors lie in shared memory
+int line_lanes_shared(int ny);
 // der(0:ny-1, 0:3, -2:2) in the slab-major order of groups of P lanes; the
 // doubles that any P takes
 std::vector<double> slab_major(const std::vector<double>& der, int ny, int P);

@@ -72,17 +72,17 @@ int fail(char* msg, int len, int rc, const char* fmt, ...) {
   return rc;
 }
 
-// lanes of a solver group: the rule of a context of one field of these sizes
+// lanes of a solver group: the rules of a context of one field of these sizes
 // (HST_LINE_LANES overrides), so the results are identical to those of such a
 // context that has not been autotuned; hst_gpu_autotune may give a context
 // another group width, and the two then agree up to rounding
-int lanes_of(int ny, long columns) {
+int lanes_of(int ny, long columns, bool d0) {
   const char* env = std::getenv("HST_LINE_LANES");
   if (env) {
     int e = std::atoi(env);
     if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && ny % e == 0 && ny / e >= 4) return e;
   }
-  return hst::line_lanes(ny, columns);
+  return d0 ? hst::line_lanes(ny, columns) : hst::line_lanes_shared(ny);
 }
 
 }  // namespace
@@ -108,7 +108,8 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
     if (a < b + bytes && b < a + bytes) return fail(msg, msg_len, HST_EARG, "src and dst overlap");
     if (c < b + bytes && b < c + dbytes) return fail(msg, msg_len, HST_EARG, "der and dst overlap");
   }
-  const int P = lanes_of(ny, (long)(nx + 1) * (2 * nz + 1));
+  const bool d0 = sys == hst::K_D0 || sys == hst::K_DY;
+  const int P = lanes_of(ny, (long)(nx + 1) * (2 * nz + 1), d0);
 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -127,7 +128,7 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
   g.rows = ny + 4;
   g.ncol = g.nxB * g.nzT;
   g.nf = (long)g.ncol * g.rows;
-  g.P = P;
+  g.P = g.PL = P;
   hst::PhysScalars ps = {};
   ps.alfa0 = alfa0;
   ps.beta0 = beta0;
@@ -136,12 +137,11 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
   d.F[0] = reinterpret_cast<double2*>(const_cast<double*>(src));
   d.F[1] = reinterpret_cast<double2*>(dst);
   d.der = const_cast<double*>(der);
-  d.derS = scratch;
+  d.derS = d.derL = scratch;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
   // der slab by slab; for the D0 matrix its slice alone, and after it the
   // factored table
-  const bool d0 = sys == hst::K_D0 || sys == hst::K_DY;
   const int slices = d0 ? 1 : 4, n = slices * 5 * hst::slab_rows(ny, P) * P, T = 256;
   if (n + (d0 ? hst::d0_table_doubles(ny) : 0) > 20 * (size_t)HST_NOALLOC_MAX_NY)
     return fail(msg, msg_len, HST_EARG, "ny = %d exceeds the static scratch", ny);

@@ -64,19 +64,19 @@ __device__ __forceinline__ Column column_of(const Geometry& g, const PhysScalars
 }
 
 template <int P>
-__device__ __forceinline__ void load_line(const double2* __restrict__ src, cxd* buf, const LineGeom& G, int s) {
+__device__ __forceinline__ void load_line(const double2* src, cxd* buf, const LineGeom& G, int s) {
 #pragma unroll 4
   for (int r = s; r < G.n; r += P) buf[G.at(r)] = src[r];
 }
 template <int P>
-__device__ __forceinline__ void store_line(double2* __restrict__ dst, const cxd* buf, const LineGeom& G, int s) {
+__device__ __forceinline__ void store_line(double2* dst, const cxd* buf, const LineGeom& G, int s) {
 #pragma unroll 4
   for (int r = s; r < G.n; r += P) dst[r] = buf[G.at(r)];
 }
 // the four ghost rows of a column (row 0 at dst) from its line (wrap_rows,
 // src/hst_mpi.f90:340-355)
 template <int P>
-__device__ __forceinline__ void store_ghosts(double2* __restrict__ dst, const cxd* buf, const LineGeom& G, cxd ph, int s) {
+__device__ __forceinline__ void store_ghosts(double2* dst, const cxd* buf, const LineGeom& G, cxd ph, int s) {
   for (int k = s; k < 4; k += P) {
     // k = 0: row ny (row 0 ph), 1: row ny+1 (row 1 ph), 2: row -1 (row ny-1 conj), 3: row -2
     const int srow = k < 2 ? k : G.n + 1 - k, drow = k < 2 ? G.n + k : 1 - k;
@@ -290,11 +290,11 @@ __global__ void __launch_bounds__(512, 1) k_dy_sums(SolveArgs a, double sx, doub
 template <int P>
 __global__ void __launch_bounds__(64) k_line_solve(Geometry g, PhysScalars ps, int sys, double lambda,
                                                    const double2* __restrict__ src, double2* __restrict__ dst, double sx,
-                                                   double sz, const double* __restrict__ derS) {
+                                                   double sz, const double* __restrict__ derL) {
   extern __shared__ __align__(16) double smem_d[];
   const LineGeom G = line_geom(g.ny, P);
   const int mM = slab_rows(g.ny, P), ny = g.ny;
-  const SlabDerT<false> DS = {derS, mM, P};
+  const SlabDerT<false> DS = {derL, mM, P};
   const int groups = blockDim.x / P, grp = threadIdx.x / P, s = threadIdx.x % P;
   const int col = blockIdx.x * groups + grp;
   if (col >= g.ncol) return;
@@ -384,6 +384,17 @@ int line_lanes(int ny, long columns) {
     }
   while (P > 4 && ny / P < 12 && columns >= 148L * 12 * (32 / (P / 2))) P >>= 1;
   return P;
+}
+
+// With the factors in shared memory (48 bytes a row beside the line's 16)
+// fewer warps fit an SM, and shorter slabs pay: as many lanes as leave eight
+// rows each (256 rows of 32896 columns: three solves 418 us with 32 lanes, 486
+// with 16).
+int line_lanes_shared(int ny) {
+  for (int mmin : {8, 4})
+    for (int c = 32; c >= 2; c >>= 1)
+      if (ny / c >= mmin) return c;
+  return 2;
 }
 
 size_t slab_der_doubles(int ny) { return (size_t)20 * (ny + 32); }
@@ -515,7 +526,7 @@ static cudaError_t launch_line_solve_t(const Geometry& g, const DeviceState& d, 
   if (per * groups > 200 * 1024) return cudaErrorInvalidValue;
   smem_limit(d, k_line_solve<P>, 200 * 1024);
   k_line_solve<P><<<(g.ncol + groups - 1) / groups, groups * P, per * groups, st>>>(g, ps, sys, lambda, d.F[src],
-                                                                                   d.F[dst], sx, sz, d.derS);
+                                                                                   d.F[dst], sx, sz, d.derL);
   return cudaGetLastError();
 }
 
@@ -556,7 +567,7 @@ cudaError_t launch_solve_half(const Geometry& g, const DeviceState& d, const Phy
 cudaError_t launch_line_solve(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int sys, double lambda,
                               int src, int dst, double sx, double sz, cudaStream_t st) {
 #define HST_CALL(P) launch_line_solve_t<P>(g, d, ps, sys, lambda, src, dst, sx, sz, st)
-  HST_LANES(g.P, HST_CALL);
+  HST_LANES(sys == K_D0 || sys == K_DY ? g.P : g.PL, HST_CALL);
 #undef HST_CALL
 }
 
