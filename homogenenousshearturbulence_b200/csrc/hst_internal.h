@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <unordered_set>
+#include <utility>
 #include <vector>
 
 #include "../../include/hst_gpu.h"
@@ -86,6 +87,27 @@ inline cudaError_t smem_limit(const DeviceState& d, K k, int bytes) {
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess && d.configured) d.configured->insert(key);
   return e;
+}
+
+// Launches kernel k so that it may start while its predecessor in the stream
+// still drains (programmatic dependent launch): its blocks take over SMs as they
+// fall free and read their tables, and wait (wait_predecessor, hst_dev.cuh)
+// before they touch anything that the substep's other kernels write or read.
+// Every kernel of a substep does, so that the wait orders a kernel after all
+// that come before it.
+template <typename... KA, typename... A>
+inline cudaError_t launch_after(void (*k)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, KA(std::forward<A>(args))...);
 }
 
 // Scalars of one substep of the column kernel.

@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
       }
     }
   };
+  wait_predecessor();
   if (lane == 0) issue(0);
   const ColConst cc = col_const(col, g, a.ps, sc, a.gdamp);
   const double al = cc.al, be = cc.be, kk = cc.kk, ni = cc.ni, gs = cc.gs;
@@ -172,10 +173,10 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
       if (!NONLIN) q[p] = QT{0, 0};
-      else if (r >= 0) q[p] = Qc[p * qs + r];
-      else q[p] = Qgc ? Qgc[p * qgs + r + 2] : Qc[p * qs + ny + r];
+      else if (r >= 0) q[p] = __ldcg(Qc + p * qs + r);
+      else q[p] = __ldcg(Qgc ? Qgc + p * qgs + r + 2 : Qc + p * qs + ny + r);
     }
-    fill(32 + lane, a.V1[cb + r], a.V2[cb + r], a.V3[cb + r], q[0], q[1], q[2], q[3], q[4], q[5], (r < 0 && !Qgc) ? -1 : 0);
+    fill(32 + lane, load_field(a.V1 + cb + r), load_field(a.V2 + cb + r), load_field(a.V3 + cb + r), q[0], q[1], q[2], q[3], q[4], q[5], (r < 0 && !Qgc) ? -1 : 0);
   }
   // the default-form shift factor exp(-i gsh y(r)) of row t 32 + lane on a
   // uniform grid: the factor of the tile's first row (lane t of tbase) times
@@ -331,8 +332,7 @@ static cudaError_t launch_rhs_t(const RhsArgs& a, const DeviceState& d, cudaStre
   const int blocks = (a.g.ncol * a.g.nmem + RT_WARPS - 1) / RT_WARPS;
   auto k = k_rhs_tiled<EXACT, NONLIN, QT>;
   smem_limit(d, k, (int)smem);
-  k<<<blocks, 32 * RT_WARPS, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k, dim3(blocks), 32 * RT_WARPS, smem, st, a);
 }
 
 cudaError_t launch_rhs_tiled(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,

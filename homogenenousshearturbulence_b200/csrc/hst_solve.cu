@@ -66,7 +66,7 @@ __device__ __forceinline__ Column column_of(const Geometry& g, const PhysScalars
 template <int P>
 __device__ __forceinline__ void load_line(const double2* src, cxd* buf, const LineGeom& G, int s) {
 #pragma unroll 4
-  for (int r = s; r < G.n; r += P) buf[G.at(r)] = src[r];
+  for (int r = s; r < G.n; r += P) buf[G.at(r)] = load_field(src + r);
 }
 template <int P>
 __device__ __forceinline__ void store_line(double2* dst, const cxd* buf, const LineGeom& G, int s) {
@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
   for (int i = threadIdx.x; i < ntab; i += blockDim.x) d0s[i] = a.d0tab[i];
   for (int i = threadIdx.x; i < nder; i += blockDim.x) der0s[i] = a.derS[i];
   if (SH) __syncthreads();
+  wait_predecessor();
   const int lineN = P * G.MS;
   cxd* const buf = reinterpret_cast<cxd*>(der0s + nder) + (size_t)grp * SHIFT_LINES * lineN;
   cxd* sb[SHIFT_LINES];
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
     for (int i = threadIdx.x; i < nder; i += blockDim.x) smem_d[i] = a.derS[i];
     __syncthreads();
   }
+  wait_predecessor();
   cxd* const buf = reinterpret_cast<cxd*>(smem_d + nder) + (size_t)grp * P * G.MS;
   cxd* const sb = buf + s * G.MS;
   const int m = G.rows(s);
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
       for (int r0 = s; r0 < ny; r0 += 8 * P) {
         cxd dvb[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) dvb[k] = r0 + k * P < ny ? v1[r0 + k * P] : mkc(0, 0);
+        for (int k = 0; k < 8; ++k) dvb[k] = r0 + k * P < ny ? load_field(v1 + r0 + k * P) : mkc(0, 0);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int r = r0 + k * P;
@@ -458,8 +460,7 @@ static cudaError_t launch_shift_t(const SolveArgs& a, const DeviceState& d, cuda
   const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
   auto k = sh ? k_shift<P, true> : k_shift<P, false>;
   smem_limit(d, k, 227 * 1024);
-  k<<<nb, 32 * W, tabs + W * SHIFT_LINES * line_bytes(g.ny, P) * (32 / P), st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k, dim3(nb), 32 * W, tabs + W * SHIFT_LINES * line_bytes(g.ny, P) * (32 / P), st, a);
 }
 
 template <int P>
@@ -504,8 +505,7 @@ static cudaError_t launch_half_t(const SolveArgs& a, const DeviceState& d, cudaS
   const size_t smem = tabs + W * line_bytes(g.ny, P) * (32 / P);
   auto k = sh ? k_solve_half<P, HALF, true> : k_solve_half<P, HALF, false>;
   smem_limit(d, k, 227 * 1024);
-  k<<<nb, 32 * W, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k, dim3(nb), 32 * W, smem, st, a);
 }
 
 template <int P>

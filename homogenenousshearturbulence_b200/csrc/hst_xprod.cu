@@ -192,11 +192,13 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
   if (tid == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
+    wait_predecessor();
     mbar_arrive_expect_tx(bar, 3u * (unsigned)(MP * sizeof(C) * nb * BX));
     for (int b = 0; b < nb; ++b)
       tma_load_4d(sh1 + b * 3 * BX * MP, &tmZ, 2 * yi0, b * BX, yt * g.nzd + kz, 3 * mem, bar);
   }
   sync();
+  wait_predecessor();
   if (!mbar_wait_bounded(bar, 0, X_WAIT_LIMIT)) {
     // record the failure and give the copy a second bounded wait before the
     // block (and its shared memory) goes away
@@ -482,8 +484,7 @@ static cudaError_t launch_x_t(const Geometry& g, const DeviceState& d, const Phy
   smem_limit(d, k_x<N, C>, (int)X::smem);
   const int nt = g.ny / (2 * X::RP);
   const dim3 grid((nt + X::G - 1) / X::G, g.nzd * g.nmem);
-  k_x<N, C><<<grid, X::T * X::G, X::smem, st>>>(g, tw + N, d.dyl, ps, want_cfl, d.cfl, d.tmZ, d.tmPp, d.err);
-  return cudaGetLastError();
+  return launch_after(k_x<N, C>, grid, X::T * X::G, X::smem, st, g, tw + N, d.dyl, ps, want_cfl, d.cfl, d.tmZ, d.tmPp, d.err);
 }
 
 cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, cudaStream_t st) {

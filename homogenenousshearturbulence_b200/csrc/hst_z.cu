@@ -177,9 +177,10 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TI, ZPlan<N, C>::MBI)
     if (k <= nz) iz = k;
     else if (k >= N - nz) iz = k - N;
     else return C{0, 0};
-    const double2 v = __ldg(V + (size_t)(iz + nz) * g.rows + l + (l >= 2 ? g.edge_gap : 0));
+    const double2 v = load_field(V + (size_t)(iz + nz) * g.rows + l + (l >= 2 ? g.edge_gap : 0));
     return C{(T)v.x, (T)v.y};
   };
+  wait_predecessor();
   z_stages<N, +1, ZPlan<N, C>::TI>(sh, tw, ld);
   const size_t zs = (size_t)g.nxB * TY;
   C* const o = Zo + ((((size_t)mem * 3 + c) * nyT + yt) * N) * zs + (size_t)ix * TY;
@@ -223,6 +224,7 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TF, ZPlan<N, C>::MBF)
     fence_mbar_init();
   }
   __syncthreads();
+  wait_predecessor();
   int t = next(blockIdx.x), tn = t;  // this tile, the next one to fetch
   if (threadIdx.x == 0)
     for (int b = 0; b < NBUF && tn < ntile; ++b) {
@@ -323,9 +325,8 @@ template <int N, typename C>
 static cudaError_t z_inv_t(const Geometry& g, const DeviceState& d, const C* tw, cudaStream_t st) {
   smem_limit(d, k_z_inv<N, C>, (int)ZShape<N, C>::tile);
   const dim3 grid(g.nxB, (g.ny + ZPlan<N, C>::TY - 1) / ZPlan<N, C>::TY, 3 * g.nmem);
-  k_z_inv<N, C><<<grid, ZPlan<N, C>::TI, ZShape<N, C>::tile, st>>>(g, d.F[0], d.F[1], d.F[2],
-                                                                  reinterpret_cast<C*>(d.Z), tw + N);
-  return cudaGetLastError();
+  return launch_after(k_z_inv<N, C>, grid, ZPlan<N, C>::TI, ZShape<N, C>::tile, st, g, d.F[0], d.F[1], d.F[2],
+                      reinterpret_cast<C*>(d.Z), tw + N);
 }
 template <int N, typename C>
 static cudaError_t z_fwd_t(const Geometry& g, const DeviceState& d, const C* tw, cudaStream_t st) {
@@ -334,8 +335,8 @@ static cudaError_t z_fwd_t(const Geometry& g, const DeviceState& d, const C* tw,
   smem_limit(d, k_z_fwd<N, C>, (int)z_fwd_smem<N, C>());
   const int ntile = (g.ny + P::TY - 1) / P::TY * ((g.nxB + 3) / 4 * 4) * 6 * g.nmem;
   const int nb = std::min(ntile, (d.nsm > 0 ? d.nsm : 148) * P::MBF);
-  k_z_fwd<N, C><<<nb, P::TF, z_fwd_smem<N, C>(), st>>>(g, reinterpret_cast<C*>(d.Q), tw + N, d.tmPz, d.err);
-  return cudaGetLastError();
+  return launch_after(k_z_fwd<N, C>, dim3(nb), P::TF, z_fwd_smem<N, C>(), st, g, reinterpret_cast<C*>(d.Q), tw + N, d.tmPz,
+                      d.err);
 }
 
 #define HST_Z_DISPATCH(F)                                    \
