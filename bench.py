@@ -66,30 +66,28 @@ def peaks():
     return 6650.0, "fallback"
 
 
-def alg_bytes(deck, nxd, nzd, split, mixed=False, shift_split=False):
+def alg_bytes(deck, nxd, nzd, mixed=False):
     """Compulsory HBM bytes per launch of each kernel and per substep.
     Ns = ny (2nz+1)(nx+1) spectral points per component, Nzx = ny nzd (nx+1).
-    With the column stage split, `rhs` streams V, Q, old in and old, rhs out
-    (15 Ns) and `column` reads rhs and writes V (5 Ns; 9 Ns with exact_shift,
-    which re-reads and rewrites old); fused, `column` moves 16 Ns.  The
-    substep figure is the four-pass model 16 (25 Ns + 18 Nzx).  Mixed
-    precision: Z, Pp and Q are 8-byte complex64, V, old and rhs stay 16-byte
-    complex128; the substep model becomes 16 13 Ns + 8 (12 Ns + 18 Nzx)."""
+    `rhs` streams V, the five products, old in and old, rhs out (14 Ns),
+    `shift` (exact_shift) rhs and old in and out (8 Ns), `column`, the two
+    passes of the solves, rhs in and V out (5 Ns).  The substep figure is the
+    four-pass model 16 (23 Ns + 16 Nzx).  Mixed precision: Z, Pp and Q are
+    8-byte complex64, V, old and rhs stay 16-byte complex128; the substep
+    model becomes 16 13 Ns + 8 (10 Ns + 16 Nzx)."""
     nx, ny, nz = deck["nx"], deck["ny"], deck["nz"]
     Ns = ny * (2 * nz + 1) * (nx + 1)
     Nzx = ny * nzd * (nx + 1)
     b, t = 16.0, (8.0 if mixed else 16.0)
     k = {
         "zinv": b * 3 * Ns + t * 3 * Nzx,
-        "xprod": t * (3 * Nzx + 6 * Nzx),
-        "zfwd": t * (6 * Nzx + 6 * Ns),
-        "rhs": b * 9 * Ns + t * 6 * Ns,
-        "column": b * ((9 if deck.get("exact_shift") and not shift_split else 5) * Ns if split else 10 * Ns)
-                  + (0 if split else t * 6 * Ns),
-        # the exact_shift shift as a kernel of its own: rhs and old in and out
+        "xprod": t * (3 * Nzx + 5 * Nzx),
+        "zfwd": t * (5 * Nzx + 5 * Ns),
+        "rhs": b * 9 * Ns + t * 5 * Ns,
+        "column": b * 5 * Ns,
         "shift": b * 8 * Ns,
     }
-    sub = b * 13 * Ns + t * (12 * Ns + 18 * Nzx)
+    sub = b * 13 * Ns + t * (10 * Ns + 16 * Nzx)
     return k, sub, Ns, Nzx
 
 
@@ -427,8 +425,7 @@ def roofline(deck, s, kt, mixed, sub_ms, config):
     """The top kernel's roofline (its algorithmic bytes per launch over its
     average launch time, against the measured HBM copy bandwidth) and the
     whole substep's (B_alg over the substep time)."""
-    per_kernel, b_sub, Ns, Nzx = alg_bytes(deck, s.nxd, s.nzd, kt.get("rhs", (0, 0))[1] > 0, mixed,
-                                           kt.get("shift", (0, 0))[1] > 0)
+    per_kernel, b_sub, Ns, Nzx = alg_bytes(deck, s.nxd, s.nzd, mixed)
     peak, peak_kind = peaks()
     top = max(kt, key=lambda k: kt[k][0])
     avg_ms = kt[top][0] / kt[top][1]

@@ -988,7 +988,7 @@ extern "C" int hst_gpu_compute_cfl(hst_ctx* ctx, double* cfl) {
   CK(cudaSetDevice(ctx->device));
   CK(cudaMemsetAsync(ctx->d.cfl, 0, sizeof(unsigned long long), ctx->stream));
   CK(timed(ctx, HST_KC_ZINV, [&] { return hst::launch_zinv(ctx->g, ctx->d, ctx->stream); }));
-  CK(timed(ctx, HST_KC_XPROD, [&] { return hst::launch_xprod(ctx->g, ctx->d, ctx->ps, 1, ctx->stream); }));
+  CK(timed(ctx, HST_KC_XPROD, [&] { return hst::launch_xprod(ctx->g, ctx->d, ctx->ps, 1, 5, ctx->stream); }));
   return read_cfl(ctx, cfl);
 }
 
@@ -1056,8 +1056,8 @@ extern "C" int hst_gpu_pressure(hst_ctx* ctx, double time, int dst) {
   double sx, sz;
   shear_shifts(ctx, time, &sx, &sz);
   CK(timed(ctx, HST_KC_ZINV, [&] { return hst::launch_zinv(g, ctx->d, ctx->stream); }));
-  CK(timed(ctx, HST_KC_XPROD, [&] { return hst::launch_xprod(g, ctx->d, ctx->ps, 0, ctx->stream); }));
-  CK(timed(ctx, HST_KC_ZFWD, [&] { return hst::launch_zfwd(g, ctx->d, ctx->stream); }));
+  CK(timed(ctx, HST_KC_XPROD, [&] { return hst::launch_xprod(g, ctx->d, ctx->ps, 0, 6, ctx->stream); }));
+  CK(timed(ctx, HST_KC_ZFWD, [&] { return hst::launch_zfwd(g, ctx->d, 6, ctx->stream); }));
   CK(hst::launch_pressure_rhs(g, ctx->d, ctx->ps, s2_of(ctx->p, time), sx, sz, ctx->stream));
   CK(timed(ctx, HST_KC_LINE_SOLVE, [&] {
     return hst::launch_line_solve(g, ctx->d, ctx->ps, hst::K_POISSON, 0.0, HST_RHS1, dst, sx, sz, ctx->stream);
@@ -1295,8 +1295,8 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
     if (!p.linear || i == 2) {
       if (i == 2) CK(cudaMemsetAsync(D.cfl, 0, sizeof(unsigned long long), ctx->stream));
       CK(timed(ctx, HST_KC_ZINV, [&] { return hst::launch_zinv(G, D, ctx->stream); }));
-      CK(timed(ctx, HST_KC_XPROD, [&] { return hst::launch_xprod(G, D, ctx->ps, i == 2, ctx->stream); }));
-      if (!p.linear) CK(timed(ctx, HST_KC_ZFWD, [&] { return hst::launch_zfwd(G, D, ctx->stream); }));
+      CK(timed(ctx, HST_KC_XPROD, [&] { return hst::launch_xprod(G, D, ctx->ps, i == 2, 5, ctx->stream); }));
+      if (!p.linear) CK(timed(ctx, HST_KC_ZFWD, [&] { return hst::launch_zfwd(G, D, 5, ctx->stream); }));
     }
     if (damp && damping_update(ctx, t)) {
       int rc = upload_gdamp(ctx);

@@ -125,13 +125,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
 // writes are visible (a launch_after kernel may start earlier)
 __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// a load of a field another kernel of the substep writes: an ordinary cached
-// load, which the wait orders, never one of read-only data
-__device__ __forceinline__ cxd load_field(const double2* p) {
-  cxd v;
-  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-  return v;
-}
+// a load of a field another kernel of the substep writes: an ordinary load,
+// which the wait orders, never one of read-only data (no __restrict__ on the
+// way to it)
+__device__ __forceinline__ cxd load_field(const double2* p) { return *p; }
 
 // line-solve kinds (src/hst_linsolve.f90:83)
 enum { K_D2V = 1, K_ETA = 2, K_POISSON = 3, K_D0 = 4, K_DY = 5 };

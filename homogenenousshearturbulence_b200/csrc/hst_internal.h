@@ -39,7 +39,7 @@ struct DeviceState {
   double2* F[7];        // V1 V2 V3 OLD1 OLD2 RHS1 RHS2, (iy fastest, ghost rows included)
   double2* Z;           // z-inverse of V: [3][nyT][nzd][nxB][Ty]
   double2* Pp;          // x-forward of the products: [6][nyT][nzd][nxB][Ty]
-  double2* Q;           // spectral products: [6][ncol][ny]
+  double2* Q;           // spectral products: [6][ncol][ny] (the first five in the substep)
   double* der;          // der(0:ny-1, 0:3, -2:2)
   double* derS;         // the same, slab-major for the line-solve groups (slab_major)
   double* derL;         // the same for groups of PL lanes
@@ -56,7 +56,8 @@ struct DeviceState {
   float2* twzf;
   unsigned long long* cfl;  // running max (bits of a non-negative double)
   int* err;                 // set by a kernel whose bounded wait ran out
-  CUtensorMap tmZ, tmPp, tmZg, tmPpg;  // TMA maps of Z, Pp and the ghost rows' buffers (make_x_maps)
+  // TMA maps of Z, Pp and the ghost rows' buffers (make_x_maps; the ...2 of two components at a time)
+  CUtensorMap tmZ, tmPp, tmPp2, tmZg, tmPpg, tmPpg2;
   CUtensorMap tmPz, tmPgz;             // of Pp and Ppg for the z-forward kernel (make_z_maps)
   // The products of the four ghost rows (-2, -1, ny, ny+1) transformed like
   // the interior ones (null when their shear-periodic images are exact):
@@ -128,8 +129,11 @@ struct PhysScalars {
 };
 
 cudaError_t launch_zinv(const Geometry& g, const DeviceState& d, cudaStream_t st);
-cudaError_t launch_xprod(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl, cudaStream_t st);
-cudaError_t launch_zfwd(const Geometry& g, const DeviceState& d, cudaStream_t st);
+// np = 5: the products uu - vv, ww - vv, uv, vw, uw that the right-hand sides
+// take, as the components 0..4 of Pp and Q; 6: uu, vv, ww, uv, vw, uw
+cudaError_t launch_xprod(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl, int np,
+                         cudaStream_t st);
+cudaError_t launch_zfwd(const Geometry& g, const DeviceState& d, int np, cudaStream_t st);
 // the right-hand sides streamed through shared memory (hst_rhs.cu)
 cudaError_t launch_rhs_tiled(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
                              int exact, int nonlin, cudaStream_t st);
@@ -200,7 +204,8 @@ bool edge_rows_needed(const Geometry& g, bool s2_active);
 // the x stage of the lengths with a compiled plan (hst_xprod.cu), the TMA maps
 // of Z and Pp that it uses, its twiddle tables (at most 2 N entries into out; their number, 0 without one)
 bool x_compiled(int N, bool fp32);
-cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, cudaStream_t st);
+cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, int np,
+                     cudaStream_t st);
 cudaError_t make_x_maps(const Geometry& g, DeviceState& d);
 // cuTensorMapEncodeTiled (null: the driver has none)
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -215,7 +220,7 @@ cudaError_t make_z_maps(const Geometry& g, DeviceState& d);
 int z_twiddles(int N, double2* out);
 int z_twiddles(int N, float2* out);
 cudaError_t launch_z_inv(const Geometry& g, const DeviceState& d, cudaStream_t st);
-cudaError_t launch_z_fwd(const Geometry& g, const DeviceState& d, cudaStream_t st);
+cudaError_t launch_z_fwd(const Geometry& g, const DeviceState& d, int np, cudaStream_t st);
 int x_twiddles(int N, double2* out);
 int x_twiddles(int N, float2* out);
 // a transform length of the mixed-precision form

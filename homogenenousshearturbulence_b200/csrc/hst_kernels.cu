@@ -54,7 +54,11 @@ __global__ void __launch_bounds__(128) k_rhs_rows(ColumnArgs a) {
 #pragma unroll 1
   for (int r = lane; r < ny; r += 32) {
     auto tv = [&](int c, int j) -> cxd { return (c == 0 ? V1c : (c == 1 ? V2c : V3c))[r + j - 2]; };
-    auto tq = [&](int p, int j) -> cxd {
+    // the components uu - vv, ww - vv, uv, vw, uw in the places of uu, ww, uv, vw,
+    // uw, with vv = 0: the right-hand sides depend on the differences alone
+    auto tq = [&](int pr, int j) -> cxd {
+      if (pr == 1) return mkc(0, 0);
+      const int p = pr > 0 ? pr - 1 : 0;
       return q_at(Qc + p * qs, a.Qg ? a.Qg + (((size_t)mem * 6 + p) * g.ncol + col) * 4 : nullptr, r + j - 2, ny, cc.ph_t);
     };
     const size_t ro = cb + r;

@@ -6,20 +6,22 @@
 //                phase shift (src/hst_equations.f90:245-257)
 //
 // One warp walks the rows of one Fourier column in tiles of 32.  The rows a
-// tile adds to the five-point window (of the three velocities, the six product
+// tile adds to the five-point window (of the three velocities, the five product
 // spectra and the two carried terms) arrive by TMA bulk copies; the tile
 // after it is in flight while this one computes.
 //
-// The six products enter the two right-hand sides through four
-// combinations of constants of the column, formed once a row before any
-// stencil is taken:
-//   rhs of d2v:  D1 A + (D2 + k^2 D0) B,  A = -alfa^2 uu + k^2 vv - beta^2 ww - 2 alfa beta uw,
+// The products enter the two right-hand sides through four combinations of
+// constants of the column, formed once a row before any stencil is taken:
+//   rhs of d2v:  D1 A + (D2 + k^2 D0) B,  A = -alfa^2 (uu - vv) - beta^2 (ww - vv) - 2 alfa beta uw,
 //                                         B = i (alfa uv + beta vw)
-//   rhs of eta:  D0 C + D1 D,             C = alfa beta (uu - ww) + (beta^2 - alfa^2) uw,
+//   rhs of eta:  D0 C + D1 D,             C = alfa beta ((uu - vv) - (ww - vv)) + (beta^2 - alfa^2) uw,
 //                                         D = i (alfa vw - beta uv)
 // and u, w through f = i (beta u - alfa w) (the mean column: f = (Re u, Re w), D =
 // -(Re uv, Re vw)), so that a row takes nine stencils instead of twenty-three.
-// What bounds it: at 768^2 x 512 the 16 B x 15 Ns that it must move.
+// What bounds it: at 768^2 x 512 the 14 Ns values of 16 B that it must move
+// (2.93 ms FP64, 5.1 TB/s; 3.67 with twenty-three stencils and six products.  2.35
+// in FP32, from 3.34); 384^2 x 256 0.536 -> 0.393 ms.  Any even ny takes this kernel:
+// the last tile is ragged (256 x 90 x 150 rows, stretched, 0.620 -> 0.155 ms).
 #include "hst_dev.cuh"
 #include "hst_internal.h"
 #include "hst_rhs.cuh"
@@ -47,14 +49,14 @@ constexpr int RT_WAIT_LIMIT = 1 << 22;
 #define RT_MINB 5
 #endif
 
-// shared memory of one warp: the raw rows of a tile (u, v, w, the six
+// shared memory of one warp: the raw rows of a tile (u, v, w, the five
 // products, the two carried terms), then the 36-row window of v, f, A, B, C, D
 // (with FP32 spectra: v and f in FP64, and all six in FP32)
 template <typename QT>
 struct RhsShape {
   static constexpr bool F32 = sizeof(QT) == 8;
   static constexpr int W = 36;
-  static constexpr size_t raw = 5 * 32 * sizeof(double2) + 6 * 32 * sizeof(QT);
+  static constexpr size_t raw = 5 * 32 * sizeof(double2) + 5 * 32 * sizeof(QT);
   static constexpr size_t win = (F32 ? 2 * W * sizeof(double2) : 0) + 6 * W * sizeof(QT);
   static constexpr size_t warp = raw + win;
 };
@@ -70,11 +72,11 @@ struct ComboConst {
   bool c00;
 };
 template <typename QT, typename R>
-__device__ __forceinline__ Combos<QT> combos(const ComboConst<R>& k, QT uu, QT vv, QT ww, QT uv, QT vw, QT uw) {
+__device__ __forceinline__ Combos<QT> combos(const ComboConst<R>& k, QT du, QT dw, QT uv, QT vw, QT uw) {
   Combos<QT> o;
-  o.A = QT{k.kk * vv.x - k.a2 * uu.x - k.b2 * ww.x - k.ab2 * uw.x, k.kk * vv.y - k.a2 * uu.y - k.b2 * ww.y - k.ab2 * uw.y};
+  o.A = QT{-(k.a2 * du.x + k.b2 * dw.x + k.ab2 * uw.x), -(k.a2 * du.y + k.b2 * dw.y + k.ab2 * uw.y)};
   o.B = QT{-(k.al * uv.y + k.be * vw.y), k.al * uv.x + k.be * vw.x};
-  o.C = QT{k.ab * (uu.x - ww.x) + k.bma * uw.x, k.ab * (uu.y - ww.y) + k.bma * uw.y};
+  o.C = QT{k.ab * (du.x - dw.x) + k.bma * uw.x, k.ab * (du.y - dw.y) + k.bma * uw.y};
   o.D = k.c00 ? QT{-uv.x, -vw.x} : QT{k.be * uv.y - k.al * vw.y, k.al * vw.x - k.be * uv.x};
   return o;
 }
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
   if (cgl >= g.ncol * g.nmem) return;
   const int mem = cgl / g.ncol, col = cgl - mem * g.ncol;
   double2* const raw = reinterpret_cast<double2*>(smt + warp * S::warp);  // u, v, w [32] each, old1, old2 [32]
-  QT* const rawq = reinterpret_cast<QT*>(raw + 5 * 32);                   // six products [32]
+  QT* const rawq = reinterpret_cast<QT*>(raw + 5 * 32);                   // five products [32]
   double2* const wv = reinterpret_cast<double2*>(smt + warp * S::warp + S::raw);  // v, f
   double2* const wf = wv + W;
   QT* const wq = reinterpret_cast<QT*>(wv) + (F32 ? 4 * W : 2 * W);  // A, B, C, D (then v, f in FP32)
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
   // window, and its carried terms
   auto issue = [&](int t) {
     const int r0 = t * 32, nr = min(32, ny - r0);
-    mbar_arrive_expect_tx(bar, (unsigned)nr * (5 * 16 + (NONLIN ? 6 * QE : 0)));
+    mbar_arrive_expect_tx(bar, (unsigned)nr * (5 * 16 + (NONLIN ? 5 * QE : 0)));
     const double2* const Vg[3] = {a.V1, a.V2, a.V3};
 #pragma unroll
     for (int c = 0; c < 3; ++c) bulk_g2s(raw + c * 32, Vg[c] + cb + r0 + 2, nr * 16, bar);
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
       // to the combinations), or the ghost rows' own spectra
       const int n1 = min(nr, ny - r0 - 2);
 #pragma unroll 1
-      for (int p = 0; p < 6; ++p) {
+      for (int p = 0; p < 5; ++p) {
         if (n1 > 0) bulk_g2s(rawq + p * 32, Qc + p * qs + r0 + 2, (unsigned)n1 * QE, bar);
         if (n1 < nr) bulk_g2s(rawq + p * 32 + n1, Qgc ? Qgc + p * qgs + 2 : Qc + p * qs, (unsigned)(nr - n1) * QE, bar);
       }
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
   const QT ph_q = QT{(R)cc.ph_t.x, (R)cc.ph_t.y};
   // row i of the window from the raw values of one row; s != 0: the row
   // lies beyond the box, its products times the wrap phase (s < 0: conjugate)
-  auto fill = [&](int i, cxd u, cxd v, cxd w, QT uu, QT vv, QT ww, QT uv, QT vw, QT uw, int s) {
+  auto fill = [&](int i, cxd u, cxd v, cxd w, QT du, QT dw, QT uv, QT vw, QT uw, int s) {
     const cxd f = cc.c00 ? mkc(u.x, w.x) : mkc(al * w.y - be * u.y, be * u.x - al * w.x);
     wv[i] = v;
     wf[i] = f;
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
       wv32[W + i] = make_float2((float)f.x, (float)f.y);
     }
     if (NONLIN) {
-      Combos<QT> k = combos<QT, R>(kc, uu, vv, ww, uv, vw, uw);
+      Combos<QT> k = combos<QT, R>(kc, du, dw, uv, vw, uw);
       if (s != 0) {
         const QT e = s < 0 ? cconj(ph_q) : ph_q;
         k.A = cmul(k.A, e);
@@ -169,14 +171,15 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
   // rows -2 .. 1 into the window's last four rows, whence each tile moves them
   if (lane < 4) {
     const int r = lane - 2;
-    QT q[6];
+    QT q[5];
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
+    for (int p = 0; p < 5; ++p) {
       if (!NONLIN) q[p] = QT{0, 0};
       else if (r >= 0) q[p] = __ldcg(Qc + p * qs + r);
       else q[p] = __ldcg(Qgc ? Qgc + p * qgs + r + 2 : Qc + p * qs + ny + r);
     }
-    fill(32 + lane, load_field(a.V1 + cb + r), load_field(a.V2 + cb + r), load_field(a.V3 + cb + r), q[0], q[1], q[2], q[3], q[4], q[5], (r < 0 && !Qgc) ? -1 : 0);
+    fill(32 + lane, load_field(a.V1 + cb + r), load_field(a.V2 + cb + r), load_field(a.V3 + cb + r), q[0], q[1], q[2], q[3], q[4],
+         (r < 0 && !Qgc) ? -1 : 0);
   }
   // the default-form shift factor exp(-i gsh y(r)) of row t 32 + lane on a
   // uniform grid: the factor of the tile's first row (lane t of tbase) times
@@ -215,7 +218,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS, RT_MINB) k_rhs_tiled(RhsArgs a)
       o1in = raw[3 * 32 + lane];
       o2in = raw[4 * 32 + lane];
       fill(4 + lane, raw[lane], raw[32 + lane], raw[64 + lane], rawq[lane], rawq[32 + lane], rawq[64 + lane],
-           rawq[96 + lane], rawq[128 + lane], rawq[160 + lane], (r0 + 2 + lane >= ny && !Qgc) ? 1 : 0);
+           rawq[96 + lane], rawq[128 + lane], (r0 + 2 + lane >= ny && !Qgc) ? 1 : 0);
     }
     __syncwarp();
     if (lane == 0 && t + 1 < ntile) {

@@ -19,6 +19,15 @@
 // solves go to a slice of global scratch a group, rewritten column after
 // column (so that it stays in L2): without them in shared memory sixteen
 // warps' lines fit an SM.
+//
+// What bounds them: the dependent operations of a row's elimination and the
+// shared-memory pipe (512 rows: 73 % busy in k_shift, 50-60 % in the halves,
+// DRAM a third), so a line is cut into uneven slabs without padding rows, the
+// factors are kept with unit diagonals (a multiplication less a row each
+// way) and the D0 stencil and node phase are taken inside the back
+// substitution: 768^2 x 512 halves 3.57 -> 3.11 ms, shift 3.17 -> 2.72; 384^2 x 256
+// 0.535 -> 0.381; sizes without the persistent form before: 1536 rows 11.1 ->
+// 2.74, 90 rows 0.399 -> 0.132.
 #include <algorithm>
 
 #include "hst_internal.h"
@@ -63,10 +72,18 @@ __device__ __forceinline__ Column column_of(const Geometry& g, const PhysScalars
   return c;
 }
 
+// (eight loads issued before the first use: the stores to shared memory may
+// alias them for all the compiler knows)
 template <int P>
 __device__ __forceinline__ void load_line(const double2* src, cxd* buf, const LineGeom& G, int s) {
-#pragma unroll 4
-  for (int r = s; r < G.n; r += P) buf[G.at(r)] = load_field(src + r);
+  for (int r0 = s; r0 < G.n; r0 += 8 * P) {
+    cxd v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = r0 + k * P < G.n ? load_field(src + r0 + k * P) : mkc(0, 0);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (r0 + k * P < G.n) buf[G.at(r0 + k * P)] = v[k];
+  }
 }
 template <int P>
 __device__ __forceinline__ void store_line(double2* dst, const cxd* buf, const LineGeom& G, int s) {

@@ -88,9 +88,10 @@ struct ZfwdDst {
 
 template <int PPT>
 __global__ void __launch_bounds__(256)
-    k_zfwd(Geometry g, const double2* __restrict__ Pp, double2* __restrict__ Q, const double2* __restrict__ twz) {
+    k_zfwd(Geometry g, int np, const double2* __restrict__ Pp, double2* __restrict__ Q,
+           const double2* __restrict__ twz) {
   extern __shared__ double2 sh[];
-  const int yt = blockIdx.x, ix = blockIdx.y, pm = blockIdx.z;
+  const int yt = blockIdx.x, ix = blockIdx.y, pm = blockIdx.z / np * 6 + blockIdx.z % np;
   const int Ty = g.Ty, NZ = g.nzd;
   const TileSrc src = {Pp + (((size_t)pm * g.nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
   const ZfwdDst dst = {Q + ((size_t)pm * g.ncol + (size_t)ix * g.nzT) * g.ny + yt * Ty, g.ny, g.nz, NZ};
@@ -130,16 +131,23 @@ struct XinvSrc {
     return C{a.x + b.y, b.x - a.y};  // conj(a) + i conj(b)
   }
 };
-// the products of row yy, pair pl (0: uu, vv; 1: ww, uv; 2: vw, uw) at x
+// the products of row yy, pair pl (0: uu, vv; 1: ww, uv; 2: vw, uw; of five
+// products 0: uu - vv, ww - vv; 1: uv, vw; 2: uw, 0) at x
 template <typename LT, typename C>
 struct ProdSrc {
   typedef typename RealOf<C>::T T;
   LT L;
   T f;
+  bool five;
   __device__ __forceinline__ C operator()(int l, int x) const {
     const int yy = l >= 3 ? 1 : 0, pl = l - 3 * yy;
     const C a = L(yy, x), b = L(2, x);
     const T u = a.x, v = a.y, w = yy ? b.y : b.x;
+    if (five) {
+      if (pl == 0) return C{(u * u - v * v) * f, (w * w - v * v) * f};
+      if (pl == 1) return C{u * v * f, v * w * f};
+      return C{u * w * f, T(0)};
+    }
     if (pl == 0) return C{u * u * f, v * v * f};
     if (pl == 1) return C{w * w * f, u * v * f};
     return C{v * w * f, u * w * f};
@@ -150,7 +158,7 @@ struct ProdSrc {
 // with the runtime plan (PPT points a thread)
 template <int PPT>
 __global__ void __launch_bounds__(320)
-    k_xprod(Geometry g, const double2* __restrict__ Z, double2* __restrict__ Pp, const double2* __restrict__ twx,
+    k_xprod(Geometry g, int np, const double2* __restrict__ Z, double2* __restrict__ Pp, const double2* __restrict__ twx,
             const double* __restrict__ dyl, PhysScalars ps, int want_cfl, unsigned long long* __restrict__ cflmax) {
   typedef double2 C;
   extern __shared__ double2 sh[];
@@ -184,7 +192,7 @@ __global__ void __launch_bounds__(320)
     if ((threadIdx.x & 31) == 0) atomicMax(cflmax, (unsigned long long)__double_as_longlong(cm));
   }
   // the six product lines, transformed forward in place
-  const ProdSrc<LT, C> ps6 = {L, ps.factor};
+  const ProdSrc<LT, C> ps6 = {L, ps.factor, np == 5};
   fft_global<-1, PPT, true, true>(NX, 6, twx, sh, ps6, L);
   __syncthreads();
   // separate the two real transforms of each line, keep kx = 0..nx
@@ -294,6 +302,7 @@ static void edge_view(const Geometry& g, const DeviceState& d, Geometry& ge, Dev
   de.Q = d.Qg;
   de.tmZ = d.tmZg;
   de.tmPp = d.tmPpg;
+  de.tmPp2 = d.tmPpg2;
   de.tmPz = d.tmPgz;
 }
 
@@ -326,34 +335,34 @@ static cudaError_t launch_zinv_main(const Geometry& g, const DeviceState& d, cud
   return cudaGetLastError();
 }
 
-static cudaError_t launch_zfwd_main(const Geometry& g, const DeviceState& d, cudaStream_t st) {
-  if (z_rows(g.nzd, g.mp != 0)) return launch_z_fwd(g, d, st);
+static cudaError_t launch_zfwd_main(const Geometry& g, const DeviceState& d, int np, cudaStream_t st) {
+  if (z_rows(g.nzd, g.mp != 0)) return launch_z_fwd(g, d, np, st);
   const int pts = g.nzd * g.Ty;
-  const dim3 grid(g.nyT, g.nxB, 6 * g.nmem);
+  const dim3 grid(g.nyT, g.nxB, np * g.nmem);
   const size_t smem = (size_t)g.Ty * (g.nzd + 1) * sizeof(double2);
   if (pts <= 16 * 256) {
     big_smem(d, k_zfwd<16>);
-    k_zfwd<16><<<grid, fft_threads(pts, 16), smem, st>>>(g, d.Pp, d.Q, d.twz);
+    k_zfwd<16><<<grid, fft_threads(pts, 16), smem, st>>>(g, np, d.Pp, d.Q, d.twz);
   } else {
     big_smem(d, k_zfwd<32>);
-    k_zfwd<32><<<grid, fft_threads(pts, 32), smem, st>>>(g, d.Pp, d.Q, d.twz);
+    k_zfwd<32><<<grid, fft_threads(pts, 32), smem, st>>>(g, np, d.Pp, d.Q, d.twz);
   }
   return cudaGetLastError();
 }
 
-static cudaError_t launch_xprod_main(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl,
+static cudaError_t launch_xprod_main(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl, int np,
                                      cudaStream_t st) {
   const int NX = 2 * g.nxd;
-  if (x_compiled(NX, g.mp != 0)) return launch_x(g, d, ph, want_cfl, st);
+  if (x_compiled(NX, g.mp != 0)) return launch_x(g, d, ph, want_cfl, np, st);
   if (g.mp) return cudaErrorInvalidValue;
   const dim3 grid(g.ny / 2, g.nzd * g.nmem);
   const size_t smem = (size_t)6 * (NX + 1) * sizeof(double2);
   if (6 * NX <= 16 * 256) {
     big_smem(d, k_xprod<16>);
-    k_xprod<16><<<grid, fft_threads(6 * NX, 16), smem, st>>>(g, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
+    k_xprod<16><<<grid, fft_threads(6 * NX, 16), smem, st>>>(g, np, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
   } else {
     big_smem(d, k_xprod<32>);
-    k_xprod<32><<<grid, fft_threads(6 * NX, 32), smem, st>>>(g, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
+    k_xprod<32><<<grid, fft_threads(6 * NX, 32), smem, st>>>(g, np, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
   }
   return cudaGetLastError();
 }
@@ -368,22 +377,22 @@ cudaError_t launch_zinv(const Geometry& g, const DeviceState& d, cudaStream_t st
   edge_view(g, d, ge, de);
   return launch_zinv_main(ge, de, st);
 }
-cudaError_t launch_xprod(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl,
+cudaError_t launch_xprod(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int want_cfl, int np,
                          cudaStream_t st) {
-  cudaError_t e = launch_xprod_main(g, d, ph, want_cfl, st);
+  cudaError_t e = launch_xprod_main(g, d, ph, want_cfl, np, st);
   if (e != cudaSuccess || !d.Qg) return e;
   Geometry ge;
   DeviceState de;
   edge_view(g, d, ge, de);
-  return launch_xprod_main(ge, de, ph, 0, st);
+  return launch_xprod_main(ge, de, ph, 0, np, st);
 }
-cudaError_t launch_zfwd(const Geometry& g, const DeviceState& d, cudaStream_t st) {
-  cudaError_t e = launch_zfwd_main(g, d, st);
+cudaError_t launch_zfwd(const Geometry& g, const DeviceState& d, int np, cudaStream_t st) {
+  cudaError_t e = launch_zfwd_main(g, d, np, st);
   if (e != cudaSuccess || !d.Qg) return e;
   Geometry ge;
   DeviceState de;
   edge_view(g, d, ge, de);
-  return launch_zfwd_main(ge, de, st);
+  return launch_zfwd_main(ge, de, np, st);
 }
 
 }  // namespace hst

@@ -1,16 +1,21 @@
 // The x stage of the hst substep for the compiled transform lengths:
 //
-//   k_x   Z -> x-inverse (c2r) of u, v, w; the six products times
-//         1/(2 nxd nzd); the CFL maximum; x-forward (r2c) of the products
-//         truncated to the nx+1 retained modes (Pp)
+//   k_x   Z -> x-inverse (c2r) of u, v, w; the products times 1/(2 nxd nzd);
+//         the CFL maximum; x-forward (r2c) of the products truncated to the
+//         nx+1 retained modes (Pp)
+//
+// The right-hand sides of the v-eta form depend on uu, vv and ww through uu - vv
+// and ww - vv alone (k^2 vv = alfa^2 vv + beta^2 vv), so the substep takes five
+// products, uu - vv, ww - vv, uv, vw, uw (NP = 5); the pressure needs all six,
+// uu, vv, ww, uv, vw, uw (NP = 6).
 //
 // (to_x_points with zero padding and RFT, build_products for both groups,
 // compute_cfl and HFT: src/hst_transforms.f90:85-133, 163-179,
 // src/hst_fft.f90:211-237).  Other lengths run k_xprod (hst_transforms.cu).
 //
 // One tile is two rows y0, y0 + 1 at one z point.  Two real lines ride on one
-// complex line, the two rows of one component: three lines in (u, v, w), six
-// out (one a product), separated by Hermitian symmetry.  N = R0 R1 R2 splits
+// complex line, the two rows of one component: three lines in (u, v, w), five
+// or six out (one a product), separated by Hermitian symmetry.  N = R0 R1 R2 splits
 // the transform into three register stages with two exchanges each way, and
 // what bounds the kernel is the shared-memory traffic of those exchanges and
 // the FP64 arithmetic, so the split is chosen to keep both small:
@@ -22,17 +27,25 @@
 //   - the last inverse stage, the products and the first forward stage are one
 //     pass: the x points v + (N/R2) r that a radix-R2 butterfly of each of
 //     the three lines leaves in a thread's registers are the inputs of the
-//     first forward radix-R2 butterfly of each of the six products;
+//     first forward radix-R2 butterfly of each product;
 //   - the stages run in place (decimation in frequency on the way in, in time
 //     on the way out), so that one barrier separates two stages, and the
-//     middle twiddles are loaded once for the nine lines.
+//     last inverse and first forward twiddles are loaded once for all lines.
 // Line layout: element (p0, j), p0 < R0, j < N/R0, at p0 S0 + j with S0 odd;
 // lanes run over p0 first in the two inner stages, over j in the outer ones,
 // which keeps 16-byte accesses (R0 = 8) and 8-byte accesses (R0 = 16) free of
 // bank conflicts.  The tile comes in and goes out by tensor copies of 32
 // bytes a mode (two rows in FP64, four in FP32 up to 768 points): lane-wise
 // loads and stores of the same 32 bytes at the 64-byte stride of the
-// [ix][Ty] layout took 75 of the kernel's 185 million L1 wavefronts.
+// [ix][Ty] layout took 75 of the kernel's 185 million L1 wavefronts and 848
+// against 668 us at 768 points.
+// Measured a substep, against a Stockham kernel of four exchanges each way and
+// staged lines (k_xprod's form), B200: 768^2 x 512 FP64 9.70 -> 4.86 ms, FP32
+// 7.26 -> 2.38; 384^2 x 256 FP64 1.10 -> 0.556 ms, FP32 0.79 -> 0.307; 1536^2 x 128
+// FP32 9.40 -> 3.11; 512 points (384 z points, 256 rows) 2.40 -> 0.387.  In FP64
+// at 768 points (six products) the L1 pipe is 74 % and the FP64 pipe 51 %
+// busy, in FP32 65 % with issue at 73 %: both near what one tile's exchanges
+// and butterflies allow, HBM at 40 %.
 #include "hst_dev.cuh"
 #include "hst_fft.cuh"
 #include "hst_internal.h"
@@ -157,11 +170,11 @@ __device__ __forceinline__ void tile_store(float2* p, bool, float2 a, float2 b) 
   *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
 }
 
-template <int N, typename C>
+template <int N, int NP, typename C>
 __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::MINB)
     k_x(Geometry g, const C* __restrict__ tw, const double* __restrict__ dyl, PhysScalars ps, int want_cfl,
         unsigned long long* __restrict__ cflmax, const __grid_constant__ CUtensorMap tmZ,
-        const __grid_constant__ CUtensorMap tmP, int* __restrict__ err) {
+        const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmP2, int* __restrict__ err) {
   typedef XShape<N, C> X;
   typedef typename RealOf<C>::T T;
   constexpr int R0 = X::R0, R1 = X::R1, R2 = X::R2, M = X::M, H = X::H, S0 = X::S0, LS = X::LS, RH = X::RH;
@@ -170,8 +183,8 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
   extern __shared__ __align__(128) double2 sh_d[];
   const int warp_tile = X::G > 1 ? threadIdx.x / TT : 0;
   const int tid = X::G > 1 ? threadIdx.x % TT : threadIdx.x;
-  // the lines of u, v, w (later uu, vv, ww), then those of uv, vw, uw; the
-  // tile comes in over the second half
+  // the lines of u, v, w (later the first three products), then those of the
+  // other products; the tile comes in over the second half
   C* const sh = reinterpret_cast<C*>(sh_d) + (size_t)warp_tile * 2 * HALF;
   C* const sh1 = sh + HALF;
   uint64_t* const bar = reinterpret_cast<uint64_t*>(reinterpret_cast<C*>(sh_d) + (size_t)X::G * 2 * HALF) + 2 * warp_tile;
@@ -206,11 +219,11 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
     mbar_wait_bounded(bar, 0, X_WAIT_LIMIT);
     return;
   }
-  // mode m of component c (of three) in a staging tile
-  auto slot = [&](int c, int m) -> int {
+  // mode m of component c (of nc) in a staging tile
+  auto slot = [&](int c, int m, int nc) -> int {
     if (NB == 1) return (c * BX + m) * MP;
     const int b = m >= BX ? 1 : 0;
-    return ((b * 3 + c) * BX + m - b * BX) * MP;
+    return ((b * nc + c) * BX + m - b * BX) * MP;
   };
   const bool rev = (threadIdx.x >> 2) & 1;
 
@@ -230,13 +243,13 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
         const int mA = j + r * M, mB = jB + r * M;
         C a, b;
         if (mA <= nx) {
-          tile_load(sh1 + slot(c, mA) + 2 * sub, rev, a, b);
+          tile_load(sh1 + slot(c, mA, 3) + 2 * sub, rev, a, b);
           A[r] = C{a.x - b.y, a.y + b.x};
           nA[r] = C{a.x + b.y, b.x - a.y};
           if (r == 0 && j == 0) A[r] = C{a.x, b.x};  // the c2r ignores the mean's imaginary part
         }
         if (mB <= nx) {
-          tile_load(sh1 + slot(c, mB) + 2 * sub, rev, a, b);
+          tile_load(sh1 + slot(c, mB, 3) + 2 * sub, rev, a, b);
           B[r] = C{a.x - b.y, a.y + b.x};
           nB[r] = C{a.x + b.y, b.x - a.y};
         }
@@ -303,12 +316,23 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
       }
     }
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      constexpr int ia[6] = {0, 1, 2, 0, 1, 0}, ib[6] = {0, 1, 2, 1, 2, 2};
+    for (int q = 0; q < NP; ++q) {
+      // NP = 6: uu, vv, ww, uv, vw, uw; NP = 5: uu - vv, ww - vv, uv, vw, uw
+      constexpr int ia[2][6] = {{0, 1, 2, 0, 1, 0}, {0, 2, 0, 1, 0, 0}}, ib[2][6] = {{0, 1, 2, 1, 2, 2}, {0, 2, 1, 2, 2, 0}};
+      const int i = ia[6 - NP][q], j = ib[6 - NP][q];
       C P[R2];
 #pragma unroll
-      for (int r = 0; r < R2; ++r)
-        P[r] = C{U[ia[q]][r].x * (U[ib[q]][r].x * f), U[ia[q]][r].y * (U[ib[q]][r].y * f)};
+      for (int r = 0; r < R2; ++r) {
+        // a difference of squares: in FP64 as one product, which leaves no spills
+        // (601 against 687 us for 768 points, 384 z points and 128 rows); in FP32
+        // as two (307 against 314 us for 384 points, 192 z points and 256 rows)
+        if (NP == 5 && q < 2 && sizeof(T) == 8)
+          P[r] = C{(U[i][r].x - U[1][r].x) * ((U[i][r].x + U[1][r].x) * f), (U[i][r].y - U[1][r].y) * ((U[i][r].y + U[1][r].y) * f)};
+        else
+          P[r] = C{U[i][r].x * (U[j][r].x * f), U[i][r].y * (U[j][r].y * f)};
+        if (NP == 5 && q < 2 && sizeof(T) == 4)
+          P[r] = C{P[r].x - U[1][r].x * (U[1][r].x * f), P[r].y - U[1][r].y * (U[1][r].y * f)};
+      }
       DFT<R2, -1>::run(P);
       C* const o = s + (q >= 3 ? HALF + (q - 3) * LS : q * LS);
       o[0] = P[0];
@@ -327,10 +351,9 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
   // middle forward stage
   if constexpr (R1 > 1) {
 #pragma unroll 1
-    for (int u = tid; u < RP * 6 * NU; u += TT) {
+    for (int u = tid; u < RP * NP * NU; u += TT) {
       const int l = u / NU, v = u - l * NU;
-      const int hf = l / (3 * RP), lh = l - hf * 3 * RP;
-      const int sub = RP > 1 ? lh / 3 : 0, c = lh - 3 * sub;
+      const int sub = RP > 1 ? l / NP : 0, q = l - NP * sub, hf = q >= 3 ? 1 : 0, c = q - 3 * hf;
       C* const s = sh + hf * HALF + sub * SP + c * LS + (v % R0) * S0 + v / R0;
       C x[R1];
 #pragma unroll
@@ -347,7 +370,7 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
 #pragma unroll 1
   for (int hf = 0; hf < 2; ++hf) {
     int sub, c, j;
-    const bool on = outer_unit<X>(tid, sub, c, j);
+    const bool on = outer_unit<X>(tid, sub, c, j) && (hf == 0 || c < NP - 3);
     const int jB = j ? M - j : H;
     C A[R0], B[R0];
     C* const half = sh + hf * HALF;
@@ -375,10 +398,10 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
         const int kA = j + r * M, kB = jB + r * M;
         const C mA = j ? B[R0 - 1 - r] : A[(R0 - r) % R0], mB = j ? A[R0 - 1 - r] : B[R0 - 1 - r];
         if (kA <= nx)
-          tile_store(half + slot(c, kA) + 2 * sub, rev, C{h * (A[r].x + mA.x), h * (A[r].y - mA.y)},
+          tile_store(half + slot(c, kA, hf ? NP - 3 : 3) + 2 * sub, rev, C{h * (A[r].x + mA.x), h * (A[r].y - mA.y)},
                      C{h * (A[r].y + mA.y), h * (mA.x - A[r].x)});
         if (kB <= nx)
-          tile_store(half + slot(c, kB) + 2 * sub, rev, C{h * (B[r].x + mB.x), h * (B[r].y - mB.y)},
+          tile_store(half + slot(c, kB, hf ? NP - 3 : 3) + 2 * sub, rev, C{h * (B[r].x + mB.x), h * (B[r].y - mB.y)},
                      C{h * (B[r].y + mB.y), h * (mB.x - B[r].x)});
       }
     }
@@ -387,7 +410,7 @@ __global__ void __launch_bounds__(XPlan<N, C>::T* XPlan<N, C>::G, XPlan<N, C>::M
   sync();
   if (tid == 0) {
     for (int b = 0; b < nb; ++b)
-      tma_store_4d(&tmP, 2 * yi0, b * BX, yt * g.nzd + kz, 6 * mem + 3, sh1 + b * 3 * BX * MP);
+      tma_store_4d(NP == 6 ? &tmP : &tmP2, 2 * yi0, b * BX, yt * g.nzd + kz, 6 * mem + 3, sh1 + b * (NP - 3) * BX * MP);
     bulk_commit();
     bulk_wait_read_all();
   }
@@ -438,7 +461,8 @@ int x_twiddles(int N, float2* out) {
 // ------------------------------------------------------------- TMA maps ----
 // Z and Pp seen as 4-D real tensors: d0 = the 2 Ty reals of one y tile
 // (innermost), d1 = ix, d2 = (y tile, kz) as yt nzd + kz, d3 = component.
-// The box is {the rows of a tile, modes, 1, three components}.
+// The box is {the rows of a tile, modes, 1, three components (two: the second
+// half of five products)}.
 EncodeTiled encode_tiled() {
   static const EncodeTiled enc = [] {
     void* fn = nullptr;
@@ -449,12 +473,12 @@ EncodeTiled encode_tiled() {
   return enc;
 }
 
-static cudaError_t encode_map(EncodeTiled enc, const Geometry& g, void* base, int comps, int Ty, int nyT, int rp,
-                              CUtensorMap* map) {
+static cudaError_t encode_map(EncodeTiled enc, const Geometry& g, void* base, int comps, int box_comps, int Ty, int nyT,
+                              int rp, CUtensorMap* map) {
   const cuuint64_t es = g.mp ? 8 : 16;  // bytes of one complex element
   cuuint64_t dims[4] = {(cuuint64_t)2 * Ty, (cuuint64_t)g.nxB, (cuuint64_t)g.nzd * nyT, (cuuint64_t)comps * g.nmem};
   cuuint64_t strides[3] = {es * Ty, es * Ty * g.nxB, es * Ty * g.nxB * g.nzd * nyT};
-  cuuint32_t box[4] = {(cuuint32_t)(4 * rp), (cuuint32_t)x_box(g.nxB), 1, 3};
+  cuuint32_t box[4] = {(cuuint32_t)(4 * rp), (cuuint32_t)x_box(g.nxB), 1, (cuuint32_t)box_comps};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(map, g.mp ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, base, dims,
                          strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -467,31 +491,36 @@ cudaError_t make_x_maps(const Geometry& g, DeviceState& d) {
   const EncodeTiled enc = encode_tiled();
   if (!enc) return cudaErrorNotSupported;
   const int rp = x_row_pairs(2 * g.nxd, g.mp != 0);
-  cudaError_t e = encode_map(enc, g, d.Z, 3, g.Ty, g.nyT, rp, &d.tmZ);
-  if (e == cudaSuccess) e = encode_map(enc, g, d.Pp, 6, g.Ty, g.nyT, rp, &d.tmPp);
+  cudaError_t e = encode_map(enc, g, d.Z, 3, 3, g.Ty, g.nyT, rp, &d.tmZ);
+  if (e == cudaSuccess) e = encode_map(enc, g, d.Pp, 6, 3, g.Ty, g.nyT, rp, &d.tmPp);
+  if (e == cudaSuccess) e = encode_map(enc, g, d.Pp, 6, 2, g.Ty, g.nyT, rp, &d.tmPp2);
   if (e == cudaSuccess && d.Zg) {  // the ghost rows' buffers: one tile
-    e = encode_map(enc, g, d.Zg, 3, g.EY, 1, rp, &d.tmZg);
-    if (e == cudaSuccess) e = encode_map(enc, g, d.Ppg, 6, g.EY, 1, rp, &d.tmPpg);
+    e = encode_map(enc, g, d.Zg, 3, 3, g.EY, 1, rp, &d.tmZg);
+    if (e == cudaSuccess) e = encode_map(enc, g, d.Ppg, 6, 3, g.EY, 1, rp, &d.tmPpg);
+    if (e == cudaSuccess) e = encode_map(enc, g, d.Ppg, 6, 2, g.EY, 1, rp, &d.tmPpg2);
   }
   return e;
 }
 
-template <int N, typename C>
+template <int N, int NP, typename C>
 static cudaError_t launch_x_t(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl,
                               const C* tw, cudaStream_t st) {
   typedef XShape<N, C> X;
   if (g.Ty % (2 * X::RP) != 0) return cudaErrorInvalidValue;
-  smem_limit(d, k_x<N, C>, (int)X::smem);
+  smem_limit(d, k_x<N, NP, C>, (int)X::smem);
   const int nt = g.ny / (2 * X::RP);
   const dim3 grid((nt + X::G - 1) / X::G, g.nzd * g.nmem);
-  return launch_after(k_x<N, C>, grid, X::T * X::G, X::smem, st, g, tw + N, d.dyl, ps, want_cfl, d.cfl, d.tmZ, d.tmPp, d.err);
+  return launch_after(k_x<N, NP, C>, grid, X::T * X::G, X::smem, st, g, tw + N, d.dyl, ps, want_cfl, d.cfl, d.tmZ, d.tmPp, d.tmPp2, d.err);
 }
 
-cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, cudaStream_t st) {
+cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars& ps, int want_cfl, int np,
+                     cudaStream_t st) {
   if (g.mp) {
     switch (2 * g.nxd) {
 #define HST_X(n) \
-  case n: return launch_x_t<n, float2>(g, d, ps, want_cfl, d.twxf, st);
+  case n:    \
+    return np == 5 ? launch_x_t<n, 5, float2>(g, d, ps, want_cfl, d.twxf, st)    \
+                   : launch_x_t<n, 6, float2>(g, d, ps, want_cfl, d.twxf, st);
       HST_X_LENGTHS32(HST_X)
 #undef HST_X
     }
@@ -499,7 +528,9 @@ cudaError_t launch_x(const Geometry& g, const DeviceState& d, const PhysScalars&
   }
   switch (2 * g.nxd) {
 #define HST_X(n) \
-  case n: return launch_x_t<n, double2>(g, d, ps, want_cfl, d.twx, st);
+  case n:    \
+    return np == 5 ? launch_x_t<n, 5, double2>(g, d, ps, want_cfl, d.twx, st)    \
+                   : launch_x_t<n, 6, double2>(g, d, ps, want_cfl, d.twx, st);
     HST_X_LENGTHS64(HST_X)
 #undef HST_X
   }

@@ -16,7 +16,12 @@
 //
 // The forward transform waits on its loads (64-byte runs 16 KB apart at
 // 768^2 x 512), so it runs on a persistent grid whose tiles land by tensor copies
-// in one of NBUF buffers while the previous tile is transformed.
+// in one of NBUF buffers while the previous tile is transformed: 4.66 -> 2.79
+// ms a substep at 768^2 x 512 FP64 (five products; 3.28 for six), 3.16 -> 1.57 FP32;
+// 0.490 -> 0.357 and 0.302 -> 0.217 ms at 384^2 x 256.  It reads and writes 80 %
+// of what a copy could in that time at 768 points.  The inverse one reads V's
+// short runs through the L1 (2.18 -> 2.10 ms at 768^2 x 512, 0.254 -> 0.232 at
+// 384^2 x 256) and is bound by them.
 #include <algorithm>
 
 #include "hst_dev.cuh"
@@ -152,22 +157,30 @@ __device__ __forceinline__ void z_last(const C* __restrict__ sh, const ST& st) {
 }
 
 // ------------------------------------------------------------- inverse ----
+// x modes that run side by side
+template <int N, typename C>
+__host__ __device__ __forceinline__ int z_inv_group(int nxB) {
+  return ZShape<N, C>::TY * (int)sizeof(C) < 64 ? 4 : nxB;
+}
 // V row of tile row i: row i of the field, or (edge view: gap = ny) rows -2,
 // -1, ny, ny + 1
 template <int N, typename C>
 __global__ void __launch_bounds__(ZPlan<N, C>::TI, ZPlan<N, C>::MBI)
-    k_z_inv(Geometry g, const double2* __restrict__ V0, const double2* __restrict__ V1, const double2* __restrict__ V2,
-            C* __restrict__ Zo, const C* __restrict__ tw) {
+    k_z_inv(Geometry g, const double2* V0, const double2* V1, const double2* V2, C* Zo, const C* __restrict__ tw) {
   typedef ZShape<N, C> Z;
   typedef typename RealOf<C>::T T;
   constexpr int TY = Z::TY;
   extern __shared__ __align__(128) double2 sh_d[];
   C* const sh = reinterpret_cast<C*>(sh_d);
   // the x modes of one y tile run side by side: consecutive blocks write
-  // adjacent runs of the [yt][kz][ix][Ty] tiles (four x modes, then the y tiles:
-  // 588 against 504 us for 64 x modes of 768 points and 512 rows)
-  const int ix = blockIdx.x, yt = blockIdx.y, c = blockIdx.z % 3, mem = blockIdx.z / 3;
-  const int nyT = (g.ny + TY - 1) / TY, nz = g.nz;
+  // adjacent runs of the [yt][kz][ix][Ty] tiles; where a run is half a 64-byte
+  // sector pair (1536 points in FP32), four x modes and then the y tiles, whose
+  // runs of V adjoin (2.07 against 2.45 ms at 1536^2 x 128; at 768 points in
+  // FP64 the other way round, 588 against 504 us for 64 x modes and 512 rows)
+  const int nyT = (g.ny + TY - 1) / TY, nz = g.nz, grp = z_inv_group<N, C>(g.nxB);
+  const int bg = blockIdx.x / grp, ix = bg / nyT * grp + blockIdx.x % grp, yt = bg % nyT;
+  const int c = blockIdx.y % 3, mem = blockIdx.y / 3;
+  if (ix >= g.nxB) return;
   const int y0 = yt * TY;
   const double2* const V = (c == 0 ? V0 : (c == 1 ? V1 : V2)) + (size_t)mem * g.nf + (size_t)ix * g.nzT * g.rows +
                            (g.edge_gap ? 0 : 2) + y0;
@@ -190,7 +203,7 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TI, ZPlan<N, C>::MBI)
 // ------------------------------------------------------------- forward ----
 template <int N, typename C>
 __global__ void __launch_bounds__(ZPlan<N, C>::TF, ZPlan<N, C>::MBF)
-    k_z_fwd(Geometry g, C* __restrict__ Q, const C* __restrict__ tw, const __grid_constant__ CUtensorMap tmP,
+    k_z_fwd(Geometry g, int np, C* __restrict__ Q, const C* __restrict__ tw, const __grid_constant__ CUtensorMap tmP,
             int* __restrict__ err) {
   typedef ZShape<N, C> Z;
   constexpr int TY = Z::TY, KB = Z::KB, NBUF = ZPlan<N, C>::NBUF;
@@ -198,15 +211,16 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TF, ZPlan<N, C>::MBF)
   C* const sh = reinterpret_cast<C*>(sh_d);
   uint64_t* const bar = reinterpret_cast<uint64_t*>(sh + (size_t)NBUF * N * TY);
   const int nyT = (g.ny + TY - 1) / TY, nz = g.nz, nxP = (g.nxB + 3) / 4 * 4;
-  const int ntile = nyT * nxP * 6 * g.nmem;
+  const int ntile = nyT * nxP * np * g.nmem;
   // tile t: four x modes of one y tile side by side (whole 256-byte runs of
   // Pp), then the y tiles, then the next four x modes
   struct Tile {
     int ix, yt, pm;
   };
   auto tile_of = [&](int t) -> Tile {
-    const int per = nyT * nxP, pm = t / per, e = t - pm * per, q = e >> 2;
-    return Tile{(q / nyT) * 4 + (e & 3), q % nyT, pm};
+    // pm: the product's component among the six of every member
+    const int per = nyT * nxP, k = t / per, e = t - k * per, q = e >> 2;
+    return Tile{(q / nyT) * 4 + (e & 3), q % nyT, k / np * 6 + k % np};
   };
   auto next = [&](int t) {  // the first tile from t on whose x mode exists
     while (t < ntile && tile_of(t).ix >= g.nxB) t += gridDim.x;
@@ -324,18 +338,19 @@ cudaError_t make_z_maps(const Geometry& g, DeviceState& d) {
 template <int N, typename C>
 static cudaError_t z_inv_t(const Geometry& g, const DeviceState& d, const C* tw, cudaStream_t st) {
   smem_limit(d, k_z_inv<N, C>, (int)ZShape<N, C>::tile);
-  const dim3 grid(g.nxB, (g.ny + ZPlan<N, C>::TY - 1) / ZPlan<N, C>::TY, 3 * g.nmem);
+  const int grp = z_inv_group<N, C>(g.nxB), nyT = (g.ny + ZPlan<N, C>::TY - 1) / ZPlan<N, C>::TY;
+  const dim3 grid((g.nxB + grp - 1) / grp * grp * nyT, 3 * g.nmem);
   return launch_after(k_z_inv<N, C>, grid, ZPlan<N, C>::TI, ZShape<N, C>::tile, st, g, d.F[0], d.F[1], d.F[2],
                       reinterpret_cast<C*>(d.Z), tw + N);
 }
 template <int N, typename C>
-static cudaError_t z_fwd_t(const Geometry& g, const DeviceState& d, const C* tw, cudaStream_t st) {
+static cudaError_t z_fwd_t(const Geometry& g, const DeviceState& d, int np, const C* tw, cudaStream_t st) {
   typedef ZPlan<N, C> P;
   static_assert(z_fwd_smem<N, C>() <= 227 * 1024, "the buffers fit one block");
   smem_limit(d, k_z_fwd<N, C>, (int)z_fwd_smem<N, C>());
-  const int ntile = (g.ny + P::TY - 1) / P::TY * ((g.nxB + 3) / 4 * 4) * 6 * g.nmem;
+  const int ntile = (g.ny + P::TY - 1) / P::TY * ((g.nxB + 3) / 4 * 4) * np * g.nmem;
   const int nb = std::min(ntile, (d.nsm > 0 ? d.nsm : 148) * P::MBF);
-  return launch_after(k_z_fwd<N, C>, dim3(nb), P::TF, z_fwd_smem<N, C>(), st, g, reinterpret_cast<C*>(d.Q), tw + N, d.tmPz,
+  return launch_after(k_z_fwd<N, C>, dim3(nb), P::TF, z_fwd_smem<N, C>(), st, g, np, reinterpret_cast<C*>(d.Q), tw + N, d.tmPz,
                       d.err);
 }
 
@@ -353,9 +368,9 @@ cudaError_t launch_z_inv(const Geometry& g, const DeviceState& d, cudaStream_t s
 #undef HST_Z32
 #undef HST_Z64
 }
-cudaError_t launch_z_fwd(const Geometry& g, const DeviceState& d, cudaStream_t st) {
-#define HST_Z32(n) case n: return z_fwd_t<n, float2>(g, d, d.twzf, st);
-#define HST_Z64(n) case n: return z_fwd_t<n, double2>(g, d, d.twz, st);
+cudaError_t launch_z_fwd(const Geometry& g, const DeviceState& d, int np, cudaStream_t st) {
+#define HST_Z32(n) case n: return z_fwd_t<n, float2>(g, d, np, d.twzf, st);
+#define HST_Z64(n) case n: return z_fwd_t<n, double2>(g, d, np, d.twz, st);
   HST_Z_DISPATCH();
 #undef HST_Z32
 #undef HST_Z64
