@@ -25,9 +25,9 @@
 // DRAM a third), so a line is cut into uneven slabs without padding rows, the
 // factors are kept with unit diagonals (a multiplication less a row each
 // way) and the D0 stencil and node phase are taken inside the back
-// substitution: 768^2 x 512 halves 3.57 -> 3.11 ms, shift 3.17 -> 2.72; 384^2 x 256
-// 0.535 -> 0.381; sizes without the persistent form before: 1536 rows 11.1 ->
-// 2.74, 90 rows 0.399 -> 0.132.
+// substitution: 768^2 x 512 halves 3.57 -> 3.15 ms, shift 3.17 -> 2.72; 384^2 x 256
+// 0.535 -> 0.371; 1536^2 x 128 (a generic form before) 11.1 -> 2.65,
+// 20300 columns of 150 rows 0.399 -> 0.130.
 #include <algorithm>
 
 #include "hst_internal.h"

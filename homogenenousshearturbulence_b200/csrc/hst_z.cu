@@ -19,9 +19,16 @@
 // in one of NBUF buffers while the previous tile is transformed: 4.66 -> 2.79
 // ms a substep at 768^2 x 512 FP64 (five products; 3.28 for six), 3.16 -> 1.57 FP32;
 // 0.490 -> 0.357 and 0.302 -> 0.217 ms at 384^2 x 256.  It reads and writes 80 %
-// of what a copy could in that time at 768 points.  The inverse one reads V's
-// short runs through the L1 (2.18 -> 2.10 ms at 768^2 x 512, 0.254 -> 0.232 at
-// 384^2 x 256) and is bound by them.
+// of what a copy could in that time at 768 points.
+//
+// The inverse one hides its loads of V (16-byte rows, runs of TY) behind other
+// blocks' arithmetic, so all R0 loads of a butterfly are issued before the
+// first is converted, and its radices keep the registers low enough for a
+// full SM of blocks where that is faster: FP32 768 points 8 x 12 x 8 and 12 x 8 x 8
+// 620 and 611 us against 636 with the forward kernel's 16 x 16 x 3 (961 with each
+// value converted as it is loaded); 384 points 8 x 12 x 4 159 us against 224
+// (226); FP64 384 points 8 x 8 x 6 216 against 220 (232); FP64 768 points stays at
+// 16 x 16 x 3 (504; 529 before; 616 with 12 x 8 x 8, which spills).
 #include <algorithm>
 
 #include "hst_dev.cuh"
@@ -30,33 +37,34 @@
 
 namespace hst {
 
-// The plan of length N: radices, rows a tile; threads a block, buffers and
-// resident blocks of the forward kernel; threads and resident blocks of the
-// inverse one.
+// The plan of length N: the forward kernel's radices; rows a tile; threads a
+// block, buffers and resident blocks of the forward kernel; radices, threads
+// and resident blocks of the inverse one.
 template <int N, typename C>
 struct ZPlan;
-#define HST_ZPLAN(N_, C_, r0, r1, r2, ty, tf, nb, mbf, ti, mbi)                      \
+#define HST_ZPLAN(N_, C_, r0, r1, r2, ty, tf, nb, mbf, i0, i1, i2, ti, mbi)          \
   template <>                                                                        \
   struct ZPlan<N_, C_> {                                                             \
     static constexpr int R0 = r0, R1 = r1, R2 = r2, TY = ty, NBUF = nb;              \
-    static constexpr int TF = tf, MBF = mbf, TI = ti, MBI = mbi;                     \
+    static constexpr int TF = tf, MBF = mbf;                                         \
+    static constexpr int I0 = i0, I1 = i1, I2 = i2, TI = ti, MBI = mbi;              \
   };
-HST_ZPLAN(48, double2, 4, 4, 3, 8, 96, 2, 8, 96, 8)
-HST_ZPLAN(64, double2, 4, 4, 4, 8, 128, 2, 6, 128, 6)
-HST_ZPLAN(96, double2, 8, 4, 3, 8, 96, 2, 6, 96, 8)
-HST_ZPLAN(128, double2, 8, 4, 4, 8, 128, 2, 5, 128, 5)
-HST_ZPLAN(192, double2, 8, 8, 3, 8, 192, 2, 4, 192, 4)
-HST_ZPLAN(256, double2, 8, 8, 4, 8, 256, 2, 3, 256, 3)
-HST_ZPLAN(384, double2, 16, 8, 3, 8, 192, 2, 2, 192, 3)
-HST_ZPLAN(512, double2, 8, 8, 8, 4, 256, 2, 3, 128, 4)
-HST_ZPLAN(768, double2, 16, 16, 3, 4, 192, 2, 2, 192, 2)
-HST_ZPLAN(1024, double2, 16, 16, 4, 4, 256, 1, 2, 256, 2)
-HST_ZPLAN(1536, double2, 16, 16, 6, 4, 384, 2, 1, 192, 2)
-HST_ZPLAN(96, float2, 8, 4, 3, 8, 96, 2, 8, 96, 8)
-HST_ZPLAN(192, float2, 8, 8, 3, 8, 192, 2, 4, 192, 5)
-HST_ZPLAN(384, float2, 16, 8, 3, 8, 192, 2, 4, 192, 5)
-HST_ZPLAN(768, float2, 16, 16, 3, 8, 384, 2, 2, 192, 4)
-HST_ZPLAN(1536, float2, 16, 16, 6, 4, 384, 2, 2, 192, 4)
+HST_ZPLAN(48, double2, 4, 4, 3, 8, 96, 2, 8, 4, 4, 3, 96, 8)
+HST_ZPLAN(64, double2, 4, 4, 4, 8, 128, 2, 6, 4, 4, 4, 128, 6)
+HST_ZPLAN(96, double2, 8, 4, 3, 8, 96, 2, 6, 8, 4, 3, 96, 8)
+HST_ZPLAN(128, double2, 8, 4, 4, 8, 128, 2, 5, 8, 4, 4, 128, 5)
+HST_ZPLAN(192, double2, 8, 8, 3, 8, 192, 2, 4, 8, 8, 3, 192, 4)
+HST_ZPLAN(256, double2, 8, 8, 4, 8, 256, 2, 3, 8, 8, 4, 256, 3)
+HST_ZPLAN(384, double2, 16, 8, 3, 8, 192, 2, 2, 8, 8, 6, 192, 4)
+HST_ZPLAN(512, double2, 8, 8, 8, 4, 256, 2, 3, 8, 8, 8, 128, 4)
+HST_ZPLAN(768, double2, 16, 16, 3, 4, 192, 2, 2, 16, 16, 3, 192, 2)
+HST_ZPLAN(1024, double2, 16, 16, 4, 4, 256, 1, 2, 16, 16, 4, 256, 2)
+HST_ZPLAN(1536, double2, 16, 16, 6, 4, 384, 2, 1, 16, 16, 6, 192, 2)
+HST_ZPLAN(96, float2, 8, 4, 3, 8, 96, 2, 8, 8, 4, 3, 96, 8)
+HST_ZPLAN(192, float2, 8, 8, 3, 8, 192, 2, 4, 8, 8, 3, 192, 5)
+HST_ZPLAN(384, float2, 16, 8, 3, 8, 192, 2, 4, 8, 12, 4, 192, 6)
+HST_ZPLAN(768, float2, 16, 16, 3, 8, 384, 2, 2, 12, 8, 8, 256, 4)
+HST_ZPLAN(1536, float2, 16, 16, 6, 4, 384, 2, 2, 16, 16, 6, 192, 4)
 #undef HST_ZPLAN
 
 #define HST_Z_LENGTHS64(F) F(48) F(64) F(96) F(128) F(192) F(256) F(384) F(512) F(768) F(1024) F(1536)
@@ -64,10 +72,10 @@ HST_ZPLAN(1536, float2, 16, 16, 6, 4, 384, 2, 2, 192, 4)
 
 constexpr int Z_WAIT_LIMIT = 1 << 22;  // polls of a tile's TMA barrier before giving up
 
-template <int N, typename C>
+template <int N, typename C, bool INV = false>
 struct ZShape {
   typedef ZPlan<N, C> P;
-  static constexpr int R0 = P::R0, R1 = P::R1, R2 = P::R2, TY = P::TY;
+  static constexpr int R0 = INV ? P::I0 : P::R0, R1 = INV ? P::I1 : P::R1, R2 = INV ? P::I2 : P::R2, TY = P::TY;
   static_assert(R0 * R1 * R2 == N, "the radices multiply to N");
   static constexpr int M = N / R0;                     // butterflies of the first stage a row
   static constexpr int KB = N <= 256 ? N : (N % 256 == 0 ? 256 : 192);  // z points of one tensor copy
@@ -80,13 +88,12 @@ constexpr size_t z_fwd_smem() {
 }
 
 // the twiddles W_N^(j p) as [p][j], j < M, p < R0 (p = 0 left out), then those
-// of the middle stage W_M^(j' p) as [p][j'], j' < R2, p < R1
-template <int N, typename C>
-static int z_twiddles_t(C* out) {
-  typedef ZShape<N, C> S;
+// of the middle stage W_M^(j' p) as [p][j'], j' < R2, p < R1: N - R2 entries
+template <int N, typename C, bool INV>
+static void z_table(C* o) {
+  typedef ZShape<N, C, INV> S;
   typedef typename RealOf<C>::T T;
   const long double w = -2.0L * 3.141592653589793238462643383279502884L;
-  C* o = out;
   auto put = [&](long e, int n) {
     const long double a = w * (long double)(e % n) / (long double)n;
     *o++ = C{(T)cosl(a), (T)sinl(a)};
@@ -95,20 +102,34 @@ static int z_twiddles_t(C* out) {
     for (int j = 0; j < S::M; ++j) put((long)j * p, N);
   for (int p = 1; p < S::R1; ++p)
     for (int j = 0; j < S::R2; ++j) put((long)j * p, S::M);
-  return (int)(o - out);
+}
+// the forward table, then (N entries on) the inverse one
+template <int N, typename C>
+static int z_twiddles_t(C* out) {
+  z_table<N, C, false>(out);
+  z_table<N, C, true>(out + N);
+  return 2 * N;
 }
 
-// the first two stages on one tile; LD(k, l) gives z point k of row l
-template <int N, int S, int T, typename C, typename LD>
+// the first two stages on one tile; LD(k, l) gives z point k of row l, all R0
+// of a butterfly loaded before the first is converted to the transform's type
+// (PAD: zero between N / 3 and 2 N / 3, where nothing is loaded)
+template <int N, int S, int T, bool PAD, typename C, typename LD>
 __device__ __forceinline__ void z_stages(C* __restrict__ sh, const C* __restrict__ tw, const LD& ld) {
-  typedef ZShape<N, C> Z;
+  typedef typename RealOf<C>::T R;
+  typedef ZShape<N, C, (S > 0)> Z;
   constexpr int R0 = Z::R0, R1 = Z::R1, R2 = Z::R2, M = Z::M, TY = Z::TY;
 #pragma unroll 1
   for (int u = threadIdx.x; u < TY * M; u += T) {
     const int l = u % TY, j = u / TY;
+    decltype(ld(0, 0)) v[R0];
+#pragma unroll
+    for (int r = 0; r < R0; ++r)
+      if (!(PAD && r * M > N / 3 && (r + 1) * M <= N - N / 3)) v[r] = ld(j + r * M, l);
+      else v[r] = {0, 0};
     C x[R0];
 #pragma unroll
-    for (int r = 0; r < R0; ++r) x[r] = ld(j + r * M, l);
+    for (int r = 0; r < R0; ++r) x[r] = C{(R)v[r].x, (R)v[r].y};
     DFT<R0, S>::run(x);
     sh[j * TY + l] = x[0];
 #pragma unroll
@@ -141,7 +162,7 @@ __device__ __forceinline__ void z_stages(C* __restrict__ sh, const C* __restrict
 // the last stage: ST(k, l, value) takes output k of row l
 template <int N, int S, int T, typename C, typename ST>
 __device__ __forceinline__ void z_last(const C* __restrict__ sh, const ST& st) {
-  typedef ZShape<N, C> Z;
+  typedef ZShape<N, C, (S > 0)> Z;
   constexpr int R0 = Z::R0, R1 = Z::R1, R2 = Z::R2, TY = Z::TY;
 #pragma unroll 2
   for (int u = threadIdx.x; u < TY * R0 * R1; u += T) {
@@ -160,7 +181,7 @@ __device__ __forceinline__ void z_last(const C* __restrict__ sh, const ST& st) {
 // x modes that run side by side
 template <int N, typename C>
 __host__ __device__ __forceinline__ int z_inv_group(int nxB) {
-  return ZShape<N, C>::TY * (int)sizeof(C) < 64 ? 4 : nxB;
+  return sizeof(C) == 8 ? 4 : nxB;
 }
 // V row of tile row i: row i of the field, or (edge view: gap = ny) rows -2,
 // -1, ny, ny + 1
@@ -172,11 +193,12 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TI, ZPlan<N, C>::MBI)
   constexpr int TY = Z::TY;
   extern __shared__ __align__(128) double2 sh_d[];
   C* const sh = reinterpret_cast<C*>(sh_d);
-  // the x modes of one y tile run side by side: consecutive blocks write
-  // adjacent runs of the [yt][kz][ix][Ty] tiles; where a run is half a 64-byte
-  // sector pair (1536 points in FP32), four x modes and then the y tiles, whose
-  // runs of V adjoin (2.07 against 2.45 ms at 1536^2 x 128; at 768 points in
-  // FP64 the other way round, 588 against 504 us for 64 x modes and 512 rows)
+  // FP64: the x modes of one y tile run side by side, so that consecutive
+  // blocks write adjacent runs of the [yt][kz][ix][Ty] tiles (768 points, 64 x
+  // modes, 512 rows: 504 us; 588 in the order below).  FP32, whose runs of V are
+  // twice as long as those it writes: four x modes and then the y tiles, whose
+  // runs of V adjoin (768 points, 128 x modes, 512 rows: 636 us against 723 in
+  // the order above; 1536^2 x 128 2.07 against 2.45 ms).
   const int nyT = (g.ny + TY - 1) / TY, nz = g.nz, grp = z_inv_group<N, C>(g.nxB);
   const int bg = blockIdx.x / grp, ix = bg / nyT * grp + blockIdx.x % grp, yt = bg % nyT;
   const int c = blockIdx.y % 3, mem = blockIdx.y / 3;
@@ -184,17 +206,14 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TI, ZPlan<N, C>::MBI)
   const int y0 = yt * TY;
   const double2* const V = (c == 0 ? V0 : (c == 1 ? V1 : V2)) + (size_t)mem * g.nf + (size_t)ix * g.nzT * g.rows +
                            (g.edge_gap ? 0 : 2) + y0;
-  auto ld = [&](int k, int l) -> C {
-    if (y0 + l >= g.ny) return C{0, 0};
-    int iz;
-    if (k <= nz) iz = k;
-    else if (k >= N - nz) iz = k - N;
-    else return C{0, 0};
-    const double2 v = load_field(V + (size_t)(iz + nz) * g.rows + l + (l >= 2 ? g.edge_gap : 0));
-    return C{(T)v.x, (T)v.y};
+  auto ld = [&](int k, int l) -> double2 {
+    const int iz = k <= nz ? k : k - N;
+    double2 v = mkc(0, 0);
+    if (iz >= -nz && y0 + l < g.ny) v = load_field(V + (size_t)(iz + nz) * g.rows + l + (l >= 2 ? g.edge_gap : 0));
+    return v;
   };
   wait_predecessor();
-  z_stages<N, +1, ZPlan<N, C>::TI>(sh, tw, ld);
+  z_stages<N, +1, ZPlan<N, C>::TI, true>(sh, tw, ld);
   const size_t zs = (size_t)g.nxB * TY;
   C* const o = Zo + ((((size_t)mem * 3 + c) * nyT + yt) * N) * zs + (size_t)ix * TY;
   z_last<N, +1, ZPlan<N, C>::TI>(sh, [&](int k, int l, C v) { o[(size_t)k * zs + l] = v; });
@@ -257,7 +276,7 @@ __global__ void __launch_bounds__(ZPlan<N, C>::TF, ZPlan<N, C>::MBF)
       return;
     }
     C* const s = sh + (size_t)b * N * TY;
-    z_stages<N, -1, ZPlan<N, C>::TF>(s, tw, [&](int k, int l) { return s[k * TY + l]; });
+    z_stages<N, -1, ZPlan<N, C>::TF, false>(s, tw, [&](int k, int l) { return s[k * TY + l]; });
     const Tile q = tile_of(t);
     const int y0 = q.yt * TY;
     C* const o = Q + ((size_t)q.pm * g.ncol + (size_t)q.ix * g.nzT) * g.ny + y0;
@@ -341,7 +360,7 @@ static cudaError_t z_inv_t(const Geometry& g, const DeviceState& d, const C* tw,
   const int grp = z_inv_group<N, C>(g.nxB), nyT = (g.ny + ZPlan<N, C>::TY - 1) / ZPlan<N, C>::TY;
   const dim3 grid((g.nxB + grp - 1) / grp * grp * nyT, 3 * g.nmem);
   return launch_after(k_z_inv<N, C>, grid, ZPlan<N, C>::TI, ZShape<N, C>::tile, st, g, d.F[0], d.F[1], d.F[2],
-                      reinterpret_cast<C*>(d.Z), tw + N);
+                      reinterpret_cast<C*>(d.Z), tw + 2 * N);
 }
 template <int N, typename C>
 static cudaError_t z_fwd_t(const Geometry& g, const DeviceState& d, int np, const C* tw, cudaStream_t st) {
