@@ -63,7 +63,7 @@ extern "C" {
 #define HST_PREC_FP64 0  /* everything in FP64: the drop-in */
 #define HST_PREC_MIXED 1 /* the x-z transforms, the products and their spectra in FP32; the right-hand
                             sides, the shear shift, the line solves and u, w in FP64.  Needs 2 nxd and
-                            nzd in {96, 192, 384, 768} and ny a multiple of 32.  No counterpart in the
+                            nzd in {96, 192, 384, 768, 1536} and ny a multiple of 32.  No counterpart in the
                             reference, which is FP64 throughout. */
 
 /* line-solve kinds, KIND_D2V .. KIND_DY (src/hst_linsolve.f90:83) */
@@ -190,9 +190,8 @@ int hst_gpu_outstats(hst_ctx* ctx, double time, double* out);
  * overwritten. */
 int hst_gpu_outstats_sums(hst_ctx* ctx, double time, double* sums, double* exz);
 
-/* Tries the launch choices that keep every buffer's layout -- the lanes of
- * a line-solver group and the points a thread of the z FFT plans --
- * on this context's sizes (`steps` time steps of `deltat` each, after one
+/* Tries the launch choice that keeps every buffer's layout -- the lanes of
+ * a line-solver group in the substep -- on this context's sizes (`steps` time steps of `deltat` each, after one
  * untimed step), keeps the fastest and restores the fields (V, OLD) and
  * the damping state.  A report of the candidates' times a step goes to
  * report[0:report_len) when report is not NULL.  It allocates a copy of
@@ -361,9 +360,9 @@ void* hst_gpu_stream(const hst_ctx* ctx);
  * up the static array's address in the context current at that moment (a
  * lookup, not an allocation; a device reset may move the array); the first
  * call in a context may load the library's device code: make it before any
- * stream capture begins.  Results equal hst_gpu_line_solve's on a context
- * that has not been autotuned (hst_gpu_autotune may pick another solver
- * group width; the two then agree up to rounding).
+ * stream capture begins.  Results equal hst_gpu_line_solve's (both
+ * take the group width of hst_gpu_line_solve, which the substep's and
+ * hst_gpu_autotune leave alone).
  * Errors: a negative HST_E* class, with a message in msg[0:msg_len) when msg
  * is not NULL.  No counterpart in the reference, whose line_solve always
  * works on its module arrays (src/hst_linsolve.f90:147). */
