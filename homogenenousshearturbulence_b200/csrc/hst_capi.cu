@@ -490,12 +490,17 @@ static void free_device(hst_ctx* c) {
   d.configured = &c->configured;
 }
 
+// what a time step runs on: every member of an ensemble at once (the base
+// buffers), or the field itself
+static const Geometry& step_geometry(const hst_ctx* ctx) { return ctx->nmem > 1 ? ctx->gb : ctx->g; }
+
 // The line solves' factor scratch for the current group width: a slice for
-// every solver group that can be resident (sixteen warps an SM), or for as
-// many as the device has room for (the solves then run on fewer groups).
+// every solver group that can be resident (sixteen warps an SM, the columns of
+// every member of an ensemble), or for as many as the device has room for (the
+// solves then run on fewer groups).
 static cudaError_t ensure_facg(hst_ctx* ctx) {
   const int nsm = ctx->d.nsm > 0 ? ctx->d.nsm : 148;
-  const size_t need = hst::solve_scratch_bytes(ctx->g, nsm);
+  const size_t need = hst::solve_scratch_bytes(step_geometry(ctx), nsm);
   if (ctx->d.facg && ctx->d.facg_doubles * sizeof(double) >= need) return cudaSuccess;
   if (ctx->d.facg) {
     cudaError_t r = cudaStreamSynchronize(ctx->stream);
@@ -1284,8 +1289,7 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
                                   {120.0 / 20.0, 90.0 / 20.0, 50.0 / 20.0}};
   const hst_gpu_params& p = ctx->p;
   const bool damp = damping_active(p);
-  // every member of an ensemble at once (the base buffers); the field itself otherwise
-  const Geometry& G = ctx->nmem > 1 ? ctx->gb : ctx->g;
+  const Geometry& G = step_geometry(ctx);
   const DeviceState& D = ctx->nmem > 1 ? ctx->db : ctx->d;
   const char* env = std::getenv("HST_RHS_TILED");
   const bool tiled = !(env && std::atoi(env) == 0);

@@ -2,8 +2,11 @@
 (hst_gpu_create_batch): every kernel of the substep covers all members in one
 launch; each member must evolve exactly as it does alone in its own
 context."""
+import json
+
 import numpy as np
 import pytest
+import torch
 
 from homogenenousshearturbulence_b200 import hst
 from tests.gpu_util import c1_deck, rel_l2, seeded_field
@@ -50,6 +53,33 @@ def test_ensemble_members_match_single_contexts(case):
         assert err <= 1e-15, (case, m, err)
         s.close()
     ens.close()
+
+
+def blocks_of_a_step(s, tmp_path):
+    """{kernel: the blocks of its launch} of one time step"""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        s.timesteps(1)
+        s.sync()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    return {name: int(np.prod(e["args"]["grid"])) for e in events if e.get("cat") == "kernel"
+            for name in ("k_shift", "k_solve_half") if name in e["name"]}
+
+
+@pytest.mark.parametrize("members,nx,ny,nz", [(8, 31, 64, 32), (12, 15, 32, 16), (8, 63, 128, 64), (1, 31, 64, 32)])
+def test_ensemble_solves_run_on_all_blocks(members, nx, ny, nz, tmp_path):
+    """The implicit solves cover an ensemble's columns with as many blocks as
+    the shift, which has the same warps and needs no factor scratch: the
+    scratch holds the columns of every member, not of one."""
+    deck = c1_deck(nx=nx, ny=ny, nz=nz, exact_shift=True)
+    torch.cuda.init()
+    s = hst.Solver(deck, members=members)
+    s.time = 0.0
+    s.timesteps(1)
+    s.sync()
+    got = blocks_of_a_step(s, tmp_path)
+    assert got["k_shift"] > 0 and got["k_solve_half"] == got["k_shift"], got
+    s.close()
 
 
 def test_ensemble_refuses_bad_members():
