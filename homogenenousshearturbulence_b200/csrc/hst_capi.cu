@@ -377,10 +377,7 @@ static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::
   // the line-solver group (HST_LINE_LANES overrides)
   g.P = hst::line_lanes(p.ny, (long)g.ncol * nmem);
   g.PL = hst::line_lanes_shared(p.ny);
-  if (const char* env = std::getenv("HST_LINE_LANES")) {
-    int e = std::atoi(env);
-    if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && p.ny % e == 0 && p.ny / e >= 4) g.P = g.PL = e;
-  }
+  if (const int e = hst::line_lanes_asked(p.ny)) g.P = g.PL = e;
   // mixed precision: the FP32 transforms of the lengths it compiles and the
   // streamed right-hand sides
   g.mp = p.precision == HST_PREC_MIXED;
@@ -1076,11 +1073,10 @@ extern "C" int hst_gpu_pressure(hst_ctx* ctx, double time, int dst) {
 static int queue_timestep(hst_ctx* ctx, double* time, double deltat);
 
 // ------------------------------------------------------------ autotune ----
-// Tries the launch choices that leave every buffer's layout unchanged -- the
-// lanes of a line-solver group (P) and the points a thread of the z
-// FFT plans -- on this context's own sizes, `steps` time steps each after
-// one untimed step, keeps the fastest, and puts the fields and the time back
-// as they were.  The report lists every candidate with its time a step.
+// Tries the launch choice that leaves every buffer's layout unchanged -- the
+// lanes of a line-solver group (P), every width that fits -- on this context's
+// own sizes, `steps` time steps each after one untimed step, keeps the
+// fastest, and puts the fields and the time back as they were.  The report lists every candidate with its time a step.
 extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* report, int report_len) {
   if (!ctx || steps < 1) return fail(ctx, HST_EARG, "autotune: bad arguments");
   if (ctx->nmem > 1) return fail(ctx, HST_EARG, "autotune: not for an ensemble context");
@@ -1109,7 +1105,7 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   // candidates
   std::vector<int> lanes;
   for (int c = 32; c >= 4; c >>= 1)
-    if (g0.ny / c >= 4) lanes.push_back(c);
+    if (hst::line_lanes_fit(g0.ny, c)) lanes.push_back(c);
   if (lanes.empty()) lanes.push_back(g0.P);
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1149,7 +1145,7 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
       best = per;
       gbest = t;
     }
-    }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   // the winner, and the state as it was

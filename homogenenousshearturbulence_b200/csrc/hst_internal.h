@@ -150,6 +150,10 @@ cudaError_t launch_solve_half(const Geometry& g, const DeviceState& d, const Phy
 int line_lanes(int ny, long columns);
 // of k_line_solve, whose factors lie in shared memory
 int line_lanes_shared(int ny);
+// whether the solvers have room for groups of P lanes; the width that
+// HST_LINE_LANES asks for, where they do (0: none)
+bool line_lanes_fit(int ny, int P);
+int line_lanes_asked(int ny);
 // der(0:ny-1, 0:3, -2:2) in the slab-major order of groups of P lanes; the
 // doubles that any P takes
 std::vector<double> slab_major(const std::vector<double>& der, int ny, int P);

@@ -36,7 +36,6 @@
 #include <stdint.h>
 
 #include <cstdarg>
-#include <cstdlib>
 #include <cstdio>
 
 #include "hst_internal.h"
@@ -77,11 +76,7 @@ int fail(char* msg, int len, int rc, const char* fmt, ...) {
 // context that has not been autotuned; hst_gpu_autotune may give a context
 // another group width, and the two then agree up to rounding
 int lanes_of(int ny, long columns, bool d0) {
-  const char* env = std::getenv("HST_LINE_LANES");
-  if (env) {
-    int e = std::atoi(env);
-    if (e >= 2 && e <= 32 && (e & (e - 1)) == 0 && ny % e == 0 && ny / e >= 4) return e;
-  }
+  if (const int e = hst::line_lanes_asked(ny)) return e;
   return d0 ? hst::line_lanes(ny, columns) : hst::line_lanes_shared(ny);
 }
 

@@ -29,6 +29,7 @@
 // 0.535 -> 0.371; 1536^2 x 128 (a generic form before) 11.1 -> 2.65,
 // 20300 columns of 150 rows 0.399 -> 0.130.
 #include <algorithm>
+#include <cstdlib>
 
 #include "hst_internal.h"
 #include "hst_line.cuh"
@@ -416,6 +417,20 @@ int line_lanes_shared(int ny) {
   return 2;
 }
 
+// A width fits where one warp's lines (32 / P of them) have room in a block's
+// shared memory beside k_dy_sums' own; every width that does also has the exact
+// quotients of LineGeom::at (checked for all even ny up to 2560: two lanes lose
+// them from 1512 rows on, four from 2128).
+static size_t line_bytes(int ny, int P) { return (size_t)P * line_geom(ny, P).MS * sizeof(double2); }
+bool line_lanes_fit(int ny, int P) { return ny / P >= 4 && line_bytes(ny, P) * (32 / P) <= 226 * 1024; }
+
+// HST_LINE_LANES, where it divides ny and fits; 0 otherwise
+int line_lanes_asked(int ny) {
+  const char* env = std::getenv("HST_LINE_LANES");
+  const int P = env ? std::atoi(env) : 0;
+  return P >= 2 && P <= 32 && (P & (P - 1)) == 0 && ny % P == 0 && line_lanes_fit(ny, P) ? P : 0;
+}
+
 size_t slab_der_doubles(int ny) { return (size_t)20 * (ny + 32); }
 size_t d0_table_doubles(int ny) {
   // d0_fields(mM, P) P, mM P < ny + P
@@ -435,7 +450,6 @@ std::vector<double> slab_major(const std::vector<double>& der, int ny, int P) {
   return o;
 }
 
-static size_t line_bytes(int ny, int P) { return (size_t)P * line_geom(ny, P).MS * sizeof(double2); }
 // double2 of factor scratch a group
 static int fac_elems(int ny, int P) { return 2 * (slab_rows(ny, P) - 2) * P; }
 

@@ -77,6 +77,47 @@ def test_lanes_follow_the_columns(columns):
     against_oracle(c1_deck(nx=nx, nz=nz, ny=128, exact_shift=True))
 
 
+@pytest.mark.parametrize("lanes", [None, "2", "4", "8", "16", "32"])
+@pytest.mark.parametrize("ny", [64, 1024, 2048])
+def test_lanes_asked_for(monkeypatch, ny, lanes):
+    """every width that HST_LINE_LANES can ask for: from about 910 rows two lanes have no room, from about 1820 four,
+    and the context then keeps its own width; the steps and every kind of line solve run either way"""
+    if lanes:
+        monkeypatch.setenv("HST_LINE_LANES", lanes)
+    deck = c1_deck(nx=3, nz=2, ny=ny, exact_shift=True, deltat=0.0005)
+    V0 = seeded_field(deck, seed=2, k0=3.0)
+    s, o = make_pair(deck, V0)
+    Vg, Vo = run_pair(s, o, deck["deltat"], 1)
+    # the tall lines are ill-conditioned in proportion to ny^2 (2e-13 at 512 rows)
+    assert rel_l2(Vg, Vo) <= 1e-12 * max(1.0, (ny / 512) ** 2)
+    shift = s.shear_shifts(0.37)
+    for c in range(3):
+        o.field(c)[...] = Vg[c]
+    for kind in (hst.KIND_D2V, hst.KIND_ETA, hst.KIND_POISSON, hst.KIND_D0, hst.KIND_DY):
+        s.upload(hst.RHS1, np.zeros(s.shape, np.complex128))
+        s.line_solve(kind, 123.4, hst.V2, hst.RHS1, shift=shift)
+        o.field(5)[...] = 0.0
+        o.line_solve(kind, 123.4, 1, 5, shift=shift)
+        assert rel_l2(s.download(hst.RHS1), o.field(5)) <= 1e-11 * max(1.0, (ny / 512) ** 2), kind
+    s.close()
+
+
+@pytest.mark.parametrize("ny", [1024, 2048])
+def test_autotune_leaves_out_what_has_no_room(ny):
+    """tall lines: four lanes have no room at 2048 rows, and the others are tried"""
+    deck = c1_deck(nx=3, nz=2, ny=ny)
+    V0 = seeded_field(deck, seed=2, k0=3.0)
+    s = hst.Solver(deck)
+    s.time = 0.0
+    s.set_velocity(V0)
+    before = s.velocity()
+    report = s.autotune(deck["deltat"], steps=1)
+    assert [f"P={P}:" in report for P in (32, 16, 8, 4)] == [True, True, True, ny == 1024], report
+    assert np.array_equal(s.velocity(), before)
+    s.timestep(deck["deltat"])
+    s.close()
+
+
 @pytest.mark.parametrize("ny,exact,linear", [(34, False, False), (34, True, False), (150, False, False), (64, True, True),
                                              (30, False, True)])
 def test_streamed_right_hand_sides_equal_row_by_row(monkeypatch, ny, exact, linear):
