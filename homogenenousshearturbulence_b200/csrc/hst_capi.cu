@@ -324,7 +324,7 @@ static int upload_gdamp(hst_ctx* ctx) {
 }
 
 // ------------------------------------------------------ geometry ----
-static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::string& why) {
+static int choose_geometry(const hst_gpu_params& p, Geometry& g, std::string& why) {
   g.nx = p.nx;
   g.ny = p.ny;
   g.nz = p.nz;
@@ -374,8 +374,10 @@ static int choose_geometry(const hst_gpu_params& p, int nmem, Geometry& g, std::
       return HST_EARG;
     }
   }
-  // the line-solver group (HST_LINE_LANES overrides)
-  g.P = hst::line_lanes(p.ny, (long)g.ncol * nmem);
+  // the line-solver group (HST_LINE_LANES overrides), from one field's columns:
+  // another width rounds differently, and a member of an ensemble has the bits
+  // that it has alone
+  g.P = hst::line_lanes(p.ny, g.ncol);
   g.PL = hst::line_lanes_shared(p.ny);
   if (const int e = hst::line_lanes_asked(p.ny)) g.P = g.PL = e;
   // mixed precision: the FP32 transforms of the lengths it compiles and the
@@ -424,7 +426,7 @@ static double dev_bytes(const Geometry& g) {
 extern "C" double hst_gpu_device_bytes(const hst_gpu_params* p) {
   Geometry g;
   std::string why;
-  if (!p || choose_geometry(*p, 1, g, why) != HST_OK) return 0.0;
+  if (!p || choose_geometry(*p, g, why) != HST_OK) return 0.0;
   return dev_bytes(g);
 }
 
@@ -550,7 +552,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   std::memset(&ctx->d, 0, sizeof ctx->d);
   ctx->d.configured = &ctx->configured;
   std::string why;
-  int rc = choose_geometry(*pin, nmem, ctx->g, why);
+  int rc = choose_geometry(*pin, ctx->g, why);
   if (rc != HST_OK) {
     std::fprintf(stderr, "hst_gpu_create: %s\n", why.c_str());
     delete ctx;
