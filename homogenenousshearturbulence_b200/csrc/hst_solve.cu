@@ -102,6 +102,26 @@ __device__ __forceinline__ void store_ghosts(double2* dst, const cxd* buf, const
   }
 }
 
+// A table into shared memory, eight 16-byte loads of a thread in flight (n
+// even, both 16-byte aligned).  Where the columns leave a block few warps, one
+// load at a time took longer than the solves: both halves of 136 columns of 512
+// rows 123 us, with this 39; of 256 rows 67 and 25; of 14661 columns of 512
+// rows 421 and 408.
+__device__ __forceinline__ void copy_table(double* dst, const double* __restrict__ src, int n) {
+  const double2* const s2 = reinterpret_cast<const double2*>(src);
+  double2* const d2 = reinterpret_cast<double2*>(dst);
+  const int T = blockDim.x;
+  for (int i0 = threadIdx.x; i0 < n / 2; i0 += 8 * T) {
+    double2 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (i0 + k * T < n / 2) v[k] = __ldg(s2 + i0 + k * T);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (i0 + k * T < n / 2) d2[i0 + k * T] = v[k];
+  }
+}
+
 // The four lines of a column one after another.  What bounds it is the
 // shared-memory traffic of the tables and the lines; two lines at a time,
 // sharing the table loads, leave nine warps an SM and measured slower (3.42
@@ -120,8 +140,8 @@ __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
   const int ntab = SH ? d0_fields(mM, P) * P : 0, nder = SH ? 5 * mM * P : 0;
   double* const d0s = smem_d;
   double* const der0s = d0s + ntab;
-  for (int i = threadIdx.x; i < ntab; i += blockDim.x) d0s[i] = a.d0tab[i];
-  for (int i = threadIdx.x; i < nder; i += blockDim.x) der0s[i] = a.derS[i];
+  copy_table(d0s, a.d0tab, ntab);
+  copy_table(der0s, a.derS, nder);
   if (SH) __syncthreads();
   wait_predecessor();
   const int lineN = P * G.MS;
@@ -179,7 +199,7 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
   const unsigned gmask = group_mask<P>();
   const int nder = SH ? half_slices(HALF) * 5 * mM * P : 0;
   if (SH) {
-    for (int i = threadIdx.x; i < nder; i += blockDim.x) smem_d[i] = a.derS[i];
+    copy_table(smem_d, a.derS, nder);
     __syncthreads();
   }
   wait_predecessor();
@@ -261,8 +281,8 @@ __global__ void __launch_bounds__(512, 1) k_dy_sums(SolveArgs a, double sx, doub
   const int nd1 = 5 * mM * P, ntab = SH ? d0_fields(mM, P) * P : 0, nder = SH ? nd1 : 0;
   double* const d0s = smem_d;
   double* const der1s = d0s + ntab;
-  for (int i = threadIdx.x; i < ntab; i += blockDim.x) d0s[i] = a.d0tab[i];
-  for (int i = threadIdx.x; i < nder; i += blockDim.x) der1s[i] = a.derS[nd1 + i];
+  copy_table(d0s, a.d0tab, ntab);
+  copy_table(der1s, a.derS + nd1, nder);
   if (SH) __syncthreads();
   cxd* const buf = reinterpret_cast<cxd*>(der1s + nder) + (size_t)grp * P * G.MS;
   cxd* const sb = buf + s * G.MS;

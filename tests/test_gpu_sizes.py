@@ -5,8 +5,11 @@ right-hand sides, each against the oracle (or the other form).  Tolerances:
 1e-12 relative L2 in FP64 and 1e-5 in mixed precision, the bounds the substep
 is held to everywhere; a few 1e-15 and 1e-8 are what these sizes show.
 """
+import ctypes as ct
+
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from homogenenousshearturbulence_b200 import hst
@@ -75,6 +78,30 @@ def test_lanes_follow_the_columns(columns):
     """128 rows: few columns (wide solver groups) and many (narrow ones)"""
     nx, nz = columns
     against_oracle(c1_deck(nx=nx, nz=nz, ny=128, exact_shift=True))
+
+
+def solve_us(nx, ny, nz):
+    """microseconds of hst_gpu_linsolve on (nx + 1)(2 nz + 1) columns of ny rows (the least of five means of ten)"""
+    s = hst.Solver(c1_deck(nx=nx, ny=ny, nz=nz, linear=True))
+    stream, best = torch.cuda.ExternalStream(s.stream), np.inf
+    for _ in range(5):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record(stream)
+        for _ in range(10):
+            assert hst.lib().hst_gpu_linsolve(s._h, ct.c_double(1000.0), ct.c_double(0.0)) == 0
+        b.record(stream)
+        s.sync()
+        best = min(best, a.elapsed_time(b) * 100.0)
+    s.close()
+    return best
+
+
+@pytest.mark.parametrize("ny", [256, 512])
+def test_few_columns_take_no_longer_than_more(ny):
+    """136 columns, a warp or two an SM, against 1281 of the same rows: the blocks' own start (the tables into shared
+    memory) must not outweigh the solves.  1.0 is what these sizes show; 2.2 and 2.5 with the tables copied one
+    load at a time."""
+    assert solve_us(7, ny, 8) <= 1.5 * solve_us(20, ny, 30)
 
 
 @pytest.mark.parametrize("lanes", [None, "2", "4", "8", "16", "32"])
