@@ -73,6 +73,18 @@ __device__ __forceinline__ Column column_of(const Geometry& g, const PhysScalars
   return c;
 }
 
+// The column that this group of a persistent grid takes first; the others
+// follow gridDim.x blocks' groups apart.  Consecutive warps' columns go to
+// consecutive blocks, so that the last round, which is seldom full, falls on all
+// SMs alike (both halves of 9664 columns of 64 rows 55 -> 42 us, of 5151 of 256
+// rows 102 -> 83; a full last round, 32896 of 256 rows, 357 and 355).
+template <int P>
+__device__ __forceinline__ int first_column() {
+  constexpr int G = 32 / P;  // groups a warp
+  const int warp = threadIdx.x >> 5;
+  return (warp * gridDim.x + blockIdx.x) * G + (threadIdx.x & 31) / P;
+}
+
 // (eight loads issued before the first use: the stores to shared memory may
 // alias them for all the compiler knows)
 template <int P>
@@ -152,7 +164,7 @@ __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
   const int m = G.rows(s), r0 = G.first(s);
   const SlabDerT<SH> DS = {SH ? der0s : a.derS, mM, P};
   const D0Table<P, SH> T = {(SH ? d0s : a.d0tab) + s};
-  for (int cg = blockIdx.x * groups + grp; cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
+  for (int cg = first_column<P>(); cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
     const Column c = column_of(g, a.ps, cg);
     const cxd pt = cexpi(-(c.al * sc.sx_t + c.be * sc.sz_t)), pn = cexpi(-(c.al * sc.sx_n + c.be * sc.sz_n));
     const double gx = c.al * sc.dgx + c.be * sc.dgz;
@@ -209,7 +221,7 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
   const SlabDerT<SH> DS = {SH ? smem_d : a.derS, mM, P};
   const int slot = blockIdx.x * groups + grp;
   double2* const fac = a.fac + (size_t)slot * a.facn + s;
-  for (int cg = slot; cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
+  for (int cg = first_column<P>(); cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
     const Column c = column_of(g, a.ps, cg);
     const cxd pn = cexpi(-(c.al * sc.sx_n + c.be * sc.sz_n));
     double2* const v1 = a.V1 + c.cb;

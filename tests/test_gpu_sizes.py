@@ -104,6 +104,14 @@ def test_few_columns_take_no_longer_than_more(ny):
     assert solve_us(7, ny, 8) <= 1.5 * solve_us(20, ny, 30)
 
 
+@pytest.mark.parametrize("columns", [((60, 60), (63, 75)), ((42, 42), (50, 50))])
+def test_a_last_round_of_columns_is_spread(columns):
+    """64 rows: 7381 and 9664 columns, 3655 and 5151, of which the larger just exceed what is resident at once: the
+    time must not double for the rest (1.2 to 1.5 is what these sizes show; 1.9 with that rest on a few SMs)"""
+    few, more = (solve_us(nx, 64, nz) for nx, nz in columns)
+    assert more <= 1.65 * few
+
+
 @pytest.mark.parametrize("lanes", [None, "2", "4", "8", "16", "32"])
 @pytest.mark.parametrize("ny", [64, 1024, 2048])
 def test_lanes_asked_for(monkeypatch, ny, lanes):
