@@ -422,11 +422,14 @@ __global__ void k_d0_table(const double* __restrict__ derS, int ny, double* __re
 // -------------------------------------------------------------- launchers ----
 // The lanes of a solver group: as many as leave at least four rows a lane,
 // then half of them while a lane has fewer than twelve rows and the columns
-// still give each of the chip's 148 SMs twelve warps: the reduction across
-// the lanes costs as much as some ten rows.  Measured for the solves: 64 rows of
-// 2080 columns 25.0 us with 16 lanes, 29.0 with 8; 128 rows of 8128 columns
-// 59 us with 8 lanes, 73 with 16, 97 with 32; 256 rows of 32896 columns 384 us
-// with 16 lanes, 434 with 32, 487 with 8; 512 rows 3.10 ms with 32, 3.71 with 16.
+// exceed what sixteen warps on each of the chip's 148 SMs take at once: the
+// reduction across the lanes costs as much as some ten rows, a second round of
+// columns half the first or more.  Measured for both solve halves, narrower and
+// wider group: 64 rows of 2080 columns 17.4 us with 8 lanes, 16.8 with 16; of 5151
+// 23.2 and 33.1; of 9664 35.0 with 4, 42.3 with 8; 128 rows of 3655 columns 29.8 with
+// 16, 40.2 with 32; of 32896 184 with 8, 198 with 16; 256 rows of 1281 columns 31.0
+// with 16, 26.4 with 32; of 32896 355 with 16, 406 with 32; 512 rows of 14661 436 with
+// 16, 392 with 32.
 int line_lanes(int ny, long columns) {
   int P = 2;
   for (int c = 32; c > 2; c >>= 1)
@@ -434,7 +437,7 @@ int line_lanes(int ny, long columns) {
       P = c;
       break;
     }
-  while (P > 4 && ny / P < 12 && columns >= 148L * 12 * (32 / (P / 2))) P >>= 1;
+  while (P > 4 && ny / P < 12 && columns > 148L * 16 * (32 / P)) P >>= 1;
   return P;
 }
 
