@@ -1,8 +1,9 @@
 // The register DFTs of the 3/2-dealiased x and z transforms (radices up to 24,
-// built from radix-2/3/4 pieces), and a Stockham FFT with a runtime plan for
-// the lengths without a compiled plan.
+// built from radix-2/3/4 pieces), and a Stockham FFT for the lengths without a
+// plan of their own in hst_xprod.cu and hst_z.cu: 12, 24, 48 and 64 known to the
+// compiler, the others with a runtime plan.
 //
-// In the runtime plan a block transforms nl lines of length N = 2^a 3^b.  Each
+// A block transforms nl lines of length N = 2^a 3^b.  Each
 // radix-R stage is one pass: a thread gathers the R inputs of its butterflies
 // into registers, applies the stage twiddles, computes a radix-R DFT in
 // registers, and scatters the outputs.  The first stage reads through a
@@ -190,9 +191,8 @@ struct FftPlan {
   int n;
   int r[4];
 };
-__host__ __device__ inline FftPlan make_plan(int N) {
-  FftPlan p;
-  p.n = 0;
+__host__ __device__ constexpr FftPlan make_plan(int N) {
+  FftPlan p = {0, {0, 0, 0, 0}};
   int m = N;
   while (m > 24 && m % 16 == 0 && p.n < 3) {
     p.r[p.n++] = 16;
@@ -283,29 +283,43 @@ __device__ __forceinline__ void fft_stage_r(int R, int N, int nl, int Ns, const 
   }
 }
 
-// The whole transform of nl lines with the runtime plan: the first stage
-// reads through src, the last writes through dst, the stages between
-// exchange through `sh` (nl lines of stride N+1).  SRC_SH / DST_SH: src
-// reads, dst writes the same shared buffer (the stage then synchronises
-// between its reads and its writes).  Requires nl N <= PPT blockDim.x.
-template <int S, int PPT, bool SRC_SH, bool DST_SH, typename LD, typename ST, typename C>
+// The whole transform of nl lines: the first stage reads through src, the
+// last writes through dst, the stages between exchange through `sh` (nl lines
+// of stride N+1).  SRC_SH / DST_SH: src reads, dst writes the same shared
+// buffer (the stage then synchronises between its reads and its writes).
+// NT: the length, with its one or two radices known to the compiler; 0: the
+// plan of the runtime length N.  Requires nl N <= PPT blockDim.x.
+template <int NT, int S, int PPT, bool SRC_SH, bool DST_SH, typename LD, typename ST, typename C>
 __device__ void fft_global(int N, int nl, const C* __restrict__ tw, C* sh, const LD& src, const ST& dst) {
-  const FftPlan P = make_plan(N);
-  const ShLinesT<C> L = {sh, N + 1};
-  int Ns = 1;
-  if (P.n == 1) {
-    fft_stage_r<S, PPT, SRC_SH && DST_SH>(P.r[0], N, nl, Ns, tw, src, dst);
-    return;
-  }
-  fft_stage_r<S, PPT, SRC_SH>(P.r[0], N, nl, Ns, tw, src, L);
-  Ns *= P.r[0];
-  __syncthreads();
-  for (int s = 1; s + 1 < P.n; ++s) {
-    fft_stage_r<S, PPT, true>(P.r[s], N, nl, Ns, tw, L, L);
-    Ns *= P.r[s];
+  if constexpr (NT > 0) {
+    constexpr FftPlan P = make_plan(NT);
+    static_assert(P.n <= 2, "short lengths");
+    if constexpr (P.n == 1) {
+      fft_stage_io<P.r[0], S, PPT, SRC_SH && DST_SH>(NT, nl, 1, tw, src, dst);
+    } else {
+      const ShLinesT<C> L = {sh, NT + 1};
+      fft_stage_io<P.r[0], S, PPT, SRC_SH>(NT, nl, 1, tw, src, L);
+      __syncthreads();
+      fft_stage_io<P.r[1], S, PPT, DST_SH>(NT, nl, P.r[0], tw, L, dst);
+    }
+  } else {
+    const FftPlan P = make_plan(N);
+    const ShLinesT<C> L = {sh, N + 1};
+    int Ns = 1;
+    if (P.n == 1) {
+      fft_stage_r<S, PPT, SRC_SH && DST_SH>(P.r[0], N, nl, Ns, tw, src, dst);
+      return;
+    }
+    fft_stage_r<S, PPT, SRC_SH>(P.r[0], N, nl, Ns, tw, src, L);
+    Ns *= P.r[0];
     __syncthreads();
+    for (int s = 1; s + 1 < P.n; ++s) {
+      fft_stage_r<S, PPT, true>(P.r[s], N, nl, Ns, tw, L, L);
+      Ns *= P.r[s];
+      __syncthreads();
+    }
+    fft_stage_r<S, PPT, DST_SH>(P.r[P.n - 1], N, nl, Ns, tw, L, dst);
   }
-  fft_stage_r<S, PPT, DST_SH>(P.r[P.n - 1], N, nl, Ns, tw, L, dst);
 }
 
 }  // namespace hst

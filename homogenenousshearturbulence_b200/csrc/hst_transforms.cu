@@ -1,5 +1,5 @@
-// The transforms of the hst substep for the lengths without a compiled plan
-// (FP64, the runtime plan), the launches of the three transform stages, and
+// The transforms of the hst substep for the lengths without a plan of their
+// own in hst_xprod.cu and hst_z.cu (FP64), the launches of the three transform stages, and
 // the line transforms of the per-piece path:
 //
 //   zinv    V (u, v, w) -> zero-padded z-inverse transform (Z)
@@ -57,17 +57,17 @@ struct TileSrc {
   __device__ __forceinline__ C operator()(int yi, int kz) const { return base[(size_t)kz * zstride + yi]; }
 };
 
-template <int PPT>
+template <int NT, int PPT>
 __global__ void __launch_bounds__(256)
     k_zinv(Geometry g, const double2* __restrict__ V0, const double2* __restrict__ V1, const double2* __restrict__ V2,
            double2* __restrict__ Z, const double2* __restrict__ twz) {
   extern __shared__ double2 sh[];
   const int ix = blockIdx.x, yt = blockIdx.y, c = blockIdx.z % 3, mem = blockIdx.z / 3;
-  const int Ty = g.Ty, NZ = g.nzd;
+  const int Ty = g.Ty, NZ = NT ? NT : g.nzd;
   const double2* V = (c == 0 ? V0 : (c == 1 ? V1 : V2)) + (size_t)mem * g.nf;
   const ZinvSrc src = {V + (size_t)ix * g.nzT * g.rows + (g.edge_gap ? 0 : 2) + yt * Ty, g.rows, g.nz, NZ, g.edge_gap};
   const TileDst dst = {Z + ((((size_t)mem * 3 + c) * g.nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
-  fft_global<+1, PPT, false, false>(NZ, Ty, twz, sh, src, dst);
+  fft_global<NT, +1, PPT, false, false>(NZ, Ty, twz, sh, src, dst);
 }
 
 // --------------------------------------------------------------- k_zfwd ----
@@ -86,16 +86,16 @@ struct ZfwdDst {
   }
 };
 
-template <int PPT>
+template <int NT, int PPT>
 __global__ void __launch_bounds__(256)
     k_zfwd(Geometry g, int np, const double2* __restrict__ Pp, double2* __restrict__ Q,
            const double2* __restrict__ twz) {
   extern __shared__ double2 sh[];
   const int yt = blockIdx.x, ix = blockIdx.y, pm = blockIdx.z / np * 6 + blockIdx.z % np;
-  const int Ty = g.Ty, NZ = g.nzd;
+  const int Ty = g.Ty, NZ = NT ? NT : g.nzd;
   const TileSrc src = {Pp + (((size_t)pm * g.nyT + yt) * NZ) * g.nxB * Ty + (size_t)ix * Ty, (size_t)g.nxB * Ty};
   const ZfwdDst dst = {Q + ((size_t)pm * g.ncol + (size_t)ix * g.nzT) * g.ny + yt * Ty, g.ny, g.nz, NZ};
-  fft_global<-1, PPT, false, false>(NZ, Ty, twz, sh, src, dst);
+  fft_global<NT, -1, PPT, false, false>(NZ, Ty, twz, sh, src, dst);
 }
 
 // -------------------------------------------------------------- k_xprod ----
@@ -154,16 +154,16 @@ struct ProdSrc {
   }
 };
 
-// The x stage of the lengths without a compiled plan (hst_xprod.cu), FP64,
-// with the runtime plan (PPT points a thread)
-template <int PPT>
+// The x stage of the lengths without a plan in hst_xprod.cu, FP64 (PPT points a
+// thread; NT: the length, 0: any)
+template <int NT, int PPT>
 __global__ void __launch_bounds__(320)
     k_xprod(Geometry g, int np, const double2* __restrict__ Z, double2* __restrict__ Pp, const double2* __restrict__ twx,
             const double* __restrict__ dyl, PhysScalars ps, int want_cfl, unsigned long long* __restrict__ cflmax) {
   typedef double2 C;
   extern __shared__ double2 sh[];
   typedef ShLinesT<C> LT;
-  const int NX = 2 * g.nxd, nx = g.nx, nxB = g.nxB, NZ = g.nzd, Ty = g.Ty;
+  const int NX = NT ? NT : 2 * g.nxd, nx = g.nx, nxB = g.nxB, NZ = g.nzd, Ty = g.Ty;
   const int nyT = g.nyT;
   const int y0 = 2 * blockIdx.x, kz = blockIdx.y % g.nzd, mem = blockIdx.y / g.nzd;
   Z += (size_t)mem * 3 * g.nzd * nyT * Ty * g.nxB;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(320)
   const LT L = {sh, NX + 1};
   // u + i v of both rows and w0 + i w1 on the physical x grid
   const XinvSrc<C> xs = {Z + tile + yi0, cs, Ty, nx, NX};
-  fft_global<+1, PPT, false, true>(NX, 3, twx, sh, xs, L);
+  fft_global<NT, +1, PPT, false, true>(NX, 3, twx, sh, xs, L);
   __syncthreads();
   if (want_cfl) {
     double cm = 0.0;
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(320)
   }
   // the six product lines, transformed forward in place
   const ProdSrc<LT, C> ps6 = {L, ps.factor, np == 5};
-  fft_global<-1, PPT, true, true>(NX, 6, twx, sh, ps6, L);
+  fft_global<NT, -1, PPT, true, true>(NX, 6, twx, sh, ps6, L);
   __syncthreads();
   // separate the two real transforms of each line, keep kx = 0..nx
   for (int e = threadIdx.x; e < nxB * 3; e += blockDim.x) {
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(256) k_piece_lines(PieceLines P, int nlines, i
   }
   __syncthreads();
   const ShLinesT<double2> L = {sh_d, LS};
-  fft_global<S, 16, true, true>(N, lpb, tw, sh_d, L, L);
+  fft_global<0, S, 16, true, true>(N, lpb, tw, sh_d, L, L);
   __syncthreads();
   if (P.kind == 1) {  // real parts: 2(nxd+1) reals a line, the two past N zero
     for (int e = threadIdx.x; e < nl * (N + 2); e += blockDim.x) {
@@ -318,6 +318,30 @@ static void big_smem(const DeviceState& d, K k) {
   smem_limit(d, k, 220 * 1024);
 }
 
+// The lengths known to the compiler, then the runtime plan with 16 or 32 points
+// a thread.  Computed at run time, the indices of a short line's few butterflies
+// cost as much as the butterflies: x at 48 points (nx 15, ny 64, nz 40) 50.3 us a
+// substep, at 24 (nx 7, ny 128, nz 128) 285, known to the compiler 35.9 and 223;
+// z inverse at 24 (nx 127, ny 128, nz 8) 37.5 and 31.2.
+#define HST_SHORT_Z(n, pts, F) \
+  switch (n) {                 \
+    case 12: F(12, 16); break; \
+    case 24: F(24, 16); break; \
+    default:                   \
+      if ((pts) <= 16 * 256) { \
+        F(0, 16);              \
+      } else {                 \
+        F(0, 32);              \
+      }                        \
+  }
+#define HST_SHORT_X(n, pts, F) \
+  if ((n) == 48) {             \
+    F(48, 16);                 \
+  } else if ((n) == 64) {      \
+    F(64, 16);                 \
+  } else                       \
+    HST_SHORT_Z(n, pts, F)
+
 bool mp_length_ok(int n) { return x_compiled(n, true) && z_rows(n, true) > 0; }
 
 static cudaError_t launch_zinv_main(const Geometry& g, const DeviceState& d, cudaStream_t st) {
@@ -325,13 +349,11 @@ static cudaError_t launch_zinv_main(const Geometry& g, const DeviceState& d, cud
   const int pts = g.nzd * g.Ty;
   const dim3 grid(g.nxB, g.nyT, 3 * g.nmem);
   const size_t smem = (size_t)g.Ty * (g.nzd + 1) * sizeof(double2);
-  if (pts <= 16 * 256) {
-    big_smem(d, k_zinv<16>);
-    k_zinv<16><<<grid, fft_threads(pts, 16), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz);
-  } else {
-    big_smem(d, k_zinv<32>);
-    k_zinv<32><<<grid, fft_threads(pts, 32), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz);
-  }
+#define HST_ZINV(NT, PPT)        \
+  big_smem(d, k_zinv<NT, PPT>); \
+  k_zinv<NT, PPT><<<grid, fft_threads(pts, PPT), smem, st>>>(g, d.F[0], d.F[1], d.F[2], d.Z, d.twz)
+  HST_SHORT_Z(g.nzd, pts, HST_ZINV)
+#undef HST_ZINV
   return cudaGetLastError();
 }
 
@@ -340,13 +362,11 @@ static cudaError_t launch_zfwd_main(const Geometry& g, const DeviceState& d, int
   const int pts = g.nzd * g.Ty;
   const dim3 grid(g.nyT, g.nxB, np * g.nmem);
   const size_t smem = (size_t)g.Ty * (g.nzd + 1) * sizeof(double2);
-  if (pts <= 16 * 256) {
-    big_smem(d, k_zfwd<16>);
-    k_zfwd<16><<<grid, fft_threads(pts, 16), smem, st>>>(g, np, d.Pp, d.Q, d.twz);
-  } else {
-    big_smem(d, k_zfwd<32>);
-    k_zfwd<32><<<grid, fft_threads(pts, 32), smem, st>>>(g, np, d.Pp, d.Q, d.twz);
-  }
+#define HST_ZFWD(NT, PPT)        \
+  big_smem(d, k_zfwd<NT, PPT>); \
+  k_zfwd<NT, PPT><<<grid, fft_threads(pts, PPT), smem, st>>>(g, np, d.Pp, d.Q, d.twz)
+  HST_SHORT_Z(g.nzd, pts, HST_ZFWD)
+#undef HST_ZFWD
   return cudaGetLastError();
 }
 
@@ -357,13 +377,11 @@ static cudaError_t launch_xprod_main(const Geometry& g, const DeviceState& d, co
   if (g.mp) return cudaErrorInvalidValue;
   const dim3 grid(g.ny / 2, g.nzd * g.nmem);
   const size_t smem = (size_t)6 * (NX + 1) * sizeof(double2);
-  if (6 * NX <= 16 * 256) {
-    big_smem(d, k_xprod<16>);
-    k_xprod<16><<<grid, fft_threads(6 * NX, 16), smem, st>>>(g, np, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
-  } else {
-    big_smem(d, k_xprod<32>);
-    k_xprod<32><<<grid, fft_threads(6 * NX, 32), smem, st>>>(g, np, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl);
-  }
+#define HST_XPROD(NT, PPT)        \
+  big_smem(d, k_xprod<NT, PPT>); \
+  k_xprod<NT, PPT><<<grid, fft_threads(6 * NX, PPT), smem, st>>>(g, np, d.Z, d.Pp, d.twx, d.dyl, ph, want_cfl, d.cfl)
+  HST_SHORT_X(NX, 6 * NX, HST_XPROD)
+#undef HST_XPROD
   return cudaGetLastError();
 }
 
