@@ -452,7 +452,7 @@ static int der_rows(const std::vector<double>& der, int ny, std::vector<double>&
     for (int u = 0; u < nu; ++u) tab[(size_t)q * nu + u] = der[(size_t)first[u] + (size_t)ny * q];
   return nu;
 }
-// uploads der's distinct-row table (stream-ordered after everything before)
+// uploads der's distinct-row table; no kernel queued before may still read it
 static cudaError_t upload_der_rows(hst_ctx* ctx);
 
 static std::vector<double2> twiddles(int n) {
@@ -785,9 +785,8 @@ static cudaError_t upload_der_rows(hst_ctx* ctx) {
   std::vector<int> idx;
   const int ny = ctx->p.ny;
   const int nu = der_rows(ctx->der, ny, tab, idx);
-  // the kernels queued before may still read the previous table
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
-  if (e == cudaSuccess && nu > 0) e = cudaMemcpy(ctx->d.derU, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaSuccess;
+  if (nu > 0) e = cudaMemcpy(ctx->d.derU, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(ctx->d.derI, idx.data(), sizeof(int) * ny, cudaMemcpyHostToDevice);
   ctx->d.nderU = e == cudaSuccess ? nu : 0;
   ctx->db.derU = ctx->d.derU;
@@ -804,6 +803,9 @@ extern "C" int hst_gpu_set_tables(hst_ctx* ctx, const double* der, const double*
   if (!ctx) return HST_EARG;
   const int ny = ctx->p.ny;
   CK(cudaSetDevice(ctx->device));
+  // the copies below are not ordered with the context's stream, whose queued
+  // kernels may still read the tables
+  CK(cudaStreamSynchronize(ctx->stream));
   if (der) {
     std::memcpy(ctx->der.data(), der, sizeof(double) * 20 * ny);
     CK(cudaMemcpy(ctx->d.der, ctx->der.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice));
@@ -1117,8 +1119,11 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
   int rc = HST_OK;
   auto apply = [&](const Geometry& t) -> cudaError_t {
     g = t;
+    // the copy is not ordered with the stream, whose queued kernels may still read the table
+    cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return e;
     auto ds = hst::slab_major(ctx->der, g.ny, g.P);
-    cudaError_t e = cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = hst::launch_d0_table(g, ctx->d, ctx->stream);
     if (e == cudaSuccess) e = ensure_facg(ctx);
     return e;

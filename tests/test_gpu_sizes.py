@@ -196,6 +196,30 @@ def test_streamed_right_hand_sides_equal_row_by_row(monkeypatch, ny, exact, line
         assert rel_l2(a, b) <= 1e-13
 
 
+@pytest.mark.parametrize("change", ["tables", "autotune"])
+def test_queued_steps_keep_their_tables(change):
+    """new tables (and the trial tables of autotuning) take effect after the steps that are still queued: the same bits
+    as when the caller waits for those steps first"""
+    deck = c1_deck(nx=31, nz=32, ny=64, exact_shift=True)
+    other = hst.Solver(dict(deck, ystretch=0.8))
+    out = []
+    for wait in (True, False):
+        s = hst.Solver(deck)
+        s.time = 0.0
+        s.set_velocity(seeded_field(deck, seed=3))
+        s.timesteps(200)
+        if wait:
+            s.sync()
+        if change == "tables":
+            s.set_tables(der=other.der, y=other.y, dyl=other.dyl)
+        else:
+            s.autotune(deck["deltat"], steps=1)
+        out.append(s.velocity())
+        s.close()
+    other.close()
+    assert np.array_equal(*out)
+
+
 def test_a_replaced_grid_is_not_taken_as_uniform():
     """a caller that replaces der, y and dyl of a uniform deck by a stretched grid's gets the stretched deck's result
     (the node phases must follow the y table, not the deck), in both forms of the shift"""
