@@ -452,7 +452,10 @@ static int der_rows(const std::vector<double>& der, int ny, std::vector<double>&
     for (int u = 0; u < nu; ++u) tab[(size_t)q * nu + u] = der[(size_t)first[u] + (size_t)ny * q];
   return nu;
 }
-// uploads der's distinct-row table; no kernel queued before may still read it
+static cudaError_t upload(hst_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+}
+// uploads der's distinct-row table (stream-ordered after everything before)
 static cudaError_t upload_der_rows(hst_ctx* ctx);
 
 static std::vector<double2> twiddles(int n) {
@@ -660,7 +663,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   {
     auto ds = hst::slab_major(ctx->der, ny, g.P);
     cudaMemcpy(d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
-    ds = hst::slab_major(ctx->der, ny, g.PL);
+    if (g.PL != g.P) ds = hst::slab_major(ctx->der, ny, g.PL);
     cudaMemcpy(d.derL, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
     etab = hst::launch_d0_table(g, d, ctx->stream);
     if (etab == cudaSuccess) etab = upload_der_rows(ctx);
@@ -786,8 +789,8 @@ static cudaError_t upload_der_rows(hst_ctx* ctx) {
   const int ny = ctx->p.ny;
   const int nu = der_rows(ctx->der, ny, tab, idx);
   cudaError_t e = cudaSuccess;
-  if (nu > 0) e = cudaMemcpy(ctx->d.derU, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(ctx->d.derI, idx.data(), sizeof(int) * ny, cudaMemcpyHostToDevice);
+  if (nu > 0) e = upload(ctx, ctx->d.derU, tab.data(), sizeof(double) * tab.size());
+  if (e == cudaSuccess) e = upload(ctx, ctx->d.derI, idx.data(), sizeof(int) * ny);
   ctx->d.nderU = e == cudaSuccess ? nu : 0;
   ctx->db.derU = ctx->d.derU;
   ctx->db.derI = ctx->d.derI;
@@ -803,16 +806,15 @@ extern "C" int hst_gpu_set_tables(hst_ctx* ctx, const double* der, const double*
   if (!ctx) return HST_EARG;
   const int ny = ctx->p.ny;
   CK(cudaSetDevice(ctx->device));
-  // the copies below are not ordered with the context's stream, whose queued
-  // kernels may still read the tables
-  CK(cudaStreamSynchronize(ctx->stream));
+  // every copy in the order of the context's stream, whose queued kernels may
+  // still read the tables (a copy from pageable memory is staged by the call)
   if (der) {
     std::memcpy(ctx->der.data(), der, sizeof(double) * 20 * ny);
-    CK(cudaMemcpy(ctx->d.der, ctx->der.data(), sizeof(double) * 20 * ny, cudaMemcpyHostToDevice));
+    CK(upload(ctx, ctx->d.der, ctx->der.data(), sizeof(double) * 20 * ny));
     auto ds = hst::slab_major(ctx->der, ny, ctx->g.P);
-    CK(cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice));
-    ds = hst::slab_major(ctx->der, ny, ctx->g.PL);
-    CK(cudaMemcpy(ctx->d.derL, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice));
+    CK(upload(ctx, ctx->d.derS, ds.data(), sizeof(double) * ds.size()));
+    if (ctx->g.PL != ctx->g.P) ds = hst::slab_major(ctx->der, ny, ctx->g.PL);
+    CK(upload(ctx, ctx->d.derL, ds.data(), sizeof(double) * ds.size()));
     CK(hst::launch_d0_table(ctx->g, ctx->d, ctx->stream));
     CK(upload_der_rows(ctx));
   }

@@ -475,13 +475,18 @@ std::vector<double> slab_major(const std::vector<double>& der, int ny, int P) {
   const int mM = slab_rows(ny, P);
   const LineGeom G = line_geom(ny, P);
   std::vector<double> o((size_t)20 * mM * P, 0.0);
-  for (int s = 0; s < P; ++s) {
-    const int m = G.m + (s < G.rem ? 1 : 0), r0 = s * G.m + std::min(s, G.rem);
-    for (int n = 0; n < 4; ++n)
-      for (int j = 0; j < 5; ++j)
-        for (int i = 0; i < m; ++i)
-          o[((size_t)(n * 5 + j) * mM + i) * P + s] = der[(size_t)(r0 + i) + (size_t)ny * (n + 4 * j)];
-  }
+  std::vector<int> first(P);
+  for (int s = 0; s < P; ++s) first[s] = s * G.m + std::min(s, G.rem);
+  // in the table's own order (written across it, it took as long as the rest of
+  // hst_gpu_set_tables); the last place of a shorter slab stays zero
+  double* q = o.data();
+  for (int n = 0; n < 4; ++n)
+    for (int j = 0; j < 5; ++j) {
+      const double* const d = der.data() + (size_t)ny * (n + 4 * j);
+      for (int i = 0; i < mM; ++i)
+        for (int s = 0; s < P; ++s, ++q)
+          if (i < G.m || s < G.rem) *q = d[first[s] + i];
+    }
   return o;
 }
 
