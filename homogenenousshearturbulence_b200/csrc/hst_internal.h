@@ -165,7 +165,7 @@ cudaError_t launch_line_solve(const Geometry& g, const DeviceState& d, const Phy
 cudaError_t launch_fill_ghosts(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int field, double sx,
                                double sz, cudaStream_t st);
 // the factored D0 matrix of the line-solve group (P of g) into d.d0tab,
-// from d.derS; d0_table_doubles: the table's size for any group of ny rows
+// from d.der; d0_table_doubles: the table's size for any group of ny rows
 cudaError_t launch_d0_table(const Geometry& g, const DeviceState& d, cudaStream_t st);
 size_t d0_table_doubles(int ny);
 // outstats (src/hst_stats.f90:136-285): block count of the moments' reduction,

@@ -65,6 +65,13 @@ struct SlabDerT {
   }
 };
 
+// D0 of the slabs straight from der (Fortran order), first row r0 of slab s
+struct SlabD0 {
+  const double* __restrict__ der;
+  int ny, r0;
+  __device__ __forceinline__ double operator()(int, int i, int, int j) const { return __ldg(der + r0 + i + ny * (4 * j)); }
+};
+
 // A system's band entries before the wrap phase are c0 D0 + c2 D2 + c4 D4 with
 // constants of the column (coef, src/hst_linsolve.f90:236-252): NT = 3 (D2V),
 // 2 (ETA, POISSON: c4 = 0) or 1 (D0, DY: D0 itself).
@@ -282,16 +289,22 @@ __host__ __device__ constexpr int d0_levels(int P) {
 }
 __host__ __device__ constexpr int d0_fields(int mM, int P) { return 9 * (mM - 2) + 7 + 8 * d0_levels(P) + 24; }
 
-template <int P>
-__device__ void d0_factor(const SlabDerT<false>& DS, int m, int mM, int s, unsigned gmask, double* __restrict__ tab) {
+template <int P, class DST>
+__device__ void d0_factor(const DST& DS, int m, int mM, int s, unsigned gmask, double* __restrict__ tab) {
   const int mi = m - 2;
   const BandConst bc = {1.0, 0.0, 0.0};
   auto put = [&](int f, double v) { tab[(size_t)f * P + s] = v; };
   double u11 = 0, u12 = 0, p1 = 0, q1 = 0, u21 = 0, u22 = 0, p2 = 0, q2 = 0;
   double w1 = 0, w2 = 0, v1 = 0, v2 = 0, sp0 = 0, sq0 = 0, sp1 = 0, sq1 = 0;
+  // (the next row's entries are loaded before this row's fields are stored: the
+  // one warp's chain of rows would wait for them)
+  double next[5];
+  band_row<1>(bc, DS, s, 0, next);
   for (int i = 0; i < mi; ++i) {
     double a[5];
-    band_row<1>(bc, DS, s, i, a);
+#pragma unroll
+    for (int j = 0; j < 5; ++j) a[j] = next[j];
+    band_row<1>(bc, DS, s, i + 1, next);  // (row mi is the first border row)
     double p = 0, q = 0, l0 = 0, l1 = 0;
     if (i == 0) {
       p = a[0];

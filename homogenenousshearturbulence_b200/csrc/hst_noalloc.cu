@@ -11,8 +11,8 @@
 // cudaMalloc/cudaFree also synchronise the device in the middle of the
 // caller's queued work.  This entry point runs the same solve kernel as
 // hst_gpu_line_solve and keeps its one piece of working memory, the
-// slab-major copy of der that the solver groups read, in a fixed array in
-// the module's static device memory.
+// slab-major copy of der that the solver groups read (D0, DY: the factored
+// matrix), in a fixed array in the module's static device memory.
 //
 // Limits and rules of use:
 //   - ny <= HST_NOALLOC_MAX_NY (2048): the scratch holds 20 * 2048 doubles
@@ -48,11 +48,11 @@ namespace {
 // der(0:ny-1, 0:3, -2:2) reordered slab-major (the order of hst::slab_major)
 __device__ __align__(256) double g_line_der[20 * HST_NOALLOC_MAX_NY];
 
-// out[((n*5 + j)*mM + i)*P + s] = der(first(s) + i, n, j - 2) for n < slices; the
-// place past the end of a shorter slab repeats its last row
-__global__ void k_slab_major(const double* __restrict__ der, double* __restrict__ out, int ny, int P, int slices) {
+// out[((n*5 + j)*mM + i)*P + s] = der(first(s) + i, n, j - 2); the place past the
+// end of a shorter slab repeats its last row
+__global__ void k_slab_major(const double* __restrict__ der, double* __restrict__ out, int ny, int P) {
   const int mM = hst::slab_rows(ny, P), e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= slices * 5 * mM * P) return;
+  if (e >= 20 * mM * P) return;
   const hst::LineGeom G = hst::line_geom(ny, P);
   const int s = e % P;
   const int i = (e / P) % mM;
@@ -135,16 +135,16 @@ extern "C" int hst_gpu_line_solve_noalloc(int nx, int ny, int nz, double alfa0, 
   d.derS = d.derL = scratch;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-  // der slab by slab; for the D0 matrix its slice alone, and after it the
-  // factored table
-  const int slices = d0 ? 1 : 4, n = slices * 5 * hst::slab_rows(ny, P) * P, T = 256;
-  if (n + (d0 ? hst::d0_table_doubles(ny) : 0) > 20 * (size_t)HST_NOALLOC_MAX_NY)
+  // der slab by slab, or for the D0 matrix the factored table alone
+  const int n = 20 * hst::slab_rows(ny, P) * P, T = 256;
+  if ((d0 ? hst::d0_table_doubles(ny) : (size_t)n) > sizeof g_line_der / sizeof(double))
     return fail(msg, msg_len, HST_EARG, "ny = %d exceeds the static scratch", ny);
-  k_slab_major<<<(n + T - 1) / T, T, 0, st>>>(der, scratch, ny, P, slices);
-  e = cudaGetLastError();
   if (d0) {
-    d.d0tab = scratch + n;
-    if (e == cudaSuccess) e = hst::launch_d0_table(g, d, st);
+    d.d0tab = scratch;
+    e = hst::launch_d0_table(g, d, st);
+  } else {
+    k_slab_major<<<(n + T - 1) / T, T, 0, st>>>(der, scratch, ny, P);
+    e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = hst::launch_line_solve(g, d, ps, sys, lambda, 0, 1, shift_x, shift_z, st);
   if (e != cudaSuccess) return fail(msg, msg_len, HST_ECUDA, "launch: %s", cudaGetErrorString(e));

@@ -115,3 +115,33 @@ def test_noalloc_at_the_largest_size():
             err = rel_l2(out.cpu().numpy(), want)
             assert err <= TOL, (kind, err)
     s.close()
+
+
+def test_noalloc_d0_of_few_columns_costs_no_more_than_d2v():
+    """528 columns of 1024 rows: the D0 and DY solves factor their matrix first, once for all columns, which must not
+    outweigh the solves themselves (1.1 times the D2V solve is what this size shows; 1.4 and 1.5 with the factoring
+    waiting for each row's loads)"""
+    import torch
+
+    deck = c1_deck(nx=15, nz=16, ny=1024)
+    s = hst.Solver(deck)
+    der = torch.from_numpy(np.ascontiguousarray(s.der).ravel()).cuda()
+    src = torch.zeros(s.shape, dtype=torch.complex128, device="cuda")
+    dst = torch.zeros_like(src)
+    s.close()
+    f, stream = noalloc(), torch.cuda.current_stream().cuda_stream
+
+    def us(kind):
+        best = np.inf
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(20):
+                assert call(f, deck, kind, 100.0, der, src, dst, (0.1, 0.2), stream)[0] == 0
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 50.0)
+        return best
+
+    d2v = us(hst.KIND_D2V)
+    assert us(hst.KIND_D0) <= 1.25 * d2v and us(hst.KIND_DY) <= 1.4 * d2v
