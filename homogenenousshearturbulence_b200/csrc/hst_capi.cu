@@ -299,24 +299,29 @@ static bool damping_update(hst_ctx* c, double t) {
   return true;
 }
 
+// The pinned copies and their events, at creation: a table can change in any
+// substep, and a step allocates nothing.
+static cudaError_t alloc_gdamp(hst_ctx* ctx) {
+  int niz;
+  damping_box(ctx->p, &ctx->gd_nix, &niz);
+  ctx->gd_nix += 1;
+  cudaError_t e = cudaMallocHost((void**)&ctx->h_gdamp, sizeof(double) * (2 * (size_t)ctx->p.nz + 1) * ctx->gd_nix * hst_ctx::GD_SLOTS);
+  for (cudaEvent_t& ev : ctx->ev_gd)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  return e;
+}
+
 // The damping table's x modes that can be damped, uploaded in stream order (an
 // oscillating S2 turns the damped region every substep): one of GD_SLOTS pinned
 // copies is refilled, once the copy from it GD_SLOTS updates ago has gone out,
 // so that the host does not wait for the stream.
 static int upload_gdamp(hst_ctx* ctx) {
   const size_t nzT = 2 * (size_t)ctx->p.nz + 1;
-  if (!ctx->h_gdamp) {
-    int niz;
-    damping_box(ctx->p, &ctx->gd_nix, &niz);
-    ctx->gd_nix += 1;
-    CK(cudaMallocHost((void**)&ctx->h_gdamp, sizeof(double) * nzT * ctx->gd_nix * hst_ctx::GD_SLOTS));
-  }
   const int k = ctx->gd_next;
   ctx->gd_next = (k + 1) % hst_ctx::GD_SLOTS;
   const size_t n = nzT * ctx->gd_nix;
   double* const slot = ctx->h_gdamp + n * k;
-  if (ctx->ev_gd[k]) CK(cudaEventSynchronize(ctx->ev_gd[k]));
-  else CK(cudaEventCreateWithFlags(&ctx->ev_gd[k], cudaEventDisableTiming));
+  CK(cudaEventSynchronize(ctx->ev_gd[k]));  // (at once, before its first record)
   std::memcpy(slot, ctx->gdamp.data(), sizeof(double) * n);
   CK(cudaMemcpyAsync(ctx->d.gdamp, slot, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaEventRecord(ctx->ev_gd[k], ctx->stream));
@@ -704,6 +709,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   if (e == cudaSuccess) e = hst::make_z_maps(ctx->gb, ctx->db);
   if (e == cudaSuccess) e = hst::make_z_maps(g, d);
   if (e == cudaSuccess) e = ensure_facg(ctx);
+  if (e == cudaSuccess && damping_active(p)) e = alloc_gdamp(ctx);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {

@@ -1,7 +1,9 @@
 """Helpers shared by the GPU tests: building matching oracle and GPU runs."""
+import json
 import math
 
 import numpy as np
+import torch
 
 import oracle
 from homogenenousshearturbulence_b200 import hst
@@ -64,3 +66,13 @@ def seeded_field(deck, seed=1, k0=4.0, energy=0.1):
     s_y = oracle.Sim(deck_to_oracle(deck)).y()
     return hst.random_field(deck["nx"], deck["ny"], deck["nz"], deck["alfa0"], deck["beta0"], deck["ly"], s_y,
                             seed=seed, k0=k0, energy=energy)
+
+
+def traced(s, steps, tmp_path):
+    """The trace events (kernels with their grids, runtime calls) of `steps` time steps of a solver."""
+    torch.cuda.init()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        s.timesteps(steps)
+        s.sync()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    return json.loads((tmp_path / "trace.json").read_text())["traceEvents"]

@@ -2,14 +2,11 @@
 (hst_gpu_create_batch): every kernel of the substep covers all members in one
 launch; each member must evolve exactly as it does alone in its own
 context."""
-import json
-
 import numpy as np
 import pytest
-import torch
 
 from homogenenousshearturbulence_b200 import hst
-from tests.gpu_util import c1_deck, rel_l2, seeded_field
+from tests.gpu_util import c1_deck, rel_l2, seeded_field, traced
 
 pytestmark = pytest.mark.gpu
 
@@ -59,12 +56,7 @@ def test_ensemble_members_match_single_contexts(case):
 
 def blocks_of_a_step(s, tmp_path):
     """{kernel: the blocks of its launch} of one time step"""
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        s.timesteps(1)
-        s.sync()
-    prof.export_chrome_trace(str(tmp_path / "trace.json"))
-    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
-    return {name: int(np.prod(e["args"]["grid"])) for e in events if e.get("cat") == "kernel"
+    return {name: int(np.prod(e["args"]["grid"])) for e in traced(s, 1, tmp_path) if e.get("cat") == "kernel"
             for name in ("k_shift", "k_solve_half") if name in e["name"]}
 
 
@@ -74,7 +66,6 @@ def test_ensemble_solves_run_on_all_blocks(members, nx, ny, nz, tmp_path):
     the shift, which has the same warps and needs no factor scratch: the
     scratch holds the columns of every member, not of one."""
     deck = c1_deck(nx=nx, ny=ny, nz=nz, exact_shift=True)
-    torch.cuda.init()
     s = hst.Solver(deck, members=members)
     s.time = 0.0
     s.timesteps(1)

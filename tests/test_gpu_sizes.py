@@ -13,7 +13,7 @@ import torch
 
 import oracle
 from homogenenousshearturbulence_b200 import hst
-from tests.gpu_util import c1_deck, make_pair, rel_l2, run_pair, seeded_field
+from tests.gpu_util import c1_deck, make_pair, rel_l2, run_pair, seeded_field, traced
 
 pytestmark = pytest.mark.gpu
 
@@ -194,6 +194,17 @@ def test_streamed_right_hand_sides_equal_row_by_row(monkeypatch, ny, exact, line
         s.close()
     for a, b in zip(*out):
         assert rel_l2(a, b) <= 1e-13
+
+
+@pytest.mark.parametrize("over", [dict(), dict(damp_hard=True, damp_kpar=2.0, damp_kperp=2.0, s2_amplitude=0.5, s2_period=0.7)])
+def test_the_first_steps_allocate_nothing(over, tmp_path):
+    """every buffer of a step, the pinned copies of a turning damping table among them, is there once the context is"""
+    s = hst.Solver(c1_deck(exact_shift=True, **over))
+    s.time = 0.1
+    calls = [e["name"] for e in traced(s, 2, tmp_path) if e.get("cat") == "cuda_runtime"]
+    s.close()
+    assert any("Launch" in c for c in calls)
+    assert not [c for c in calls if "Malloc" in c or "HostAlloc" in c], calls
 
 
 @pytest.mark.parametrize("change", ["tables", "autotune"])
