@@ -473,7 +473,7 @@ static std::vector<double2> twiddles(int n) {
 }
 
 static void free_device(hst_ctx* c) {
-  if (c->nmem > 1) {
+  if (c->nmem > 1 && c->db.F[0]) {  // (set once every buffer is there)
     // the per-member buffers belong to the base; the view only points into them
     DeviceState& d = c->d;
     for (int i = 0; i < 7; ++i) d.F[i] = c->db.F[i];
@@ -649,15 +649,13 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   ok = ok && alloc((void**)&d.cfl, 2 * sizeof(unsigned long long));
   if (ok) d.err = reinterpret_cast<int*>(d.cfl + 1);
   if (!ok) {
-    free_device(ctx);
-    std::fprintf(stderr, "hst_gpu_create: device allocation of %.2f GB refused\n", dev_bytes(g) / 1e9);
-    delete ctx;
+    std::fprintf(stderr, "hst_gpu_create: device allocation of %.2f GB refused\n", nmem * dev_bytes(g) / 1e9);
+    hst_gpu_destroy(ctx);
     return HST_ENOMEM;
   }
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMallocHost((void**)&ctx->h_cfl, 2 * sizeof(unsigned long long)) != cudaSuccess) {
-    free_device(ctx);
-    delete ctx;
+    hst_gpu_destroy(ctx);
     return HST_ECUDA;
   }
   for (int i = 0; i < 7; ++i) cudaMemsetAsync(d.F[i], 0, sizeof(double2) * g.nf * nm, ctx->stream);
@@ -714,8 +712,7 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     std::fprintf(stderr, "hst_gpu_create: %s\n", cudaGetErrorString(e));
-    free_device(ctx);
-    delete ctx;
+    hst_gpu_destroy(ctx);
     return HST_ECUDA;
   }
   *out = ctx;

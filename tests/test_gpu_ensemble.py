@@ -4,6 +4,7 @@ launch; each member must evolve exactly as it does alone in its own
 context."""
 import numpy as np
 import pytest
+import torch
 
 from homogenenousshearturbulence_b200 import hst
 from tests.gpu_util import c1_deck, rel_l2, seeded_field, traced
@@ -73,6 +74,18 @@ def test_ensemble_solves_run_on_all_blocks(members, nx, ny, nz, tmp_path):
     got = blocks_of_a_step(s, tmp_path)
     assert got["k_shift"] > 0 and got["k_solve_half"] == got["k_shift"], got
     s.close()
+
+
+def test_a_refused_ensemble_gives_its_memory_back():
+    """more members than the device holds: the creation is refused half way, and what it had allocated is free again"""
+    hst.Solver(c1_deck(), members=2).close()
+    free = torch.cuda.mem_get_info()[0]
+    deck = c1_deck()
+    members = int(1.1 * free / hst.device_bytes(**{k: deck[k] for k in ("nx", "ny", "nz", "alfa0", "beta0", "ly")}))
+    with pytest.raises(hst.HstError) as e:
+        hst.Solver(deck, members=min(members, 4096))
+    assert e.value.code == hst.ENOMEM
+    assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)
 
 
 def test_ensemble_refuses_bad_members():
