@@ -19,7 +19,6 @@ __device__ __forceinline__ cxd cneg(cxd a) { return mkc(-a.x, -a.y); }
 __device__ __forceinline__ cxd cmuli(double b, cxd a) { return mkc(-b * a.y, b * a.x); }
 // a - s * b (s real)
 __device__ __forceinline__ cxd cfms(cxd a, double s, cxd b) { return mkc(a.x - s * b.x, a.y - s * b.y); }
-__device__ __forceinline__ cxd cdivr(cxd a, double d) { return mkc(a.x / d, a.y / d); }
 // max that propagates NaN (fmax returns the other operand), as a positive
 // quiet NaN
 __device__ __forceinline__ double nan_max(double a, double b) {
@@ -30,16 +29,6 @@ __device__ __forceinline__ cxd cexpi(double x) {
   double s, c;
   sincos(x, &s, &c);
   return mkc(c, s);
-}
-// complex division with range reduction (Smith)
-__device__ __forceinline__ cxd cdiv(cxd a, cxd b) {
-  if (fabs(b.x) >= fabs(b.y)) {
-    double r = b.y / b.x, d = b.x + b.y * r;
-    return mkc((a.x + a.y * r) / d, (a.y - a.x * r) / d);
-  } else {
-    double r = b.x / b.y, d = b.x * r + b.y;
-    return mkc((a.x * r + a.y) / d, (a.y * r - a.x) / d);
-  }
 }
 // the same operations on complex64 (the transforms of the mixed-precision form)
 typedef float2 cxf;
@@ -122,7 +111,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
 }
 
 // waits until the kernels before this one in the stream have finished and their
-// writes are visible (a launch_after kernel may start earlier)
+// writes are visible (a launch_after kernel may start a little earlier)
 __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // a load of a field another kernel of the substep writes: an ordinary load,

@@ -417,11 +417,9 @@ __device__ void d0_factor(const DST& DS, int m, int mM, int s, unsigned gmask, d
   put2(f + 20, shfl_m2(gmask, Di, q, P));
 }
 
-// The solve with the D0 matrix from the table of d0_factor, on NR lines at
-// once (sb[k] each as line_solve's sb): the lines share every table load and
-// run as independent dependency chains.  d0_forward runs the forward sweep and
-// the reduction and leaves each lane the borders of its slab (c: its own last
-// two rows, y: those of the slab below).
+// The solve with the D0 matrix from the table of d0_factor (sb as line_solve's).
+// d0_forward runs the forward sweep and the reduction and leaves each lane the
+// borders of its slab (c: its own last two rows, y: those of the slab below).
 template <int P, bool SH>
 struct D0Table {
   const double* __restrict__ ts;  // tab + s
@@ -435,54 +433,45 @@ struct D0Table {
     return M2{(*this)(f), (*this)(f + 1), (*this)(f + 2), (*this)(f + 3)};
   }
 };
-template <int P, int NR, class TAB>
-__device__ __forceinline__ void d0_forward(cxd ph, const TAB& T, int mM, int m, cxd* const* sb, int s, unsigned gmask,
-                                           V2c* c, V2c* y) {
+template <int P, class TAB>
+__device__ __forceinline__ void d0_forward(cxd ph, const TAB& T, int mM, int m, cxd* sb, int s, unsigned gmask, V2c& c,
+                                           V2c& y) {
   const int mi = m - 2;
-  cxd x1[NR], x2[NR], sx0[NR], sx1[NR];
+  cxd x1, x2, sx0, sx1;
   {
     const double rp0 = T(2), l1 = T(10), rp1 = T(11), w = T(12);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      x2[k] = cscale(rp0, sb[k][0]);
-      sb[k][0] = x2[k];
-      x1[k] = cscale(rp1, cfms(sb[k][1], l1, x2[k]));
-      sb[k][1] = x1[k];
-      sx0[k] = mkc(x2[k].x + w * x1[k].x, x2[k].y + w * x1[k].y);
-      sx1[k] = x1[k];
-    }
+    x2 = cscale(rp0, sb[0]);
+    sb[0] = x2;
+    x1 = cscale(rp1, cfms(sb[1], l1, x2));
+    sb[1] = x1;
+    sx0 = mkc(x2.x + w * x1.x, x2.y + w * x1.y);
+    sx1 = x1;
   }
 #pragma unroll 2
   for (int i = 2; i < mi; ++i) {
     const double l0 = T(9 * i + 0), l1 = T(9 * i + 1), rp = T(9 * i + 2), w = T(9 * i + 3), v = T(9 * i + 4);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const cxd bx = cscale(rp, cfms(cfms(sb[k][i], l0, x2[k]), l1, x1[k]));
-      sb[k][i] = bx;
-      sx0[k] = mkc(sx0[k].x + w * bx.x, sx0[k].y + w * bx.y);
-      sx1[k] = mkc(sx1[k].x + v * bx.x, sx1[k].y + v * bx.y);
-      x2[k] = x1[k];
-      x1[k] = bx;
-    }
+    const cxd bx = cscale(rp, cfms(cfms(sb[i], l0, x2), l1, x1));
+    sb[i] = bx;
+    sx0 = mkc(sx0.x + w * bx.x, sx0.y + w * bx.y);
+    sx1 = mkc(sx1.x + v * bx.x, sx1.y + v * bx.y);
+    x2 = x1;
+    x1 = bx;
   }
   const int B = 9 * (mM - 2);
-  V2c r[NR];
+  V2c r;
   {
     const double u21 = T(B), c1m4 = T(B + 1), c1m3 = T(B + 2), c10 = T(B + 3), c2m3 = T(B + 4), c20 = T(B + 5),
                  c21 = T(B + 6);
     const int t = (s + 1) & (P - 1);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      cxd TX0 = shfl_c(gmask, sx0[k], t, P), TX1 = shfl_c(gmask, sx1[k], t, P);
-      if (s == P - 1) {
-        TX0 = cmul(TX0, ph);
-        TX1 = cmul(TX1, ph);
-      }
-      const cxd XM2 = csub(x2[k], cscale(u21, x1[k]));
-      const cxd RB1 = sb[k][mi], RB2 = sb[k][mi + 1];
-      r[k].u = mkc(RB1.x - c1m4 * XM2.x - c1m3 * x1[k].x - c10 * TX0.x, RB1.y - c1m4 * XM2.y - c1m3 * x1[k].y - c10 * TX0.y);
-      r[k].v = mkc(RB2.x - c2m3 * x1[k].x - c20 * TX0.x - c21 * TX1.x, RB2.y - c2m3 * x1[k].y - c20 * TX0.y - c21 * TX1.y);
+    cxd TX0 = shfl_c(gmask, sx0, t, P), TX1 = shfl_c(gmask, sx1, t, P);
+    if (s == P - 1) {
+      TX0 = cmul(TX0, ph);
+      TX1 = cmul(TX1, ph);
     }
+    const cxd XM2 = csub(x2, cscale(u21, x1));
+    const cxd RB1 = sb[mi], RB2 = sb[mi + 1];
+    r.u = mkc(RB1.x - c1m4 * XM2.x - c1m3 * x1.x - c10 * TX0.x, RB1.y - c1m4 * XM2.y - c1m3 * x1.y - c10 * TX0.y);
+    r.v = mkc(RB2.x - c2m3 * x1.x - c20 * TX0.x - c21 * TX1.x, RB2.y - c2m3 * x1.y - c20 * TX0.y - c21 * TX1.y);
   }
   const cxd phc = cconj(ph);
   int f = B + 7;
@@ -490,11 +479,8 @@ __device__ __forceinline__ void d0_forward(cxd ph, const TAB& T, int mM, int m, 
   for (int d = 1; 2 * d < P; d <<= 1, f += 8) {
     const int sm = (s - d) & (P - 1), sp = (s + d) & (P - 1);
     const M2 A = T.m2(f), Gm = T.m2(f + 4);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const V2c rm = shfl_rhs(gmask, r[k], sm, P, s < d, phc), rq = shfl_rhs(gmask, r[k], sp, P, s + d >= P, ph);
-      r[k] = v2sub(v2sub(r[k], m2vec(A, rm)), m2vec(Gm, rq));
-    }
+    const V2c rm = shfl_rhs(gmask, r, sm, P, s < d, phc), rq = shfl_rhs(gmask, r, sp, P, s + d >= P, ph);
+    r = v2sub(v2sub(r, m2vec(A, rm)), m2vec(Gm, rq));
   }
   {
     const int q = s ^ (P >> 1);
@@ -511,14 +497,10 @@ __device__ __forceinline__ void d0_forward(cxd ph, const TAB& T, int mM, int m, 
     const C2 S = c2mul(M, Mq);
     const C2 S1 = {mkc(1.0 - S.a.x, -S.a.y), cneg(S.b), cneg(S.c), mkc(1.0 - S.d.x, -S.d.y)};
     const M2 Di = T.m2(f + 16), Dq = T.m2(f + 20);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const V2c rr = m2vec(Di, r[k]), rq = m2vec(Dq, shfl_v2(gmask, r[k], q, P));
-      c[k] = c2solve1(S1, v2sub(rr, c2vec(M, rq)));
-    }
+    const V2c rr = m2vec(Di, r), rq = m2vec(Dq, shfl_v2(gmask, r, q, P));
+    c = c2solve1(S1, v2sub(rr, c2vec(M, rq)));
   }
-#pragma unroll
-  for (int k = 0; k < NR; ++k) y[k] = shfl_rhs(gmask, c[k], (s - 1) & (P - 1), P, s == 0, phc);
+  y = shfl_rhs(gmask, c, (s - 1) & (P - 1), P, s == 0, phc);
 }
 // one row of the back substitution: row i of the slab from its forward value,
 // the borders below and the two rows above
@@ -533,101 +515,90 @@ __device__ __forceinline__ void line_solve_d0(cxd ph, const double* __restrict__
                                               unsigned gmask) {
   const int mi = m - 2;
   const D0Table<P, SH> T = {tab + s};
-  cxd* const sbs[1] = {sb};
-  V2c c[1], y[1];
-  d0_forward<P, 1>(ph, T, mM, m, sbs, s, gmask, c, y);
-  cxd xk1 = c[0].u, xk2 = c[0].v;
+  V2c c, y;
+  d0_forward<P>(ph, T, mM, m, sb, s, gmask, c, y);
+  cxd xk1 = c.u, xk2 = c.v;
   sb[mi] = xk1;
   sb[mi + 1] = xk2;
 #pragma unroll 2
   for (int i = mi - 1; i >= 0; --i) {
-    const cxd xk = d0_back(T, i, sb[i], y[0], xk1, xk2);
+    const cxd xk = d0_back(T, i, sb[i], y, xk1, xk2);
     sb[i] = xk;
     xk2 = xk1;
     xk1 = xk;
   }
 }
 
-// NR lines shifted in place (shift_unweighted, src/hst_equations.f90:263-293):
+// A line shifted in place (shift_unweighted, src/hst_equations.f90:263-293):
 // the D0 solve with the wrap pt, row r times the node phase, the D0 stencil
 // with the ghost images of pn.  The stencil follows two rows behind the back
 // substitution in registers; the rows at the slab's ends wait for the
 // neighbours' (the sums run over j = -2..2 in order).  node(i): the phase of row
 // i of the slab, asked for from the last row down.
-template <int P, int NR, class TAB, class DST, class NODE>
-__device__ __forceinline__ void shift_lines(cxd pt, cxd pn, const TAB& T, const DST& DS, int mM, int m, cxd* const* sb,
-                                            int s, unsigned gmask, NODE& node) {
-  V2c c[NR], y[NR];
-  d0_forward<P, NR>(pt, T, mM, m, sb, s, gmask, c, y);
-  cxd xk1[NR], xk2[NR];              // rows i + 1, i + 2 of the solution
-  cxd z1[NR], z2[NR], z3[NR], z4[NR];  // rows i + 1 .. i + 4 times their phases
-  cxd top0[NR], top1[NR];            // rows m - 2, m - 1 likewise
+template <int P, class TAB, class DST, class NODE>
+__device__ __forceinline__ void shift_line(cxd pt, cxd pn, const TAB& T, const DST& DS, int mM, int m, cxd* sb, int s,
+                                           unsigned gmask, NODE& node) {
+  V2c c, y;
+  d0_forward<P>(pt, T, mM, m, sb, s, gmask, c, y);
+  cxd xk1, xk2;        // rows i + 1, i + 2 of the solution
+  cxd z1, z2, z3, z4;  // rows i + 1 .. i + 4 times their phases
+  cxd top0, top1;      // rows m - 2, m - 1 likewise
   {
     const cxd e1 = node(m - 1), e0 = node(m - 2), f1 = node(m - 3), f0 = node(m - 4);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      top1[k] = cmul(c[k].v, e1);
-      top0[k] = cmul(c[k].u, e0);
-      const cxd a = d0_back(T, m - 3, sb[k][m - 3], y[k], c[k].u, c[k].v);
-      const cxd b = d0_back(T, m - 4, sb[k][m - 4], y[k], a, c[k].u);
-      xk1[k] = b;
-      xk2[k] = a;
-      z4[k] = top1[k];
-      z3[k] = top0[k];
-      z2[k] = cmul(a, f1);
-      z1[k] = cmul(b, f0);
-      // the sums of rows m - 1 and m - 2 over the rows of this slab
-      const double h0 = DS(s, m - 1, 0, 0), h1 = DS(s, m - 1, 0, 1), h2 = DS(s, m - 1, 0, 2);
-      const double g0 = DS(s, m - 2, 0, 0), g1 = DS(s, m - 2, 0, 1), g2 = DS(s, m - 2, 0, 2), g3 = DS(s, m - 2, 0, 3);
-      sb[k][m - 1] = mkc(h0 * z2[k].x + h1 * z3[k].x + h2 * z4[k].x, h0 * z2[k].y + h1 * z3[k].y + h2 * z4[k].y);
-      sb[k][m - 2] = mkc(g0 * z1[k].x + g1 * z2[k].x + g2 * z3[k].x + g3 * z4[k].x,
-                         g0 * z1[k].y + g1 * z2[k].y + g2 * z3[k].y + g3 * z4[k].y);
-    }
+    top1 = cmul(c.v, e1);
+    top0 = cmul(c.u, e0);
+    const cxd a = d0_back(T, m - 3, sb[m - 3], y, c.u, c.v);
+    const cxd b = d0_back(T, m - 4, sb[m - 4], y, a, c.u);
+    xk1 = b;
+    xk2 = a;
+    z4 = top1;
+    z3 = top0;
+    z2 = cmul(a, f1);
+    z1 = cmul(b, f0);
+    // the sums of rows m - 1 and m - 2 over the rows of this slab
+    const double h0 = DS(s, m - 1, 0, 0), h1 = DS(s, m - 1, 0, 1), h2 = DS(s, m - 1, 0, 2);
+    const double g0 = DS(s, m - 2, 0, 0), g1 = DS(s, m - 2, 0, 1), g2 = DS(s, m - 2, 0, 2), g3 = DS(s, m - 2, 0, 3);
+    sb[m - 1] = mkc(h0 * z2.x + h1 * z3.x + h2 * z4.x, h0 * z2.y + h1 * z3.y + h2 * z4.y);
+    sb[m - 2] = mkc(g0 * z1.x + g1 * z2.x + g2 * z3.x + g3 * z4.x, g0 * z1.y + g1 * z2.y + g2 * z3.y + g3 * z4.y);
   }
 #pragma unroll 2
   for (int i = m - 5; i >= 0; --i) {
     const cxd e = node(i);
     const double c0 = DS(s, i + 2, 0, 0), c1 = DS(s, i + 2, 0, 1), c2 = DS(s, i + 2, 0, 2), c3 = DS(s, i + 2, 0, 3),
                  c4 = DS(s, i + 2, 0, 4);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const cxd x = d0_back(T, i, sb[k][i], y[k], xk1[k], xk2[k]);
-      const cxd z = cmul(x, e);
-      sb[k][i + 2] = mkc(c0 * z.x + c1 * z1[k].x + c2 * z2[k].x + c3 * z3[k].x + c4 * z4[k].x,
-                         c0 * z.y + c1 * z1[k].y + c2 * z2[k].y + c3 * z3[k].y + c4 * z4[k].y);
-      xk2[k] = xk1[k];
-      xk1[k] = x;
-      z4[k] = z3[k];
-      z3[k] = z2[k];
-      z2[k] = z1[k];
-      z1[k] = z;
-    }
+    const cxd x = d0_back(T, i, sb[i], y, xk1, xk2);
+    const cxd z = cmul(x, e);
+    sb[i + 2] = mkc(c0 * z.x + c1 * z1.x + c2 * z2.x + c3 * z3.x + c4 * z4.x,
+                    c0 * z.y + c1 * z1.y + c2 * z2.y + c3 * z3.y + c4 * z4.y);
+    xk2 = xk1;
+    xk1 = x;
+    z4 = z3;
+    z3 = z2;
+    z2 = z1;
+    z1 = z;
   }
   // the slab's ends
   const int up = (s + 1) & (P - 1), dn = (s - 1) & (P - 1);
-#pragma unroll
-  for (int k = 0; k < NR; ++k) {
-    cxd a0 = shfl_c(gmask, z1[k], up, P), a1 = shfl_c(gmask, z2[k], up, P);
-    cxd b0 = shfl_c(gmask, top0[k], dn, P), b1 = shfl_c(gmask, top1[k], dn, P);
-    if (s == P - 1) {
-      a0 = cmul(a0, pn);
-      a1 = cmul(a1, pn);
-    }
-    if (s == 0) {
-      b0 = cmul(b0, cconj(pn));
-      b1 = cmul(b1, cconj(pn));
-    }
-    const double h3 = DS(s, m - 1, 0, 3), h4 = DS(s, m - 1, 0, 4), g4 = DS(s, m - 2, 0, 4);
-    const cxd t1 = sb[k][m - 1], t0 = sb[k][m - 2];
-    sb[k][m - 1] = mkc(t1.x + h3 * a0.x + h4 * a1.x, t1.y + h3 * a0.y + h4 * a1.y);
-    sb[k][m - 2] = mkc(t0.x + g4 * a0.x, t0.y + g4 * a0.y);
-    const double p0 = DS(s, 0, 0, 0), p1 = DS(s, 0, 0, 1), p2 = DS(s, 0, 0, 2), p3 = DS(s, 0, 0, 3), p4 = DS(s, 0, 0, 4);
-    const double q0 = DS(s, 1, 0, 0), q1 = DS(s, 1, 0, 1), q2 = DS(s, 1, 0, 2), q3 = DS(s, 1, 0, 3), q4 = DS(s, 1, 0, 4);
-    sb[k][0] = mkc(p0 * b0.x + p1 * b1.x + p2 * z1[k].x + p3 * z2[k].x + p4 * z3[k].x,
-                   p0 * b0.y + p1 * b1.y + p2 * z1[k].y + p3 * z2[k].y + p4 * z3[k].y);
-    sb[k][1] = mkc(q0 * b1.x + q1 * z1[k].x + q2 * z2[k].x + q3 * z3[k].x + q4 * z4[k].x,
-                   q0 * b1.y + q1 * z1[k].y + q2 * z2[k].y + q3 * z3[k].y + q4 * z4[k].y);
+  cxd a0 = shfl_c(gmask, z1, up, P), a1 = shfl_c(gmask, z2, up, P);
+  cxd b0 = shfl_c(gmask, top0, dn, P), b1 = shfl_c(gmask, top1, dn, P);
+  if (s == P - 1) {
+    a0 = cmul(a0, pn);
+    a1 = cmul(a1, pn);
   }
+  if (s == 0) {
+    b0 = cmul(b0, cconj(pn));
+    b1 = cmul(b1, cconj(pn));
+  }
+  const double h3 = DS(s, m - 1, 0, 3), h4 = DS(s, m - 1, 0, 4), g4 = DS(s, m - 2, 0, 4);
+  const cxd t1 = sb[m - 1], t0 = sb[m - 2];
+  sb[m - 1] = mkc(t1.x + h3 * a0.x + h4 * a1.x, t1.y + h3 * a0.y + h4 * a1.y);
+  sb[m - 2] = mkc(t0.x + g4 * a0.x, t0.y + g4 * a0.y);
+  const double p0 = DS(s, 0, 0, 0), p1 = DS(s, 0, 0, 1), p2 = DS(s, 0, 0, 2), p3 = DS(s, 0, 0, 3), p4 = DS(s, 0, 0, 4);
+  const double q0 = DS(s, 1, 0, 0), q1 = DS(s, 1, 0, 1), q2 = DS(s, 1, 0, 2), q3 = DS(s, 1, 0, 3), q4 = DS(s, 1, 0, 4);
+  sb[0] = mkc(p0 * b0.x + p1 * b1.x + p2 * z1.x + p3 * z2.x + p4 * z3.x,
+              p0 * b0.y + p1 * b1.y + p2 * z1.y + p3 * z2.y + p4 * z3.y);
+  sb[1] = mkc(q0 * b1.x + q1 * z1.x + q2 * z2.x + q3 * z3.x + q4 * z4.x,
+              q0 * b1.y + q1 * z1.y + q2 * z2.y + q3 * z3.y + q4 * z4.y);
 }
 
 // The five-point stencil n (0: D0, 1: D1) of a line held slab by slab in

@@ -138,7 +138,7 @@ __device__ __forceinline__ void copy_table(double* dst, const double* __restrict
 // shared-memory traffic of the tables and the lines; two lines at a time,
 // sharing the table loads, leave nine warps an SM and measured slower (3.42
 // against 2.62 ms at 768^2 x 512).
-constexpr int SHIFT_LINES = 1, SHIFT_WARPS = 16;
+constexpr int SHIFT_WARPS = 16;
 // SH: the tables in shared memory (the most rows have no room there)
 template <int P, bool SH>
 __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
@@ -156,11 +156,8 @@ __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
   copy_table(der0s, a.derS, nder);
   if (SH) __syncthreads();
   wait_predecessor();
-  const int lineN = P * G.MS;
-  cxd* const buf = reinterpret_cast<cxd*>(der0s + nder) + (size_t)grp * SHIFT_LINES * lineN;
-  cxd* sb[SHIFT_LINES];
-#pragma unroll
-  for (int k = 0; k < SHIFT_LINES; ++k) sb[k] = buf + k * lineN + s * G.MS;
+  cxd* const buf = reinterpret_cast<cxd*>(der0s + nder) + (size_t)grp * P * G.MS;
+  cxd* const sb = buf + s * G.MS;
   const int m = G.rows(s), r0 = G.first(s);
   const SlabDerT<SH> DS = {SH ? der0s : a.derS, mM, P};
   const D0Table<P, SH> T = {(SH ? d0s : a.d0tab) + s};
@@ -173,14 +170,9 @@ __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
     const cxd etop = sc.yuni ? cexpi(-gx * a.y[r0 + m + 1]) : mkc(1.0, 0.0);
     const cxd step = sc.yuni ? cexpi(gx * (sc.ytile / 32.0)) : mkc(1.0, 0.0);
 #pragma unroll 1
-    for (int q = 0; q < 4; q += SHIFT_LINES) {
-      double2* f[SHIFT_LINES];
-#pragma unroll
-      for (int k = 0; k < SHIFT_LINES; ++k) {
-        const int l = q + k;
-        f[k] = (l == 0 ? a.O1 : (l == 1 ? a.O2 : (l == 2 ? a.R1 : a.R2))) + c.cb;
-        load_line<P>(f[k], buf + k * lineN, G, s);
-      }
+    for (int q = 0; q < 4; ++q) {
+      double2* const f = (q == 0 ? a.O1 : (q == 1 ? a.O2 : (q == 2 ? a.R1 : a.R2))) + c.cb;
+      load_line<P>(f, buf, G, s);
       __syncwarp(gmask);
       cxd e = etop;
       auto node = [&](int i) -> cxd {
@@ -189,10 +181,9 @@ __global__ void __launch_bounds__(32 * SHIFT_WARPS, 1) k_shift(SolveArgs a) {
         e = cmul(e, step);
         return v;
       };
-      shift_lines<P, SHIFT_LINES>(pt, pn, T, DS, mM, m, sb, s, gmask, node);
+      shift_line<P>(pt, pn, T, DS, mM, m, sb, s, gmask, node);
       __syncwarp(gmask);
-#pragma unroll
-      for (int k = 0; k < SHIFT_LINES; ++k) store_line<P>(f[k], buf + k * lineN, G, s);
+      store_line<P>(f, buf, G, s);
       __syncwarp(gmask);
     }
   }
@@ -498,8 +489,8 @@ static int fac_elems(int ny, int P) { return 2 * (slab_rows(ny, P) - 2) * P; }
 // warps a block (one block an SM): as many as `most` whose groups' lines fit
 // beside `tabs` bytes of tables, and no more than spread the columns over the
 // SMs; 0 when not even one fits
-static int solve_warps(const Geometry& g, int nsm, size_t tabs, int lines = 1, int most = 16) {
-  const size_t warp = lines * line_bytes(g.ny, g.P) * (32 / g.P);
+static int solve_warps(const Geometry& g, int nsm, size_t tabs, int most = 16) {
+  const size_t warp = line_bytes(g.ny, g.P) * (32 / g.P);
   if (tabs + warp > 227 * 1024) return 0;
   const long groups = ((long)g.ncol * g.nmem + nsm - 1) / nsm;  // columns an SM
   const long want = (groups * g.P + 31) / 32;
@@ -522,18 +513,18 @@ static cudaError_t launch_shift_t(const SolveArgs& a, const DeviceState& d, cuda
   const Geometry& g = a.g;
   const int mM = slab_rows(g.ny, P), nsm = sm_count(d);
   size_t tabs = ((size_t)d0_fields(mM, P) * P + (size_t)5 * mM * P) * sizeof(double);
-  int W = solve_warps(g, nsm, tabs, SHIFT_LINES, SHIFT_WARPS);
-  const bool sh = W >= 4 || W == solve_warps(g, nsm, 0, SHIFT_LINES, SHIFT_WARPS);
+  int W = solve_warps(g, nsm, tabs, SHIFT_WARPS);
+  const bool sh = W >= 4 || W == solve_warps(g, nsm, 0, SHIFT_WARPS);
   if (!sh) {  // the tables through L1
     tabs = 0;
-    W = solve_warps(g, nsm, 0, SHIFT_LINES, SHIFT_WARPS);
+    W = solve_warps(g, nsm, 0, SHIFT_WARPS);
   }
   if (W < 1) return cudaErrorInvalidValue;
   const int groups = W * 32 / P;
   const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
   auto k = sh ? k_shift<P, true> : k_shift<P, false>;
   smem_limit(d, k, 227 * 1024);
-  return launch_after(k, dim3(nb), 32 * W, tabs + W * SHIFT_LINES * line_bytes(g.ny, P) * (32 / P), st, a);
+  return launch_after(k, dim3(nb), 32 * W, tabs + W * line_bytes(g.ny, P) * (32 / P), st, a);
 }
 
 template <int P>
