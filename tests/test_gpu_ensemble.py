@@ -15,7 +15,7 @@ CASES = {
     "default": dict(),
     "exact_s2_edges": dict(exact_shift=True, s2_amplitude=0.5, s2_period=0.7),  # nzd = 3 nz: ghost-row transforms
     "mixed": dict(precision="mixed", exact_shift=True),
-    "tall_persistent": dict(nx=15, nz=16, ny=512, exact_shift=True),  # 16-row slabs: the persistent solve stage
+    "tall": dict(nx=15, nz=16, ny=512, exact_shift=True),  # slabs of 16 rows
     # 3655 columns a member: three members together have enough for a narrower solver group than one
     "more_columns": dict(nx=42, nz=42),
     "hard_damping": dict(damp_kpar=3.0, damp_kperp=2.0, damp_hard=True, s2_amplitude=0.4, s2_period=0.5),

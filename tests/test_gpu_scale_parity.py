@@ -89,8 +89,8 @@ def check_both(name, substeps=30):
 def test_384x384x256_against_oracle():
     """The 384^2 x 256 workload (deck nx = 127, nz = 128, ny = 256), 30
     substeps: FP64 <= 1e-12 and mixed <= 1e-5 relative L2 against the
-    oracle.  Runs the FP64 k_zinv/k_zfwd 384-point 16-points-a-thread plans and
-    the 8-point x plan at 384 that the timed configuration uses."""
+    oracle.  Runs the 384-point x and z plans that the timed
+    configuration uses."""
     print(check_both("c2"))
 
 
