@@ -1085,7 +1085,8 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat);
 // Tries the launch choice that leaves every buffer's layout unchanged -- the
 // lanes of a line-solver group (P), every width that fits -- on this context's
 // own sizes, `steps` time steps each after one untimed step, keeps the
-// fastest, and puts the fields and the time back as they were.  The report lists every candidate with its time a step.
+// fastest, and puts the fields and the time back as they were.  The report
+// lists every candidate with its time a step.
 extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* report, int report_len) {
   if (!ctx || steps < 1) return fail(ctx, HST_EARG, "autotune: bad arguments");
   if (ctx->nmem > 1) return fail(ctx, HST_EARG, "autotune: not for an ensemble context");

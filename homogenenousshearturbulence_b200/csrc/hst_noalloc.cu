@@ -71,10 +71,10 @@ int fail(char* msg, int len, int rc, const char* fmt, ...) {
   return rc;
 }
 
-// lanes of a solver group: the rules of a context of one field of these sizes
-// (HST_LINE_LANES overrides), so the results are identical to those of such a
-// context that has not been autotuned; hst_gpu_autotune may give a context
-// another group width, and the two then agree up to rounding
+// lanes of a solver group: the rules of a context of these sizes (HST_LINE_LANES
+// overrides), so the results are identical to those of such a context.  D0 and
+// DY take the substep's width, which hst_gpu_autotune may change in a context;
+// the two then agree up to rounding
 int lanes_of(int ny, long columns, bool d0) {
   if (const int e = hst::line_lanes_asked(ny)) return e;
   return d0 ? hst::line_lanes(ny, columns) : hst::line_lanes_shared(ny);

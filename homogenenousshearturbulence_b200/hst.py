@@ -558,8 +558,8 @@ class Solver:
         return dict(zip(self.SUM_NAMES, sums)), exz
 
     def autotune(self, deltat=None, steps: int = 3) -> str:
-        """Pick the fastest line-solver group width and FFT plans for this
-        context's sizes (the fields are left as they were); returns the report."""
+        """Pick the fastest line-solver group width for this context's sizes
+        (the fields are left as they were); returns the report."""
         dt = self.deltat if deltat is None else float(deltat)
         buf = ct.create_string_buffer(4096)
         self._check(lib().hst_gpu_autotune(self._h, dt, int(steps), buf, 4096), "autotune")

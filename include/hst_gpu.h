@@ -101,8 +101,9 @@ int hst_gpu_create(const hst_gpu_params* p, hst_ctx** out);
  * physics, time step; their own initial fields) in one context, advanced
  * together -- hst_gpu_timestep / _timesteps run every member, each kernel
  * of the substep covering all members in one launch, and the CFL number is
- * the largest over the members.  The per-field device memory is nmem times
- * that of a single field; the tables are shared.  Every other entry point
+ * the largest over the members.  Each member evolves bit for bit as it does
+ * alone.  The per-field device memory is nmem times that of a single field;
+ * the tables are shared.  Every other entry point
  * (upload, download, fill_ghosts, line_solve, outstats, pressure, restart
  * files, the pieces, the asynchronous I/O) acts on the member chosen by
  * hst_gpu_select_member (member 0 at first).  hst_gpu_autotune refuses an
@@ -191,9 +192,10 @@ int hst_gpu_outstats(hst_ctx* ctx, double time, double* out);
 int hst_gpu_outstats_sums(hst_ctx* ctx, double time, double* sums, double* exz);
 
 /* Tries the launch choice that keeps every buffer's layout -- the lanes of
- * a line-solver group in the substep -- on this context's sizes (`steps` time steps of `deltat` each, after one
- * untimed step), keeps the fastest and restores the fields (V, OLD) and
- * the damping state.  A report of the candidates' times a step goes to
+ * a line-solver group in the substep -- on this context's sizes (`steps`
+ * time steps of `deltat` each, after one untimed step; widths without room
+ * are left out), keeps the fastest and restores the fields (V, OLD) and the
+ * damping state.  A report of the candidates' times a step goes to
  * report[0:report_len) when report is not NULL.  It allocates a copy of
  * five fields while it runs.  No counterpart in the reference. */
 int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* report, int report_len);
@@ -323,11 +325,11 @@ double hst_gpu_s2_integral(const hst_ctx* ctx, double t1, double t2);
 #define HST_KC_ZINV 0       /* z-inverse transform of V */
 #define HST_KC_XPROD 1      /* x transforms + products + CFL */
 #define HST_KC_ZFWD 2       /* z-forward transform of the products */
-#define HST_KC_COLUMN 3     /* the fused column kernel (right-hand sides, shift, solves, u, w) */
-#define HST_KC_LINE_SOLVE 4 /* hst_gpu_line_solve */
+#define HST_KC_COLUMN 3     /* the implicit solves, u and w (two kernels); hst_gpu_shear_shift */
+#define HST_KC_LINE_SOLVE 4 /* hst_gpu_line_solve, the solves of outstats and the pressure */
 #define HST_KC_GHOSTS 5     /* hst_gpu_fill_ghosts */
-#define HST_KC_RHS 6        /* the right-hand sides streamed row by row (when the column stage is split) */
-#define HST_KC_SHIFT 7      /* the exact_shift shear shift, when it runs as a kernel of its own */
+#define HST_KC_RHS 6        /* the right-hand sides */
+#define HST_KC_SHIFT 7      /* the exact_shift shear shift */
 #define HST_KC_N 8
 
 /* Per-kernel device time: with profiling on, every launch is bracketed by
@@ -360,9 +362,10 @@ void* hst_gpu_stream(const hst_ctx* ctx);
  * up the static array's address in the context current at that moment (a
  * lookup, not an allocation; a device reset may move the array); the first
  * call in a context may load the library's device code: make it before any
- * stream capture begins.  Results equal hst_gpu_line_solve's (both
- * take the group width of hst_gpu_line_solve, which the substep's and
- * hst_gpu_autotune leave alone).
+ * stream capture begins.  Results equal those of hst_gpu_line_solve in a
+ * context of these sizes bit for bit: HST_KIND_D2V, _ETA and _POISSON always,
+ * HST_KIND_D0 and _DY until hst_gpu_autotune picks another solver group width
+ * for that context (the two then agree up to rounding).
  * Errors: a negative HST_E* class, with a message in msg[0:msg_len) when msg
  * is not NULL.  No counterpart in the reference, whose line_solve always
  * works on its module arrays (src/hst_linsolve.f90:147). */
