@@ -15,8 +15,6 @@ __device__ __forceinline__ cxd cmul(cxd a, cxd b) { return mkc(a.x * b.x - a.y *
 __device__ __forceinline__ cxd cscale(double s, cxd a) { return mkc(s * a.x, s * a.y); }
 __device__ __forceinline__ cxd cconj(cxd a) { return mkc(a.x, -a.y); }
 __device__ __forceinline__ cxd cneg(cxd a) { return mkc(-a.x, -a.y); }
-// (0 + i b) * a
-__device__ __forceinline__ cxd cmuli(double b, cxd a) { return mkc(-b * a.y, b * a.x); }
 // a - s * b (s real)
 __device__ __forceinline__ cxd cfms(cxd a, double s, cxd b) { return mkc(a.x - s * b.x, a.y - s * b.y); }
 // max that propagates NaN (fmax returns the other operand), as a positive
