@@ -492,43 +492,8 @@ static void free_device(hst_ctx* c) {
                 d.derL};
   for (void* q : ps)
     if (q) cudaFree(q);
-  if (d.facg) cudaFree(d.facg);
   std::memset(&d, 0, sizeof d);
   d.configured = &c->configured;
-}
-
-// what a time step runs on: every member of an ensemble at once (the base
-// buffers), or the field itself
-static const Geometry& step_geometry(const hst_ctx* ctx) { return ctx->nmem > 1 ? ctx->gb : ctx->g; }
-
-// The line solves' factor scratch for the current group width: a slice for
-// every solver group that can be resident (sixteen warps an SM, the columns of
-// every member of an ensemble), or for as many as the device has room for (the
-// solves then run on fewer groups).
-static cudaError_t ensure_facg(hst_ctx* ctx) {
-  const int nsm = ctx->d.nsm > 0 ? ctx->d.nsm : 148;
-  const size_t need = hst::solve_scratch_bytes(step_geometry(ctx), nsm);
-  if (ctx->d.facg && ctx->d.facg_doubles * sizeof(double) >= need) return cudaSuccess;
-  if (ctx->d.facg) {
-    cudaError_t r = cudaStreamSynchronize(ctx->stream);
-    if (r != cudaSuccess) return r;
-    cudaFree(ctx->d.facg);
-    ctx->d.facg = nullptr;
-    ctx->d.facg_doubles = 0;
-  }
-  cudaError_t r = cudaSuccess;
-  for (size_t bytes = need; bytes >= need / nsm / 16; bytes /= 2) {
-    r = cudaMalloc((void**)&ctx->d.facg, bytes);
-    if (r == cudaSuccess) {
-      ctx->d.facg_doubles = bytes / sizeof(double);
-      break;
-    }
-    cudaGetLastError();
-    ctx->d.facg = nullptr;
-  }
-  ctx->db.facg = ctx->d.facg;
-  ctx->db.facg_doubles = ctx->d.facg_doubles;
-  return r;
 }
 
 // whether the y table is the uniform grid r ly / ny to rounding
@@ -706,7 +671,6 @@ static int create_context(const hst_gpu_params* pin, int nmem, hst_ctx** out) {
   if (e == cudaSuccess) e = hst::make_x_maps(g, d);
   if (e == cudaSuccess) e = hst::make_z_maps(ctx->gb, ctx->db);
   if (e == cudaSuccess) e = hst::make_z_maps(g, d);
-  if (e == cudaSuccess) e = ensure_facg(ctx);
   if (e == cudaSuccess && damping_active(p)) e = alloc_gdamp(ctx);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -1131,7 +1095,6 @@ extern "C" int hst_gpu_autotune(hst_ctx* ctx, double deltat, int steps, char* re
     auto ds = hst::slab_major(ctx->der, g.ny, g.P);
     e = cudaMemcpy(ctx->d.derS, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = hst::launch_d0_table(g, ctx->d, ctx->stream);
-    if (e == cudaSuccess) e = ensure_facg(ctx);
     return e;
   };
   for (int P : lanes) {
@@ -1298,7 +1261,8 @@ static int queue_timestep(hst_ctx* ctx, double* time, double deltat) {
                                   {120.0 / 20.0, 90.0 / 20.0, 50.0 / 20.0}};
   const hst_gpu_params& p = ctx->p;
   const bool damp = damping_active(p);
-  const Geometry& G = step_geometry(ctx);
+  // every member of an ensemble at once (the base buffers); the field itself otherwise
+  const Geometry& G = ctx->nmem > 1 ? ctx->gb : ctx->g;
   const DeviceState& D = ctx->nmem > 1 ? ctx->db : ctx->d;
   const char* env = std::getenv("HST_RHS_TILED");
   const bool tiled = !(env && std::atoi(env) == 0);

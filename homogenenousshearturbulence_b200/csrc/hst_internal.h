@@ -73,9 +73,6 @@ struct DeviceState {
   // kernels whose shared-memory limit has been raised in this context
   // (owned by the context; null: raise it at every launch)
   std::unordered_set<const void*>* configured;
-  // the line solves' factor scratch (a slice a resident solver group)
-  double* facg;
-  size_t facg_doubles;
 };
 
 // Raises kernel k's dynamic shared-memory limit to `bytes`, once per context
@@ -143,7 +140,8 @@ cudaError_t launch_rhs_tiled(const Geometry& g, const DeviceState& d, const Phys
 cudaError_t launch_rhs_rows(const Geometry& g, const DeviceState& d, const PhysScalars& ph, const SubstepScalars& sc,
                             int exact, int nonlin, cudaStream_t st);
 // the implicit half (hst_solve.cu): the exact_shift shift of RHS1/2, OLD1/2,
-// and the solves in two passes (half 0, then 1) from RHS1/2 into V1..V3
+// and the solves in two passes (half 0, then 1) from RHS1/2 into V1..V3, whose
+// factors go to Pp
 cudaError_t launch_shift(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
                          cudaStream_t st);
 cudaError_t launch_solve_half(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc,
@@ -160,8 +158,6 @@ int line_lanes_asked(int ny);
 // doubles that any P takes
 std::vector<double> slab_major(const std::vector<double>& der, int ny, int P);
 size_t slab_der_doubles(int ny);
-// bytes of the solves' factor scratch (DeviceState::facg)
-size_t solve_scratch_bytes(const Geometry& g, int nsm);
 cudaError_t launch_line_solve(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int sys, double lambda,
                               int src, int dst, double sx, double sz, cudaStream_t st);
 cudaError_t launch_fill_ghosts(const Geometry& g, const DeviceState& d, const PhysScalars& ph, int field, double sx,

@@ -18,7 +18,10 @@
 // warps share the tables in shared memory; the factors of the D2V and ETA
 // solves go to a slice of global scratch a group, rewritten column after
 // column (so that it stays in L2): without them in shared memory sixteen
-// warps' lines fit an SM.
+// warps' lines fit an SM.  The scratch is the product buffer Pp, whose contents
+// are dead from the z-forward transform to the next x stage: a group's slice is
+// that of its first column, at most 32 bytes a row and column, where Pp has at
+// least 48 (in FP32 48 nzd for the 2 nz + 1 columns of an x mode, nzd >= 3 nz).
 //
 // What bounds them: the dependent operations of a row's elimination and the
 // shared-memory pipe (512 rows: 73 % busy in k_shift, 50-60 % in the halves,
@@ -44,7 +47,7 @@ struct SolveArgs {
   const double* derS;
   const double* d0tab;
   const double* y;
-  double2* fac;  // factor scratch, facn double2 a group
+  double2* fac;  // factor scratch, facn double2 a group: the product buffer Pp, which is free between the transforms
   int facn;
 };
 
@@ -210,9 +213,9 @@ __global__ void __launch_bounds__(512, 1) k_solve_half(SolveArgs a) {
   cxd* const sb = buf + s * G.MS;
   const int m = G.rows(s);
   const SlabDerT<SH> DS = {SH ? smem_d : a.derS, mM, P};
-  const int slot = blockIdx.x * groups + grp;
-  double2* const fac = a.fac + (size_t)slot * a.facn + s;
-  for (int cg = first_column<P>(); cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
+  const int first = first_column<P>();
+  double2* const fac = a.fac + (size_t)first * a.facn + s;
+  for (int cg = first; cg < g.ncol * g.nmem; cg += gridDim.x * groups) {
     const Column c = column_of(g, a.ps, cg);
     const cxd pn = cexpi(-(c.al * sc.sx_n + c.be * sc.sz_n));
     double2* const v1 = a.V1 + c.cb;
@@ -497,14 +500,9 @@ static int solve_warps(const Geometry& g, int nsm, size_t tabs, int most = 16) {
   return (int)std::min<long>({most, want, (long)((227 * 1024 - tabs) / warp)});
 }
 
-size_t solve_scratch_bytes(const Geometry& g, int nsm) {
-  const size_t most = (size_t)nsm * 16 * (32 / g.P), cols = (size_t)g.ncol * g.nmem + 16 * (32 / g.P);
-  return std::min(most, cols) * fac_elems(g.ny, g.P) * sizeof(double2);
-}
-
 static SolveArgs solve_args(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc) {
   return {g,      ps,     sc,     d.F[0], d.F[1],  d.F[2], d.F[3],
-          d.F[4], d.F[5], d.F[6], d.derS, d.d0tab, d.y,    reinterpret_cast<double2*>(d.facg), fac_elems(g.ny, g.P)};
+          d.F[4], d.F[5], d.F[6], d.derS, d.d0tab, d.y,    d.Pp, fac_elems(g.ny, g.P)};
 }
 static int sm_count(const DeviceState& d) { return d.nsm > 0 ? d.nsm : 148; }
 
@@ -559,13 +557,9 @@ static cudaError_t launch_half_t(const SolveArgs& a, const DeviceState& d, cudaS
     tabs = 0;
     W = solve_warps(g, nsm, 0);
   }
-  if (W < 1 || !a.fac) return cudaErrorInvalidValue;
-  int groups = W * 32 / P;
-  // no more groups than the scratch has slices for
-  const long slices = (long)(d.facg_doubles / 2 / a.facn);
-  while (W > 1 && slices < groups) groups = --W * 32 / P;
-  const int nb = (int)std::min<long>({nsm, (g.ncol * g.nmem + groups - 1) / groups, slices / groups});
-  if (nb < 1) return cudaErrorInvalidValue;
+  if (W < 1) return cudaErrorInvalidValue;
+  const int groups = W * 32 / P;
+  const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
   const size_t smem = tabs + W * line_bytes(g.ny, P) * (32 / P);
   auto k = sh ? k_solve_half<P, HALF, true> : k_solve_half<P, HALF, false>;
   smem_limit(d, k, 227 * 1024);

@@ -76,6 +76,22 @@ def test_ensemble_solves_run_on_all_blocks(members, nx, ny, nz, tmp_path):
     s.close()
 
 
+def test_a_context_holds_what_it_says():
+    """hst_gpu_device_bytes and the rounding of some twenty-five allocations to 2 MiB (12 MB here) are all that a
+    context takes: the solves' factors lie in the product buffer (a scratch of their own took 34 MB more)"""
+    deck = c1_deck(nx=63, nz=64, ny=256, exact_shift=True)
+    s = hst.Solver(deck)  # loads the kernels
+    s.timesteps(1)
+    s.sync()
+    s.close()
+    free = torch.cuda.mem_get_info()[0]
+    s = hst.Solver(deck)
+    took = free - torch.cuda.mem_get_info()[0]
+    s.close()
+    said = hst.device_bytes(**{k: deck[k] for k in ("nx", "ny", "nz", "alfa0", "beta0", "ly")})
+    assert said <= took + (2 << 20) and took <= said + (28 << 20), (said, took)
+
+
 def test_a_refused_ensemble_gives_its_memory_back():
     """more members than the device holds: the creation is refused half way, and what it had allocated is free again"""
     hst.Solver(c1_deck(), members=2).close()
