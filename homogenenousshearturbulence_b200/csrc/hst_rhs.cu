@@ -19,8 +19,9 @@
 // and u, w through f = i (beta u - alfa w) (the mean column: f = (Re u, Re w), D =
 // -(Re uv, Re vw)), so that a row takes nine stencils instead of twenty-three.
 // What bounds it: at 768^2 x 512 the 14 Ns values of 16 B that it must move
-// (2.93 ms FP64, 5.1 TB/s; 3.67 with twenty-three stencils and six products.  2.35
-// in FP32, from 3.34); 384^2 x 256 0.536 -> 0.393 ms.  Any even ny takes this kernel:
+// (2.93 ms FP64, 5.1 TB/s, 3.1 in a long run under the power cap; 3.67 with
+// twenty-three stencils and six products.  2.37 in FP32, from 3.34); 384^2 x 256
+// 0.536 -> 0.393 ms.  Any even ny takes this kernel:
 // the last tile is ragged (nx 100, nz 75, 150 stretched rows: 0.620 -> 0.155 ms).
 #include "hst_dev.cuh"
 #include "hst_internal.h"

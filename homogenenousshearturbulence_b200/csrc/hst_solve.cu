@@ -24,13 +24,13 @@
 // least 48 (in FP32 48 nzd for the 2 nz + 1 columns of an x mode, nzd >= 3 nz).
 //
 // What bounds them: the dependent operations of a row's elimination and the
-// shared-memory pipe (512 rows: 73 % busy in k_shift, 50-60 % in the halves,
+// shared-memory pipe (512 rows: 69 % busy in k_shift, 54-64 % in the halves,
 // DRAM a third), so a line is cut into uneven slabs without padding rows, the
 // factors are kept with unit diagonals (a multiplication less a row each
 // way) and the D0 stencil and node phase are taken inside the back
-// substitution: 768^2 x 512 halves 3.57 -> 3.15 ms, shift 3.17 -> 2.72; 384^2 x 256
-// 0.535 -> 0.371; 1536^2 x 128 (a generic form before) 11.1 -> 2.65,
-// 20300 columns of 150 rows 0.399 -> 0.130.
+// substitution: 768^2 x 512 halves 3.57 -> 3.15 ms, shift 3.17 -> 2.92; 384^2 x 256
+// 0.535 -> 0.358; 1536^2 x 128 (a generic form before) 11.1 -> 2.53,
+// 15251 columns of 150 rows 0.399 -> 0.115.
 #include <algorithm>
 #include <cstdlib>
 
@@ -140,7 +140,7 @@ __device__ __forceinline__ void copy_table(double* dst, const double* __restrict
 // The four lines of a column one after another.  What bounds it is the
 // shared-memory traffic of the tables and the lines; two lines at a time,
 // sharing the table loads, leave nine warps an SM and measured slower (3.42
-// against 2.62 ms at 768^2 x 512).
+// against 2.92 ms at 768^2 x 512).
 constexpr int SHIFT_WARPS = 16;
 // SH: the tables in shared memory (the most rows have no room there)
 template <int P, bool SH>

@@ -43,9 +43,9 @@
 // staged lines (k_xprod's form), B200: 768^2 x 512 FP64 9.70 -> 4.86 ms, FP32
 // 7.26 -> 2.38; 384^2 x 256 FP64 1.10 -> 0.556 ms, FP32 0.79 -> 0.307; 1536^2 x 128
 // FP32 9.40 -> 3.11; 512 x 256 x 200 2.40 -> 0.387.  In FP64
-// at 768 points (six products) the L1 pipe is 74 % and the FP64 pipe 51 %
-// busy, in FP32 65 % with issue at 73 %: both near what one tile's exchanges
-// and butterflies allow, HBM at 40 %.
+// at 768 points the L1 pipe is 70 % and the FP64 pipe 53 % busy, in FP32 62 %
+// with issue at 70 %: both near what one tile's exchanges and butterflies allow,
+// HBM at 40 %.
 #include "hst_dev.cuh"
 #include "hst_fft.cuh"
 #include "hst_internal.h"

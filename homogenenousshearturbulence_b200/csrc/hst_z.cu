@@ -16,9 +16,9 @@
 //
 // The forward transform waits on its loads (64-byte runs 16 KB apart at
 // 768^2 x 512), so it runs on a persistent grid whose tiles land by tensor copies
-// in one of NBUF buffers while the previous tile is transformed: 4.66 -> 2.79
-// ms a substep at 768^2 x 512 FP64 (five products; 3.28 for six), 3.16 -> 1.57 FP32;
-// 0.490 -> 0.357 and 0.302 -> 0.217 ms at 384^2 x 256.  It reads and writes 80 %
+// in one of NBUF buffers while the previous tile is transformed: 4.66 -> 2.80
+// ms a substep at 768^2 x 512 FP64 (five products; 3.28 for six), 3.16 -> 1.58 FP32;
+// 0.490 -> 0.357 and 0.302 -> 0.215 ms at 384^2 x 256.  It reads and writes 74 %
 // of what a copy could in that time at 768 points.
 //
 // The inverse one hides its loads of V (16-byte rows, runs of TY) behind other
