@@ -102,12 +102,13 @@ int hst_gpu_create(const hst_gpu_params* p, hst_ctx** out);
  * together -- hst_gpu_timestep / _timesteps run every member, each kernel
  * of the substep covering all members in one launch, and the CFL number is
  * the largest over the members.  Each member evolves bit for bit as it does
- * alone.  The per-field device memory is nmem times that of a single field;
- * the tables are shared.  Every other entry point
- * (upload, download, fill_ghosts, line_solve, outstats, pressure, restart
- * files, the pieces, the asynchronous I/O) acts on the member chosen by
- * hst_gpu_select_member (member 0 at first).  hst_gpu_autotune refuses an
- * ensemble.  No counterpart in the reference, which runs one field a job. */
+ * alone (in a context that has not been autotuned).  The per-field device
+ * memory is nmem times that of a single field; the tables are shared.  Every
+ * other entry point (upload, download, fill_ghosts, line_solve, outstats,
+ * pressure, restart files, the pieces, the asynchronous I/O) acts on the
+ * member chosen by hst_gpu_select_member (member 0 at first).
+ * hst_gpu_autotune refuses an ensemble.  No counterpart in the reference,
+ * which runs one field a job. */
 int hst_gpu_create_batch(const hst_gpu_params* p, int nmem, hst_ctx** out);
 int hst_gpu_select_member(hst_ctx* ctx, int member);
 int hst_gpu_members(const hst_ctx* ctx);

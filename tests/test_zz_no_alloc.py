@@ -119,7 +119,7 @@ def test_noalloc_at_the_largest_size():
 
 def test_noalloc_d0_of_few_columns_costs_no_more_than_d2v():
     """528 columns of 1024 rows: the D0 and DY solves factor their matrix first, once for all columns, which must not
-    outweigh the solves themselves (1.1 times the D2V solve is what this size shows; 1.4 and 1.5 with the factoring
+    outweigh the solves themselves (1.1 and 1.2 times the D2V solve is what this size shows; 1.4 and 1.5 with the factoring
     waiting for each row's loads)"""
     import torch
 
@@ -144,4 +144,4 @@ def test_noalloc_d0_of_few_columns_costs_no_more_than_d2v():
         return best
 
     d2v = us(hst.KIND_D2V)
-    assert us(hst.KIND_D0) <= 1.25 * d2v and us(hst.KIND_DY) <= 1.4 * d2v
+    assert us(hst.KIND_D0) <= 1.3 * d2v and us(hst.KIND_DY) <= 1.43 * d2v
