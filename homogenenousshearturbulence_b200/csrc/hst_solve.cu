@@ -78,9 +78,9 @@ __device__ __forceinline__ Column column_of(const Geometry& g, const PhysScalars
 
 // The column that this group of a persistent grid takes first; the others
 // follow gridDim.x blocks' groups apart.  Consecutive warps' columns go to
-// consecutive blocks, so that the last round, which is seldom full, falls on all
-// SMs alike (both halves of 9664 columns of 64 rows 55 -> 42 us, of 5151 of 256
-// rows 102 -> 83; a full last round, 32896 of 256 rows, 357 and 355).
+// consecutive blocks, so that the last round falls on all SMs alike (both
+// halves of 9664 columns of 64 rows 55 -> 42 us, of 5151 of 256 rows 102 -> 83; a
+// full last round, 32896 of 256 rows, 357 and 355).
 template <int P>
 __device__ __forceinline__ int first_column() {
   constexpr int G = 32 / P;  // groups a warp
@@ -421,11 +421,11 @@ __global__ void k_d0_table(const double* __restrict__ der, int ny, double* __res
 // exceed what sixteen warps on each of the chip's 148 SMs take at once: the
 // reduction across the lanes costs as much as some ten rows, a second round of
 // columns half the first or more.  Measured for both solve halves, narrower and
-// wider group: 64 rows of 2080 columns 17.4 us with 8 lanes, 16.8 with 16; of 5151
-// 23.2 and 33.1; of 9664 35.0 with 4, 42.3 with 8; 128 rows of 3655 columns 29.8 with
-// 16, 40.2 with 32; of 32896 184 with 8, 198 with 16; 256 rows of 1281 columns 31.0
-// with 16, 26.4 with 32; of 32896 355 with 16, 406 with 32; 512 rows of 14661 436 with
-// 16, 392 with 32.
+// wider group: 64 rows of 2080 columns 17.1 us with 8 lanes, 16.6 with 16; of 5151
+// 23.0 and 32.6; of 9664 35.8 with 4, 37.5 with 8; 128 rows of 3655 columns 29.4 with
+// 16, 39.4 with 32; of 32896 180 with 8, 198 with 16; 256 rows of 1281 columns 30.8
+// with 16, 25.8 with 32; of 32896 350 with 16, 405 with 32; 512 rows of 14661 426 with
+// 16, 334 with 32.
 int line_lanes(int ny, long columns) {
   int P = 2;
   for (int c = 32; c > 2; c >>= 1)
@@ -500,6 +500,16 @@ static int solve_warps(const Geometry& g, int nsm, size_t tabs, int most = 16) {
   return (int)std::min<long>({most, want, (long)((227 * 1024 - tabs) / warp)});
 }
 
+// As many of W warps as give every round that W warps take the same columns: a
+// nearly empty last round costs as much as half a full one, and holds the whole
+// SM against other streams' kernels.  Both halves of 9664 columns of 512 rows 272
+// -> 235 us, the shift 259 -> 223; of 20301 of 64 rows 79 -> 73; three fields of nx
+// 27, ny 92, nz 431 in turn, exact shift, 10.5 -> 9.4 ms a pass.
+static int even_warps(const Geometry& g, int nsm, int W) {
+  const int cols = (g.ncol * g.nmem + nsm - 1) / nsm, round = W * 32 / g.P, rounds = (cols + round - 1) / round;
+  return ((cols + rounds - 1) / rounds * g.P + 31) / 32;
+}
+
 static SolveArgs solve_args(const Geometry& g, const DeviceState& d, const PhysScalars& ps, const SubstepScalars& sc) {
   return {g,      ps,     sc,     d.F[0], d.F[1],  d.F[2], d.F[3],
           d.F[4], d.F[5], d.F[6], d.derS, d.d0tab, d.y,    d.Pp, fac_elems(g.ny, g.P)};
@@ -518,6 +528,7 @@ static cudaError_t launch_shift_t(const SolveArgs& a, const DeviceState& d, cuda
     W = solve_warps(g, nsm, 0, SHIFT_WARPS);
   }
   if (W < 1) return cudaErrorInvalidValue;
+  W = even_warps(g, nsm, W);
   const int groups = W * 32 / P;
   const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
   auto k = sh ? k_shift<P, true> : k_shift<P, false>;
@@ -558,6 +569,7 @@ static cudaError_t launch_half_t(const SolveArgs& a, const DeviceState& d, cudaS
     W = solve_warps(g, nsm, 0);
   }
   if (W < 1) return cudaErrorInvalidValue;
+  W = even_warps(g, nsm, W);
   const int groups = W * 32 / P;
   const int nb = std::min(nsm, (g.ncol * g.nmem + groups - 1) / groups);
   const size_t smem = tabs + W * line_bytes(g.ny, P) * (32 / P);

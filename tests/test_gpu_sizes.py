@@ -127,9 +127,28 @@ def test_few_columns_take_no_longer_than_more(ny):
 @pytest.mark.parametrize("columns", [((60, 60), (63, 75)), ((42, 42), (50, 50))])
 def test_a_last_round_of_columns_is_spread(columns):
     """64 rows: 7381 and 9664 columns, 3655 and 5151, of which the larger just exceed what is resident at once: the
-    time must not double for the rest (1.2 to 1.5 is what these sizes show; 1.9 with that rest on a few SMs)"""
+    time must not double for the rest (1.0 and 1.3 is what these sizes show; 1.9 with that rest on a few SMs)"""
     few, more = (solve_us(nx, 64, nz) for nx, nz in columns)
     assert more <= 1.65 * few
+
+
+@pytest.mark.parametrize("nx,ny,nz,lanes", [(50, 256, 50, 16), (63, 64, 75, 8), (100, 96, 100, 8), (20, 512, 60, 32)])
+def test_rounds_of_columns_are_alike(monkeypatch, nx, ny, nz, lanes, tmp_path):
+    """columns above one round: the shift's and the solves' blocks have the warps that fill every round (0.9 of the
+    places and more; 0.5 to 0.8 with as many warps as fit)"""
+    monkeypatch.setenv("HST_LINE_LANES", str(lanes))
+    s = hst.Solver(c1_deck(nx=nx, ny=ny, nz=nz, exact_shift=True, linear=True))
+    s.timesteps(1)
+    s.sync()
+    columns, seen = (nx + 1) * (2 * nz + 1), set()
+    for e in traced(s, 1, tmp_path):
+        for name in ("k_shift", "k_solve_half"):
+            if e.get("cat") == "kernel" and name in e["name"]:
+                places = e["args"]["grid"][0] * e["args"]["block"][0] // lanes
+                assert columns >= 0.9 * places * -(-columns // places), (name, places)
+                seen.add(name)
+    s.close()
+    assert len(seen) == 2
 
 
 @pytest.mark.parametrize("lanes", [None, "2", "4", "8", "16", "32"])
